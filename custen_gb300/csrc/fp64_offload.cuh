@@ -6,13 +6,12 @@
 // and a reciprocal 5.6 of them. The functions below give the same bits with fewer:
 //   to_double / to_float   conversions rewritten on the IEEE 754 encodings           0 instead of 1
 //   div_by_float           correctly rounded c / d, d a float value                  3 instead of 10.4
-//   reciprocal             correctly rounded 1 / x                                   5 instead of 5.6 (+ the range check's)
-//   Divider                correctly rounded a / b; several a share b                3 + 3 per a instead of 9.4 per a
+//   reciprocal             correctly rounded 1 / x                                   4 instead of 5.6 (+ the range check's)
+//   Divider                correctly rounded a / b; several a share b                2 + 3 per a instead of 9.4 per a
 // Arguments outside the ranges named at each function take the compiler's own operation.
 //
-// Method: Newton's iteration for the reciprocal from an FP32 seed, taken to third order in one step
-// (1/b = y0 (1 + e + e^2 + ...), e = 1 - b y0), then one residual correction of the quotient with a fused
-// multiply-add (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
+// Method: Newton's iteration for the reciprocal (1/b = y (1 + e + e^2 + ...), e = 1 - b y), carried to about 47 bits
+// in pairs of floats, then one residual correction of the quotient with a fused multiply-add (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
 // IBM J. Res. Dev. 34, 1990). The error bounds that make the results correctly rounded stand at each function.
 #pragma once
 
@@ -105,38 +104,54 @@ __device__ __forceinline__ double times4(double x) {
     return __hiloint2double(zero ? hi : hi + (2 << 20), lo);
 }
 
-// 1/b to within 2^-69 before its one rounding, for |b| in [2^-100, 2^100): y0 = RN(1/RN32(b)), e = 1 - b y0 is
-// exact (|e| < 2^-22, a multiple of 2^-76 in units of its magnitude), y = RN(y0 + y0 (e + e^2)), neglecting e^3.
+// 1/b to within 2^-92 before its one rounding, for |b| in [2^-60, 2^60). An FP32 pair first: b = bh + bl with bh
+// the truncated float, yh = RN(1/bh), e = (1 - bh yh) - bl yh to 2^-47 (the parenthesis is exact), 1/b = yh + yl
+// with yl = yh (e + e^2), renormalised so that |yl| is at most half a unit of yh; the sum is formed by adding yl,
+// in units of yh's double, to yh's encoding (twice below a power of two, where a unit counts half). Then one
+// Newton step on the FP64 pipe.
 __device__ __forceinline__ double reciprocal_seed(double b, double one) {
-    const double y0 = to_double_normal(__frcp_rn(to_float_inrange(b)));
-    const double e = fma(-b, y0, one);
-    return fma(y0, fma(e, e, e), y0);
+    const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
+    const unsigned ub = (__funnelshift_l(lo, hi, 3) + 0x40000000u) & 0x7fffffffu;   // |b| truncated to float
+    const float bh = __uint_as_float(ub);
+    const float y1 = __frcp_rn(bh);
+    const float bl = (float)(lo & 0x1fffffffu) * __uint_as_float((ub & 0x7f800000u) - (52u << 23));
+    const float e = __fmaf_rn(-bl, y1, __fmaf_rn(-bh, y1, 1.0f));
+    const float y2 = __fmul_rn(y1, __fmaf_rn(e, e, e));
+    const float yh = __fadd_rn(y1, y2);
+    const float yl = __fsub_rn(y2, __fsub_rn(yh, y1));
+    const unsigned uy = __float_as_uint(yh);
+    const float unit = __uint_as_float(((2u * 127u + 52u) << 23) - (uy & 0x7f800000u));
+    int off = __float2int_rn(yl * unit);
+    if (off < 0 && (uy & 0x7fffffu) == 0u) off *= 2;
+    const long long yb = ((long long)((uy >> 3) + 0x38000000u) << 32 | (long long)(uy << 29)) + off;
+    const double y = __longlong_as_double(yb | (long long)((unsigned long long)(hi >> 31) << 63));
+    return fma(y, fma(-b, y, one), y);
 }
 
 // Correctly rounded 1 / x. A reciprocal y within one unit in the last place becomes the correctly rounded one
 // by one more iteration, except where the fraction of x is all ones (Markstein's theorem); those and arguments
-// outside [2^-100, 2^100) take the operator.
+// outside [2^-60, 2^60) take the operator.
 __device__ __forceinline__ double reciprocal(double x, double one) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
-    if (!exponent_in<-100, 100>(hi) || ((hi & 0xfffff) == 0xfffff && lo == -1)) return hw_divide(1.0, x);
+    if (!exponent_in<-60, 60>(hi) || ((hi & 0xfffff) == 0xfffff && lo == -1)) return hw_divide(1.0, x);
     const double y = reciprocal_seed(x, one);
     return fma(fma(-x, y, one), y, y);
 }
 
-// Correctly rounded quotients by one divisor. |b| in [2^-100, 2^100) and |a| in [2^-800, 2^800) or zero;
+// Correctly rounded quotients by one divisor. |b| in [2^-60, 2^60) and |a| in [2^-800, 2^800) or zero;
 // anything else takes the operator. q0 = RN(a y) is within one unit of a/b, so the residual is exact, and the
 // corrected quotient is correctly rounded where y is RN(1/b) (Markstein). y is, except where 1/b lies within
-// 2^-69 (relative) of a midpoint, where it may be the other neighbour; q0 + r y then still differs from a/b by at
+// 2^-92 (relative) of a midpoint, where it may be the other neighbour; q0 + r y then still differs from a/b by at
 // most 2^-105 (relative), which changes a rounding only if a/b lies that near a midpoint as well. Divisors just
 // below a power of two, b = 2^j (1 - k 2^-53) with small odd k, are systematically like that (1/b and quotients
 // of simple numerators fall next to midpoints): fractions whose upper 20 bits are ones take the operator. For
-// the others both coincidences together are about one quotient in 2^60.
+// the others both coincidences together are about one quotient in 2^90.
 struct Divider {
     double b, y;
     bool ok;
     __device__ __forceinline__ Divider(double b_, double one) : b(b_) {
         const int hi = __double2hiint(b_);
-        ok = exponent_in<-100, 100>(hi) && (hi & 0xfffff) != 0xfffff;
+        ok = exponent_in<-60, 60>(hi) && (hi & 0xfffff) != 0xfffff;
         y = reciprocal_seed(b_, one);   // unused unless ok
     }
     __device__ __forceinline__ double operator()(double a) const {

@@ -10,11 +10,15 @@
 // inverted once, the solve multiplies instead of dividing (rounding differs from the reference by about
 // one unit in the last place per row).
 //
-// GB300 shape: one thread per system, coalesced across systems (the layout's purpose). The per-row
-// recurrence is a dependent chain, so each thread issues the loads of the next KR rows before the chain
-// consumes them, and keeps the rows the chain refers back to in registers instead of re-reading them.
-// With divisions (about 10 FP64 operations each) the exact variants are FP64-bound; the reciprocal
-// variant is bound by HBM.
+// GB300 shape: one thread per system, coalesced across systems (the layout's purpose), one warp per CTA so that a
+// batch spreads evenly over the SMs. The per-row recurrence is a dependent chain; the rows ahead of it are copied
+// into a shared-memory ring while it runs, and the rows it refers back to stay in registers. The divisions of the
+// exact variants are the correctly rounded ones of fp64_offload.cuh (5 FP64 operations, 8 for the two that
+// share a pivot, against 9.4 each for the operator). The exact variants are bound by the FP64 pipe (12 and 9
+// operations a row), the reciprocal variant by HBM.
+// Measured, 262144 systems of 256 rows, G rows/s (before: operator divisions, loads staged in registers):
+// factorisation 27.9 -> 47.5, exact solve 44.2 -> 62.1, inverted-pivot solve 80.8 -> 93.9 (6.8 TB/s); 4096 systems of
+// 512 rows: 4.6 -> 6.0, 3.6 -> 7.7, 4.6 -> 13.8.
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -24,169 +28,183 @@
 #include <string>
 
 #include "../../include/custen_gb300.h"
+#include "fp64_offload.cuh"
 
 namespace custen {
 namespace pent {
 namespace {
 
-constexpr int kThreads = 128;
+constexpr int kThreads = 128;    // pivot inversion
+constexpr int kLine = 32;        // systems per CTA of the factorisation and the solves: one warp
 
-// KR: rows whose loads are issued ahead of the dependent chain.
-template <int KR>
-__global__ void __launch_bounds__(kThreads) factor_kernel(double* __restrict__ ds, double* __restrict__ dl,
-                                                          double* __restrict__ d, double* __restrict__ du,
-                                                          double* __restrict__ dw, int m, int batch) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// 1.0, read into a register: an FP64 instruction with a literal operand issues about 19% slower.
+__device__ double g_one = 1.0;
+
+// Rows in flight: every thread copies the values of the next D rows of its own system into its own slots of a
+// shared-memory ring (cp.async, one group per row), so the loads take no registers and no barrier. A row beyond
+// the end leaves an empty group, which keeps the group count per row fixed.
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void wait_group() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Expressions and order of the reference's pentFactorBatch (cuPentBatch.cu:35-113): rows 0 and 1 lack the terms
+// of the rows before them, row m-2 has no dw, row m-1 neither du nor dw.
+template <int D>
+__global__ void __launch_bounds__(kLine) factor_kernel(const double* __restrict__ ds, double* dl, double* d, double* du,
+                                                       double* dw, int m, int batch) {
+    __shared__ double ring[D][5][kLine];
+    const int t = threadIdx.x;
+    const int s = blockIdx.x * kLine + t;
     if (s >= batch) return;
     const size_t B = (size_t)batch;
-    // row 0
-    double d0 = d[s];
-    double du0 = du[s] / d0;
-    double dw0 = dw[s] / d0;
-    du[s] = du0;
-    dw[s] = dw0;
-    // row 1
-    size_t r = B + s;
-    const double dl1 = dl[r];
-    double d1 = d[r] - dl1 * du0;
-    double du1 = (du[r] - dl1 * dw0) / d1;
-    double dw1 = dw[r] / d1;
-    d[r] = d1;
-    du[r] = du1;
-    dw[r] = dw1;
-    // interior rows 2 .. m-3 (cuPentBatch.cu:75-80); (du, dw) of the two previous rows stay in registers
-    // (duP2, dwP2 = row i-2; duP1, dwP1 = row i-1)
-    double duP2 = du0, dwP2 = dw0, duP1 = du1, dwP1 = dw1;
-    for (int i0 = 2; i0 < m - 2; i0 += KR) {
-        double vs[KR], vl[KR], vd[KR], vu[KR], vw[KR];
-#pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 + k;
-            if (i < m - 2) {
-                const size_t q = (size_t)i * B + s;
-                vs[k] = ds[q];
-                vl[k] = dl[q];
-                vd[k] = d[q];
-                vu[k] = du[q];
-                vw[k] = dw[q];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 + k;
-            if (i >= m - 2) break;
+    const double one = *(const volatile double*)&g_one;
+    auto issue = [&](int i) {
+        if (i < m) {
             const size_t q = (size_t)i * B + s;
-            const double l = vl[k] - vs[k] * duP2;
-            const double dd = vd[k] - vs[k] * dwP2 - l * duP1;
-            const double ww = vw[k] / dd;
-            const double uu = (vu[k] - l * dwP1) / dd;
+            double(*r)[kLine] = ring[i % D];
+            if (i >= 2) copy8(&r[0][t], ds + q);
+            if (i >= 1) copy8(&r[1][t], dl + q);
+            copy8(&r[2][t], d + q);
+            if (i < m - 1) copy8(&r[3][t], du + q);
+            if (i < m - 2) copy8(&r[4][t], dw + q);
+        }
+        commit();
+    };
+#pragma unroll
+    for (int i = 0; i < D; ++i) issue(i);
+    // (du, dw) of the two previous rows: P2 = row i-2, P1 = row i-1
+    double duP2 = 0.0, dwP2 = 0.0, duP1 = 0.0, dwP1 = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < m; ++i) {
+        wait_group<D - 1>();
+        const size_t q = (size_t)i * B + s;
+        const double(*r)[kLine] = ring[i % D];
+        double dd = r[2][t], l = 0.0;
+        if (i >= 2) {   // interior rows (:75-80)
+            const double vs = r[0][t];
+            l = r[1][t] - vs * duP2;
+            dd = dd - vs * dwP2 - l * duP1;
             dl[q] = l;
             d[q] = dd;
-            dw[q] = ww;
-            du[q] = uu;
-            duP2 = duP1;
-            dwP2 = dwP1;
-            duP1 = uu;
-            dwP1 = ww;
+        } else if (i == 1) {
+            l = r[1][t];
+            dd = dd - l * duP1;
+            d[q] = dd;
         }
-    }
-    // second last row (:86-92): no dw
-    {
-        const size_t q = (size_t)(m - 2) * B + s;
-        const double l = dl[q] - ds[q] * duP2;
-        const double dd = d[q] - ds[q] * dwP2 - l * duP1;
-        const double uu = (du[q] - l * dwP1) / dd;
-        dl[q] = l;
-        d[q] = dd;
-        du[q] = uu;
+        const f64::Divider by(dd, one);
         duP2 = duP1;
+        const double dwL = dwP1;
         dwP2 = dwP1;
-        duP1 = uu;
-    }
-    // last row (:94-99): dl and d only
-    {
-        const size_t q = (size_t)(m - 1) * B + s;
-        const double l = dl[q] - ds[q] * duP2;
-        dl[q] = l;
-        d[q] = d[q] - ds[q] * dwP2 - l * duP1;
+        if (i < m - 2) {
+            dwP1 = by(r[4][t]);
+            dw[q] = dwP1;
+        }
+        if (i < m - 1) {
+            const double vu = r[3][t];
+            duP1 = by(i >= 1 ? vu - l * dwL : vu);
+            du[q] = duP1;
+        }
+        issue(i + D);
     }
 }
 
-template <int KR>
-__global__ void __launch_bounds__(kThreads) solve_kernel(const double* __restrict__ ds, const double* __restrict__ dl,
-                                                         const double* __restrict__ d, const double* __restrict__ du,
-                                                         const double* __restrict__ dw, double* __restrict__ b, int m,
-                                                         int batch, int rcp) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+// pentSolveBatch (cuPentBatch.cu:119-198): forward substitution (:153-171), then backward (:178-196). RCP: d holds
+// the inverted pivots. Each thread re-reads in the backward pass what it stored itself in the forward pass.
+template <int D, bool RCP>
+__global__ void __launch_bounds__(kLine) solve_kernel(const double* __restrict__ ds, const double* __restrict__ dl,
+                                                      const double* __restrict__ d, const double* __restrict__ du,
+                                                      const double* __restrict__ dw, double* b, int m, int batch) {
+    __shared__ double ring[D][4][kLine];
+    const int t = threadIdx.x;
+    const int s = blockIdx.x * kLine + t;
     if (s >= batch) return;
     const size_t B = (size_t)batch;
-    // forward substitution (cuPentBatch.cu:153-171)
-    double b0 = rcp ? b[s] * d[s] : b[s] / d[s];
-    b[s] = b0;
-    double b1 = rcp ? (b[B + s] - dl[B + s] * b0) * d[B + s] : (b[B + s] - dl[B + s] * b0) / d[B + s];
-    b[B + s] = b1;
-    double p2 = b0, p1 = b1;
-    for (int i0 = 2; i0 < m; i0 += KR) {
-        double vs[KR], vl[KR], vd[KR], vb[KR];
-#pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 + k;
-            if (i < m) {
-                const size_t q = (size_t)i * B + s;
-                vs[k] = ds[q];
-                vl[k] = dl[q];
-                vd[k] = d[q];
-                vb[k] = b[q];
-            }
+    const double one = *(const volatile double*)&g_one;
+    auto issue = [&](int i) {
+        if (i < m) {
+            const size_t q = (size_t)i * B + s;
+            double(*r)[kLine] = ring[i % D];
+            if (i >= 2) copy8(&r[0][t], ds + q);
+            if (i >= 1) copy8(&r[1][t], dl + q);
+            copy8(&r[2][t], d + q);
+            copy8(&r[3][t], b + q);
         }
+        commit();
+    };
 #pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 + k;
-            if (i >= m) break;
-            const double t = vb[k] - vs[k] * p2 - vl[k] * p1;
-            const double v = rcp ? t * vd[k] : t / vd[k];
-            b[(size_t)i * B + s] = v;
-            p2 = p1;
-            p1 = v;
-        }
+    for (int i = 0; i < D; ++i) issue(i);
+    double p2 = 0.0, p1 = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < m; ++i) {
+        wait_group<D - 1>();
+        const double(*r)[kLine] = ring[i % D];
+        double v = r[3][t];
+        if (i >= 2) v = v - r[0][t] * p2 - r[1][t] * p1;
+        else if (i == 1) v = v - r[1][t] * p1;
+        v = RCP ? v * r[2][t] : f64::Divider(r[2][t], one)(v);
+        b[(size_t)i * B + s] = v;
+        p2 = p1;
+        p1 = v;
+        issue(i + D);
     }
-    // backward substitution (:178-196); rows m-1 and m-2 first
-    double a1 = p1;                                   // row m-1
-    double a0 = b[(size_t)(m - 2) * B + s] - du[(size_t)(m - 2) * B + s] * a1;   // row m-2
-    b[(size_t)(m - 2) * B + s] = a0;
-    // a0 = row i+1, a1 = row i+2
-    double n1 = a0, n2 = a1;
-    for (int i0 = m - 3; i0 >= 0; i0 -= KR) {
-        double vu[KR], vw[KR], vb[KR];
-#pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 - k;
-            if (i >= 0) {
-                const size_t q = (size_t)i * B + s;
-                vu[k] = du[q];
-                vw[k] = dw[q];
-                vb[k] = b[q];
-            }
+    wait_group<0>();
+    // row m-1 is done; p1, p2: rows i+1, i+2
+    auto issue_back = [&](int k) {   // k rows above row m-2
+        const int i = m - 2 - k;
+        if (i >= 0) {
+            const size_t q = (size_t)i * B + s;
+            double(*r)[kLine] = ring[k % D];
+            copy8(&r[0][t], du + q);
+            if (k > 0) copy8(&r[1][t], dw + q);
+            copy8(&r[2][t], b + q);
         }
+        commit();
+    };
 #pragma unroll
-        for (int k = 0; k < KR; ++k) {
-            const int i = i0 - k;
-            if (i < 0) break;
-            const double v = vb[k] - vu[k] * n1 - vw[k] * n2;
-            b[(size_t)i * B + s] = v;
-            n2 = n1;
-            n1 = v;
-        }
+    for (int k = 0; k < D; ++k) issue_back(k);
+    p2 = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < m - 1; ++k) {
+        wait_group<D - 1>();
+        const double(*r)[kLine] = ring[k % D];
+        double v = r[2][t] - r[0][t] * p1;
+        if (k > 0) v = v - r[1][t] * p2;
+        b[(size_t)(m - 2 - k) * B + s] = v;
+        p2 = p1;
+        p1 = v;
+        issue_back(k + D);
     }
 }
 
 __global__ void __launch_bounds__(kThreads) invert_kernel(double* __restrict__ d, size_t count) {
+    const double one = *(const volatile double*)&g_one;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < count; q += (size_t)gridDim.x * blockDim.x)
-        d[q] = 1.0 / d[q];
+        d[q] = f64::reciprocal(d[q], one);
 }
 
 thread_local std::string g_err;
-std::atomic<int> g_kr[3] = {8, 2, 2};   // prefetch depth: factor, exact solve, inverted-pivot solve (measured best)
+std::atomic<int> g_kr[3] = {0, 0, 0};   // rows in flight of factor, exact solve, inverted-pivot solve; 0: by the rule
+
+// Rows in flight: 8 while at most two warps share an FP64 sub-partition (4 per SM) and the copies' latency shows,
+// else 4, since a deep ring limits the resident warps. Measured (us, 4 / 8 rows): inverted-pivot solve 179 / 152 with
+// 4096 systems of 512 rows, 41 / 38 with 20000 of 100, 369 / 451 with 131072 of 256; exact solve 287 / 271, 65 / 64,
+// 561 / 629; factorisation 352 / 352, 78 / 79, 709 / 760.
+int rows_in_flight(int which, int blocks) {
+    const int set = g_kr[which].load();
+    if (set) return set;
+    static std::atomic<int> sms[64] = {};   // threads that race store the same value
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        n = sms[dev].load(std::memory_order_relaxed);
+        if (n == 0 && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+            sms[dev].store(n, std::memory_order_relaxed);
+    }
+    return blocks <= 8 * n ? 8 : 4;
+}
 
 template <typename F2, typename F4, typename F8>
 void by_depth(int kr, F2 f2, F4 f4, F8 f8) {
@@ -224,7 +242,7 @@ extern "C" {
 
 const char* custen_pent_last_error(void) { return g_err.c_str(); }
 
-// Prefetch depth (rows of loads issued ahead of the chain: 2, 4 or 8) of the factorisation (which = 0),
+// Prefetch depth (rows in flight ahead of the chain: 2, 4 or 8) of the factorisation (which = 0),
 // the exact solve (1) and the inverted-pivot solve (2). Results do not depend on it.
 int custen_pent_set_depth(int which, int rows) {
     if (which < 0 || which > 2 || (rows != 2 && rows != 4 && rows != 8)) {
@@ -238,12 +256,12 @@ int custen_pent_set_depth(int which, int rows) {
 int custen_pent_factor_batch(double* ds, double* dl, double* d, double* du, double* dw, int m, int batch,
                              void* stream) {
     if (int st = check_args(ds, dl, d, du, dw, m, batch)) return st;
-    const int blocks = (batch + kThreads - 1) / kThreads;
+    const int blocks = (batch + kLine - 1) / kLine;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     by_depth(
-        g_kr[0], [&] { factor_kernel<2><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, m, batch); },
-        [&] { factor_kernel<4><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, m, batch); },
-        [&] { factor_kernel<8><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, m, batch); });
+        rows_in_flight(0, blocks), [&] { factor_kernel<2><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, m, batch); },
+        [&] { factor_kernel<4><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, m, batch); },
+        [&] { factor_kernel<8><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, m, batch); });
     return check(cudaGetLastError(), "Launching the batched factorisation");
 }
 
@@ -254,12 +272,12 @@ int custen_pent_solve_batch(const double* ds, const double* dl, const double* d,
         g_err = "right-hand side pointer must not be NULL";
         return 2;
     }
-    const int blocks = (batch + kThreads - 1) / kThreads;
+    const int blocks = (batch + kLine - 1) / kLine;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     by_depth(
-        g_kr[1], [&] { solve_kernel<2><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, b, m, batch, 0); },
-        [&] { solve_kernel<4><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, b, m, batch, 0); },
-        [&] { solve_kernel<8><<<blocks, kThreads, 0, st>>>(ds, dl, d, du, dw, b, m, batch, 0); });
+        rows_in_flight(1, blocks), [&] { solve_kernel<2, false><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, b, m, batch); },
+        [&] { solve_kernel<4, false><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, b, m, batch); },
+        [&] { solve_kernel<8, false><<<blocks, kLine, 0, st>>>(ds, dl, d, du, dw, b, m, batch); });
     return check(cudaGetLastError(), "Launching the batched solve");
 }
 
@@ -282,12 +300,12 @@ int custen_pent_solve_batch_rcp(const double* ds, const double* dl, const double
         g_err = "right-hand side pointer must not be NULL";
         return 2;
     }
-    const int blocks = (batch + kThreads - 1) / kThreads;
+    const int blocks = (batch + kLine - 1) / kLine;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     by_depth(
-        g_kr[2], [&] { solve_kernel<2><<<blocks, kThreads, 0, st>>>(ds, dl, rd, du, dw, b, m, batch, 1); },
-        [&] { solve_kernel<4><<<blocks, kThreads, 0, st>>>(ds, dl, rd, du, dw, b, m, batch, 1); },
-        [&] { solve_kernel<8><<<blocks, kThreads, 0, st>>>(ds, dl, rd, du, dw, b, m, batch, 1); });
+        rows_in_flight(2, blocks), [&] { solve_kernel<2, true><<<blocks, kLine, 0, st>>>(ds, dl, rd, du, dw, b, m, batch); },
+        [&] { solve_kernel<4, true><<<blocks, kLine, 0, st>>>(ds, dl, rd, du, dw, b, m, batch); },
+        [&] { solve_kernel<8, true><<<blocks, kLine, 0, st>>>(ds, dl, rd, du, dw, b, m, batch); });
     return check(cudaGetLastError(), "Launching the batched solve");
 }
 

@@ -13,12 +13,12 @@
 //     second differences are formed once per tile into shared memory (the reference forms five differences and
 //     three second differences per point and direction);
 //   - the 36 conversions per point between double and the float smoothness terms, and all but 3 operations of
-//     each division, run on the integer and FP32 pipes (fp64_offload.cuh).
+//     each division (4 of the reciprocal's), run on the integer and FP32 pipes (fp64_offload.cuh).
 // The reconstruction keeps the reference's operation order, including its single-precision powf on the
 // smoothness terms, so that results are bit-identical to the reference's kernel on the same GPU.
 // Measured (2048^2): 1418 us with hardware conversions and divisions (about 200 FP64 instructions per point),
-// 913 us with those moved off the FP64 pipe (112), 832 us with the shared second differences and the shorter
-// division (5.0 Gpts/s; 8192 x 4096: 5.4).
+// 913 us with those moved off the FP64 pipe (112), 820 us with the shared second differences and the shorter
+// divisions (5.1 Gpts/s; 8192 x 4096: 5.4).
 #include <cuda_runtime.h>
 
 #include <atomic>

@@ -213,8 +213,8 @@ int custen_pent_invert_pivots(double* d, int m, int batch, void* stream);
 int custen_pent_solve_batch_rcp(const double* ds, const double* dl, const double* rd, const double* du,
                                 const double* dw, double* b, int m, int batch, void* stream);
 const char* custen_pent_last_error(void);
-/* Rows of loads issued ahead of the recurrence (2, 4 or 8) in the factorisation (which = 0), the exact
- * solve (1) and the inverted-pivot solve (2); results do not depend on it. */
+/* Rows in flight ahead of the recurrence (2, 4 or 8) in the factorisation (which = 0), the exact solve (1)
+ * and the inverted-pivot solve (2); chosen by the batch size unless set. Results do not depend on it. */
 int custen_pent_set_depth(int which, int rows);
 
 /* ---- Cahn-Hilliard ADI solver: batches of periodic grids of different sizes ----
