@@ -2,7 +2,7 @@
 //
 // Requests (grid size n, step count, initial field, arrival time) arrive over time. The loop admits
 // arrived requests first-come first-served while their device memory fits the HBM budget: their two
-// field buffers, work field, h field and row ends are allocated stream-ordered (cudaMallocAsync, no device
+// field buffers, work field and h field are allocated stream-ordered (cudaMallocAsync, no device
 // synchronisation) and their pre-factored solver table is shared by every resident grid of the same
 // size. All resident grids then advance together, a chunk of steps at a time, through the same
 // persistent kernels as the batch solver (ch_solver.cu): one launch per kernel covers every grid.
@@ -12,6 +12,7 @@
 //
 // The solver is the reference's (cuPentCahnADI/src/cuPentCahnADI.cu:197-627); the request loop has
 // no counterpart in the reference, whose driver runs one simulation per process.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>   // header-only; the ranges cost nothing unless a profiler is attached
 
@@ -66,6 +67,7 @@ struct Request {
     std::vector<double> result;
     size_t bytes = 0;
     GridDev g{};
+    CUtensorMap maps[2];             // of g.tmp, unless g.general
     std::string table_key;
 };
 
@@ -89,11 +91,11 @@ struct Server {
     std::vector<int> active;        // request ids resident on the device
     std::map<std::string, TableRef> tables;
     GridDev* grids_d = nullptr;
+    CUtensorMap* maps_d = nullptr;
     Item* items_rhs_d = nullptr;
     Item* items_rows_d = nullptr;
-    size_t cap_grids = 0, cap_rhs = 0, cap_rows = 0;
-    int n_rhs = 0, n_rows = 0;
-    unsigned int* counters = nullptr;
+    size_t cap_grids = 0, cap_maps = 0, cap_rhs = 0, cap_rows = 0;
+    int n_rhs = 0, n_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
     double* mass_d = nullptr;
     int sms = 0;
     // statistics of the last run
@@ -122,8 +124,8 @@ static int srv_arg(const std::string& m) {
         if (_e != cudaSuccess) return srv_fail(_e, what); \
     } while (0)
 
-// per grid: cCurr, cOld, the work field and the h field of the two-pass right-hand side, plus 2 n row ends
-static size_t grid_bytes(int n) { return 4 * (size_t)n * n * sizeof(double) + 2 * (size_t)n * sizeof(double); }
+// per grid: cCurr, cOld, the work field and the h field of the two-pass right-hand side
+static size_t grid_bytes(int n) { return 4 * (size_t)n * n * sizeof(double); }
 
 static int grow(void** p, size_t* cap, size_t need, size_t elem, cudaStream_t s) {
     if (need <= *cap) return 0;
@@ -139,21 +141,31 @@ static int rebuild(Server* S) {
     std::vector<int> order = S->active;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return S->reqs[a].n > S->reqs[b].n; });
     std::vector<GridDev> grids;
+    std::vector<CUtensorMap> maps;
     std::vector<Item> rhs, rows;
     for (size_t k = 0; k < order.size(); ++k) {
         const Request& r = S->reqs[order[k]];
         grids.push_back(r.g);
+        maps.insert(maps.end(), r.maps, r.maps + 2);
         const int bpr = r.n / BLK;
         for (int b = 0; b < bpr * bpr; ++b) rhs.push_back({(int)k, b});
-        for (int b = 0; b < bpr; ++b) rows.push_back({(int)k, b});
+        if (!r.g.general)
+            for (int b = 0; b < bpr; ++b) rows.push_back({(int)k, b});
     }
+    S->n_general = 0;
+    for (size_t k = 0; k < grids.size(); ++k)
+        if (grids[k].general)
+            for (int b = 0; b < grids[k].n / BLK; ++b, ++S->n_general) rows.push_back({(int)k, b});
     int st;
     if ((st = grow((void**)&S->grids_d, &S->cap_grids, grids.size(), sizeof(GridDev), S->stream))) return st;
+    if ((st = grow((void**)&S->maps_d, &S->cap_maps, maps.size(), sizeof(CUtensorMap), S->stream))) return st;
     if ((st = grow((void**)&S->items_rhs_d, &S->cap_rhs, rhs.size(), sizeof(Item), S->stream))) return st;
     if ((st = grow((void**)&S->items_rows_d, &S->cap_rows, rows.size(), sizeof(Item), S->stream))) return st;
     // pageable copies: the host vectors may be released as soon as the calls return
     SRV_TRY(cudaMemcpyAsync(S->grids_d, grids.data(), grids.size() * sizeof(GridDev), cudaMemcpyHostToDevice,
                             S->stream), "Uploading grid descriptors");
+    SRV_TRY(cudaMemcpyAsync(S->maps_d, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice,
+                            S->stream), "Uploading tensor maps");
     SRV_TRY(cudaMemcpyAsync(S->items_rhs_d, rhs.data(), rhs.size() * sizeof(Item), cudaMemcpyHostToDevice, S->stream),
             "Uploading work list");
     SRV_TRY(cudaMemcpyAsync(S->items_rows_d, rows.data(), rows.size() * sizeof(Item), cudaMemcpyHostToDevice,
@@ -176,6 +188,7 @@ static int admit(Server* S, int id, double now) {
     snprintf(key, sizeof(key), "%d/%.17g", r.n, r.lx);
     r.table_key = key;
     TableRef& t = S->tables[key];
+    const bool general = line_is_general(r.n, r.lx, S->gamma, S->dt_factor, S->rhs_fp32 != 0);
     cudaError_t e = cudaSuccess;
     const char* what = "";
     auto step = [&](cudaError_t x, const char* w) {
@@ -190,7 +203,7 @@ static int admit(Server* S, int id, double now) {
     };
     bool new_table = false;
     if (!t.ptr) {
-        std::vector<double> h = build_table(r.n, r.lx, S->gamma, S->dt_factor);
+        std::vector<double> h = build_table(r.n, r.lx, S->gamma, S->dt_factor, general);
         t.bytes = h.size() * sizeof(double);
         step(alloc(&t.ptr, t.bytes), "Allocating a solver table");
         if (e == cudaSuccess) {
@@ -200,9 +213,9 @@ static int admit(Server* S, int id, double now) {
         }
     }
     const size_t f = (size_t)r.n * r.n * sizeof(double);
-    double* p[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // cCurr, cOld, tmp, row ends, h
-    for (int k = 0; k < 5 && e == cudaSuccess; ++k)
-        step(alloc(&p[k], k == 3 ? 2 * (size_t)r.n * sizeof(double) : f), "Allocating a grid");
+    double* p[4] = {nullptr, nullptr, nullptr, nullptr};   // cCurr, cOld, tmp, h
+    for (int k = 0; k < 4 && e == cudaSuccess; ++k) step(alloc(&p[k], f), "Allocating a grid");
+    if (e == cudaSuccess && !general && !sweep_maps(r.maps, p[2], r.n)) step(cudaErrorNotSupported, "Encoding tensor maps");
     double m = 0.0;
     if (e == cudaSuccess) {
         if (!r.c0.empty()) {
@@ -244,10 +257,10 @@ static int admit(Server* S, int id, double now) {
     r.g.buf[S->parity] = p[0];        // cCurr
     r.g.buf[S->parity ^ 1] = p[1];    // cOld
     r.g.tmp = p[2];
-    r.g.ends = p[3];
-    r.g.hbuf = p[4];
+    r.g.hbuf = r.g.ends = p[3];   // the sweeps' closure amplitudes lie in the h field, which they do not read
     r.g.tab = t.ptr;
     r.g.n = r.n;
+    r.g.general = general;
     r.mean0 = m / ((double)r.n * r.n);
     r.bytes = grid_bytes(r.n);
     S->used += (double)r.bytes;
@@ -273,7 +286,7 @@ static int retire(Server* S, int id, double now_after) {
     SRV_TRY(cudaStreamSynchronize(S->stream), "Retiring");
     r.mean_end = m / ((double)r.n * r.n);
     r.done_t = now_after;
-    for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.ends, r.g.hbuf}) SRV_TRY(cudaFreeAsync(p, S->stream), "Freeing a grid");
+    for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.hbuf}) SRV_TRY(cudaFreeAsync(p, S->stream), "Freeing a grid");
     S->used -= (double)r.bytes;
     TableRef& t = S->tables[r.table_key];
     if (--t.refs == 0) {
@@ -319,7 +332,7 @@ static bool write_snapshot(Server* S, Request& r, std::string* err) {
 // Take a resident request out of the run as failed: release its memory, record why.
 static int drop(Server* S, int id, const std::string& why, double now) {
     Request& r = S->reqs[id];
-    for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.ends, r.g.hbuf}) SRV_TRY(cudaFreeAsync(p, S->stream), "Freeing a grid");
+    for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.hbuf}) SRV_TRY(cudaFreeAsync(p, S->stream), "Freeing a grid");
     S->used -= (double)r.bytes;
     TableRef& t = S->tables[r.table_key];
     if (--t.refs == 0) {
@@ -335,16 +348,11 @@ static int drop(Server* S, int id, const std::string& why, double now) {
 }
 
 static int enqueue_steps(Server* S, int k) {
+    const ChConfig cfg = ch_config(kChBatchDefault);
+    const ChWork w{S->grids_d, S->items_rhs_d, S->items_rows_d, S->maps_d, S->n_rhs, S->n_rows, S->n_general};
     for (int s = 0; s < k; ++s) {
-        SRV_TRY(cudaMemsetAsync(S->counters, 0, kChCounters * sizeof(unsigned int), S->stream), "Resetting counters");
-        // Fewer 32-line warps than FP64 sub-partitions (4 per SM): the sweeps are bound by a warp's own FP64
-        // instruction count, so the y sweep's correction and update run as element-wise kernels. Every
-        // configuration computes the same values, so a request's result does not depend on the choice.
-        const ChConfig cfg = ch_config(S->n_rows < 4 * S->sms ? kChSplitConfig : kChBatchDefault);
-        SRV_TRY(launch_ch_step(cfg, S->rhs_fp32 != 0, S->grids_d, S->items_rhs_d, S->n_rhs, S->items_rows_d,
-                               S->n_rows, S->parity, S->counters, S->sms, S->stream),
-                "Launching a step");
-        S->launches += ch_launches_per_step(cfg);
+        SRV_TRY(launch_ch_step(cfg, S->rhs_fp32 != 0, w, S->parity, S->sms, S->stream), "Launching a step");
+        S->launches += ch_launches_per_step(cfg, w, S->sms);
         S->parity ^= 1;
     }
     return 0;
@@ -474,7 +482,6 @@ int custen_ch_server_create(void** out, double hbm_budget_bytes, int rhs_dtype, 
     S->chunk = chunk_steps;
     S->keep_results = keep_results;
     cudaError_t e = cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocAsync(&S->counters, kChCounters * sizeof(unsigned int), S->stream);
     if (e == cudaSuccess) e = cudaMallocAsync(&S->mass_d, sizeof(double), S->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(S->stream);
     if (e != cudaSuccess) {
@@ -629,14 +636,14 @@ int custen_ch_server_destroy(void* h) {
     cudaStreamSynchronize(S->stream);
     for (int id : S->active) {
         Request& r = S->reqs[id];
-        for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.ends, r.g.hbuf}) cudaFreeAsync(p, S->stream);
+        for (double* p : {r.g.buf[0], r.g.buf[1], r.g.tmp, r.g.hbuf}) cudaFreeAsync(p, S->stream);
     }
     for (auto& t : S->tables)
         if (t.second.ptr) cudaFreeAsync(t.second.ptr, S->stream);
     if (S->grids_d) cudaFreeAsync(S->grids_d, S->stream);
+    if (S->maps_d) cudaFreeAsync(S->maps_d, S->stream);
     if (S->items_rhs_d) cudaFreeAsync(S->items_rhs_d, S->stream);
     if (S->items_rows_d) cudaFreeAsync(S->items_rows_d, S->stream);
-    cudaFreeAsync(S->counters, S->stream);
     cudaFreeAsync(S->mass_d, S->stream);
     cudaStreamSynchronize(S->stream);
     cudaStreamDestroy(S->stream);

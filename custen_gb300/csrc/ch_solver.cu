@@ -4,44 +4,36 @@
 // cuPentSpeedUp/serialCahnADITiming/serialCahnADI.c:1010-1047), per grid of n x n points:
 //   cBar = 2 cCurr - cOld
 //   rhs  = Lin5x5(cBar) + Nl3x3(cCurr^3 - cCurr) - (2/3)(cCurr - cOld)
-//   (1 + s Dx4)(1 + s Dy4) delta = rhs   -- two cyclic pentadiagonal sweeps, x then y, each solved as
-//       the (n-2) x (n-2) banded block (pre-factored, cuPentBatch.cu:35-198) plus the 2 x 2 Schur
-//       complement on the last two unknowns (BatchHyper.cu:195-259, 421-514)
+//   (1 + s Dx4)(1 + s Dy4) delta = rhs   -- two cyclic pentadiagonal sweeps, x then y
 //   cNew = cBar + delta;  cOld <- cCurr;  cCurr <- cNew
 //
 // GB300 shape: FP64 FMAs (about 2 per clock per SM) bound this solver, not HBM, so the kernels
-// minimise FP64 operations (about 32 per point and step, against about 100 in the reference: the two
-// explicit stencils as two 5-point Laplacians, cBar and c^3 - c computed once per point, divisions
-// replaced by reciprocals) and keep every SM sub-partition busy:
-//   K1 ch_rhs_kernel     -- right-hand side, 32 x 32 blocks, lane = column, all points in parallel.
-//   K2 ch_xsolve_kernel  -- x sweep, one warp per 32 rows (lane = row) walking 32-column chunks
-//                           transposed through shared memory; leaves the banded solution y and the
-//                           two corner values of every row.
-//   K3 ch_ysolve_kernel  -- y sweep, one warp per 32 columns (lane = column, coalesced), applying the
-//                           x sweep's rank-2 correction as it reads, then cNew = cBar + delta written
-//                           over cOld (the two field buffers swap roles every step).
-// Each kernel is persistent over a work list that covers all grids (largest first, claimed through
-// an atomic counter), so grids of different sizes share one launch. A step is three launches (four with
-// the two-pass right-hand side, six with the split y sweep as well); pairs of steps are captured in a CUDA
-// graph.
-//
-// The sweeps come in three forms, all computing the same values (ChConfig, tuned per batch):
-// staged through registers (the kernels K2/K3 below), pipelined (the next chunk copied into shared
-// memory with cp.async while the current one runs), and pipelined with the chunk's table entries held
-// in registers by every lane (no per-element shuffles; the default, configuration 12).
+// minimise FP64 operations (about 27 per point and step, against about 100 in the reference: the two
+// explicit stencils as two 5-point Laplacians, cBar and c^3 - c computed once per point, the line operators
+// factored with constant coefficients) and keep every SM sub-partition busy:
+//   K1 ch_rhs_kernel / ch_h_kernel + ch_rhs2_kernel -- right-hand side, 32 x 32 blocks, lane = column, all points
+//                           in parallel.
+//   K2 ch_xsweep_kernel  -- x sweep, two chains (warps) per 32 rows, lane = row.
+//   K3 ch_ysweep_kernel  -- y sweep, two chains per 32 columns, lane = column.
+//   K4 ch_update_kernel  -- cNew = cBar + delta, written over cOld (the two field buffers swap roles every step).
+// Each launch covers all grids of a work list (largest first), so grids of different sizes share it; pairs of steps
+// are captured in a CUDA graph.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <complex>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/custen_gb300.h"
 #include "ch_internal.cuh"
 #include "checked.cuh"
+#include "stencil_launch.cuh"   // mbarrier and TMA helpers, the tensor map encoder
 
 namespace custen {
 namespace ch {
@@ -72,37 +64,28 @@ __device__ double g_rhs_factors[3] = {2.0, -4.0, -2.0 / 3.0};
 
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restrict__ grids,
-                                                          const Item* __restrict__ items, int n_items, int parity,
-                                                          unsigned int* counter) {
+                                                          const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T cb[36][37];        // cBar over the block and a 2-point halo
     __shared__ T hh[34][35];        // sigma_nl * (c^3 - c), then h, over the block and a 1-point halo
     __shared__ double dco[32][33];  // cCurr - cOld at the block's points (FP64 in both variants)
-    __shared__ int s_item;
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
     const double m_four_d = factors[1], m_two_thirds_d = factors[2];
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();
-        if (it >= n_items) break;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
+        const int n = gd.n;
         // selects rather than gd.buf[parity]: a run-time index would put the descriptor in local memory
         const double* cur = parity ? gd.buf[1] : gd.buf[0];
         const double* old = parity ? gd.buf[0] : gd.buf[1];
         const double* tab = gd.tab;
         const int bpr = n / BLK;
         const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        // sigma_lin and sigma_nl, exactly: the far weight of the biharmonic is -sigma_lin, the north weight
-        // of the Laplacian sigma_nl (the table stores the weights as pattern * sigma)
-        const T s_lin = (T)(-tab[7 * m + 8 + 2]);
-        const T s_nl = (T)tab[7 * m + 33 + 1];
+        const T s_lin = (T)tab[TAB_SLIN];
+        const T s_nl = (T)tab[TAB_SNL];
         // stage the 36 x 36 window (periodic wrap)
 #pragma unroll 4
         for (int e = tid; e < 36 * 36; e += NT) {
@@ -154,31 +137,24 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
 // Pass 1: h = sigma_nl * (c^3 - c) - sigma_lin * Lap(cBar), cBar over the block and a 1-point halo.
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restrict__ grids,
-                                                        const Item* __restrict__ items, int n_items, int parity,
-                                                        unsigned int* counter) {
+                                                        const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T cb[34][35];
     __shared__ T gg[32][33];   // sigma_nl * (c^3 - c)
-    __shared__ int s_item;
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();
-        if (it >= n_items) break;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
+        const int n = gd.n;
         const double* cur = parity ? gd.buf[1] : gd.buf[0];
         const double* old = parity ? gd.buf[0] : gd.buf[1];
         const double* tab = gd.tab;
         const int bpr = n / BLK;
         const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const T s_lin = (T)(-tab[7 * m + 8 + 2]);
-        const T s_nl = (T)tab[7 * m + 33 + 1];
+        const T s_lin = (T)tab[TAB_SLIN];
+        const T s_nl = (T)tab[TAB_SNL];
 #pragma unroll 4
         for (int e = tid; e < 34 * 34; e += NT) {
             const int r = e / 34, c = e - r * 34;
@@ -207,22 +183,15 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
 // 1-point halo from the h buffer.
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __restrict__ grids,
-                                                           const Item* __restrict__ items, int n_items, int parity,
-                                                           unsigned int* counter) {
+                                                           const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T hh[34][35];
     __shared__ T dco[32][33];
-    __shared__ int s_item;
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const T m_four = (T)factors[1], m_two_thirds = (T)factors[2];
-    for (;;) {
-        if (tid == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncthreads();
-        const int it = s_item;
-        __syncthreads();
-        if (it >= n_items) break;
+    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
         const int n = gd.n;
@@ -305,23 +274,19 @@ __device__ __forceinline__ void rhs2_issue(double* buf, const GridDev& gd, const
 template <int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* __restrict__ grids,
                                                                 const Item* __restrict__ items, int n_items,
-                                                                int parity, unsigned int* counter) {
+                                                                int parity) {
     extern __shared__ __align__(16) double rhs2_smem[];
-    __shared__ int s_next[2];
     const int tid = threadIdx.x;
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const double m_four = factors[1], m_two_thirds = factors[2];
-    if (tid == 0) s_next[1] = (int)atomicAdd(counter, 1u);
-    __syncthreads();
-    int it_cur = s_next[1];
+    int it_cur = blockIdx.x;
     if (it_cur < n_items) rhs2_issue<NW>(rhs2_smem, grids[items[it_cur].grid], items[it_cur], parity, tid);
     cp_async_commit();
     for (int k = 0;; ++k) {
-        if (it_cur >= n_items) break;   // uniform: every thread read the same claim
-        if (tid == 0) s_next[k & 1] = (int)atomicAdd(counter, 1u);
-        __syncthreads();   // the claim is visible; every thread is done with the other half of the buffer
-        const int it_next = s_next[k & 1];
+        if (it_cur >= n_items) break;
+        __syncthreads();   // every thread is done with the other half of the buffer
+        const int it_next = it_cur + gridDim.x;
         if (it_next < n_items)
             rhs2_issue<NW>(rhs2_smem + ((k + 1) & 1) * kRhs2PipeWords, grids[items[it_next].grid], items[it_next],
                            parity, tid);
@@ -353,440 +318,463 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 }
 
 // ------------------------------------------------------------------------------------------------
-// K2: x sweep (lane = row), 32-column chunks through shared memory
+// K2 / K3: the line solves
 // ------------------------------------------------------------------------------------------------
-// The recurrences are latency chains of FP64 operations; everything else is taken off their path:
-// the 32 solver-table entries of a chunk are loaded once, coalesced (lane k holds entry k), and
-// broadcast with shuffles as the chain walks the chunk, and a chunk's 32 x 32 field values are all
-// in flight before the chain starts.
-__global__ void __launch_bounds__(BLK) ch_xsolve_kernel(const GridDev* __restrict__ grids,
-                                                        const Item* __restrict__ items, int n_items,
-                                                        unsigned int* counter) {
-    __shared__ double blk[BLK][BLK + 1];
-    __shared__ int s_item;
-    const int lane = threadIdx.x;
-    const unsigned FULL = 0xffffffffu;
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        double* rows = gd.tmp + (size_t)item.block * BLK * n;   // 32 rows, stride n
-        const int nchunk = n / BLK;
-        // forward elimination of the banded (n-2) x (n-2) block, row = lane
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        for (int ch = 0; ch < nchunk; ++ch) {
-            const int cx = ch * BLK;
-            const int il = cx + lane;
-            const double tds = il < m ? ds[il] : 0.0, tdl = il < m ? dl[il] : 0.0, trd = il < m ? rd[il] : 0.0;
-            double v[BLK];
+// Each line is a circulant pentadiagonal system A x = r, A = 1 + sigma_lin D^4 (the two unknowns that the reference
+// splits off, BatchHyper.cu:195-259, are its way of closing the same circulant). Its symbol is positive, so it
+// factors as A = G P(z) P(1/z) with P(z) = 1 + p1 / z + p2 / z^2 causal and minimum phase (line_factor, below):
+// constant coefficients, two multiply-adds per element and direction, no pivots and no tables, against five and
+// a table row for the banded factors. The constant G is applied once, in the update.
+//
+// A line is solved by two chains that meet in its middle (one warp each, a lane per line):
+//   - cut the ring between its last and first element and let the right-hand side be zero beyond both ends: on that
+//     infinite line chain A runs u = r / P(z) from the left end to the middle, chain B the mirrored w = r / P(1/z)
+//     from the right end. v = A^-1 r satisfies P(1/z) v = u left of the middle and P(z) v = w right of it, which
+//     makes the four values of v around the middle a constant 4 x 4 system in the chains' last two values each
+//     (TAB_MID); from there each chain runs back to its end;
+//   - close the ring: the periodic solution is v summed over all its translates by n. To the right of the line v
+//     decays as the homogeneous solutions of P, so the translates from the left add alpha1 f1(i) + alpha2 f2(i) with
+//     (alpha1, alpha2) = (1 - M^n)^-1 (v[n-1], v[n-2]) (TAB_CLOSE; M the one-step matrix), and the mirrored sum at
+//     the other end adds beta1 f1(n-1-i) + beta2 f2(n-1-i). f1 and f2 fall off; beyond TAB_REACH entries (2^-62 of
+//     their peak) they are left out.
+// The x sweep's closure is applied where the y sweep reads, the y sweep's in the update. Per point that is 8
+// multiply-adds for the recurrences and 2 for each end within reach, against 10 and 4, and a line's dependent chain
+// is half as long. The arithmetic is a function of n, lx, gamma and dt alone, so a grid's result does not depend
+// on its batch.
+//
+// A warp's FP64 instruction holds its sub-partition's FP64 pipe for 64 cycles however few lanes it has, so with
+// fewer chains than FP64 sub-partitions (4 per SM) a step takes the chain's instruction count: n / 2 elements
+// of 4 instructions per sweep. Measured, us per step (before: banded factors, one warp per 32 lines): one grid of 256^2
+// 66 (159), 512^2 118 (298), 1024^2 252 (601), 2048^2 577 (1331); 96 grids of 64^2 .. 1024^2 1680 (1973).
+
+// Chunks of kChunk elements of a warp's 32 lines move between the work field and a shared-memory ring of kStages
+// stages by the tensor memory accelerator, one copy per chunk each way, issued by a copy warp per chain (two chain
+// warps and two copy warps make a CTA): the recurrence has the issue slots to itself, and a chain alone on its
+// sub-partition keeps the FP64 pipe busy. Measured, x sweep of one 512^2 grid (32 us of FP64 instructions): 44 us;
+// the copies issued by the chain warp itself 48 us; its lanes copying with 8-byte cp.async and stores 63 us; with bulk
+// copies of 128 bytes per lane 106 us (each occupies the copy engine for about 50 cycles). A
+// chunk is solved in place in its stage and copied back from there. At the middle the last kStages chunks are
+// still in the ring; the backward pass starts from them and they never make the round trip through the work field.
+constexpr int kChunk = 16, kStages = 4;
+using Forward = std::true_type;
+using Backward = std::false_type;
+
+__device__ __forceinline__ void pair_barrier() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+
+__device__ __forceinline__ void bulk_load(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(smem)),
+                 "l"(gmem), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* smem) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(smem_u32(smem))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// this thread's copies out of shared memory have read their source / have completed
+__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// The map lies in device memory that the host writes between launches: made visible to the copy engine.
+__device__ __forceinline__ void acquire_map(const CUtensorMap* map) {
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map))
+                 : "memory");
+}
+
+// The value next to the chain's end and the one behind it, from the chains' ends (TAB_MID row 0 and 1).
+__device__ __forceinline__ double mid_value(const double* q, double own1, double own2, double oth1, double oth2) {
+    return fma(q[0], own1, fma(q[1], own2, fma(q[2], oth1, q[3] * oth2)));
+}
+
+// The ring of one chain: full[s] completes when a chunk has arrived in stage s, done[s] when it has been solved
+// there and may be copied out.
+struct ChainBars {
+    uint64_t full[kStages], done[kStages];
+};
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.release.cta.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Waits on the stages' barriers in turn; after one has expired (stencil_tma.cuh) none waits any more, so the
+// warps of a CTA run to their end and meet at its barriers whatever happened; the results are void then.
+struct RingWait {
+    unsigned parity = 0;   // per stage: the phase its next completion ends
+    bool ok = true;
+    __device__ __forceinline__ void operator()(uint64_t* bars, int st) {
+        if (ok) ok = mbar_wait(&bars[st], (parity >> st) & 1u);
+        parity ^= 1u << st;
+    }
+    __device__ __forceinline__ void report() const {
+        if (!ok) atomicOr(&g_custen_device_error, kErrMbarrierTimeout);
+    }
+};
+
+// The copy warp of a chain (one lane): load(c, stage, pass) starts the copy of chunk c on the stage's full
+// barrier, store(c, stage) the copy back. A stage is refilled once its store has read it.
+template <class Load, class Store>
+__device__ __forceinline__ void run_copies(int nchunk, ChainBars& bars, Load load, Store store) {
+    RingWait done;
+    for (int c = 0; c < kStages && c < nchunk; ++c) load(c, c, Forward{});
+    for (int c = 0; c < nchunk - kStages; ++c) {
+        const int st = c % kStages;
+        done(bars.done, st);
+        fence_proxy_async_smem();
+        store(c, st);
+        bulk_wait_read_all();
+        load(c + kStages, st, Forward{});
+    }
+    bulk_wait_all();   // the backward pass reads the forward pass's chunks again
+    for (int c = nchunk - 1; c >= 0; --c) {
+        const int st = c % kStages;
+        done(bars.done, st);
+        fence_proxy_async_smem();
+        store(c, st);
+        if (c >= kStages) {
+            bulk_wait_read_all();
+            load(c - kStages, st, Backward{});
+        }
+    }
+    bulk_wait_all();
+    done.report();
+}
+
+// The chain itself (a lane per line): solve(stage, a1, a2, pass) runs the recurrence over a chunk in place, from
+// the last two values; v1, v2: the values at the chain's outer end.
+template <class Solve>
+__device__ __forceinline__ void run_chain(int nchunk, ChainBars& bars, double (*own)[BLK], double (*other)[BLK], int lane,
+                                          const double* mid, double& v1, double& v2, Solve solve) {
+    RingWait full;
+    auto solved = [&](int st) {
+        __syncwarp();   // every lane's writes
+        if (lane == 0) mbar_arrive(&bars.done[st]);
+    };
+    double u1 = 0.0, u2 = 0.0;
+    for (int c = 0; c < nchunk; ++c) {
+        const int st = c % kStages;
+        full(bars.full, st);
+        solve(st, u1, u2, Forward{});
+        if (c < nchunk - kStages) solved(st);
+    }
+    own[0][lane] = u1;
+    own[1][lane] = u2;
+    pair_barrier();
+    const double o1 = other[0][lane], o2 = other[1][lane];
+    v1 = mid_value(mid, u1, u2, o1, o2);
+    v2 = mid_value(mid + 4, u1, u2, o1, o2);
+    for (int c = nchunk - 1; c >= 0; --c) {
+        const int st = c % kStages;
+        if (c < nchunk - kStages) full(bars.full, st);
+        solve(st, v1, v2, Backward{});
+        solved(st);
+    }
+    if (lane == 0) full.report();
+}
+
+// The recurrence over kChunk values in registers, w[0] first: v = w + np1 v1 + np2 v2.
+__device__ __forceinline__ void recur(double (&w)[kChunk], double np1, double np2, double& v1, double& v2) {
 #pragma unroll
-            for (int rr = 0; rr < BLK; ++rr) v[rr] = rows[(size_t)rr * n + il];
+    for (int k = 0; k < kChunk; ++k) {
+        w[k] = fma(np1, v1, fma(np2, v2, w[k]));
+        v2 = v1;
+        v1 = w[k];
+    }
+}
+
+// x sweep: DIR = 1 is chain A (columns upwards), -1 chain B. A stage holds 32 rows of 128 bytes in the 128-byte
+// swizzle (the 16-byte unit u of row r lies at u ^ (r & 7)), in which a lane per row reads and writes 16 bytes at a
+// time without bank conflicts.
+template <int DIR>
+__device__ __forceinline__ int chunk_origin(int n, int c) { return DIR > 0 ? c * kChunk : n - (c + 1) * kChunk; }
+
+template <int DIR>
+__device__ __forceinline__ void xsweep_copies(const GridDev& gd, const CUtensorMap* map, int block,
+                                              double (*stage)[BLK][kChunk], ChainBars& bars) {
+    const int n = gd.n;
+    auto load = [&](int c, int st, auto) {
+        mbar_arrive_expect_tx(&bars.full[st], BLK * kChunk * sizeof(double));
+        tma_load_2d(&stage[st][0][0], map, chunk_origin<DIR>(n, c), block * BLK, &bars.full[st]);
+    };
+    auto store = [&](int c, int st) {
+        const int x = chunk_origin<DIR>(n, c);
+        if (!in_bounds(x, 0, n - kChunk + 1) || !in_bounds(block * BLK, 0, n - BLK + 1)) return;
+        tma_store_2d(map, x, block * BLK, &stage[st][0][0]);
+        bulk_commit();
+    };
+    run_copies(n / 2 / kChunk, bars, load, store);
+}
+
+template <int DIR>
+__device__ __forceinline__ void xsweep_chain(const GridDev& gd, int block, int lane, double (*stage)[BLK][kChunk],
+                                             ChainBars& bars, double (*own)[BLK], double (*other)[BLK]) {
+    const int n = gd.n;
+    const double np1 = gd.tab[TAB_NP1], np2 = gd.tab[TAB_NP2];
+    const int swz = lane & 7;
+    auto solve = [&](int st, double& a1, double& a2, auto forward) {
+        double2* p = reinterpret_cast<double2*>(&stage[st][lane][0]);
+        constexpr bool up = (DIR > 0) == decltype(forward)::value;
+        double w[kChunk];
 #pragma unroll
-            for (int rr = 0; rr < BLK; ++rr) blk[rr][lane] = v[rr];
-            __syncwarp();
+        for (int k = 0; k < kChunk / 2; ++k) {
+            const double2 q = p[(up ? k : kChunk / 2 - 1 - k) ^ swz];
+            w[2 * k] = up ? q.x : q.y;
+            w[2 * k + 1] = up ? q.y : q.x;
+        }
+        recur(w, np1, np2, a1, a2);
 #pragma unroll
-            for (int k = 0; k < BLK; ++k) {
-                const int i = cx + k;
-                const double x = blk[lane][k];
-                const double a_s = __shfl_sync(FULL, tds, k), a_l = __shfl_sync(FULL, tdl, k);
-                const double a_r = __shfl_sync(FULL, trd, k);
-                if (i < m) {
-                    double t = fma(-a_s, b2, x);
-                    t = fma(-a_l, b1, t);
-                    t *= a_r;
-                    b2 = b1;
-                    b1 = t;
-                    blk[lane][k] = t;
-                } else if (i == m) {
-                    r2 = x;
-                } else {
-                    r1 = x;
-                }
+        for (int k = 0; k < kChunk / 2; ++k)
+            p[(up ? k : kChunk / 2 - 1 - k) ^ swz] =
+                up ? make_double2(w[2 * k], w[2 * k + 1]) : make_double2(w[2 * k + 1], w[2 * k]);
+    };
+    double v1, v2;
+    run_chain(n / 2 / kChunk, bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
+    const double* cl = gd.tab + TAB_CLOSE;
+    const int y = block * BLK + lane;
+    if (in_bounds(4 * y + 3, 0, 4 * n)) {
+        gd.ends[4 * y + (DIR > 0 ? 2 : 0)] = fma(cl[0], v1, cl[1] * v2);
+        gd.ends[4 * y + (DIR > 0 ? 3 : 1)] = fma(cl[2], v1, cl[3] * v2);
+    }
+}
+
+__device__ __forceinline__ void init_ring(ChainBars (&bars)[2]) {
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 2; ++k)
+            for (int st = 0; st < kStages; ++st) {
+                mbar_init(&bars[k].full[st], 1);
+                mbar_init(&bars[k].done[st], 1);
             }
-            __syncwarp();
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
+
+// The ring's base, aligned for the 128-byte swizzle inside 1 KB of slack (as in stencil_tma.cuh, through an opaque
+// value, since the compiler may not assume more than the declared alignment).
+__device__ __forceinline__ double* ring_base(unsigned char* raw) {
+    uint32_t addr = smem_u32(raw);
+    asm volatile("" : "+r"(addr));
+    return reinterpret_cast<double*>(raw + ((1024u - (addr & 1023u)) & 1023u));
+}
+
+constexpr int kStageWords = BLK * kChunk;
+constexpr size_t kSweepBytes = 2 * kStages * kStageWords * sizeof(double) + 1024;   // dynamic shared memory
+
+constexpr int kSweepThreads = 4 * BLK;   // warps: chain A, chain B, the copies of A, the copies of B
+
+__global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev* __restrict__ grids,
+                                                                  const Item* __restrict__ items,
+                                                                  const CUtensorMap* maps) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    __shared__ double ex[2][2][BLK];
+    __shared__ __align__(8) ChainBars bars[2];
+    init_ring(bars);
+    const int lane = threadIdx.x & (BLK - 1), warp = threadIdx.x / BLK;
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    const CUtensorMap* map = maps + 2 * item.grid;
+    auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base(sweep_smem));
+    if (warp == 0) xsweep_chain<1>(gd, item.block, lane, stage, bars[0], ex[0], ex[1]);
+    else if (warp == 1) xsweep_chain<-1>(gd, item.block, lane, stage + kStages, bars[1], ex[1], ex[0]);
+    else if (lane == 0) {
+        acquire_map(map);
+        if (warp == 2) xsweep_copies<1>(gd, map, item.block, stage, bars[0]);
+        else xsweep_copies<-1>(gd, map, item.block, stage + kStages, bars[1]);
+    }
+}
+
+// y sweep: DIR = 1 is chain A (rows upwards). CLOSE: the x sweep's closure is added to the right-hand side as a
+// chunk is read, in the columns within reach of either end, by the rows' amplitudes (copied with the chunk).
+// Without it ch_xclose_kernel has added it, with the same operations.
+struct CloseEnds {
+    bool left, right;   // whether the block's columns lie within reach of either end
+    __device__ __forceinline__ CloseEnds(const GridDev& gd, int block) {
+        const int reach = (int)gd.tab[TAB_REACH];
+        left = block * BLK < reach;
+        right = (block + 1) * BLK > gd.n - reach;
+    }
+};
+
+template <int DIR, bool CLOSE>
+__device__ __forceinline__ void ysweep_copies(const GridDev& gd, const CUtensorMap* map, int block,
+                                              double (*stage)[kChunk][BLK], double (*amp)[kChunk][4], ChainBars& bars) {
+    const int n = gd.n;
+    const CloseEnds ends(gd, block);
+    auto load = [&](int c, int st, auto forward) {
+        const int y = chunk_origin<DIR>(n, c);
+        const bool amps = CLOSE && decltype(forward)::value && (ends.left || ends.right);
+        mbar_arrive_expect_tx(&bars.full[st], kChunk * BLK * sizeof(double) + (amps ? kChunk * 4 * sizeof(double) : 0));
+        tma_load_2d(&stage[st][0][0], map, block * BLK, y, &bars.full[st]);
+        if (amps) bulk_load(&amp[st][0][0], gd.ends + 4 * y, kChunk * 4 * sizeof(double), &bars.full[st]);
+    };
+    auto store = [&](int c, int st) {
+        const int y = chunk_origin<DIR>(n, c);
+        if (!in_bounds(y, 0, n - kChunk + 1) || !in_bounds(block * BLK, 0, n - BLK + 1)) return;
+        tma_store_2d(map, block * BLK, y, &stage[st][0][0]);
+        bulk_commit();
+    };
+    run_copies(n / 2 / kChunk, bars, load, store);
+}
+
+template <int DIR, bool CLOSE>
+__device__ __forceinline__ void ysweep_chain(const GridDev& gd, int block, int lane, double (*stage)[kChunk][BLK],
+                                             double (*amp)[kChunk][4], ChainBars& bars, double (*own)[BLK],
+                                             double (*other)[BLK]) {
+    const int n = gd.n;
+    const double np1 = gd.tab[TAB_NP1], np2 = gd.tab[TAB_NP2];
+    const int x = block * BLK + lane;
+    double l1 = 0.0, l2 = 0.0, r1 = 0.0, r2 = 0.0;
+    const CloseEnds ends_of(gd, block);
+    const bool left = ends_of.left, right = ends_of.right;   // uniform over the warp
+    if (CLOSE) {
+        const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
+        l1 = f1[x]; l2 = f2[x]; r1 = f1[n - 1 - x]; r2 = f2[n - 1 - x];
+    }
+    auto solve = [&](int st, double& a1, double& a2, auto forward) {
+        constexpr bool up = (DIR > 0) == decltype(forward)::value;
+        double w[kChunk];
 #pragma unroll
-            for (int rr = 0; rr < BLK; ++rr)
-                if (in_bounds((long long)(item.block * BLK + rr) * n + il, 0, (long long)n * n))
-                    rows[(size_t)rr * n + il] = blk[rr][lane];
-            __syncwarp();
-        }
-        // backward substitution, chunks in reverse
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        for (int ch = nchunk - 1; ch >= 0; --ch) {
-            const int cx = ch * BLK;
-            const int il = cx + lane;
-            const double tdu = il < m ? du[il] : 0.0, tdw = il < m ? dw[il] : 0.0;
-            double v[BLK];
+        for (int k = 0; k < kChunk; ++k) w[k] = stage[st][up ? k : kChunk - 1 - k][lane];
+        if (CLOSE && decltype(forward)::value && (left || right)) {
 #pragma unroll
-            for (int rr = 0; rr < BLK; ++rr) v[rr] = rows[(size_t)rr * n + il];
-#pragma unroll
-            for (int rr = 0; rr < BLK; ++rr) blk[rr][lane] = v[rr];
-            __syncwarp();
-#pragma unroll
-            for (int k = BLK - 1; k >= 0; --k) {
-                const int i = cx + k;
-                const double a_u = __shfl_sync(FULL, tdu, k), a_w = __shfl_sync(FULL, tdw, k);
-                if (i < m) {
-                    double y = fma(-a_u, f1, blk[lane][k]);
-                    y = fma(-a_w, f2, y);
-                    f2 = f1;
-                    f1 = y;
-                    blk[lane][k] = y;
-                    if (i == 0) y0v = y;
-                    if (i == 1) y1v = y;
-                    if (i == m - 2) ym2 = y;
-                    if (i == m - 1) ym1 = y;
-                }
+            for (int k = 0; k < kChunk; ++k) {
+                const double* e = amp[st][up ? k : kChunk - 1 - k];
+                if (left) w[k] = fma(l1, e[0], fma(l2, e[1], w[k]));
+                if (right) w[k] = fma(r1, e[2], fma(r2, e[3], w[k]));
             }
-            __syncwarp();
+        }
+        recur(w, np1, np2, a1, a2);
 #pragma unroll
-            for (int rr = 0; rr < BLK; ++rr)
-                if (in_bounds((long long)(item.block * BLK + rr) * n + il, 0, (long long)n * n))
-                    rows[(size_t)rr * n + il] = blk[rr][lane];
-            __syncwarp();
-        }
-        // the last two unknowns through the 2 x 2 Schur complement (BatchHyper.cu:195-227)
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        double* row = rows + (size_t)lane * n;
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        row[n - 2] = x2;
-        row[n - 1] = x1;
-        // kept apart as well: the y sweep overwrites columns n-2 and n-1 of tmp while other warps still
-        // need them for the rank-2 correction
-        const int gy = item.block * BLK + lane;
-        if (in_bounds(2 * gy + 1, 0, 2 * n)) {
-            gd.ends[2 * gy] = x2;
-            gd.ends[2 * gy + 1] = x1;
-        }
+        for (int k = 0; k < kChunk; ++k) stage[st][up ? k : kChunk - 1 - k][lane] = w[k];
+    };
+    double v1, v2;
+    run_chain(n / 2 / kChunk, bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
+    const double* cl = gd.tab + TAB_CLOSE;
+    double* ends = gd.ends + 4 * n;
+    if (in_bounds(4 * x + 3, 0, 4 * n)) {
+        ends[4 * x + (DIR > 0 ? 2 : 0)] = fma(cl[0], v1, cl[1] * v2);
+        ends[4 * x + (DIR > 0 ? 3 : 1)] = fma(cl[2], v1, cl[3] * v2);
+    }
+}
+
+template <bool CLOSE>
+__global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev* __restrict__ grids,
+                                                                  const Item* __restrict__ items,
+                                                                  const CUtensorMap* maps) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    __shared__ __align__(16) double amp[CLOSE ? 2 * kStages : 1][kChunk][4];
+    __shared__ double ex[2][2][BLK];
+    __shared__ __align__(8) ChainBars bars[2];
+    init_ring(bars);
+    const int lane = threadIdx.x & (BLK - 1), warp = threadIdx.x / BLK;
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    const CUtensorMap* map = maps + 2 * item.grid + 1;
+    auto* stage = reinterpret_cast<double(*)[kChunk][BLK]>(ring_base(sweep_smem));
+    auto* amp_b = amp + (CLOSE ? kStages : 0);
+    if (warp == 0) ysweep_chain<1, CLOSE>(gd, item.block, lane, stage, amp, bars[0], ex[0], ex[1]);
+    else if (warp == 1) ysweep_chain<-1, CLOSE>(gd, item.block, lane, stage + kStages, amp_b, bars[1], ex[1], ex[0]);
+    else if (lane == 0) {
+        acquire_map(map);
+        if (warp == 2) ysweep_copies<1, CLOSE>(gd, map, item.block, stage, amp, bars[0]);
+        else ysweep_copies<-1, CLOSE>(gd, map, item.block, stage + kStages, amp_b, bars[1]);
+    }
+}
+
+// The x sweep's closure as an element-wise kernel over the 32 x 32 blocks, for batches with few chains (it spreads
+// over every SM, where in the y sweep it would lengthen the chains).
+__global__ void __launch_bounds__(256) ch_xclose_kernel(const GridDev* __restrict__ grids,
+                                                        const Item* __restrict__ items) {
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    if (gd.general) return;
+    const int n = gd.n;
+    const int bpr = n / BLK;
+    const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
+    const int reach = (int)gd.tab[TAB_REACH];
+    const bool left = x0 < reach, right = x0 + BLK > n - reach;
+    if (!left && !right) return;
+    const int x = x0 + (threadIdx.x & (BLK - 1));
+    const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
+    const double l1 = f1[x], l2 = f2[x], r1 = f1[n - 1 - x], r2 = f2[n - 1 - x];
+    const int r0 = threadIdx.x / BLK;
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = gd.tmp[(size_t)(y0 + r0 + 8 * k) * n + x];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int y = y0 + r0 + 8 * k;
+        const double* e = gd.ends + 4 * y;
+        if (left) v[k] = fma(l1, e[0], fma(l2, e[1], v[k]));
+        if (right) v[k] = fma(r1, e[2], fma(r2, e[3], v[k]));
+        if (in_bounds((long long)y * n + x, 0, (long long)n * n)) gd.tmp[(size_t)y * n + x] = v[k];
+    }
+}
+
+// K4: cNew = cBar + delta written over cOld (cuPentCahnADI.cu:58-69, 89-100), one 32 x 32 block per CTA: delta is
+// kappa times the y solution with its closure, for the rows within reach of either end.
+__global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restrict__ grids,
+                                                        const Item* __restrict__ items, int parity) {
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    if (gd.general) return;   // its y sweep has updated the field
+    const int n = gd.n;
+    const int bpr = n / BLK;
+    const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
+    const int x = x0 + (threadIdx.x & (BLK - 1));
+    const int reach = (int)gd.tab[TAB_REACH];
+    const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
+    const bool top = y0 < reach, bottom = y0 + BLK > n - reach;
+    const double two = ((const volatile double*)g_rhs_factors)[0];
+    const double kappa = gd.tab[TAB_KAPPA];
+    const double* e = gd.ends + 4 * n + 4 * x;
+    double a1 = 0.0, a2 = 0.0, b1 = 0.0, b2 = 0.0;
+    if (top) { a1 = e[0]; a2 = e[1]; }
+    if (bottom) { b1 = e[2]; b2 = e[3]; }
+    const double* cur = parity ? gd.buf[1] : gd.buf[0];
+    double* old = parity ? gd.buf[0] : gd.buf[1];
+    const int r0 = threadIdx.x / BLK;
+    double v[4], cv[4], ov[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const size_t q = (size_t)(y0 + r0 + 8 * k) * n + x;
+        v[k] = gd.tmp[q];
+        cv[k] = cur[q];
+        ov[k] = old[q];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int y = y0 + r0 + 8 * k;
+        const long long q = (long long)y * n + x;
+        double d = v[k];
+        if (top) d = fma(f1[y], a1, fma(f2[y], a2, d));
+        if (bottom) d = fma(f1[n - 1 - y], b1, fma(f2[n - 1 - y], b2, d));
+        if (in_bounds(q, 0, (long long)n * n)) old[q] = fma(kappa, d, fma(two, cv[k], -ov[k]));
     }
 }
 
 // ------------------------------------------------------------------------------------------------
-// K3: y sweep (lane = column) + the update
+// General sweeps: the line solved as the (n-2) x (n-2) banded block with its pre-computed factors plus the 2 x 2
+// Schur complement on the last two unknowns (cuPentBatch.cu:35-198, BatchHyper.cu:195-259, 421-514). For
+//   - a negative sigma_lin (a negative gamma or time step): the symbol may vanish and has no real causal factor;
+//   - the precision variant: it rounds the fields to FP32 every step, which turns any other last bit of a solve into
+//     a difference of FP32 rounding size (2e-7 after 40 steps), so its results are tied to these operations.
+// One warp per 32 lines; table entries are held in registers, field values come through cp.async.
 // ------------------------------------------------------------------------------------------------
-// Rows are taken 32 at a time: the batch's field values are loaded into registers first (32 loads
-// in flight per lane) and the batch's table entries / row ends are loaded coalesced and broadcast
-// with shuffles, so the FP64 recurrence does not wait on memory.
-// CH rows per batch (16 or 32): the three CH-deep register arrays of the update set the register use,
-// hence how many warps fit on an SM (the tuned choice, ChConfig).
-template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_kernel(const GridDev* __restrict__ grids,
-                                                        const Item* __restrict__ items, int n_items, int parity,
-                                                        unsigned int* counter) {
-    __shared__ int s_item;
-    const int lane = threadIdx.x;
-    const unsigned FULL = 0xffffffffu;
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        const double* inv1 = tab + 5 * m;
-        const double* inv2 = tab + 6 * m;
-        const int x = item.block * BLK + lane;
-        double* t = gd.tmp;
-        const double* ends = gd.ends;
-        // x sweep's rank-2 correction for this column (BatchHyper.cu:233-259): applied on read
-        const bool corr = x < m;
-        const double cx1 = corr ? inv1[x] : 0.0;
-        const double cx2 = corr ? inv2[x] : 0.0;
-        const int nb = n / CH;
-        // forward elimination along y
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        for (int bb = 0; bb < nb; ++bb) {
-            const int yb = bb * CH, yl = yb + lane;
-            const double tds = yl < m ? ds[yl] : 0.0, tdl = yl < m ? dl[yl] : 0.0, trd = yl < m ? rd[yl] : 0.0;
-            const double e2 = yl < n ? ends[2 * yl] : 0.0, e1 = yl < n ? ends[2 * yl + 1] : 0.0;
-            double v[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) v[k] = t[(size_t)(yb + k) * n + x];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int y = yb + k;
-                const double c2 = __shfl_sync(FULL, e2, k), c1 = __shfl_sync(FULL, e1, k);
-                const double a_s = __shfl_sync(FULL, tds, k), a_l = __shfl_sync(FULL, tdl, k);
-                const double a_r = __shfl_sync(FULL, trd, k);
-                const double val = corr ? fma(-cx1, c2, fma(-cx2, c1, v[k])) : v[k];
-                if (y < m) {
-                    double w = fma(-a_s, b2, val);
-                    w = fma(-a_l, b1, w);
-                    w *= a_r;
-                    b2 = b1;
-                    b1 = w;
-                    v[k] = w;
-                } else if (y == m) {
-                    r2 = val;
-                } else {
-                    r1 = val;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k)
-                if (yb + k < m && in_bounds((long long)(yb + k) * n + x, 0, (long long)n * n))
-                    t[(size_t)(yb + k) * n + x] = v[k];
-        }
-        // backward substitution
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        for (int bb = nb - 1; bb >= 0; --bb) {
-            const int yb = bb * CH, yl = yb + lane;
-            const double tdu = yl < m ? du[yl] : 0.0, tdw = yl < m ? dw[yl] : 0.0;
-            double v[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) v[k] = (yb + k < m) ? t[(size_t)(yb + k) * n + x] : 0.0;
-#pragma unroll
-            for (int k = CH - 1; k >= 0; --k) {
-                const int y = yb + k;
-                const double a_u = __shfl_sync(FULL, tdu, k), a_w = __shfl_sync(FULL, tdw, k);
-                if (y < m) {
-                    double w = fma(-a_u, f1, v[k]);
-                    w = fma(-a_w, f2, w);
-                    f2 = f1;
-                    f1 = w;
-                    v[k] = w;
-                    if (y == m - 1) ym1 = w;
-                    if (y == m - 2) ym2 = w;
-                    if (y == 1) y1v = w;
-                    if (y == 0) y0v = w;
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k)
-                if (yb + k < m && in_bounds((long long)(yb + k) * n + x, 0, (long long)n * n))
-                    t[(size_t)(yb + k) * n + x] = v[k];
-        }
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        // cNew = cBar + delta over cOld (cuPentCahnADI.cu:58-69, 89-100)
-        const double two = ((const volatile double*)g_rhs_factors)[0];   // register operand, as in K1
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        double* old = parity ? gd.buf[0] : gd.buf[1];
-        for (int bb = 0; bb < nb; ++bb) {
-            const int yb = bb * CH, yl = yb + lane;
-            const double ti1 = yl < m ? inv1[yl] : 0.0, ti2 = yl < m ? inv2[yl] : 0.0;
-            double v[CH], cv[CH], ov[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const size_t q = (size_t)(yb + k) * n + x;
-                v[k] = (yb + k < m) ? t[q] : 0.0;
-                cv[k] = cur[q];
-                ov[k] = old[q];
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int y = yb + k;
-                const double a1 = __shfl_sync(FULL, ti1, k), a2 = __shfl_sync(FULL, ti2, k);
-                double dlt;
-                if (y < m) dlt = fma(-a1, x2, fma(-a2, x1, v[k]));
-                else dlt = (y == m) ? x2 : x1;
-                const double cbar = fma(two, cv[k], -ov[k]);
-                if (in_bounds((long long)y * n + x, 0, (long long)n * n)) old[(size_t)y * n + x] = cbar + dlt;
-            }
-        }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
-// K2 / K3, pipelined: the same sweeps with the field values of chunk c+1 copied into shared memory
-// (cp.async, double buffered) while the recurrence runs over chunk c
-// ------------------------------------------------------------------------------------------------
-// The recurrences are latency-bound: a warp's chain issues one dependent FP64 operation at a time, so
-// the FP64 pipe stays busy only while other warps have work. In the kernels above a chunk's loads start
-// when its chain is about to run, and the values they stage in registers (32 per lane) limit the warps
-// per SM. Here the loads of the next chunk are in flight during the current chain, they occupy no
-// registers, and the table entries of the next chunk are read one chunk ahead. The arithmetic, its order
-// and so every result are those of the kernels above.
-
-// x sweep (lane = row) over XC-column chunks. Each lane copies, and later writes back, the elements
-// e = lane + 32 j of a chunk (row e / XC, column e % XC): one row segment (XC = 32) or two (XC = 16) per
-// instruction, coalesced; a lane reads back in the backward pass exactly what it stored in the forward
-// pass, so program order alone orders those accesses.
+// x sweep (lane = row) over XC-column chunks.
 template <int XC>
-__global__ void __launch_bounds__(BLK) ch_xsolve_pipe_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items, int n_items,
-                                                             unsigned int* counter) {
-    __shared__ double blk[2][BLK][XC + 1];
-    __shared__ int s_item;
-    const int lane = threadIdx.x;
-    const unsigned FULL = 0xffffffffu;
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        double* rows = gd.tmp + (size_t)item.block * BLK * n;   // 32 rows, stride n
-        const int nchunk = n / XC;
-        // element e = lane + 32 j sits at row j * RPI + lr, column lc of the chunk
-        constexpr int RPI = BLK / XC;
-        const int lr = lane / XC, lc = lane % XC;
-        const size_t step = (size_t)RPI * n;
-        auto issue = [&](int c, int b) {
-            const double* src = rows + (size_t)lr * n + c * XC + lc;
-#pragma unroll 4
-            for (int j = 0; j < XC; ++j, src += step) cp_async8(&blk[b][j * RPI + lr][lc], src);
-            cp_async_commit();
-        };
-        auto write_back = [&](int c, int b) {
-            double* dst = rows + (size_t)lr * n + c * XC + lc;
-#pragma unroll 4
-            for (int j = 0; j < XC; ++j, dst += step)
-                if (in_bounds(dst - gd.tmp, 0, (long long)n * n)) *dst = blk[b][j * RPI + lr][lc];
-        };
-        // forward elimination of the banded (n-2) x (n-2) block
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        issue(0, 0);
-        double tds = lane < m ? ds[lane] : 0.0, tdl = lane < m ? dl[lane] : 0.0, trd = lane < m ? rd[lane] : 0.0;
-        for (int c = 0; c < nchunk; ++c) {
-            const int b = c & 1, cx = c * XC;
-            double nds = 0.0, ndl = 0.0, nrd = 0.0;
-            if (c + 1 < nchunk) {
-                issue(c + 1, b ^ 1);
-                const int il = cx + XC + lane;
-                if (il < m && lane < XC) { nds = ds[il]; ndl = dl[il]; nrd = rd[il]; }
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncwarp();
-#pragma unroll
-            for (int k = 0; k < XC; ++k) {
-                const int i = cx + k;
-                const double x = blk[b][lane][k];
-                const double a_s = __shfl_sync(FULL, tds, k), a_l = __shfl_sync(FULL, tdl, k);
-                const double a_r = __shfl_sync(FULL, trd, k);
-                if (i < m) {
-                    double t = fma(-a_s, b2, x);
-                    t = fma(-a_l, b1, t);
-                    t *= a_r;
-                    b2 = b1;
-                    b1 = t;
-                    blk[b][lane][k] = t;
-                } else if (i == m) {
-                    r2 = x;
-                } else {
-                    r1 = x;
-                }
-            }
-            __syncwarp();
-            write_back(c, b);
-            __syncwarp();   // buffer b is refilled next iteration
-            tds = nds; tdl = ndl; trd = nrd;
-        }
-        // backward substitution, chunks in reverse
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        issue(nchunk - 1, 0);
-        int il0 = (nchunk - 1) * XC + lane;
-        double tdu = (il0 < m && lane < XC) ? du[il0] : 0.0, tdw = (il0 < m && lane < XC) ? dw[il0] : 0.0;
-        for (int j = 0; j < nchunk; ++j) {
-            const int c = nchunk - 1 - j, b = j & 1, cx = c * XC;
-            double ndu = 0.0, ndw = 0.0;
-            if (c > 0) {
-                issue(c - 1, b ^ 1);
-                const int il = cx - XC + lane;
-                if (il < m && lane < XC) { ndu = du[il]; ndw = dw[il]; }
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncwarp();
-#pragma unroll
-            for (int k = XC - 1; k >= 0; --k) {
-                const int i = cx + k;
-                const double a_u = __shfl_sync(FULL, tdu, k), a_w = __shfl_sync(FULL, tdw, k);
-                if (i < m) {
-                    double y = fma(-a_u, f1, blk[b][lane][k]);
-                    y = fma(-a_w, f2, y);
-                    f2 = f1;
-                    f1 = y;
-                    blk[b][lane][k] = y;
-                    if (i == 0) y0v = y;
-                    if (i == 1) y1v = y;
-                    if (i == m - 2) ym2 = y;
-                    if (i == m - 1) ym1 = y;
-                }
-            }
-            __syncwarp();
-            write_back(c, b);
-            __syncwarp();
-            tdu = ndu; tdw = ndw;
-        }
-        // the last two unknowns through the 2 x 2 Schur complement (BatchHyper.cu:195-227)
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        double* row = rows + (size_t)lane * n;
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        row[n - 2] = x2;
-        row[n - 1] = x1;
-        const int gy = item.block * BLK + lane;
-        if (in_bounds(2 * gy + 1, 0, 2 * n)) {
-            gd.ends[2 * gy] = x2;
-            gd.ends[2 * gy + 1] = x1;
-        }
-    }
-}
-
-// The same x sweep with XC-column chunks (8 or 16) whose table entries every lane holds in registers, read with
-// uniform (broadcast) loads when the chunk starts and before its field copies are awaited: the chain
-// then takes no shuffle. The arithmetic is that of the kernels above.
-template <int XC>
-__global__ void __launch_bounds__(BLK) ch_xsolve_pipe_rt_kernel(const GridDev* __restrict__ grids,
-                                                                const Item* __restrict__ items, int n_items,
-                                                                unsigned int* counter) {
+__global__ void __launch_bounds__(BLK) ch_xsolve_general_kernel(const GridDev* __restrict__ grids,
+                                                                const Item* __restrict__ items) {
     constexpr int RPI = BLK / XC;
     __shared__ double blk[2][BLK][XC + 1];
-    __shared__ int s_item;
     const int lane = threadIdx.x;
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
+    {
+        const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
         const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
+        const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
         const double* dl = tab + m;
         const double* rd = tab + 2 * m;
@@ -902,188 +890,19 @@ __global__ void __launch_bounds__(BLK) ch_xsolve_pipe_rt_kernel(const GridDev* _
     }
 }
 
-// y sweep (lane = column) with CH-row batches copied one batch ahead. Each lane reads only its own
-// column, which it copied itself, so no warp barrier is needed around the buffers; results are stored
-// to global memory as the chain produces them. The update runs in register batches of 8 rows.
+// y sweep (lane = column) over CH-row chunks, with the x sweep's rank-2 correction on read and the update.
 template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_pipe_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items, int n_items, int parity,
-                                                             unsigned int* counter) {
+__global__ void __launch_bounds__(BLK) ch_ysolve_general_kernel(const GridDev* __restrict__ grids,
+                                                             const Item* __restrict__ items, int parity) {
     __shared__ double vb[2][CH][BLK];
-    __shared__ int s_item;
-    constexpr int UD = 8;
-    const int lane = threadIdx.x;
-    const unsigned FULL = 0xffffffffu;
-    const double two = ((const volatile double*)g_rhs_factors)[0];
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        const double* inv1 = tab + 5 * m;
-        const double* inv2 = tab + 6 * m;
-        const int x = item.block * BLK + lane;
-        double* t = gd.tmp;
-        const double* ends = gd.ends;
-        const bool corr = x < m;
-        const double cx1 = corr ? inv1[x] : 0.0;
-        const double cx2 = corr ? inv2[x] : 0.0;
-        const int nb = n / CH;
-        auto issue = [&](int bb, int b, bool below_m) {
-            const int yb = bb * CH;
-            const double* src = t + (size_t)yb * n + x;
-#pragma unroll 4
-            for (int k = 0; k < CH; ++k, src += n)
-                if (!below_m || yb + k < m) cp_async8(&vb[b][k][lane], src);
-            cp_async_commit();
-        };
-        // forward elimination along y
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        issue(0, 0, false);
-        double tds = 0.0, tdl = 0.0, trd = 0.0, e2 = 0.0, e1 = 0.0;
-        if (lane < CH) {
-            if (lane < m) { tds = ds[lane]; tdl = dl[lane]; trd = rd[lane]; }
-            e2 = ends[2 * lane];
-            e1 = ends[2 * lane + 1];
-        }
-        for (int bb = 0; bb < nb; ++bb) {
-            const int b = bb & 1, yb = bb * CH;
-            double nds = 0.0, ndl = 0.0, nrd = 0.0, ne2 = 0.0, ne1 = 0.0;
-            if (bb + 1 < nb) {
-                issue(bb + 1, b ^ 1, false);
-                const int yl = yb + CH + lane;
-                if (lane < CH) {
-                    if (yl < m) { nds = ds[yl]; ndl = dl[yl]; nrd = rd[yl]; }
-                    ne2 = ends[2 * yl];
-                    ne1 = ends[2 * yl + 1];
-                }
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int y = yb + k;
-                const double c2 = __shfl_sync(FULL, e2, k), c1 = __shfl_sync(FULL, e1, k);
-                const double a_s = __shfl_sync(FULL, tds, k), a_l = __shfl_sync(FULL, tdl, k);
-                const double a_r = __shfl_sync(FULL, trd, k);
-                const double vk = vb[b][k][lane];
-                const double val = corr ? fma(-cx1, c2, fma(-cx2, c1, vk)) : vk;
-                if (y < m) {
-                    double w = fma(-a_s, b2, val);
-                    w = fma(-a_l, b1, w);
-                    w *= a_r;
-                    b2 = b1;
-                    b1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                } else if (y == m) {
-                    r2 = val;
-                } else {
-                    r1 = val;
-                }
-            }
-            tds = nds; tdl = ndl; trd = nrd; e2 = ne2; e1 = ne1;
-        }
-        // backward substitution (rows below m only; the lane re-reads what it stored above)
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        issue(nb - 1, 0, true);
-        int yl0 = (nb - 1) * CH + lane;
-        double tdu = (lane < CH && yl0 < m) ? du[yl0] : 0.0, tdw = (lane < CH && yl0 < m) ? dw[yl0] : 0.0;
-        for (int j = 0; j < nb; ++j) {
-            const int bb = nb - 1 - j, b = j & 1, yb = bb * CH;
-            double ndu = 0.0, ndw = 0.0;
-            if (bb > 0) {
-                issue(bb - 1, b ^ 1, true);
-                const int yl = yb - CH + lane;
-                if (lane < CH && yl < m) { ndu = du[yl]; ndw = dw[yl]; }
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-#pragma unroll
-            for (int k = CH - 1; k >= 0; --k) {
-                const int y = yb + k;
-                const double a_u = __shfl_sync(FULL, tdu, k), a_w = __shfl_sync(FULL, tdw, k);
-                if (y < m) {
-                    double w = fma(-a_u, f1, vb[b][k][lane]);
-                    w = fma(-a_w, f2, w);
-                    f2 = f1;
-                    f1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                    if (y == m - 1) ym1 = w;
-                    if (y == m - 2) ym2 = w;
-                    if (y == 1) y1v = w;
-                    if (y == 0) y0v = w;
-                }
-            }
-            tdu = ndu; tdw = ndw;
-        }
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        // cNew = cBar + delta over cOld (cuPentCahnADI.cu:58-69, 89-100)
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        double* old = parity ? gd.buf[0] : gd.buf[1];
-        for (int yb = 0; yb < n; yb += UD) {
-            const int yl = yb + (lane & (UD - 1));
-            const double ti1 = yl < m ? inv1[yl] : 0.0, ti2 = yl < m ? inv2[yl] : 0.0;
-            double v[UD], cv[UD], ov[UD];
-#pragma unroll
-            for (int k = 0; k < UD; ++k) {
-                const size_t q = (size_t)(yb + k) * n + x;
-                v[k] = (yb + k < m) ? t[q] : 0.0;
-                cv[k] = cur[q];
-                ov[k] = old[q];
-            }
-#pragma unroll
-            for (int k = 0; k < UD; ++k) {
-                const int y = yb + k;
-                const double a1 = __shfl_sync(FULL, ti1, k), a2 = __shfl_sync(FULL, ti2, k);
-                double dlt;
-                if (y < m) dlt = fma(-a1, x2, fma(-a2, x1, v[k]));
-                else dlt = (y == m) ? x2 : x1;
-                const double cbar = fma(two, cv[k], -ov[k]);
-                if (in_bounds((long long)y * n + x, 0, (long long)n * n)) old[(size_t)y * n + x] = cbar + dlt;
-            }
-        }
-    }
-}
-
-// The same y sweep with the batch's table entries (pivots, multipliers, x-sweep row ends, update
-// factors) held in registers by every lane, read with uniform loads before the batch's copies are
-// awaited: the chain takes no shuffle. The arithmetic is that of the kernels above.
-template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_pipe_rt_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items, int n_items, int parity,
-                                                             unsigned int* counter) {
-    __shared__ double vb[2][CH][BLK];
-    __shared__ int s_item;
     constexpr int UD = 8;
     const int lane = threadIdx.x;
     const double two = ((const volatile double*)g_rhs_factors)[0];
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
+    {
+        const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
         const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
+        const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
         const double* dl = tab + m;
         const double* rd = tab + 2 * m;
@@ -1223,28 +1042,23 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_pipe_rt_kernel(const GridDev* _
     }
 }
 
-// ------------------------------------------------------------------------------------------------
-// K3 split in three (configurations with ysplit): for batches too small to fill the GPU with line warps.
-// ch_xcorr_kernel applies the x sweep's rank-2 correction to the work field, ch_ysolve_split_kernel runs
-// the y recurrences alone and leaves each column's two cyclic unknowns in GridDev::ends, and
-// ch_update_kernel forms cNew = cBar + delta. The expressions are those of ch_ysolve_pipe_rt_kernel, so
-// the results are the same bit for bit. A warp's FP64 instruction holds its sub-partition's FP64 pipe for
-// 64 cycles however few lanes it has, so a column's time in the y sweep is its warp's FP64 instruction
-// count: 5 per element here against 11 in the fused kernel, while the correction and the update spread
-// over every SM as element-wise kernels.
-// ------------------------------------------------------------------------------------------------
+// The y sweep in three, for batches too small to fill the GPU with line warps: ch_xcorr_general_kernel applies the
+// x sweep's rank-2 correction to the work field, ch_ysolve_split_general_kernel runs the recurrences alone and
+// leaves each column's two cyclic unknowns in GridDev::ends, ch_update_general_kernel forms cNew = cBar + delta.
+// Same expressions, same bits.
 // One 32 x 32 block of a grid per CTA (the right-hand side's work list): t[y][x] -= inv1[x] x2(y) +
 // inv2[x] x1(y) for the columns x < n - 2 of the block's rows, as fma(-inv1, x2, fma(-inv2, x1, t)).
-__global__ void __launch_bounds__(256) ch_xcorr_kernel(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(256) ch_xcorr_general_kernel(const GridDev* __restrict__ grids,
                                                        const Item* __restrict__ items) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    if (!gd.general) return;
     const int n = gd.n, m = n - 2;
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     const int x = x0 + (threadIdx.x & (BLK - 1));
     if (x >= m) return;
-    const double cx1 = gd.tab[5 * m + x], cx2 = gd.tab[6 * m + x];
+    const double cx1 = gd.tab[kTabParams + 5 * m + x], cx2 = gd.tab[kTabParams + 6 * m + x];
     for (int r = threadIdx.x / BLK; r < BLK; r += blockDim.x / BLK) {
         const int y = y0 + r;
         const long long q = (long long)y * n + x;
@@ -1255,10 +1069,11 @@ __global__ void __launch_bounds__(256) ch_xcorr_kernel(const GridDev* __restrict
 
 // One 32 x 32 block per CTA: cNew = cBar + delta written over cOld (cuPentCahnADI.cu:58-69, 89-100), delta
 // from the banded y solution in the work field and the column's cyclic unknowns in GridDev::ends.
-__global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* __restrict__ grids,
                                                         const Item* __restrict__ items, int parity) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    if (!gd.general) return;
     const int n = gd.n, m = n - 2;
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
@@ -1271,7 +1086,7 @@ __global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restric
         const int y = y0 + r;
         const long long q = (long long)y * n + x;
         double dlt;
-        if (y < m) dlt = fma(-gd.tab[5 * m + y], x2, fma(-gd.tab[6 * m + y], x1, gd.tmp[q]));
+        if (y < m) dlt = fma(-gd.tab[kTabParams + 5 * m + y], x2, fma(-gd.tab[kTabParams + 6 * m + y], x1, gd.tmp[q]));
         else dlt = (y == m) ? x2 : x1;
         const double cbar = fma(two, cur[q], -old[q]);
         if (in_bounds(q, 0, (long long)n * n)) old[q] = cbar + dlt;
@@ -1279,22 +1094,15 @@ __global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restric
 }
 
 template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_split_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items, int n_items, int parity,
-                                                             unsigned int* counter) {
+__global__ void __launch_bounds__(BLK) ch_ysolve_split_general_kernel(const GridDev* __restrict__ grids,
+                                                             const Item* __restrict__ items) {
     __shared__ double vb[2][CH][BLK];
-    __shared__ int s_item;
     const int lane = threadIdx.x;
-    for (;;) {
-        if (lane == 0) s_item = (int)atomicAdd(counter, 1u);
-        __syncwarp();
-        const int it = s_item;
-        __syncwarp();
-        if (it >= n_items) break;
-        const Item item = items[it];
+    {
+        const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
         const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab;
+        const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
         const double* dl = tab + m;
         const double* rd = tab + 2 * m;
@@ -1336,7 +1144,7 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_split_kernel(const GridDev* __r
                 const double a_s = ts[k], a_l = tl[k];
                 const double a_r = tr[k];
                 const double vk = vb[b][k][lane];
-                const double val = vk;   // corrected by ch_xcorr_kernel
+                const double val = vk;   // corrected by ch_xcorr_general_kernel
                 if (y < m) {
                     double w = fma(-a_s, b2, val);
                     w = fma(-a_l, b1, w);
@@ -1392,42 +1200,43 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_split_kernel(const GridDev* __r
         const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
         const double x2 = om[0] * nx2 + om[1] * nx1;
         const double x1 = om[2] * nx2 + om[3] * nx1;
-        // the column's two cyclic unknowns, for ch_update_kernel (the x sweep's row ends were consumed
-        // by ch_xcorr_kernel, so their buffer is free)
+        // the column's two cyclic unknowns, for ch_update_general_kernel (the x sweep's row ends were consumed
+        // by ch_xcorr_general_kernel, so their buffer is free)
         gd.ends[2 * x] = x2;
         gd.ends[2 * x + 1] = x1;
     }
 }
 
-int ch_launches_per_step(const ChConfig& c) { return 3 + (c.rhs_split ? 1 : 0) + (c.ysplit ? 2 : 0); }
+// Whether the element-wise parts of a sweep run as kernels of their own: with fewer chains than FP64 sub-partitions
+// (4 per SM) a sweep takes as long as one chain, so they are taken out of it.
+static bool few_chains(int chains, int sms) { return chains < 4 * sms; }
+static bool close_apart(const ChConfig& c, const ChWork& w, int sms) {
+    return c.close == 2 || (c.close == 0 && few_chains(2 * (w.n_lines - w.n_general), sms));
+}
+
+int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms) {
+    return (c.rhs_split ? 2 : 1) + (w.n_lines > w.n_general ? 3 + close_apart(c, w, sms) : 0) +
+           (w.n_general > 0 ? (few_chains(w.n_general, sms) ? 4 : 2) : 0);
+}
 
 ChConfig ch_config(int index) {
-    // {warps per right-hand-side CTA, y-sweep rows per batch, sweep kind, x-sweep columns per chunk (kinds 2,
-    // 3), two-pass right-hand side}
+    // {warps per right-hand-side CTA, right-hand-side passes, x closure}
     static const ChConfig tab[kChConfigs] = {
-        {1, 32, 0, 16}, {2, 32, 0, 16}, {4, 32, 0, 16}, {1, 16, 0, 16}, {2, 16, 0, 16}, {4, 16, 0, 16},
-        {2, 16, 1, 16}, {4, 16, 1, 16}, {2, 32, 1, 16}, {4, 32, 1, 16}, {4, 16, 2, 16}, {4, 32, 2, 16},
-        {4, 8, 3, 16},  {4, 16, 3, 16}, {4, 8, 3, 8},   {4, 4, 3, 8},   {4, 4, 3, 16},
-        {4, 8, 3, 16, 1}, {2, 8, 3, 16, 1}, {4, 8, 3, 16, 2}, {8, 8, 3, 16, 2}, {8, 8, 3, 16, 2, 1}};
+        {1, 0, 1}, {2, 0, 1}, {4, 0, 1}, {8, 0, 1}, {1, 1, 1}, {2, 1, 1}, {4, 1, 1}, {8, 1, 1}, {2, 2, 1}, {4, 2, 1}, {8, 2, 1},
+        {1, 0, 2}, {4, 0, 0}, {2, 0, 2}, {4, 0, 2}, {8, 0, 2}, {2, 1, 2}, {4, 1, 2}, {8, 1, 2}, {4, 2, 2}, {8, 2, 0}, {8, 2, 2}};
     return tab[(index >= 0 && index < kChConfigs) ? index : 0];
 }
 
 void config_name(const ChConfig& c, char* name, size_t len) {
-    if (c.pipe >= 2)
-        snprintf(name, len, "rhs_warps%d%s_ychunk%d_pipe_regtab%s_xchunk%d%s", c.rhs_warps,
-                 c.rhs_split == 2 ? "_2pass_pipe" : (c.rhs_split ? "_2pass" : ""),
-                 c.y_chunk, c.pipe == 3 ? "_xy" : "", c.x_chunk, c.ysplit ? "_ysplit" : "");
-    else
-        snprintf(name, len, "rhs_warps%d_ychunk%d%s", c.rhs_warps, c.y_chunk, c.pipe ? "_pipe" : "");
+    snprintf(name, len, "rhs_warps%d%s%s", c.rhs_warps, c.rhs_split == 2 ? "_2pass_pipe" : (c.rhs_split ? "_2pass" : ""),
+             c.close == 2 ? "_close_apart" : (c.close ? "_close_fused" : ""));
 }
 
-// The two passes of the split right-hand side; pass 2 claims work through the step's fourth counter.
-// Pass 2 runs in FP64 in both variants: the precision variant's h buffer holds FP32 values, whose FP64
-// Laplacian is exact, so its mass is conserved to FP64 rounding (the one-pass kernel does the same).
-// Pass 2 pipelined: dynamic shared memory beyond 48 KB, allowed once per device and kernel.
+// The two passes of the split right-hand side. Pass 2 runs in FP64 in both variants: the precision variant's h
+// buffer holds FP32 values, whose FP64 Laplacian is exact, so its mass is conserved to FP64 rounding (the
+// one-pass kernel does the same). Pass 2 pipelined: dynamic shared memory beyond 48 KB, allowed once per device.
 template <int NW>
-static cudaError_t launch_rhs2_pipe(int grid, const GridDev* g, const Item* it, int n, int parity, unsigned int* ctr,
-                                    cudaStream_t s) {
+static cudaError_t launch_rhs2_pipe(int grid, const GridDev* g, const Item* it, int n, int parity, cudaStream_t s) {
     static std::atomic<int> ready[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1438,103 +1247,71 @@ static cudaError_t launch_rhs2_pipe(int grid, const GridDev* g, const Item* it, 
         if (e != cudaSuccess) return e;
         ready[dev].store(1, std::memory_order_release);
     }
-    ch_rhs2_pipe_kernel<NW><<<grid, NW * BLK, kRhs2PipeBytes, s>>>(g, it, n, parity, ctr);
+    ch_rhs2_pipe_kernel<NW><<<grid, NW * BLK, kRhs2PipeBytes, s>>>(g, it, n, parity);
     return cudaGetLastError();
 }
 
-template <typename T>
-static cudaError_t launch_rhs2(int nw, int grid, const GridDev* g, const Item* it, int n, int parity,
-                               unsigned int* ctr, cudaStream_t s, bool pipe, int sms) {
-    if (pipe) {   // four CTAs per SM fit the double buffer
-        const int gp = std::max(1, std::min(n, sms * 4));
-        if (nw == 8) {
-            ch_h_kernel<T, 8><<<grid, 8 * BLK, 0, s>>>(g, it, n, parity, ctr);
-            return launch_rhs2_pipe<8>(gp, g, it, n, parity, ctr + 3, s);
-        }
-        if (nw == 4) {
-            ch_h_kernel<T, 4><<<grid, 4 * BLK, 0, s>>>(g, it, n, parity, ctr);
-            return launch_rhs2_pipe<4>(gp, g, it, n, parity, ctr + 3, s);
-        }
-        ch_h_kernel<T, 2><<<grid, 2 * BLK, 0, s>>>(g, it, n, parity, ctr);
-        return launch_rhs2_pipe<2>(gp, g, it, n, parity, ctr + 3, s);
-    }
-    if (nw == 4) {
-        ch_h_kernel<T, 4><<<grid, 4 * BLK, 0, s>>>(g, it, n, parity, ctr);
-        ch_rhs2_kernel<double, 4><<<grid, 4 * BLK, 0, s>>>(g, it, n, parity, ctr + 3);
-    } else {
-        ch_h_kernel<T, 2><<<grid, 2 * BLK, 0, s>>>(g, it, n, parity, ctr);
-        ch_rhs2_kernel<double, 2><<<grid, 2 * BLK, 0, s>>>(g, it, n, parity, ctr + 3);
-    }
-    return cudaGetLastError();
-}
-
-template <typename T>
-static void launch_rhs(int nw, int grid, const GridDev* g, const Item* it, int n, int parity, unsigned int* ctr,
-                       cudaStream_t s) {
-    switch (nw) {
-    case 1: ch_rhs_kernel<T, 1><<<grid, BLK, 0, s>>>(g, it, n, parity, ctr); break;
-    case 4: ch_rhs_kernel<T, 4><<<grid, 4 * BLK, 0, s>>>(g, it, n, parity, ctr); break;
-    default: ch_rhs_kernel<T, 2><<<grid, 2 * BLK, 0, s>>>(g, it, n, parity, ctr); break;
-    }
-}
-
-cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const GridDev* grids, const Item* items_rhs, int n_rhs,
-                           const Item* items_rows, int n_rows, int parity, unsigned int* counters, int sms,
-                           cudaStream_t s) {
-    // persistent grids over the work lists; CTAs beyond the resident ones find the lists empty
-    const int g1 = std::max(1, std::min(n_rhs, sms * 32 / c.rhs_warps));
-    const int g23 = std::max(1, std::min(n_rows, sms * 16));
-    if (c.rhs_split) {
-        const cudaError_t e2 =
-            rhs_fp32 ? launch_rhs2<float>(c.rhs_warps, g1, grids, items_rhs, n_rhs, parity, counters, s,
-                                          c.rhs_split == 2, sms)
-                     : launch_rhs2<double>(c.rhs_warps, g1, grids, items_rhs, n_rhs, parity, counters, s,
-                                           c.rhs_split == 2, sms);
-        if (e2 != cudaSuccess) return e2;
-    } else if (rhs_fp32) {
-        launch_rhs<float>(c.rhs_warps, g1, grids, items_rhs, n_rhs, parity, counters, s);
-    } else {
-        launch_rhs<double>(c.rhs_warps, g1, grids, items_rhs, n_rhs, parity, counters, s);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (c.pipe) {
-        // 64-100 registers and 8-17 KB of shared memory per one-warp CTA: up to 32 CTAs per SM
-        const int gp = std::max(1, std::min(n_rows, sms * 32));
-        if (c.ysplit) {   // x sweep, x correction, y recurrences, update (register-table sweeps, 8-row y batches)
-            if (c.x_chunk == 8) ch_xsolve_pipe_rt_kernel<8><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-            else ch_xsolve_pipe_rt_kernel<16><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_xcorr_kernel<<<n_rhs, 256, 0, s>>>(grids, items_rhs);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_ysolve_split_kernel<8><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_update_kernel<<<n_rhs, 256, 0, s>>>(grids, items_rhs, parity);
-            return cudaGetLastError();
-        }
-        if (c.pipe >= 2 && c.x_chunk == 8)
-            ch_xsolve_pipe_rt_kernel<8><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-        else if (c.pipe >= 2)
-            ch_xsolve_pipe_rt_kernel<16><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-        else if (c.y_chunk == 32) ch_xsolve_pipe_kernel<32><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-        else ch_xsolve_pipe_kernel<16><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if (c.pipe == 3 && c.y_chunk == 4)
-            ch_ysolve_pipe_rt_kernel<4><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-        else if (c.pipe == 3 && c.y_chunk == 8)
-            ch_ysolve_pipe_rt_kernel<8><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-        else if (c.pipe == 3)
-            ch_ysolve_pipe_rt_kernel<16><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-        else if (c.y_chunk == 32)
-            ch_ysolve_pipe_kernel<32><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-        else ch_ysolve_pipe_kernel<16><<<gp, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
+template <typename T, int NW>
+static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, int sms, cudaStream_t s) {
+    // persistent grids over the work list
+    const int n = w.n_blocks, grid = std::max(1, std::min(n, sms * 32 / NW));
+    if (!c.rhs_split) {
+        ch_rhs_kernel<T, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
         return cudaGetLastError();
     }
-    ch_xsolve_kernel<<<g23, BLK, 0, s>>>(grids, items_rows, n_rows, counters + 1);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (c.y_chunk == 32) ch_ysolve_kernel<32><<<g23, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
-    else ch_ysolve_kernel<16><<<g23, BLK, 0, s>>>(grids, items_rows, n_rows, parity, counters + 2);
+    ch_h_kernel<T, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    if (c.rhs_split == 2)   // four CTAs per SM fit the double buffer
+        return launch_rhs2_pipe<NW>(std::max(1, std::min(n, sms * 4)), w.grids, w.blocks, n, parity, s);
+    ch_rhs2_kernel<double, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
     return cudaGetLastError();
+}
+
+template <typename T>
+static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, int sms, cudaStream_t s) {
+    switch (c.rhs_warps) {
+    case 1: return launch_rhs<T, 1>(c, w, parity, sms, s);
+    case 2: return launch_rhs<T, 2>(c, w, parity, sms, s);
+    case 4: return launch_rhs<T, 4>(c, w, parity, sms, s);
+    default: return launch_rhs<T, 8>(c, w, parity, sms, s);
+    }
+}
+
+cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, int parity, int sms, cudaStream_t s) {
+    cudaError_t e = rhs_fp32 ? launch_rhs<float>(c, w, parity, sms, s) : launch_rhs<double>(c, w, parity, sms, s);
+    if (e != cudaSuccess) return e;
+    const int n = w.n_lines - w.n_general;
+    if (n > 0) {   // one CTA (two chains) per 32 lines, largest grids first
+        ch_xsweep_kernel<<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (close_apart(c, w, sms)) {
+            ch_xclose_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            ch_ysweep_kernel<false><<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+        } else {
+            ch_ysweep_kernel<true><<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+        }
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        ch_update_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks, parity);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (w.n_general > 0) {
+        const Item* lines = w.lines + n;
+        ch_xsolve_general_kernel<16><<<w.n_general, BLK, 0, s>>>(w.grids, lines);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (few_chains(w.n_general, sms)) {
+            ch_xcorr_general_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            ch_ysolve_split_general_kernel<8><<<w.n_general, BLK, 0, s>>>(w.grids, lines);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            ch_update_general_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks, parity);
+        } else {
+            ch_ysolve_general_kernel<8><<<w.n_general, BLK, 0, s>>>(w.grids, lines, parity);
+        }
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 // Compensated (Neumaier) sum of one grid, one CTA of 256 threads; combined with a two-sum tree.
@@ -1572,13 +1349,99 @@ __global__ void __launch_bounds__(256) ch_mass_kernel(const double* __restrict__
 // Host side
 // ------------------------------------------------------------------------------------------------
 
-// Solver table for an n x n grid of side lx with D = 1, gamma, dt = dt_factor * dx (the reference
-// defaults are gamma = 0.01, dt = 0.1 dx: cuPentCahnADI.cu:204-221), written into t (tab_size(n)
-// doubles) with `work` (7 * (n - 2) doubles) as scratch.
-static void fill_table(double* t, double* work, int n, double lx, double gamma, double dt_factor) {
+// sigma_lin of an n x n grid of side lx with D = 1, gamma, dt = dt_factor * dx (the reference defaults are gamma =
+// 0.01, dt = 0.1 dx: cuPentCahnADI.cu:204-221).
+static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
+    const double D = 1.0, dx = lx / n, dt = dt_factor * dx;
+    return 2.0 * dt * D * gamma / (3.0 * (dx * dx * dx * dx));
+}
+
+bool line_is_general(int n, double lx, double gamma, double dt_factor, bool rhs_fp32) {
+    return rhs_fp32 || !(sigma_lin(n, lx, gamma, dt_factor) >= 0.0);
+}
+
+// Causal factor of the circulant line operator 1 + s D^4, s >= 0: its symbol 1 + s w^2, w = 2 - z - 1/z, vanishes at
+// w = +-i / sqrt(s); P(z) = (1 - z1 / z)(1 - conj(z1) / z) with z1 the root inside the unit circle of z + 1/z = 2 - w.
+static void line_factor(double s, double* p1, double* p2) {
+    *p1 = *p2 = 0.0;
+    if (s < 1e-36) return;   // P = 1 to double precision
+    const long double a = 0.5L / sqrtl((long double)s);
+    const std::complex<long double> t(1.0L, -a), r = std::sqrt(std::complex<long double>(-a * a, -2.0L * a));
+    const std::complex<long double> big = std::norm(t + r) > std::norm(t - r) ? t + r : t - r;
+    const std::complex<long double> z = 1.0L / big;
+    *p1 = (double)(-2.0L * z.real());
+    *p2 = (double)std::norm(z);
+}
+
+// The factored sweeps' part of the table: parameters and homogeneous solutions (see K2 / K3).
+static void fill_line_table(double* t, int n, double s) {
+    double p1d, p2d;
+    line_factor(s, &p1d, &p2d);
+    const long double p1 = p1d, p2 = p2d;
+    t[TAB_NP1] = -p1d;
+    t[TAB_NP2] = -p2d;
+    const long double at1 = 1.0L + p1 + p2;   // P(1): G P(1)^2 = 1, the operator on constants
+    t[TAB_KAPPA] = (double)(at1 * at1 * at1 * at1);
+    // the four values around the middle (X1, X2 | Y1, Y2) from the chains' ends (a1, a2 | b1, b2)
+    long double m[4][8] = {{1, 0, p1, p2, 1, 0, 0, 0},
+                           {p1, 1, p2, 0, 0, 1, 0, 0},
+                           {p1, p2, 1, 0, 0, 0, 1, 0},
+                           {p2, 0, p1, 1, 0, 0, 0, 1}};
+    for (int c = 0; c < 4; ++c) {
+        int piv = c;
+        for (int r = c + 1; r < 4; ++r)
+            if (fabsl(m[r][c]) > fabsl(m[piv][c])) piv = r;
+        for (int k = 0; k < 8; ++k) std::swap(m[c][k], m[piv][k]);
+        const long double inv = 1.0L / m[c][c];
+        for (int k = 0; k < 8; ++k) m[c][k] *= inv;
+        for (int r = 0; r < 4; ++r) {
+            if (r == c) continue;
+            const long double f = m[r][c];
+            for (int k = 0; k < 8; ++k) m[r][k] -= f * m[c][k];
+        }
+    }
+    for (int k = 0; k < 4; ++k) {
+        t[TAB_MID + k] = (double)m[2][4 + k];
+        t[TAB_MID + 4 + k] = (double)m[3][4 + k];
+    }
+    // f1, f2: P f = 0 from (f[-1], f[-2]) = (1, 0) and (0, 1)
+    double *f1 = t + kTabParams, *f2 = f1 + n;
+    long double a1 = 1.0L, a2 = 0.0L, b1 = 0.0L, b2 = 1.0L, peak = 1.0L;
+    for (int i = 0; i < n; ++i) {
+        const long double a = -p1 * a1 - p2 * a2, b = -p1 * b1 - p2 * b2;
+        a2 = a1;
+        a1 = a;
+        b2 = b1;
+        b1 = b;
+        f1[i] = (double)a;
+        f2[i] = (double)b;
+        peak = std::max(peak, std::max(fabsl(a), fabsl(b)));
+    }
+    int reach = n;
+    while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp((double)peak, -62)) --reach;
+    t[TAB_REACH] = reach;
+    // (1 - M^n)^-1, M^n = [f1[n-1] f2[n-1]; f1[n-2] f2[n-2]]
+    const long double c00 = 1.0L - a1, c01 = -b1, c10 = -a2, c11 = 1.0L - b2, det = c00 * c11 - c01 * c10;
+    t[TAB_CLOSE] = (double)(c11 / det);
+    t[TAB_CLOSE + 1] = (double)(-c01 / det);
+    t[TAB_CLOSE + 2] = (double)(-c10 / det);
+    t[TAB_CLOSE + 3] = (double)(c00 / det);
+}
+
+// Solver table for an n x n grid (layout in ch_internal.cuh), written into t (tab_size(n) doubles) with `work`
+// (7 * (n - 2) doubles) as scratch.
+static void fill_table(double* t, double* work, int n, double lx, double gamma, double dt_factor, bool general) {
     const int m = n - 2;
     const double D = 1.0, dx = lx / n, dt = dt_factor * dx;
-    const double sl = 2.0 * dt * D * gamma / (3.0 * (dx * dx * dx * dx));
+    const double sl = sigma_lin(n, lx, gamma, dt_factor);
+    for (int k = 0; k < tab_size(n); ++k) t[k] = 0.0;
+    t[TAB_SLIN] = sl;
+    t[TAB_SNL] = (dt / 3.0) * D * (2.0 / (dx * dx));
+    if (!general) {
+        fill_line_table(t, n, sl);
+        return;
+    }
+    t += kTabParams;
     const double a = sl, b = -4 * sl, c = 1 + 6 * sl, d = -4 * sl, e = sl;
     double *ds = work, *dl = work + m, *dg = work + 2 * m, *du = work + 3 * m, *dw = work + 4 * m;
     double *inv1 = work + 5 * m, *inv2 = work + 6 * m;
@@ -1620,7 +1483,6 @@ static void fill_table(double* t, double* work, int n, double lx, double gamma, 
     const double z22 = d * inv2[0] + e * inv2[1] + a * inv2[m - 1];
     const double y11 = c - z11, y12 = d - z12, y21 = b - z21, y22 = c - z22;
     const double det = 1.0 / (y11 * y22 - y21 * y12);
-    for (int k = 0; k < tab_size(n); ++k) t[k] = 0.0;
     for (int i = 0; i < m; ++i) {
         t[i] = (i > 1) ? ds[i] : 0.0;
         t[m + i] = (i > 0) ? dl[i] : 0.0;
@@ -1636,17 +1498,30 @@ static void fill_table(double* t, double* work, int n, double lx, double gamma, 
     om[2] = -y21 * det;
     om[3] = y11 * det;
     om[4] = a; om[5] = b; om[6] = d; om[7] = e;
-    static const double wl[25] = {0, 0, -1, 0, 0, 0, -2, 8, -2, 0, -1, 8, -20, 8, -1, 0, -2, 8, -2, 0, 0, 0, -1, 0, 0};
-    static const double wn[9] = {0, 1, 0, 1, -4, 1, 0, 1, 0};
-    const double snl = (dt / 3.0) * D * (2.0 / (dx * dx));
-    for (int k = 0; k < 25; ++k) t[7 * m + 8 + k] = wl[k] * sl;
-    for (int k = 0; k < 9; ++k) t[7 * m + 33 + k] = wn[k] * snl;
 }
 
-std::vector<double> build_table(int n, double lx, double gamma, double dt_factor) {
+std::vector<double> build_table(int n, double lx, double gamma, double dt_factor, bool general) {
     std::vector<double> t(tab_size(n)), work(7 * (n - 2));
-    fill_table(t.data(), work.data(), n, lx, gamma, dt_factor);
+    fill_table(t.data(), work.data(), n, lx, gamma, dt_factor, general);
     return t;
+}
+
+// Tensor maps of a grid's work field for the sweeps: [0] 16 columns by 32 rows in the 128-byte swizzle (x), [1] 32
+// columns by 16 rows (y). False when the driver cannot encode them.
+bool sweep_maps(CUtensorMap maps[2], double* tmp, int n) {
+    auto enc = tensor_map_encoder();
+    if (!enc) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)n};
+    cuuint64_t strides[1] = {(cuuint64_t)n * sizeof(double)};
+    cuuint32_t estr[2] = {1, 1};
+    for (int k = 0; k < 2; ++k) {
+        cuuint32_t box[2] = {(cuuint32_t)(k ? BLK : kChunk), (cuuint32_t)(k ? kChunk : BLK)};
+        if (enc(&maps[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, tmp, dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, k ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    return true;
 }
 
 struct Batch {
@@ -1660,10 +1535,10 @@ struct Batch {
     std::vector<double*> allocs;
     std::vector<std::pair<std::string, double*>> tables;   // key "n/lx/gamma/dtf" -> device table
     GridDev* grids_d = nullptr;
+    CUtensorMap* maps_d = nullptr;   // two per grid (sweep_maps)
     Item* items_rhs = nullptr;
     Item* items_rows = nullptr;   // K2 and K3 share the per-grid block lists (row / column blocks)
-    int n_items_rhs = 0, n_items_rows = 0;
-    unsigned int* counters = nullptr;   // 3 counters per step of a captured pair
+    int n_items_rhs = 0, n_items_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
     double* mass_d = nullptr;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -1673,12 +1548,10 @@ struct Batch {
     unsigned long long launches = 0;
 };
 
-// The default: configuration 20, or with fewer 32-line warps than FP64 sub-partitions (4 per SM) its split
-// y sweep (configuration 21), which a warp's FP64 instruction count bounds there (a 2048^2 grid alone: 1.32
-// against 1.87 ms per step). Both compute the same values.
-static ChConfig batch_config(const Batch* b) {
-    if (b->cfg >= 0) return ch_config(b->cfg);
-    return ch_config(b->n_items_rows < 4 * b->sms ? kChSplitConfig : kChBatchDefault);
+static ChConfig batch_config(const Batch* b) { return ch_config(b->cfg >= 0 ? b->cfg : kChBatchDefault); }
+
+static ChWork batch_work(const Batch* b) {
+    return ChWork{b->grids_d, b->items_rhs, b->items_rows, b->maps_d, b->n_items_rhs, b->n_items_rows, b->n_general};
 }
 
 static thread_local std::string g_ch_err;
@@ -1697,11 +1570,8 @@ static int ch_fail_arg(const std::string& msg) {
         if (_e != cudaSuccess) return ch_fail(_e, what); \
     } while (0)
 
-static int enqueue_step(Batch* b, int parity, int slot) {
-    unsigned int* ctr = b->counters + kChCounters * slot;
-    CH_TRY(cudaMemsetAsync(ctr, 0, kChCounters * sizeof(unsigned int), b->stream), "Resetting work counters");
-    CH_TRY(launch_ch_step(batch_config(b), b->rhs_fp32 != 0, b->grids_d, b->items_rhs, b->n_items_rhs, b->items_rows,
-                          b->n_items_rows, parity, ctr, b->sms, b->stream),
+static int enqueue_step(Batch* b, int parity) {
+    CH_TRY(launch_ch_step(batch_config(b), b->rhs_fp32 != 0, batch_work(b), parity, b->sms, b->stream),
            "Launching a step");
     return 0;
 }
@@ -1711,8 +1581,8 @@ static int capture_pairs(Batch* b) {
         if (b->graph_exec[p]) continue;
         cudaGraph_t g;
         CH_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "Beginning graph capture");
-        int st = enqueue_step(b, p, 0);
-        if (st == 0) st = enqueue_step(b, p ^ 1, 1);
+        int st = enqueue_step(b, p);
+        if (st == 0) st = enqueue_step(b, p ^ 1);
         cudaError_t e = cudaStreamEndCapture(b->stream, &g);
         if (st != 0) return st;
         CH_TRY(e, "Ending graph capture");
@@ -1730,22 +1600,23 @@ static int capture_pairs(Batch* b) {
 // that owns every device allocation through its own budgeted pool, or a latency-critical loop that
 // must never enter cudaMalloc / cudaFree (they synchronise the device). For them one step of one
 // grid runs with all of its work buffers in this file-scope array: the right-hand side / x-sweep
-// field, the row ends, the solver table, the descriptor, the work lists and the work counters.
+// field, the closure amplitudes, the solver table, the descriptor, the work lists
+// and the tensor maps.
 // Maximum grid: kNoAllocMaxN x kNoAllocMaxN. Every GPU that loads the library holds the array
-// (about 532 KiB) until the process exits.
+// (about 544 KiB) until the process exits.
 constexpr int kNoAllocMaxN = 256;
 constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr size_t kNoAllocTmpOff = 0;
 constexpr size_t kNoAllocEndsOff = align256(kNoAllocTmpOff + sizeof(double) * kNoAllocMaxN * kNoAllocMaxN);
-constexpr size_t kNoAllocTabOff = align256(kNoAllocEndsOff + sizeof(double) * 2 * kNoAllocMaxN);
-constexpr int kNoAllocTabLen = 7 * (kNoAllocMaxN - 2) + 42;
+constexpr size_t kNoAllocTabOff = align256(kNoAllocEndsOff + sizeof(double) * 8 * kNoAllocMaxN);
+constexpr int kNoAllocTabLen = kTabParams + 7 * (kNoAllocMaxN - 2) + 8;
 constexpr size_t kNoAllocGridOff = align256(kNoAllocTabOff + sizeof(double) * kNoAllocTabLen);
 constexpr int kNoAllocBlocks = (kNoAllocMaxN / BLK) * (kNoAllocMaxN / BLK);
 constexpr int kNoAllocRows = kNoAllocMaxN / BLK;
 constexpr size_t kNoAllocRhsOff = align256(kNoAllocGridOff + sizeof(GridDev));
 constexpr size_t kNoAllocRowsOff = align256(kNoAllocRhsOff + sizeof(Item) * kNoAllocBlocks);
-constexpr size_t kNoAllocCtrOff = align256(kNoAllocRowsOff + sizeof(Item) * kNoAllocRows);
-constexpr size_t kNoAllocBytes = align256(kNoAllocCtrOff + kChCounters * sizeof(unsigned int));
+constexpr size_t kNoAllocMapsOff = align256(kNoAllocRowsOff + sizeof(Item) * kNoAllocRows);
+constexpr size_t kNoAllocBytes = align256(kNoAllocMapsOff + 2 * sizeof(CUtensorMap));
 
 static __device__ __align__(256) unsigned char g_ch_noalloc_scratch[kNoAllocBytes];
 
@@ -1790,13 +1661,14 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     b->grids_h.resize(nsims);
     for (int s = 0; s < nsims; ++s) {
         const int ns = n[s];
+        const bool general = line_is_general(ns, b->lx[s], gamma, dt_factor, b->rhs_fp32 != 0);
         char key[128];
         snprintf(key, sizeof(key), "%d/%.17g/%.17g/%.17g", ns, b->lx[s], gamma, dt_factor);
         double* tab = nullptr;
         for (auto& t : b->tables)
             if (t.first == key) tab = t.second;
         if (!tab) {
-            std::vector<double> h = build_table(ns, b->lx[s], gamma, dt_factor);
+            std::vector<double> h = build_table(ns, b->lx[s], gamma, dt_factor, general);
             cudaError_t e = cudaMalloc(&tab, h.size() * sizeof(double));
             if (e != cudaSuccess) return cleanup_fail(ch_fail(e, "Allocating solver table"));
             e = cudaMemcpy(tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
@@ -1805,15 +1677,16 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
         }
         GridDev g{};
         const size_t bytes = (size_t)ns * ns * sizeof(double);
-        for (int k = 0; k < 5; ++k) {   // cCurr / cOld, tmp, row ends, h of the two-pass right-hand side
+        for (int k = 0; k < 4; ++k) {   // cCurr / cOld, tmp, h of the two-pass right-hand side
             double* p = nullptr;
-            cudaError_t e = cudaMalloc(&p, k == 3 ? 2 * ns * sizeof(double) : bytes);
+            cudaError_t e = cudaMalloc(&p, bytes);
             if (e != cudaSuccess) return cleanup_fail(ch_fail(e, "Allocating grid fields"));
             b->allocs.push_back(p);
-            if (k < 2) g.buf[k] = p; else if (k == 2) g.tmp = p; else if (k == 3) g.ends = p; else g.hbuf = p;
+            if (k < 2) g.buf[k] = p; else if (k == 2) g.tmp = p; else g.hbuf = g.ends = p;
         }
         g.tab = tab;
         g.n = ns;
+        g.general = general;
         b->grids_h[s] = g;
     }
     // work lists, largest grids first
@@ -1824,8 +1697,12 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     for (int s : order) {
         const int bpr = n[s] / BLK;
         for (int k = 0; k < bpr * bpr; ++k) rhs.push_back({s, k});
-        for (int k = 0; k < bpr; ++k) rows.push_back({s, k});
+        if (!b->grids_h[s].general)
+            for (int k = 0; k < bpr; ++k) rows.push_back({s, k});
     }
+    for (int s : order)
+        if (b->grids_h[s].general)
+            for (int k = 0; k < n[s] / BLK; ++k, ++b->n_general) rows.push_back({s, k});
     b->n_items_rhs = (int)rhs.size();
     b->n_items_rows = (int)rows.size();
     cudaError_t e = cudaMalloc(&b->grids_d, nsims * sizeof(GridDev));
@@ -1835,8 +1712,13 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     if (e == cudaSuccess) e = cudaMalloc(&b->items_rows, rows.size() * sizeof(Item));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->items_rows, rows.data(), rows.size() * sizeof(Item), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&b->counters, 2 * kChCounters * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMalloc(&b->mass_d, sizeof(double));
+    std::vector<CUtensorMap> maps(2 * (size_t)nsims);
+    for (int s = 0; s < nsims && e == cudaSuccess; ++s)
+        if (!b->grids_h[s].general && !sweep_maps(&maps[2 * s], b->grids_h[s].tmp, n[s])) e = cudaErrorNotSupported;
+    if (e == cudaSuccess) e = cudaMalloc(&b->maps_d, maps.size() * sizeof(CUtensorMap));
+    if (e == cudaSuccess)
+        e = cudaMemcpy(b->maps_d, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cleanup_fail(ch_fail(e, "Allocating work lists"));
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->device);
     *out = b;
@@ -1919,7 +1801,7 @@ int custen_ch_batch_step(void* h, int steps, int use_graph) {
     if (!b || steps < 0) return ch_fail_arg("invalid arguments");
     cudaSetDevice(b->device);
     int left = steps;
-    const int per_step = ch_launches_per_step(batch_config(b));   // kernel launches in one step
+    const int per_step = ch_launches_per_step(batch_config(b), batch_work(b), b->sms);   // kernel launches in one step
     if (use_graph && left >= 2) {
         int st = capture_pairs(b);
         if (st) return st;
@@ -1931,7 +1813,7 @@ int custen_ch_batch_step(void* h, int steps, int use_graph) {
         }
     }
     while (left > 0) {
-        int st = enqueue_step(b, b->parity, 0);
+        int st = enqueue_step(b, b->parity);
         if (st) return st;
         b->launches += per_step;
         b->parity ^= 1;
@@ -1994,8 +1876,9 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
     // host-side inputs in stack buffers (no heap either)
     double tab[kNoAllocTabLen];
     double work[7 * (kNoAllocMaxN - 2)];
-    fill_table(tab, work, n, lx, gamma, dt_factor);
     GridDev g{};
+    g.general = line_is_general(n, lx, gamma, dt_factor, false);
+    fill_table(tab, work, n, lx, gamma, dt_factor, g.general != 0);
     g.buf[0] = const_cast<double*>(c_cur);
     g.buf[1] = c_new;
     g.tmp = reinterpret_cast<double*>(base + kNoAllocTmpOff);
@@ -2018,15 +1901,20 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
            "Uploading the work list");
     CH_TRY(cudaMemcpyAsync(base + kNoAllocRowsOff, rows, sizeof(Item) * bpr, cudaMemcpyHostToDevice, s),
            "Uploading the work list");
-    // the work counters must start at zero on every call (the array keeps the previous call's values)
-    unsigned int* ctr = reinterpret_cast<unsigned int*>(base + kNoAllocCtrOff);
-    CH_TRY(cudaMemsetAsync(ctr, 0, kChCounters * sizeof(unsigned int), s), "Clearing the work counters");
     const GridDev* gd = reinterpret_cast<const GridDev*>(base + kNoAllocGridOff);
     const Item* it_rhs = reinterpret_cast<const Item*>(base + kNoAllocRhsOff);
     const Item* it_rows = reinterpret_cast<const Item*>(base + kNoAllocRowsOff);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    CH_TRY(launch_ch_step(kChDefault, false, gd, it_rhs, bpr * bpr, it_rows, bpr, 0, ctr, sms, s), "Launching the step");
+    CUtensorMap maps[2];
+    if (!g.general) {
+        if (!sweep_maps(maps, g.tmp, n)) return ch_fail(cudaErrorNotSupported, "Encoding the tensor maps");
+        CH_TRY(cudaMemcpyAsync(base + kNoAllocMapsOff, maps, sizeof(maps), cudaMemcpyHostToDevice, s),
+               "Uploading the tensor maps");
+    }
+    const ChWork w{gd, it_rhs, it_rows, reinterpret_cast<const CUtensorMap*>(base + kNoAllocMapsOff),
+                   bpr * bpr, bpr, g.general ? bpr : 0};
+    CH_TRY(launch_ch_step(ch_config(kChOneGrid), false, w, 0, sms, s), "Launching the step");
     return 0;
 }
 
@@ -2139,9 +2027,9 @@ int custen_ch_batch_destroy(void* h) {
     for (double* p : b->allocs) cudaFree(p);
     for (auto& t : b->tables) cudaFree(t.second);
     cudaFree(b->grids_d);
+    cudaFree(b->maps_d);
     cudaFree(b->items_rhs);
     cudaFree(b->items_rows);
-    cudaFree(b->counters);
     cudaFree(b->mass_d);
     if (b->own_stream) cudaStreamDestroy(b->stream);
     delete b;
