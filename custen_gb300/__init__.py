@@ -250,8 +250,9 @@ def selftest_wait_expiry(rounds: int = 1 << 12) -> int:
 
 
 def selftest_fp64(samples: int = 1 << 24, seed: int = 1) -> list:
-    """Mismatches of the kernels' own conversions and divisions against the hardware's (all expected 0)."""
-    c = (ctypes.c_ulonglong * 5)()
+    """Mismatches of the kernels' own conversions, divisions, sums and products against the hardware's (all
+    expected 0)."""
+    c = (ctypes.c_ulonglong * 6)()
     st = lib().custen_selftest_fp64(ctypes.c_ulonglong(seed), ctypes.c_longlong(samples), c)
     if st != 0:
         raise CustenError(f"FP64 self-test failed to run (status {st})")

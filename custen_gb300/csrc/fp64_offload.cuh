@@ -1,4 +1,9 @@
-// FP64 work moved off the FP64 pipe, with bit-identical results.
+// FP64 work moved off the FP64 pipe or to its cheapest instruction, with bit-identical results.
+//
+// Sums and products as multiply-adds (F64): a multiply-add whose three operands are registers runs at 597 G/s on
+// GB300, an addition or a multiplication at 503 (as does a multiply-add with a literal, parameter or zero
+// operand). So a + b is fma(a, 1, b) and a b is fma(a, b, -0.0), with 1 and -0.0 in registers that the compiler
+// cannot fold: the same values for all operands, signed zeros, infinities and NaN included.
 //
 // On GB300 one FP64 instruction of a warp holds its sub-partition's FP64 pipe for 64 cycles, while an
 // integer or FP32 instruction takes one or two issue cycles. Conversions between float and double are FP64
@@ -19,6 +24,20 @@
 
 namespace custen {
 namespace f64 {
+
+static __device__ double g_f64_constants[2] = {1.0, -0.0};
+
+struct F64 {
+    double one, nzero;
+    __device__ __forceinline__ F64() {
+        const volatile double* c = g_f64_constants;
+        one = c[0];
+        nzero = c[1];
+    }
+    __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+    __device__ __forceinline__ double sub(double a, double b) const { return fma(b, -one, a); }
+    __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nzero); }
+};
 
 // The compiler's own operations, for arguments outside the ranges below. Out of line: inlined, they are
 // evaluated unconditionally and selected afterwards, which keeps their FP64 instructions (measured in the WENO
@@ -79,7 +98,7 @@ __device__ __forceinline__ float to_float(double x) {
 //   of two would need a float d between 2^-j and its successor. y is within 2^-47 of 1/d, q0 = RN(c y) within
 //   2^-46 of c/d; the residual r = c - d q0 has at most 77 - 46 bits and is exact. q0 + r y is within 2^-93 of
 //   c/d, and c/d, whose divisor has 24 bits, lies at least 2^-78 from a midpoint of two doubles: q is RN(c/d).
-__device__ __forceinline__ double div_by_float(double c, float d) {
+__device__ __forceinline__ double div_by_float(const F64& f, double c, float d) {
     const unsigned u = __float_as_uint(d);
     if (u - ((127u - 40u) << 23) >= (100u << 23)) return hw_divide(c, hw_to_double(d));
     const float yh = __frcp_rn(d);
@@ -92,7 +111,7 @@ __device__ __forceinline__ double div_by_float(double c, float d) {
     const long long yb = ((long long)((uy >> 3) + 0x38000000u) << 32 | (long long)(uy << 29)) + off;
     const double y = __longlong_as_double(yb);
     const double dd = to_double_normal(d);
-    const double q0 = c * y;
+    const double q0 = f.mul(c, y);
     return fma(fma(-dd, q0, c), y, q0);
 }
 
@@ -109,7 +128,7 @@ __device__ __forceinline__ double times4(double x) {
 // with yl = yh (e + e^2), renormalised so that |yl| is at most half a unit of yh; the sum is formed by adding yl,
 // in units of yh's double, to yh's encoding (twice below a power of two, where a unit counts half). Then one
 // Newton step on the FP64 pipe.
-__device__ __forceinline__ double reciprocal_seed(double b, double one) {
+__device__ __forceinline__ double reciprocal_seed(const F64& f, double b) {
     const unsigned hi = (unsigned)__double2hiint(b), lo = (unsigned)__double2loint(b);
     const unsigned ub = (__funnelshift_l(lo, hi, 3) + 0x40000000u) & 0x7fffffffu;   // |b| truncated to float
     const float bh = __uint_as_float(ub);
@@ -125,17 +144,17 @@ __device__ __forceinline__ double reciprocal_seed(double b, double one) {
     if (off < 0 && (uy & 0x7fffffu) == 0u) off *= 2;
     const long long yb = ((long long)((uy >> 3) + 0x38000000u) << 32 | (long long)(uy << 29)) + off;
     const double y = __longlong_as_double(yb | (long long)((unsigned long long)(hi >> 31) << 63));
-    return fma(y, fma(-b, y, one), y);
+    return fma(y, fma(-b, y, f.one), y);
 }
 
 // Correctly rounded 1 / x. A reciprocal y within one unit in the last place becomes the correctly rounded one
 // by one more iteration, except where the fraction of x is all ones (Markstein's theorem); those and arguments
 // outside [2^-60, 2^60) take the operator.
-__device__ __forceinline__ double reciprocal(double x, double one) {
+__device__ __forceinline__ double reciprocal(const F64& f, double x) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
     if (!exponent_in<-60, 60>(hi) || ((hi & 0xfffff) == 0xfffff && lo == -1)) return hw_divide(1.0, x);
-    const double y = reciprocal_seed(x, one);
-    return fma(fma(-x, y, one), y, y);
+    const double y = reciprocal_seed(f, x);
+    return fma(fma(-x, y, f.one), y, y);
 }
 
 // Correctly rounded quotients by one divisor. |b| in [2^-60, 2^60) and |a| in [2^-800, 2^800) or zero;
@@ -149,16 +168,17 @@ __device__ __forceinline__ double reciprocal(double x, double one) {
 struct Divider {
     double b, y;
     bool ok;
-    __device__ __forceinline__ Divider(double b_, double one) : b(b_) {
+    double nzero;
+    __device__ __forceinline__ Divider(const F64& f, double b_) : b(b_), nzero(f.nzero) {
         const int hi = __double2hiint(b_);
         ok = exponent_in<-60, 60>(hi) && (hi & 0xfffff) != 0xfffff;
-        y = reciprocal_seed(b_, one);   // unused unless ok
+        y = reciprocal_seed(f, b_);   // unused unless ok
     }
     __device__ __forceinline__ double operator()(double a) const {
         const unsigned hi = (unsigned)__double2hiint(a), lo = (unsigned)__double2loint(a);
         const bool zero = ((hi << 1) | lo) == 0u;
         if (!(ok && (exponent_in<-800, 800>((int)hi) || zero))) return hw_divide(a, b);
-        const double q0 = a * y;
+        const double q0 = fma(a, y, nzero);
         const double q = fma(fma(-b, q0, a), y, q0);
         return zero ? q0 : q;   // a zero keeps its sign
     }

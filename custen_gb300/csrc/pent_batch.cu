@@ -17,7 +17,7 @@
 // share a pivot, against 9.4 each for the operator). The exact variants are bound by the FP64 pipe (12 and 9
 // operations a row), the reciprocal variant by HBM.
 // Measured, 262144 systems of 256 rows, G rows/s (before: operator divisions, loads staged in registers):
-// factorisation 27.9 -> 47.5, exact solve 44.2 -> 62.1, inverted-pivot solve 80.8 -> 93.9 (6.8 TB/s); 4096 systems of
+// factorisation 27.9 -> 48.6, exact solve 44.2 -> 62.7, inverted-pivot solve 80.8 -> 93.9 (6.8 TB/s); 4096 systems of
 // 512 rows: 4.6 -> 6.0, 3.6 -> 7.7, 4.6 -> 13.8.
 #include <cuda_runtime.h>
 
@@ -36,9 +36,6 @@ namespace {
 
 constexpr int kThreads = 128;    // pivot inversion
 constexpr int kLine = 32;        // systems per CTA of the factorisation and the solves: one warp
-
-// 1.0, read into a register: an FP64 instruction with a literal operand issues about 19% slower.
-__device__ double g_one = 1.0;
 
 // Rows in flight: every thread copies the values of the next D rows of its own system into its own slots of a
 // shared-memory ring (cp.async, one group per row), so the loads take no registers and no barrier. A row beyond
@@ -61,7 +58,7 @@ __global__ void __launch_bounds__(kLine) factor_kernel(const double* __restrict_
     const int s = blockIdx.x * kLine + t;
     if (s >= batch) return;
     const size_t B = (size_t)batch;
-    const double one = *(const volatile double*)&g_one;
+    const f64::F64 f;
     auto issue = [&](int i) {
         if (i < m) {
             const size_t q = (size_t)i * B + s;
@@ -95,7 +92,7 @@ __global__ void __launch_bounds__(kLine) factor_kernel(const double* __restrict_
             dd = dd - l * duP1;
             d[q] = dd;
         }
-        const f64::Divider by(dd, one);
+        const f64::Divider by(f, dd);
         duP2 = duP1;
         const double dwL = dwP1;
         dwP2 = dwP1;
@@ -123,7 +120,7 @@ __global__ void __launch_bounds__(kLine) solve_kernel(const double* __restrict__
     const int s = blockIdx.x * kLine + t;
     if (s >= batch) return;
     const size_t B = (size_t)batch;
-    const double one = *(const volatile double*)&g_one;
+    const f64::F64 f;
     auto issue = [&](int i) {
         if (i < m) {
             const size_t q = (size_t)i * B + s;
@@ -145,7 +142,7 @@ __global__ void __launch_bounds__(kLine) solve_kernel(const double* __restrict__
         double v = r[3][t];
         if (i >= 2) v = v - r[0][t] * p2 - r[1][t] * p1;
         else if (i == 1) v = v - r[1][t] * p1;
-        v = RCP ? v * r[2][t] : f64::Divider(r[2][t], one)(v);
+        v = RCP ? f.mul(v, r[2][t]) : f64::Divider(f, r[2][t])(v);
         b[(size_t)i * B + s] = v;
         p2 = p1;
         p1 = v;
@@ -181,9 +178,9 @@ __global__ void __launch_bounds__(kLine) solve_kernel(const double* __restrict__
 }
 
 __global__ void __launch_bounds__(kThreads) invert_kernel(double* __restrict__ d, size_t count) {
-    const double one = *(const volatile double*)&g_one;
+    const f64::F64 f;
     for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < count; q += (size_t)gridDim.x * blockDim.x)
-        d[q] = f64::reciprocal(d[q], one);
+        d[q] = f64::reciprocal(f, d[q]);
 }
 
 thread_local std::string g_err;

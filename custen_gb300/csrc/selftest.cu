@@ -58,9 +58,11 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
     return __double_as_longlong(a) == __double_as_longlong(b) || (isnan(a) && isnan(b));
 }
 
-// out[0 .. 4]: mismatches of to_float, to_double_pos (plain and quartered), div_by_float, reciprocal, Divider
+// out[0 .. 5]: mismatches of to_float, to_double_pos (plain and quartered), div_by_float, reciprocal, Divider, and
+// of the sums, differences and products as multiply-adds
 __global__ void fp64_offload_kernel(unsigned long long seed, long long samples, unsigned long long* out) {
     const double cs[3] = {0.1, 0.6, 0.3};
+    const f64::F64 f64c;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < samples;
          i += (long long)gridDim.x * blockDim.x) {
         const unsigned long long r = mix64(seed + 8ull * (unsigned long long)i);
@@ -72,9 +74,12 @@ __global__ void fp64_offload_kernel(unsigned long long seed, long long samples, 
         if (!same_bits(f64::to_double_pos(p), (double)p) || !same_bits(f64::to_double_pos<-2>(p), 0.25 * (double)p))
             atomicAdd(&out[1], 1ull);
         for (int k = 0; k < 3; ++k)
-            if (!same_bits(f64::div_by_float(cs[k], p), cs[k] / (double)p)) atomicAdd(&out[2], 1ull);
-        if (!same_bits(f64::reciprocal(b, 1.0), 1.0 / b)) atomicAdd(&out[3], 1ull);
-        if (!same_bits(f64::Divider(b, 1.0)(a), a / b)) atomicAdd(&out[4], 1ull);
+            if (!same_bits(f64::div_by_float(f64c, cs[k], p), cs[k] / (double)p)) atomicAdd(&out[2], 1ull);
+        if (!same_bits(f64::reciprocal(f64c, b), 1.0 / b)) atomicAdd(&out[3], 1ull);
+        if (!same_bits(f64::Divider(f64c, b)(a), a / b)) atomicAdd(&out[4], 1ull);
+        if (!same_bits(f64c.add(a, b), __dadd_rn(a, b)) || !same_bits(f64c.sub(a, b), __dsub_rn(a, b)) ||
+            !same_bits(f64c.mul(a, b), __dmul_rn(a, b)))
+            atomicAdd(&out[5], 1ull);
     }
 }
 
@@ -93,18 +98,19 @@ extern "C" int custen_selftest_wait_expiry(long long rounds, unsigned int* flags
     return e == cudaSuccess ? 0 : 1;
 }
 
-// Compares fp64_offload.cuh with the compiler's operators on `samples` operands; mismatches[0 .. 4] receive
-// the counts for the conversions to float and to double, c / float, 1 / x and a / b (all expected zero).
+// Compares fp64_offload.cuh with the compiler's operators on `samples` operands; mismatches[0 .. 5] receive
+// the counts for the conversions to float and to double, c / float, 1 / x, a / b, and a + b, a - b, a b (all
+// expected zero).
 extern "C" int custen_selftest_fp64(unsigned long long seed, long long samples, unsigned long long* mismatches) {
     if (samples < 1 || samples > (1ll << 34) || !mismatches) return 2;
     unsigned long long* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, 5 * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemset(d, 0, 5 * sizeof(unsigned long long));
+    cudaError_t e = cudaMalloc(&d, 6 * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMemset(d, 0, 6 * sizeof(unsigned long long));
     if (e == cudaSuccess) {
         custen::fp64_offload_kernel<<<1216, 256>>>(seed, samples, d);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(mismatches, d, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(mismatches, d, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
     cudaFree(d);
     return e == cudaSuccess ? 0 : 1;
 }

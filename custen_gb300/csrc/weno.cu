@@ -7,7 +7,7 @@
 // upwind selection, 2d_xyADVWENO_p_kernel.cu:286-348 and :352-414).
 //
 // GB300 shape: about 100 FP64 operations per point against 32 bytes of compulsory traffic, so the FP64 pipe
-// bounds this operator by a wide margin (87% active in ncu, issue slots 30%). The kernel therefore spends no
+// bounds this operator by a wide margin (issue slots 30%). The kernel therefore spends no
 // FP64 work twice or where another pipe can do it:
 //   - a 64 x TH tile with its 3-point periodic halo is staged once, and the x and y differences and the squared
 //     second differences are formed once per tile into shared memory (the reference forms five differences and
@@ -17,8 +17,8 @@
 // The reconstruction keeps the reference's operation order, including its single-precision powf on the
 // smoothness terms, so that results are bit-identical to the reference's kernel on the same GPU.
 // Measured (2048^2): 1418 us with hardware conversions and divisions (about 200 FP64 instructions per point),
-// 913 us with those moved off the FP64 pipe (112), 820 us with the shared second differences and the shorter
-// divisions (5.1 Gpts/s; 8192 x 4096: 5.4).
+// 913 us with those moved off the FP64 pipe (112), 817 us with the shared second differences and the shorter
+// divisions (103; 5.1 Gpts/s; 4096^2: 5.3, about 94% of the rate of multiply-adds).
 #include <cuda_runtime.h>
 
 #include <atomic>
@@ -50,18 +50,19 @@ struct WenoTile {
 // thread (WenoCoeffs::load): an FP64 FMA or add with a literal or kernel-parameter operand issues about
 // 19% slower on GB300 than one whose operands are all registers (507 against 602-628 G FMA/s
 // measured). The values are the literals of the reference's expressions, so every result is the same.
-__device__ double g_weno_coeffs[15] = {1.0 / 3.0, 7.0 / 6.0, 11.0 / 6.0, 1.0 / 6.0, 5.0 / 6.0,
+__device__ double g_weno_coeffs[14] = {1.0 / 3.0, 7.0 / 6.0, 11.0 / 6.0, 1.0 / 6.0, 5.0 / 6.0,
                                        2.0,       4.0,       3.0,        13.0 / 12.0, 0.25,
-                                       1e-06,     0.1,       0.6,        0.3,         1.0};
+                                       1e-06,     0.1,       0.6,        0.3};
 
 struct WenoCoeffs {
     double third, seven_sixths, eleven_sixths, sixth, five_sixths, two, four, three, thirteen_twelfths,
-        eps, g1, g2, g3, one;
+        eps, g1, g2, g3;
+    f64::F64 f;
     __device__ __forceinline__ void load() {
         const volatile double* k = g_weno_coeffs;
         third = k[0]; seven_sixths = k[1]; eleven_sixths = k[2]; sixth = k[3]; five_sixths = k[4];
         two = k[5]; four = k[6]; three = k[7]; thirteen_twelfths = k[8];
-        eps = k[10]; g1 = k[11]; g2 = k[12]; g3 = k[13]; one = k[14];
+        eps = k[10]; g1 = k[11]; g2 = k[12]; g3 = k[13];
     }
 };
 
@@ -79,20 +80,23 @@ __device__ __forceinline__ double quarter_square(double t) { return f64::to_doub
 // squared (indicator + 1e-6) taken by powf in single precision.
 __device__ __forceinline__ double weno5(const WenoCoeffs& k, double a, double b, double c, double d, double e, float s1,
                                         float s2, float s3) {
-    const double q1 = k.third * a - k.seven_sixths * b + k.eleven_sixths * c;
-    const double q2 = -k.sixth * b + k.five_sixths * c + k.third * d;
-    const double q3 = k.third * c + k.five_sixths * d - k.sixth * e;
+    // each sum of products is the contraction fma(x, y, z w) the compiler gives the reference's expression
+    const f64::F64& f = k.f;
+    const double q1 = fma(k.eleven_sixths, c, fma(k.third, a, -f.mul(k.seven_sixths, b)));
+    const double q2 = fma(k.third, d, fma(k.five_sixths, c, -f.mul(k.sixth, b)));
+    const double q3 = fma(-k.sixth, e, fma(k.third, c, f.mul(k.five_sixths, d)));
 
-    const double is1 = fma(k.thirteen_twelfths, f64::to_double_pos(s1), quarter_square(a - k.four * b + k.three * c));
-    const double is2 = fma(k.thirteen_twelfths, f64::to_double_pos(s2), quarter_square(b - d));
-    const double is3 = fma(k.thirteen_twelfths, f64::to_double_pos(s3), quarter_square(fma(k.three, c, -f64::times4(d)) + e));
+    const double is1 = fma(k.thirteen_twelfths, f64::to_double_pos(s1), quarter_square(fma(k.three, c, fma(-k.four, b, a))));
+    const double is2 = fma(k.thirteen_twelfths, f64::to_double_pos(s2), quarter_square(f.sub(b, d)));
+    const double is3 =
+        fma(k.thirteen_twelfths, f64::to_double_pos(s3), quarter_square(f.add(fma(k.three, c, -f64::times4(d)), e)));
 
-    const double g1 = f64::div_by_float(k.g1, square(is1 + k.eps));
-    const double g2 = f64::div_by_float(k.g2, square(is2 + k.eps));
-    const double g3 = f64::div_by_float(k.g3, square(is3 + k.eps));
-    const double norm = f64::reciprocal(g1 + g2 + g3, k.one);
-    const double w1 = g1 * norm, w2 = g2 * norm, w3 = g3 * norm;
-    return q1 * w1 + q2 * w2 + q3 * w3;
+    const double g1 = f64::div_by_float(f, k.g1, square(f.add(is1, k.eps)));
+    const double g2 = f64::div_by_float(f, k.g2, square(f.add(is2, k.eps)));
+    const double g3 = f64::div_by_float(f, k.g3, square(f.add(is3, k.eps)));
+    const double norm = f64::reciprocal(f, f.add(f.add(g1, g2), g3));
+    const double w1 = f.mul(g1, norm), w2 = f.mul(g2, norm), w3 = f.mul(g3, norm);
+    return fma(q3, w3, fma(q1, w1, f.mul(q2, w2)));
 }
 
 __device__ __forceinline__ int wrap_col(int c, int nx) {
@@ -127,6 +131,9 @@ __global__ void __launch_bounds__(kWenoThreads, 2) weno_adv_kernel(double* __res
     float* syb = syf + G::SYH * kWenoTW;
     const int x0 = blockIdx.x * kWenoTW, y0 = blockIdx.y * TH;
     const int tid = threadIdx.x;
+    WenoCoeffs k;
+    k.load();
+    const double dx = k.f.add(cdx, k.f.nzero), dy = k.f.add(cdy, k.f.nzero);   // the parameters in registers
 
     // stage the tile and its halo: staged (r, c) is field row y0-3+r, column x0-3+c (wrapped)
     for (int e = tid; e < G::SH * kWenoSW; e += kWenoThreads) {
@@ -144,34 +151,33 @@ __global__ void __launch_bounds__(kWenoThreads, 2) weno_adv_kernel(double* __res
     for (int e = tid; e < TH * kWenoDXW; e += kWenoThreads) {
         const int r = e / kWenoDXW, c = e - r * kWenoDXW;
         const double* row = tile + (r + kWenoHalo) * kWenoSW;
-        dxs[e] = (row[c + 1] - row[c]) * cdx;
+        dxs[e] = k.f.mul(k.f.sub(row[c + 1], row[c]), dx);
     }
     for (int e = tid; e < G::DYH * kWenoTW; e += kWenoThreads) {
         const int r = e / kWenoTW, c = e - r * kWenoTW;
-        dys[e] = (tile[(r + 1) * kWenoSW + c + kWenoHalo] - tile[r * kWenoSW + c + kWenoHalo]) * cdy;
+        dys[e] = k.f.mul(k.f.sub(tile[(r + 1) * kWenoSW + c + kWenoHalo], tile[r * kWenoSW + c + kWenoHalo]), dy);
     }
     __syncthreads();
 
-    WenoCoeffs k;
-    k.load();
     // squared second differences of every cell, once in each orientation (the order of the sum differs): the
     // three smoothness indicators of a point take them from its window's three middle cells
     for (int e = tid; e < TH * kWenoSXW; e += kWenoThreads) {
         const int r = e / kWenoSXW, c = e - r * kWenoSXW;   // cell: column x0 - 1 + c
         const double* d = dxs + r * kWenoDXW + c;
-        sxf[e] = square(d[0] - k.two * d[1] + d[2]);
-        sxb[e] = square(d[2] - k.two * d[1] + d[0]);
+        sxf[e] = square(k.f.add(fma(-k.two, d[1], d[0]), d[2]));
+        sxb[e] = square(k.f.add(fma(-k.two, d[1], d[2]), d[0]));
     }
     for (int e = tid; e < G::SYH * kWenoTW; e += kWenoThreads) {   // cell: row y0 - 1 + e / TW
         const double* d = dys + e;
-        syf[e] = square(d[0] - k.two * d[kWenoTW] + d[2 * kWenoTW]);
-        syb[e] = square(d[2 * kWenoTW] - k.two * d[kWenoTW] + d[0]);
+        syf[e] = square(k.f.add(fma(-k.two, d[kWenoTW], d[0]), d[2 * kWenoTW]));
+        syb[e] = square(k.f.add(fma(-k.two, d[kWenoTW], d[2 * kWenoTW]), d[0]));
     }
     __syncthreads();
 
     const int tx = tid % kWenoTW;
     const int x = x0 + tx;
     if (x >= nx) return;
+#pragma unroll(TH == 16 ? 2 : 1)
     for (int ty = tid / kWenoTW; ty < TH; ty += kWenoThreads / kWenoTW) {
         const int y = y0 + ty;
         if (y >= rows) break;
@@ -198,7 +204,7 @@ __global__ void __launch_bounds__(kWenoThreads, 2) weno_adv_kernel(double* __res
                                 vy ? dc[4 * kWenoTW] : dc[kWenoTW], vy ? tf[0] : tb[3 * kWenoTW],
                                 vy ? tf[kWenoTW] : tb[2 * kWenoTW], vy ? tf[2 * kWenoTW] : tb[kWenoTW]);
         // (2d_xyADVWENO_p_kernel.cu:424)
-        out[q] = uu * fx + vv * fy;
+        out[q] = fma(uu, fx, k.f.mul(vv, fy));
     }
 }
 
@@ -230,10 +236,10 @@ cudaError_t launch_weno_adv(const StencilArgs& a, cudaStream_t s) {
     // Rows per tile: two CTAs are resident per SM (304 on GB300) and each tile is a long stretch of FP64 work, so
     // few tiles leave SMs idle and few waves end in an uneven one; a lower tile forms more differences of its halo
     // twice. Measured (us, 8 / 16 / 32 rows): 300^2 40 / 44 / 77, 600^2 101 / 122 / 123, 1000 x 777 187 / 189 / 201
-    // (400 tiles of 32 rows), 1500 x 1400 453 / 431 / 454 (1056), 2048^2 896 / 853 / 832 (2048).
+    // (400 tiles of 32 rows), 1500 x 1400 453 / 431 / 454 (1056), 2048^2 - / 817 / 838 (2048), 4096^2 - / 3199 / 3141.
     const long long tiles = (long long)((a.nx + kWenoTW - 1) / kWenoTW) * ((a.rows + 31) / 32);
     if (tiles < 512) return launch_tile<8>(a, s, dev);
-    if (tiles < 1536) return launch_tile<16>(a, s, dev);
+    if (tiles < 4096) return launch_tile<16>(a, s, dev);
     return launch_tile<32>(a, s, dev);
 }
 

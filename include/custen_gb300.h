@@ -190,9 +190,10 @@ int custen_device_error(unsigned int* flags, int clear);
  * raised and the kernel returns. *flags receives the flags afterwards (left set). No copy fails and
  * nothing traps; the context stays usable. */
 int custen_selftest_wait_expiry(long long rounds, unsigned int* flags);
-/* Self-test of the kernels' conversions and divisions that avoid the FP64 pipe (csrc/fp64_offload.cuh)
- * against the compiler's operators on `samples` generated operands (1 .. 2^34): mismatches[0..4] receive
- * the counts for double -> float, float -> double, c / float, 1 / x and a / b; all are expected zero. */
+/* Self-test of the kernels' conversions, divisions, sums and products that spare the FP64 pipe
+ * (csrc/fp64_offload.cuh) against the compiler's operators on `samples` generated operands (1 .. 2^34):
+ * mismatches[0..5] receive the counts for double -> float, float -> double, c / float, 1 / x, a / b, and a + b,
+ * a - b and a b; all are expected zero. */
 int custen_selftest_fp64(unsigned long long seed, long long samples, unsigned long long* mismatches);
 
 /* ---- batched pentadiagonal systems (cuPentBatch, cuPentCahnADI/src/cuPentBatch.cu) ----
