@@ -31,7 +31,7 @@ enum : int {
     TAB_NP1 = 2,     // -p1, -p2 of the causal factor P(z) = 1 + p1 / z + p2 / z^2 of the line operator
     TAB_NP2 = 3,
     TAB_KAPPA = 4,   // 1 / G^2: the two line operators are G P(z) P(1/z)
-    TAB_REACH = 5,   // entries of f1, f2 that are not negligible (a whole number)
+    TAB_REACH = 5,   // entries of f1, f2 that are not negligible (the bits of an integer)
     TAB_MID = 6,     // 2 x 4: the other chain's two values next to the middle from (own, own, other, other) ends
     TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the chain's outer end
     kTabParams = 32

@@ -33,6 +33,7 @@
 #include "../../include/custen_gb300.h"
 #include "ch_internal.cuh"
 #include "checked.cuh"
+#include "fp64_offload.cuh"
 #include "stencil_launch.cuh"   // mbarrier and TMA helpers, the tensor map encoder
 
 namespace custen {
@@ -62,6 +63,27 @@ namespace ch {
 // so the results, are the same as with literals.
 __device__ double g_rhs_factors[3] = {2.0, -4.0, -2.0 / 3.0};
 
+// Sums and products: FP64 ones as multiply-adds (fp64_offload.cuh; h kernel 459 -> 425 us and pass 2 320 -> 296 us at
+// 24 grids of 1024^2), FP32 ones as they are.
+template <typename T>
+struct Arith {
+    __device__ __forceinline__ T add(T a, T b) const { return a + b; }
+    __device__ __forceinline__ T sub(T a, T b) const { return a - b; }
+    __device__ __forceinline__ T mul(T a, T b) const { return a * b; }
+};
+template <>
+struct Arith<double> : f64::F64 {};
+
+// c^3 - c, times s; the five-point Laplacian N + S + W + E - 4 C
+template <typename T>
+__device__ __forceinline__ T scaled_cube_minus(const Arith<T>& ar, T s, T c) {
+    return ar.mul(s, fma(ar.mul(c, c), c, -c));
+}
+template <typename T>
+__device__ __forceinline__ T laplacian(const Arith<T>& ar, T m_four, T c, T n, T s, T w, T e) {
+    return fma(m_four, c, ar.add(ar.add(n, s), ar.add(w, e)));
+}
+
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restrict__ grids,
                                                           const Item* __restrict__ items, int n_items, int parity) {
@@ -74,6 +96,8 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
     const double m_four_d = factors[1], m_two_thirds_d = factors[2];
+    const Arith<T> ar;
+    const Arith<double> ar_d;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -97,15 +121,15 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
             const double ov = old[(size_t)gy * n + gx];
             const T c32 = (T)cv, o32 = (T)ov;
             cb[r][c] = fma(two, c32, -o32);
-            if (r >= 1 && r < 35 && c >= 1 && c < 35) hh[r - 1][c - 1] = s_nl * fma(c32 * c32, c32, -c32);
-            if (r >= 2 && r < 34 && c >= 2 && c < 34) dco[r - 2][c - 2] = cv - ov;
+            if (r >= 1 && r < 35 && c >= 1 && c < 35) hh[r - 1][c - 1] = scaled_cube_minus(ar, s_nl, c32);
+            if (r >= 2 && r < 34 && c >= 2 && c < 34) dco[r - 2][c - 2] = ar_d.sub(cv, ov);
         }
         __syncthreads();
         // h = sigma_nl * g - sigma_lin * Lap(cBar) over the 34 x 34 block + halo
 #pragma unroll 4
         for (int e = tid; e < 34 * 34; e += NT) {
             const int r = e / 34, c = e - r * 34;
-            const T lap = fma(m_four, cb[r + 1][c + 1], (cb[r][c + 1] + cb[r + 2][c + 1]) + (cb[r + 1][c] + cb[r + 1][c + 2]));
+            const T lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
             hh[r][c] = fma(-s_lin, lap, hh[r][c]);
         }
         __syncthreads();
@@ -117,9 +141,8 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
         double* out = gd.tmp + (size_t)y0 * n + x0 + j;
 #pragma unroll 4
         for (int rr = warp; rr < BLK; rr += NW) {
-            const double lap = fma(m_four_d, (double)hh[rr + 1][j + 1],
-                                   ((double)hh[rr][j + 1] + (double)hh[rr + 2][j + 1]) +
-                                       ((double)hh[rr + 1][j] + (double)hh[rr + 1][j + 2]));
+            const double lap = laplacian(ar_d, m_four_d, (double)hh[rr + 1][j + 1], (double)hh[rr][j + 1],
+                                         (double)hh[rr + 2][j + 1], (double)hh[rr + 1][j], (double)hh[rr + 1][j + 2]);
             if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
             out[(size_t)rr * n] = fma(m_two_thirds_d, dco[rr][j], lap);
         }
@@ -144,6 +167,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
     const int tid = threadIdx.x;
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
+    const Arith<T> ar;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -165,13 +189,13 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
             const double ov = old[(size_t)gy * n + gx];
             const T c32 = (T)cv, o32 = (T)ov;
             cb[r][c] = fma(two, c32, -o32);
-            if (r >= 1 && r < 33 && c >= 1 && c < 33) gg[r - 1][c - 1] = s_nl * fma(c32 * c32, c32, -c32);
+            if (r >= 1 && r < 33 && c >= 1 && c < 33) gg[r - 1][c - 1] = scaled_cube_minus(ar, s_nl, c32);
         }
         __syncthreads();
 #pragma unroll 4
         for (int e = tid; e < 32 * 32; e += NT) {
             const int r = e / 32, c = e - r * 32;
-            const T lap = fma(m_four, cb[r + 1][c + 1], (cb[r][c + 1] + cb[r + 2][c + 1]) + (cb[r + 1][c] + cb[r + 1][c + 2]));
+            const T lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
             const long long q = (long long)(y0 + r) * n + x0 + c;
             if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)fma(-s_lin, lap, gg[r][c]);
         }
@@ -191,6 +215,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __rest
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const T m_four = (T)factors[1], m_two_thirds = (T)factors[2];
+    const Arith<T> ar;
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -208,7 +233,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __rest
             hh[r][c] = (T)gd.hbuf[(size_t)gy * n + gx];
             if (r >= 1 && r < 33 && c >= 1 && c < 33) {
                 const T c32 = (T)cur[(size_t)gy * n + gx], o32 = (T)old[(size_t)gy * n + gx];
-                dco[r - 1][c - 1] = c32 - o32;
+                dco[r - 1][c - 1] = ar.sub(c32, o32);
             }
         }
         __syncthreads();
@@ -216,7 +241,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __rest
         double* out = gd.tmp + (size_t)y0 * n + x0 + j;
 #pragma unroll 4
         for (int rr = warp; rr < BLK; rr += NW) {
-            const T lap = fma(m_four, hh[rr + 1][j + 1], (hh[rr][j + 1] + hh[rr + 2][j + 1]) + (hh[rr + 1][j] + hh[rr + 1][j + 2]));
+            const T lap = laplacian(ar, m_four, hh[rr + 1][j + 1], hh[rr][j + 1], hh[rr + 2][j + 1], hh[rr + 1][j], hh[rr + 1][j + 2]);
             if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
             out[(size_t)rr * n] = (double)fma(m_two_thirds, dco[rr][j], lap);
         }
@@ -280,6 +305,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const double m_four = factors[1], m_two_thirds = factors[2];
+    const Arith<double> ar;
     int it_cur = blockIdx.x;
     if (it_cur < n_items) rhs2_issue<NW>(rhs2_smem, grids[items[it_cur].grid], items[it_cur], parity, tid);
     cp_async_commit();
@@ -305,10 +331,9 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
         double* out = gd.tmp + (size_t)y0 * n + x0 + j;
 #pragma unroll 4
         for (int rr = warp; rr < BLK; rr += NW) {
-            const double lap = fma(m_four, hh[(rr + 1) * 35 + j + 1],
-                                   (hh[rr * 35 + j + 1] + hh[(rr + 2) * 35 + j + 1]) +
-                                       (hh[(rr + 1) * 35 + j] + hh[(rr + 1) * 35 + j + 2]));
-            const double dco = cu[rr * 33 + j] - ol[rr * 33 + j];
+            const double lap = laplacian(ar, m_four, hh[(rr + 1) * 35 + j + 1], hh[rr * 35 + j + 1], hh[(rr + 2) * 35 + j + 1],
+                                         hh[(rr + 1) * 35 + j], hh[(rr + 1) * 35 + j + 2]);
+            const double dco = ar.sub(cu[rr * 33 + j], ol[rr * 33 + j]);
             if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
             out[(size_t)rr * n] = fma(m_two_thirds, dco, lap);
         }
@@ -345,7 +370,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 // A warp's FP64 instruction holds its sub-partition's FP64 pipe for 64 cycles however few lanes it has, so with
 // fewer chains than FP64 sub-partitions (4 per SM) a step takes the chain's instruction count: n / 2 elements
 // of 4 instructions per sweep. Measured, us per step (before: banded factors, one warp per 32 lines): one grid of 256^2
-// 66 (159), 512^2 118 (298), 1024^2 252 (601), 2048^2 577 (1331); 96 grids of 64^2 .. 1024^2 1680 (1973).
+// 65 (159), 512^2 118 (298), 1024^2 249 (601), 2048^2 555 (1331); 96 grids of 64^2 .. 1024^2 1475 (1973).
 
 // Chunks of kChunk elements of a warp's 32 lines move between the work field and a shared-memory ring of kStages
 // stages by the tensor memory accelerator, one copy per chunk each way, issued by a copy warp per chain (two chain
@@ -551,16 +576,18 @@ __device__ __forceinline__ void init_ring(ChainBars (&bars)[2]) {
     __syncthreads();
 }
 
-// The ring's base, aligned for the 128-byte swizzle inside 1 KB of slack (as in stencil_tma.cuh, through an opaque
+// The ring's base, aligned inside its slack (x: 1 KB for the 128-byte swizzle; y: 128 bytes; as in stencil_tma.cuh, through an opaque
 // value, since the compiler may not assume more than the declared alignment).
+template <uint32_t kRingAlign>
 __device__ __forceinline__ double* ring_base(unsigned char* raw) {
     uint32_t addr = smem_u32(raw);
     asm volatile("" : "+r"(addr));
-    return reinterpret_cast<double*>(raw + ((1024u - (addr & 1023u)) & 1023u));
+    return reinterpret_cast<double*>(raw + ((kRingAlign - (addr & (kRingAlign - 1))) & (kRingAlign - 1)));
 }
 
 constexpr int kStageWords = BLK * kChunk;
-constexpr size_t kSweepBytes = 2 * kStages * kStageWords * sizeof(double) + 1024;   // dynamic shared memory
+constexpr size_t kRingBytes = 2 * kStages * kStageWords * sizeof(double);
+constexpr size_t kXSweepBytes = kRingBytes + 1024, kYSweepBytes = kRingBytes + 128;   // dynamic shared memory
 
 constexpr int kSweepThreads = 4 * BLK;   // warps: chain A, chain B, the copies of A, the copies of B
 
@@ -575,7 +602,7 @@ __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev*
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
     const CUtensorMap* map = maps + 2 * item.grid;
-    auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base(sweep_smem));
+    auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base<1024>(sweep_smem));
     if (warp == 0) xsweep_chain<1>(gd, item.block, lane, stage, bars[0], ex[0], ex[1]);
     else if (warp == 1) xsweep_chain<-1>(gd, item.block, lane, stage + kStages, bars[1], ex[1], ex[0]);
     else if (lane == 0) {
@@ -588,10 +615,25 @@ __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev*
 // y sweep: DIR = 1 is chain A (rows upwards). CLOSE: the x sweep's closure is added to the right-hand side as a
 // chunk is read, in the columns within reach of either end, by the rows' amplitudes (copied with the chunk).
 // Without it ch_xclose_kernel has added it, with the same operations.
+__device__ __forceinline__ int reach_of(const GridDev& gd) { return (int)__double_as_longlong(gd.tab[TAB_REACH]); }
+
+// The closure of one end over N values, or of none: branches around whole loops, since the compiler turns a
+// condition at each value into both ends' multiply-adds and selections.
+template <int N, class Amp>
+__device__ __forceinline__ void close_end(bool within, double (&v)[N], double f1, double f2, Amp amp) {
+    if (within) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const double2 a = amp(k);
+            v[k] = fma(f1, a.x, fma(f2, a.y, v[k]));
+        }
+    }
+}
+
 struct CloseEnds {
     bool left, right;   // whether the block's columns lie within reach of either end
     __device__ __forceinline__ CloseEnds(const GridDev& gd, int block) {
-        const int reach = (int)gd.tab[TAB_REACH];
+        const int reach = reach_of(gd);
         left = block * BLK < reach;
         right = (block + 1) * BLK > gd.n - reach;
     }
@@ -637,13 +679,10 @@ __device__ __forceinline__ void ysweep_chain(const GridDev& gd, int block, int l
         double w[kChunk];
 #pragma unroll
         for (int k = 0; k < kChunk; ++k) w[k] = stage[st][up ? k : kChunk - 1 - k][lane];
-        if (CLOSE && decltype(forward)::value && (left || right)) {
-#pragma unroll
-            for (int k = 0; k < kChunk; ++k) {
-                const double* e = amp[st][up ? k : kChunk - 1 - k];
-                if (left) w[k] = fma(l1, e[0], fma(l2, e[1], w[k]));
-                if (right) w[k] = fma(r1, e[2], fma(r2, e[3], w[k]));
-            }
+        if (CLOSE && decltype(forward)::value) {
+            auto e = [&](int k) { return reinterpret_cast<const double2*>(amp[st][up ? k : kChunk - 1 - k]); };
+            close_end(left, w, l1, l2, [&](int k) { return e(k)[0]; });
+            close_end(right, w, r1, r2, [&](int k) { return e(k)[1]; });
         }
         recur(w, np1, np2, a1, a2);
 #pragma unroll
@@ -664,18 +703,20 @@ __global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev*
                                                                   const Item* __restrict__ items,
                                                                   const CUtensorMap* maps) {
     extern __shared__ __align__(16) unsigned char sweep_smem[];
-    __shared__ __align__(16) double amp[CLOSE ? 2 * kStages : 1][kChunk][4];
-    __shared__ double ex[2][2][BLK];
+    // A chain leaves its end values for the other in its own amplitude area, which the backward pass does not use:
+    // 37 KB per CTA, so six fit an SM.
+    __shared__ __align__(16) double amp[CLOSE ? 2 * kStages : 4][kChunk][4];
     __shared__ __align__(8) ChainBars bars[2];
     init_ring(bars);
     const int lane = threadIdx.x & (BLK - 1), warp = threadIdx.x / BLK;
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
     const CUtensorMap* map = maps + 2 * item.grid + 1;
-    auto* stage = reinterpret_cast<double(*)[kChunk][BLK]>(ring_base(sweep_smem));
-    auto* amp_b = amp + (CLOSE ? kStages : 0);
-    if (warp == 0) ysweep_chain<1, CLOSE>(gd, item.block, lane, stage, amp, bars[0], ex[0], ex[1]);
-    else if (warp == 1) ysweep_chain<-1, CLOSE>(gd, item.block, lane, stage + kStages, amp_b, bars[1], ex[1], ex[0]);
+    auto* stage = reinterpret_cast<double(*)[kChunk][BLK]>(ring_base<128>(sweep_smem));
+    auto* amp_b = amp + (CLOSE ? kStages : 2);
+    auto *ex_a = reinterpret_cast<double(*)[BLK]>(amp), *ex_b = reinterpret_cast<double(*)[BLK]>(amp_b);
+    if (warp == 0) ysweep_chain<1, CLOSE>(gd, item.block, lane, stage, amp, bars[0], ex_a, ex_b);
+    else if (warp == 1) ysweep_chain<-1, CLOSE>(gd, item.block, lane, stage + kStages, amp_b, bars[1], ex_b, ex_a);
     else if (lane == 0) {
         acquire_map(map);
         if (warp == 2) ysweep_copies<1, CLOSE>(gd, map, item.block, stage, amp, bars[0]);
@@ -685,7 +726,7 @@ __global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev*
 
 // The x sweep's closure as an element-wise kernel over the 32 x 32 blocks, for batches with few chains (it spreads
 // over every SM, where in the y sweep it would lengthen the chains).
-__global__ void __launch_bounds__(256) ch_xclose_kernel(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(256, 6) ch_xclose_kernel(const GridDev* __restrict__ grids,
                                                         const Item* __restrict__ items) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
@@ -693,7 +734,7 @@ __global__ void __launch_bounds__(256) ch_xclose_kernel(const GridDev* __restric
     const int n = gd.n;
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-    const int reach = (int)gd.tab[TAB_REACH];
+    const int reach = reach_of(gd);
     const bool left = x0 < reach, right = x0 + BLK > n - reach;
     if (!left && !right) return;
     const int x = x0 + (threadIdx.x & (BLK - 1));
@@ -703,19 +744,19 @@ __global__ void __launch_bounds__(256) ch_xclose_kernel(const GridDev* __restric
     double v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = gd.tmp[(size_t)(y0 + r0 + 8 * k) * n + x];
+    auto e = [&](int k) { return reinterpret_cast<const double2*>(gd.ends + 4 * (y0 + r0 + 8 * k)); };
+    close_end(left, v, l1, l2, [&](int k) { return e(k)[0]; });
+    close_end(right, v, r1, r2, [&](int k) { return e(k)[1]; });
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int y = y0 + r0 + 8 * k;
-        const double* e = gd.ends + 4 * y;
-        if (left) v[k] = fma(l1, e[0], fma(l2, e[1], v[k]));
-        if (right) v[k] = fma(r1, e[2], fma(r2, e[3], v[k]));
-        if (in_bounds((long long)y * n + x, 0, (long long)n * n)) gd.tmp[(size_t)y * n + x] = v[k];
+        const long long q = (long long)(y0 + r0 + 8 * k) * n + x;
+        if (in_bounds(q, 0, (long long)n * n)) gd.tmp[q] = v[k];
     }
 }
 
 // K4: cNew = cBar + delta written over cOld (cuPentCahnADI.cu:58-69, 89-100), one 32 x 32 block per CTA: delta is
 // kappa times the y solution with its closure, for the rows within reach of either end.
-__global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __restrict__ grids,
                                                         const Item* __restrict__ items, int parity) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
@@ -724,15 +765,11 @@ __global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restric
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     const int x = x0 + (threadIdx.x & (BLK - 1));
-    const int reach = (int)gd.tab[TAB_REACH];
+    const int reach = reach_of(gd);
     const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
     const bool top = y0 < reach, bottom = y0 + BLK > n - reach;
     const double two = ((const volatile double*)g_rhs_factors)[0];
     const double kappa = gd.tab[TAB_KAPPA];
-    const double* e = gd.ends + 4 * n + 4 * x;
-    double a1 = 0.0, a2 = 0.0, b1 = 0.0, b2 = 0.0;
-    if (top) { a1 = e[0]; a2 = e[1]; }
-    if (bottom) { b1 = e[2]; b2 = e[3]; }
     const double* cur = parity ? gd.buf[1] : gd.buf[0];
     double* old = parity ? gd.buf[0] : gd.buf[1];
     const int r0 = threadIdx.x / BLK;
@@ -744,14 +781,24 @@ __global__ void __launch_bounds__(256) ch_update_kernel(const GridDev* __restric
         cv[k] = cur[q];
         ov[k] = old[q];
     }
+    const double2* e = reinterpret_cast<const double2*>(gd.ends + 4 * n + 4 * x);
+    if (top) {
+        const double2 a = e[0];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = fma(f1[y0 + r0 + 8 * k], a.x, fma(f2[y0 + r0 + 8 * k], a.y, v[k]));
+    }
+    if (bottom) {
+        const double2 a = e[1];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = n - 1 - (y0 + r0 + 8 * k);
+            v[k] = fma(f1[i], a.x, fma(f2[i], a.y, v[k]));
+        }
+    }
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int y = y0 + r0 + 8 * k;
-        const long long q = (long long)y * n + x;
-        double d = v[k];
-        if (top) d = fma(f1[y], a1, fma(f2[y], a2, d));
-        if (bottom) d = fma(f1[n - 1 - y], b1, fma(f2[n - 1 - y], b2, d));
-        if (in_bounds(q, 0, (long long)n * n)) old[q] = fma(kappa, d, fma(two, cv[k], -ov[k]));
+        const long long q = (long long)(y0 + r0 + 8 * k) * n + x;
+        if (in_bounds(q, 0, (long long)n * n)) old[q] = fma(kappa, v[k], fma(two, cv[k], -ov[k]));
     }
 }
 
@@ -1283,14 +1330,14 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
     if (e != cudaSuccess) return e;
     const int n = w.n_lines - w.n_general;
     if (n > 0) {   // one CTA (two chains) per 32 lines, largest grids first
-        ch_xsweep_kernel<<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+        ch_xsweep_kernel<<<n, kSweepThreads, kXSweepBytes, s>>>(w.grids, w.lines, w.maps);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if (close_apart(c, w, sms)) {
             ch_xclose_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_ysweep_kernel<false><<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+            ch_ysweep_kernel<false><<<n, kSweepThreads, kYSweepBytes, s>>>(w.grids, w.lines, w.maps);
         } else {
-            ch_ysweep_kernel<true><<<n, kSweepThreads, kSweepBytes, s>>>(w.grids, w.lines, w.maps);
+            ch_ysweep_kernel<true><<<n, kSweepThreads, kYSweepBytes, s>>>(w.grids, w.lines, w.maps);
         }
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         ch_update_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks, parity);
@@ -1419,7 +1466,8 @@ static void fill_line_table(double* t, int n, double s) {
     }
     int reach = n;
     while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp((double)peak, -62)) --reach;
-    t[TAB_REACH] = reach;
+    const long long reach_bits = reach;   // as bits: a conversion on the device would take the FP64 pipe
+    memcpy(&t[TAB_REACH], &reach_bits, sizeof(reach_bits));
     // (1 - M^n)^-1, M^n = [f1[n-1] f2[n-1]; f1[n-2] f2[n-2]]
     const long double c00 = 1.0L - a1, c01 = -b1, c10 = -a2, c11 = 1.0L - b2, det = c00 * c11 - c01 * c10;
     t[TAB_CLOSE] = (double)(c11 / det);
