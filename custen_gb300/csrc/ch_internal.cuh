@@ -47,7 +47,14 @@ struct Item {
     int block;   // right-hand side and update: 32 x 32 block index (row-major over the grid); sweeps: row / column block
 };
 
-__global__ void ch_mass_kernel(const double* __restrict__ f, long long count, double* out);
+// Sum of `count` values into out->sum (zeroed before the first call; one sum at a time on a scratch).
+constexpr int kMassBlocks = 256, kMassSpan = 2048;
+struct MassScratch {
+    double sum;
+    unsigned int arrived;
+    double part[kMassBlocks][2];
+};
+cudaError_t launch_ch_mass(const double* f, long long count, MassScratch* out, cudaStream_t s);
 
 // Kernel configuration of a step: warps per right-hand-side CTA, one or two passes of it, and where the x sweep's
 // closure is applied. Every configuration computes the same values; the batch tuner times them.

@@ -96,7 +96,7 @@ struct Server {
     Item* items_rows_d = nullptr;
     size_t cap_grids = 0, cap_maps = 0, cap_rhs = 0, cap_rows = 0;
     int n_rhs = 0, n_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
-    double* mass_d = nullptr;
+    MassScratch* mass_d = nullptr;
     int sms = 0;
     // statistics of the last run
     double makespan = 0.0;
@@ -230,8 +230,8 @@ static int admit(Server* S, int id, double now) {
             step(cudaMemcpyAsync(p[1], r.c_old0.data(), f, cudaMemcpyHostToDevice, S->stream), "Uploading cOld");
         else
             step(cudaMemcpyAsync(p[1], p[0], f, cudaMemcpyDeviceToDevice, S->stream), "Copying c0");
-        if (e == cudaSuccess) ch_mass_kernel<<<1, 256, 0, S->stream>>>(p[0], (long long)r.n * r.n, S->mass_d);
-        step(cudaMemcpyAsync(&m, S->mass_d, sizeof(double), cudaMemcpyDeviceToHost, S->stream), "Reading mass");
+        if (e == cudaSuccess) step(launch_ch_mass(p[0], (long long)r.n * r.n, S->mass_d, S->stream), "Summing the mass");
+        step(cudaMemcpyAsync(&m, &S->mass_d->sum, sizeof(double), cudaMemcpyDeviceToHost, S->stream), "Reading mass");
         step(cudaStreamSynchronize(S->stream), "Admitting");
     }
     if (e != cudaSuccess) {
@@ -275,9 +275,9 @@ static int admit(Server* S, int id, double now) {
 static int retire(Server* S, int id, double now_after) {
     Request& r = S->reqs[id];
     const double* cur = r.g.buf[S->parity];
-    ch_mass_kernel<<<1, 256, 0, S->stream>>>(cur, (long long)r.n * r.n, S->mass_d);
+    SRV_TRY(launch_ch_mass(cur, (long long)r.n * r.n, S->mass_d, S->stream), "Summing the mass");
     double m = 0.0;
-    SRV_TRY(cudaMemcpyAsync(&m, S->mass_d, sizeof(double), cudaMemcpyDeviceToHost, S->stream), "Reading mass");
+    SRV_TRY(cudaMemcpyAsync(&m, &S->mass_d->sum, sizeof(double), cudaMemcpyDeviceToHost, S->stream), "Reading mass");
     if (S->keep_results) {
         r.result.resize((size_t)r.n * r.n);
         SRV_TRY(cudaMemcpyAsync(r.result.data(), cur, r.result.size() * sizeof(double), cudaMemcpyDeviceToHost,
@@ -482,7 +482,8 @@ int custen_ch_server_create(void** out, double hbm_budget_bytes, int rhs_dtype, 
     S->chunk = chunk_steps;
     S->keep_results = keep_results;
     cudaError_t e = cudaStreamCreateWithFlags(&S->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMallocAsync(&S->mass_d, sizeof(double), S->stream);
+    if (e == cudaSuccess) e = cudaMallocAsync(&S->mass_d, sizeof(MassScratch), S->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->mass_d, 0, sizeof(MassScratch), S->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(S->stream);
     if (e != cudaSuccess) {
         delete S;

@@ -1361,24 +1361,17 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
     return e;
 }
 
-// Compensated (Neumaier) sum of one grid, one CTA of 256 threads; combined with a two-sum tree.
+// Compensated (Neumaier) sum of one grid: every thread, then every CTA, then the CTA that finishes last over the
+// CTAs' partial sums, combines with two-sums and carries the rounding errors apart. One CTA over the whole grid took
+// 0.5 ms at 512^2, bound by its own six FP64 operations per value; a CTA per kMassSpan values, at most kMassBlocks, takes 28 us with its
+// launch and read-back (547 before; 2048^2: 90 against 8449).
 __device__ __forceinline__ void two_sum(double a, double b, double& s, double& err) {
     s = a + b;
     const double bb = s - a;
     err = (a - (s - bb)) + (b - bb);
 }
 
-__global__ void __launch_bounds__(256) ch_mass_kernel(const double* __restrict__ f, long long count, double* out) {
-    __shared__ double ss[256], sc[256];
-    double s = 0.0, c = 0.0;
-    for (long long k = threadIdx.x; k < count; k += blockDim.x) {
-        double t, e;
-        two_sum(s, f[k], t, e);
-        s = t;
-        c += e;
-    }
-    ss[threadIdx.x] = s;
-    sc[threadIdx.x] = c;
+__device__ __forceinline__ void mass_reduce(double (&ss)[256], double (&sc)[256]) {
     __syncthreads();
     for (int w = 128; w > 0; w >>= 1) {
         if (threadIdx.x < w) {
@@ -1389,7 +1382,44 @@ __global__ void __launch_bounds__(256) ch_mass_kernel(const double* __restrict__
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[0] = ss[0] + sc[0];
+}
+
+__global__ void __launch_bounds__(256) ch_mass_kernel(const double* __restrict__ f, long long count, MassScratch* out) {
+    __shared__ double ss[256], sc[256];
+    __shared__ bool last;
+    const int t = threadIdx.x;
+    double s = 0.0, c = 0.0;
+    for (long long k = blockIdx.x * 256ll + t; k < count; k += gridDim.x * 256ll) {
+        double v, e;
+        two_sum(s, f[k], v, e);
+        s = v;
+        c += e;
+    }
+    ss[t] = s;
+    sc[t] = c;
+    mass_reduce(ss, sc);
+    if (t == 0) {
+        out->part[blockIdx.x][0] = ss[0];
+        out->part[blockIdx.x][1] = sc[0];
+        __threadfence();
+        last = atomicAdd(&out->arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    ss[t] = t < gridDim.x ? __ldcg(&out->part[t][0]) : 0.0;
+    sc[t] = t < gridDim.x ? __ldcg(&out->part[t][1]) : 0.0;
+    mass_reduce(ss, sc);
+    if (t == 0) {
+        out->sum = ss[0] + sc[0];
+        out->arrived = 0;   // for the next sum on this stream
+    }
+}
+
+cudaError_t launch_ch_mass(const double* f, long long count, MassScratch* out, cudaStream_t s) {
+    const long long want = (count + kMassSpan - 1) / kMassSpan;
+    ch_mass_kernel<<<(int)std::min<long long>(want, kMassBlocks), 256, 0, s>>>(f, count, out);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1587,7 +1617,7 @@ struct Batch {
     Item* items_rhs = nullptr;
     Item* items_rows = nullptr;   // K2 and K3 share the per-grid block lists (row / column blocks)
     int n_items_rhs = 0, n_items_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
-    double* mass_d = nullptr;
+    MassScratch* mass_d = nullptr;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};   // pair of steps starting at parity 0 / 1
@@ -1760,7 +1790,8 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     if (e == cudaSuccess) e = cudaMalloc(&b->items_rows, rows.size() * sizeof(Item));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->items_rows, rows.data(), rows.size() * sizeof(Item), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&b->mass_d, sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&b->mass_d, sizeof(MassScratch));
+    if (e == cudaSuccess) e = cudaMemset(b->mass_d, 0, sizeof(MassScratch));
     std::vector<CUtensorMap> maps(2 * (size_t)nsims);
     for (int s = 0; s < nsims && e == cudaSuccess; ++s)
         if (!b->grids_h[s].general && !sweep_maps(&maps[2 * s], b->grids_h[s].tmp, n[s])) e = cudaErrorNotSupported;
@@ -1882,10 +1913,9 @@ int custen_ch_batch_mean(void* h, int sim, double* mean) {
     Batch* b = static_cast<Batch*>(h);
     if (!b || sim < 0 || sim >= (int)b->n.size() || !mean) return ch_fail_arg("invalid arguments");
     const long long count = (long long)b->n[sim] * b->n[sim];
-    ch_mass_kernel<<<1, 256, 0, b->stream>>>(b->grids_h[sim].buf[b->parity], count, b->mass_d);
-    CH_TRY(cudaGetLastError(), "Launching mass sum");
+    CH_TRY(launch_ch_mass(b->grids_h[sim].buf[b->parity], count, b->mass_d, b->stream), "Launching mass sum");
     double s = 0.0;
-    CH_TRY(cudaMemcpyAsync(&s, b->mass_d, sizeof(double), cudaMemcpyDeviceToHost, b->stream), "Reading mass");
+    CH_TRY(cudaMemcpyAsync(&s, &b->mass_d->sum, sizeof(double), cudaMemcpyDeviceToHost, b->stream), "Reading mass");
     CH_TRY(cudaStreamSynchronize(b->stream), "Synchronising mass");
     *mean = s / (double)count;
     return 0;

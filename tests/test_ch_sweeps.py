@@ -1,6 +1,8 @@
 """The Cahn-Hilliard line solves at the sizes where their schedule changes (fewer, as many and more chunks per
 chain than ring stages) and over parameters that change the reach of the periodic closure: against a Fourier
 solution of the same scheme, which shares nothing with the factored sweeps (GPU)."""
+import math
+
 import numpy as np
 import pytest
 
@@ -73,4 +75,16 @@ def test_mixed_signs_in_one_batch(gpu):
     for k, (n, c) in enumerate(zip(sizes, c0)):
         r, _ = fourier_steps(c, 3, lx[k], 0.01, 0.1)
         assert np.linalg.norm(b.state(k)[0] - r) <= REL_L2 * np.linalg.norm(r), n
+    b.close()
+
+
+@pytest.mark.parametrize("n", [64, 96, 736])
+def test_mean_over_few_and_many_blocks(gpu, n):
+    """The compensated sum over 2, 5 and 256 CTAs (the cap), twice on the same scratch: exact to rounding."""
+    c = np.random.default_rng(n).uniform(-0.1, 0.1, (n, n))
+    b = cs.CahnHilliardBatch([n])
+    b.set_state(0, c)
+    exact = math.fsum(c.ravel()) / (n * n)
+    for _ in range(2):
+        assert abs(b.mean(0) - exact) <= 4e-16 * np.abs(c).mean()
     b.close()
