@@ -27,16 +27,17 @@ stencil_ldg_kernel(const __grid_constant__ StencilArgs a) {
     T* list_w = reinterpret_cast<T*>(smem + g.listw_off(a));
     const int tid = threadIdx.x + threadIdx.y * NTX;
     const bool is_fun = variant_is_fun(a.variant) && !a.pre;
+    const Zeros<T> zeros;
     const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
     stage_tile_ldg<T, TW, TH, NT, VEC>(a, tile, g, x0, y0, tid);
     const int nlist = stage_coefficients<T, NT>(a, coef_s, list_off, list_w, g.SW, tid, is_fun);  // syncs
     if (a.pre) {
-        apply_cube<T, NT>(tile, g.SR * g.SW, tid);
+        apply_cube<T, NT>(tile, g.SR * g.SW, tid, zeros);
         __syncthreads();
     }
     const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
     compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, threadIdx.x,
-                                           threadIdx.y, is_fun, all_write);
+                                           threadIdx.y, is_fun, all_write, zeros);
 }
 
 // Largest dynamic shared memory a block may opt in to on the current device.

@@ -182,6 +182,7 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
                                      round_up_int(a.ncoef * (int)sizeof(int), 16));
     const int tid = threadIdx.x + threadIdx.y * NTX;
     constexpr bool is_fun = (MODE == MODE_FUN);
+    const Zeros<T> zeros;
 
     if (tid == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
@@ -217,7 +218,7 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
             __syncthreads();
         }
         if (a.pre) {
-            apply_cube<T, NT>(tile, (int)stage_elems, tid);
+            apply_cube<T, NT>(tile, (int)stage_elems, tid, zeros);
             __syncthreads();
         }
         const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
@@ -226,13 +227,13 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
                 using SH = typename ShapeOf<MODE>::type;
                 if (sizeof(T) == 4 || nlist == SH::H * SH::V)
                     compute_window_store<T, TW, TH, RPT, VEC, SH>(a, tile, coef_s, g, x0, y0, threadIdx.x,
-                                                                  threadIdx.y, all_write);
+                                                                  threadIdx.y, all_write, zeros);
                 else
                     compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0,
-                                                           threadIdx.x, threadIdx.y, false, all_write);
+                                                           threadIdx.x, threadIdx.y, false, all_write, zeros);
             } else {
                 compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0,
-                                                       threadIdx.x, threadIdx.y, is_fun, all_write);
+                                                       threadIdx.x, threadIdx.y, is_fun, all_write, zeros);
             }
         }
         fence_proxy_async_smem();
