@@ -6,7 +6,7 @@
 // buffers is safe: the last timed launch leaves the correct output.
 //
 // Modes (custen_set_autotune, or the CUSTEN_AUTOTUNE environment variable at first use):
-//   0  look the key up in the cache; default configuration when absent (the default mode)
+//   0  look the key up in the cache; the default configuration for the size when absent (the default mode)
 //   1  as 0, and tune keys that are absent (at the handle's first Compute), then store them
 //   2  tune every new handle, overwriting the cache entry
 // Cache file: custen_set_tune_cache(path), else CUSTEN_TUNE_CACHE, else
@@ -182,8 +182,20 @@ int tune(const StencilArgs& a, int dtype, cudaStream_t s, int reps, std::vector<
 
 }  // namespace
 
+// The configuration of a launch nothing has been tuned for, by its number of points: small fields need many small
+// tiles to occupy the SMs, large ones amortise a tile's halo and barrier over more points. Measured, twelve operators
+// in us, configurations 0 (64 x 32 points in FP64, 128 x 32 in FP32), 1 (half as wide) and 5 (32 x 16, 64 x 16):
+//   FP64  256^2 92 / 78 / 60   1024^2 209 / 194 / 192   1536^2 364 / 355 / 361   3072^2 1266 / 1258 / 1273
+//         4096^2 2144 / 2165 / 2204   8192^2 8207 / 8298 / -
+//   FP32  256^2 65 / 63 / 51   1536^2 99 / 94 / 93   2048^2 127 / 126 / 132   4096^2 316 / 319 / 366
+static int default_config(const StencilArgs& a, int dtype) {
+    const double points = (double)a.nx * a.rows;
+    if (dtype == DT_F64) return points < 1.5e6 ? 5 : (points < 1.2e7 ? 1 : 0);
+    return points < 3e6 ? 5 : (points < 6e6 ? 1 : 0);
+}
+
 // The configuration for a device-resident launch: from the cache, from tuning (modes 1, 2 or force),
-// else the default. Returns the index.
+// else the default for its size. Returns the index.
 int choose_config(const StencilArgs& a, int dtype, cudaStream_t s, bool force, int reps) {
     std::lock_guard<std::mutex> lock(g_mu);
     const int m = force ? 2 : mode();
@@ -191,15 +203,15 @@ int choose_config(const StencilArgs& a, int dtype, cudaStream_t s, bool force, i
     const std::string key = make_key(a, dtype);
     auto it = g_cache.find(key);
     if (m < 2 && it != g_cache.end()) return it->second.index;
-    if (m == 0) return 0;
+    if (m == 0) return default_config(a, dtype);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
         cudaGetLastError();
-        return it != g_cache.end() ? it->second.index : 0;
+        return it != g_cache.end() ? it->second.index : default_config(a, dtype);
     }
     std::vector<float> ms;
     const int best = tune(a, dtype, s, reps > 0 ? reps : 3, &ms);
-    if (best < 0) return 0;
+    if (best < 0) return default_config(a, dtype);
     Entry en;
     en.config = config_name(dtype, best);
     en.index = best;

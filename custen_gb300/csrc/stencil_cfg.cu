@@ -1,6 +1,6 @@
 // One entry of the stencil configuration table (stencil_configs.h), selected at compile time by
 // CUSTEN_CFG_DTYPE (0 FP64, 1 FP32) and CUSTEN_CFG_INDEX: the TMA-staged kernels of every mode and
-// the plain-load fallback for that tile shape. The build compiles this file once per entry.
+// the cp.async-staged kernels for that tile shape. The build compiles this file once per entry.
 #include "stencil_configs.h"
 #include "stencil_launch.cuh"
 
@@ -29,7 +29,7 @@ cudaError_t CUSTEN_CFG_FN(CUSTEN_CFG_DTYPE, CUSTEN_CFG_INDEX)(const StencilArgs&
     *path = 1;
     if (e != cudaErrorNotSupported) return e;
     *path = 0;
-    return launch_ldg<CfgT, kCfg.tw, kCfg.th, kCfg.rpt, kCfg.vec>(a, s);
+    return launch_async<CfgT, kCfg.tw, kCfg.th, kCfg.rpt, kCfg.vec>(a, s);
 }
 
 }  // namespace custen

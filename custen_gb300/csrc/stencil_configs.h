@@ -4,7 +4,8 @@
 // the depth of its register window) and the vector width (vec adjacent outputs per thread, one
 // vec-wide load / store): the CTA has (tw / vec) x (th / rpt) threads, which is the role of the
 // reference's BLOCK_X x BLOCK_Y. Every configuration computes each point with the same FMA chain, so
-// the choice changes time, never results. Entry 0 is the default.
+// the choice changes time, never results. An untuned launch
+// takes entry 0, 1 or 5 by its size (autotune.cu).
 //
 // stencil_cfg.cu is compiled once per entry (CUSTEN_CFG_DTYPE, CUSTEN_CFG_INDEX); stencil_dispatch.cu
 // routes a launch to the entry a handle uses.

@@ -10,8 +10,8 @@
 // Each CTA owns an output tile of TW x TH points. It stages the (TH+T+B) x (LP+TW+RP) input window
 // in shared memory -- the rows from the launch's own rows or from the top/bottom halo pointers, the
 // columns wrapped (periodic) or zero-filled (non-periodic) -- then every thread produces VEC adjacent
-// columns x RPT rows with 16-byte vector stores. Halo tiles are staged by TMA (stencil_tma.cuh) when
-// the geometry allows; this file holds the compute/store stage and the plain-load staging path.
+// columns x RPT rows with 16-byte vector stores. The windows are staged by TMA when rows are 16-byte aligned
+// (stencil_tma.cuh), else by cp.async (stencil_async.cuh); this file holds the compute/store stage.
 #pragma once
 
 #include "builtin_funs.cuh"
@@ -43,7 +43,6 @@ struct TileGeom {
         SW = LP + TW + RP;
         SR = TH + a.T + a.B;
     }
-    __host__ __device__ size_t tile_bytes() const { return (size_t)SR * SW * sizeof(T); }
     // TMA path, periodic in x: per stage, the side areas that the wrap-around boxes fill (LP x SR and
     // RP x SR elements, each rounded up to 128 bytes); zero when the launch does not wrap.
     __host__ __device__ int wrap_l_bytes(const StencilArgs& a) const {
@@ -52,16 +51,13 @@ struct TileGeom {
     __host__ __device__ int wrap_r_bytes(const StencilArgs& a) const {
         return a.wrap_x && RP > 0 ? round_up_int(RP * SR * (int)sizeof(T), 128) : 0;
     }
-    // tile | coefficients (ncoef T) | compact list offsets (ncoef int) | compact list weights (ncoef T)
-    __host__ __device__ size_t coef_off(const StencilArgs&) const { return round_up_int((int)tile_bytes(), 16); }
-    __host__ __device__ size_t list_off(const StencilArgs& a) const {
-        return coef_off(a) + round_up_int(a.ncoef * (int)sizeof(T), 16);
-    }
-    __host__ __device__ size_t listw_off(const StencilArgs& a) const {
+    // coefficients (ncoef T) | compact list offsets (ncoef int) | compact list weights (ncoef T), after the ring
+    __host__ __device__ static size_t list_off(const StencilArgs& a) { return round_up_int(a.ncoef * (int)sizeof(T), 16); }
+    __host__ __device__ static size_t listw_off(const StencilArgs& a) {
         return list_off(a) + round_up_int(a.ncoef * (int)sizeof(int), 16);
     }
-    __host__ __device__ size_t total_bytes(const StencilArgs& a) const {
-        return listw_off(a) + round_up_int(a.ncoef * (int)sizeof(T), 16) + 16;
+    __host__ __device__ static size_t coef_bytes(const StencilArgs& a) {
+        return listw_off(a) + round_up_int(a.ncoef * (int)sizeof(T), 16);
     }
 };
 
@@ -79,29 +75,42 @@ __device__ __forceinline__ const T* launch_row(const StencilArgs& a, int gyl) {
     return nullptr;
 }
 
-// Stage coefficients and, for weight variants, the compact list of non-zero weights in weight order.
+// Stage coefficients and, for weight variants, count the non-zero weights; with `list` also their compact list in
+// weight order (one warp, 32 weights at a time). Returns the count (0 for device functions).
 template <typename T, int NT>
 __device__ __forceinline__ int stage_coefficients(const StencilArgs& a, T* coef_s, int* list_off, T* list_w,
-                                                  int SW, int tid, bool is_fun) {
+                                                  int SW, int tid, bool is_fun, bool shape) {
     const T* c = reinterpret_cast<const T*>(a.coef);
-    for (int k = tid; k < a.ncoef; k += NT) coef_s[k] = c[k];
-    __syncthreads();
+    int mine = 0;
+    for (int k = tid; k < a.ncoef; k += NT) {
+        coef_s[k] = c[k];
+        mine += c[k] != T(0);
+    }
     __shared__ int s_count;
-    if (!is_fun && tid == 0) {
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    if (is_fun) return 0;
+    if (mine) atomicAdd(&s_count, mine);
+    __syncthreads();
+    const int count = s_count;
+    if (shape && (sizeof(T) == 4 || count == a.H * a.V)) return count;   // compute_tile takes the shape's own loop
+    if (tid < 32) {
         int n = 0;
-        for (int k = 0; k < a.ncoef; ++k) {
-            T w = coef_s[k];
+        for (int k0 = 0; k0 < a.ncoef; k0 += 32) {
+            const int k = k0 + tid;
+            const T w = k < a.ncoef ? coef_s[k] : T(0);
+            const unsigned on = __ballot_sync(0xffffffffu, w != T(0));
             if (w != T(0)) {
-                int j = k / a.H, i = k - j * a.H;
-                list_off[n] = j * SW + i;
-                list_w[n] = w;
-                ++n;
+                const int at = n + __popc(on & ((1u << tid) - 1u));
+                const int j = k / a.H, i = k - j * a.H;
+                list_off[at] = j * SW + i;
+                list_w[at] = w;
             }
+            n += __popc(on);
         }
-        s_count = n;
     }
     __syncthreads();
-    return is_fun ? 0 : s_count;
+    return count;
 }
 
 // 0.0 and -0.0 in registers that the compiler cannot fold. A multiply-add whose addend is the zero register (the
@@ -132,43 +141,6 @@ __device__ __forceinline__ void apply_cube(T* tile, int count, int tid, const Ze
     for (int e = tid; e < count; e += NT) {
         const T c = tile[e];
         tile[e] = fma(fma(c, c, zeros.neg), c, -c);
-    }
-}
-
-// Plain-load staging of the window (16-byte vector loads where the whole vector is in range).
-template <typename T, int TW, int TH, int NT, int VEC>
-__device__ __forceinline__ void stage_tile_ldg(const StencilArgs& a, T* tile, const TileGeom<T, TW, TH>& g,
-                                               int x0, int y0, int tid) {
-    using V = typename VecN<T, VEC>::type;
-    const int cvecs = g.SW / VEC;
-    const int total = g.SR * cvecs;
-    for (int e = tid; e < total; e += NT) {
-        int r = e / cvecs;
-        int c = (e - r * cvecs) * VEC;
-        int gx = x0 - g.LP + c;
-        const T* rowp = launch_row<T>(a, y0 - a.T + r);
-        if (!span_ok((long long)r * g.SW + c, VEC, (long long)g.SR * g.SW)) continue;
-        T* dst = tile + r * g.SW + c;
-        if (rowp == nullptr) {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) dst[v] = T(0);
-            continue;
-        }
-        if (a.vec_ok && gx >= 0 && gx + VEC <= a.nx) {
-            *reinterpret_cast<V*>(dst) = __ldg(reinterpret_cast<const V*>(rowp + gx));
-        } else {
-#pragma unroll
-            for (int v = 0; v < VEC; ++v) {
-                int x = gx + v;
-                T val = T(0);
-                if (x >= 0 && x < a.nx) val = __ldg(rowp + x);
-                else if (a.wrap_x) {
-                    int xw = x < 0 ? x + a.nx : x - a.nx;
-                    if (xw >= 0 && xw < a.nx) val = __ldg(rowp + xw);
-                }
-                dst[v] = val;
-            }
-        }
     }
 }
 
@@ -361,5 +333,33 @@ __device__ __forceinline__ void compute_window_store(const StencilArgs& a, const
     }
     store_outputs<T, RPT, VEC>(a, acc, x0 + c0, y0 + r0, all_write_tile);
 }
+
+// One staged tile with a kernel mode: MODE_LIST (weights, generic window), MODE_FUN (device function), or a
+// compile-time shape. FP64 shape kernels fall back to the list when a weight is zero (FP64 FMAs are the bottleneck
+// on GB300; dropping exact zeros is bit-neutral for finite inputs).
+template <typename T, int TW, int TH, int RPT, int VEC, int MODE>
+__device__ __forceinline__ void compute_tile(const StencilArgs& a, T* tile, T* coef_s, const int* list_off,
+                                             const T* list_w, int nlist, const TileGeom<T, TW, TH>& g, int x0, int y0,
+                                             bool all_write, const Zeros<T>& zeros) {
+    if constexpr (MODE >= MODE_FIRST_SHAPE) {
+        using SH = typename ShapeOf<MODE>::type;
+        if (sizeof(T) == 4 || nlist == SH::H * SH::V) {
+            compute_window_store<T, TW, TH, RPT, VEC, SH>(a, tile, coef_s, g, x0, y0, threadIdx.x, threadIdx.y, all_write,
+                                                          zeros);
+            return;
+        }
+    }
+    compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, threadIdx.x, threadIdx.y,
+                                           MODE == MODE_FUN, all_write, zeros);
+}
+
+// Resident CTAs the register allocation must allow: 768 threads per SM (512 for the device-function
+// mode, whose indirect calls need more registers).
+constexpr int min_blocks_for(int threads, bool fun) { return (fun ? 512 : 768) / threads > 0 ? (fun ? 512 : 768) / threads : 1; }
+
+// A stencil launch may start while the launch before it on the stream still runs (programmatic dependent launch):
+// its set-up overlaps that launch's end; everything it reads or writes in memory comes after launch_wait().
+__device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 }  // namespace custen

@@ -7,38 +7,12 @@
 #include <atomic>
 #include <cstring>
 
+#include "stencil_async.cuh"
 #include "stencil_configs.h"
 #include "stencil_kernel.cuh"
 #include "stencil_tma.cuh"
 
 namespace custen {
-
-// Plain-load staged kernel: handles every geometry (odd widths, unaligned rows, any halo).
-template <typename T, int TW, int TH, int RPT, int VEC>
-__global__ void __launch_bounds__((TW / VEC) * (TH / RPT), min_blocks_for((TW / VEC) * (TH / RPT), true))
-stencil_ldg_kernel(const __grid_constant__ StencilArgs a) {
-    constexpr int NTX = TW / VEC;
-    constexpr int NT = NTX * (TH / RPT);
-    extern __shared__ __align__(16) unsigned char smem[];
-    TileGeom<T, TW, TH> g(a);
-    T* tile = reinterpret_cast<T*>(smem);
-    T* coef_s = reinterpret_cast<T*>(smem + g.coef_off(a));
-    int* list_off = reinterpret_cast<int*>(smem + g.list_off(a));
-    T* list_w = reinterpret_cast<T*>(smem + g.listw_off(a));
-    const int tid = threadIdx.x + threadIdx.y * NTX;
-    const bool is_fun = variant_is_fun(a.variant) && !a.pre;
-    const Zeros<T> zeros;
-    const int x0 = blockIdx.x * TW, y0 = blockIdx.y * TH;
-    stage_tile_ldg<T, TW, TH, NT, VEC>(a, tile, g, x0, y0, tid);
-    const int nlist = stage_coefficients<T, NT>(a, coef_s, list_off, list_w, g.SW, tid, is_fun);  // syncs
-    if (a.pre) {
-        apply_cube<T, NT>(tile, g.SR * g.SW, tid, zeros);
-        __syncthreads();
-    }
-    const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
-    compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, threadIdx.x,
-                                           threadIdx.y, is_fun, all_write, zeros);
-}
 
 // Largest dynamic shared memory a block may opt in to on the current device.
 inline int smem_optin_limit() {
@@ -60,18 +34,6 @@ inline cudaError_t ensure_smem(Kernel k, size_t smem) {
     if (smem <= 48 * 1024) return cudaSuccess;
     if (smem > (size_t)smem_optin_limit()) return cudaErrorInvalidConfiguration;
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-}
-
-template <typename T, int TW, int TH, int RPT, int VEC>
-cudaError_t launch_ldg(const StencilArgs& a, cudaStream_t s) {
-    TileGeom<T, TW, TH> g(a);
-    const size_t smem = g.total_bytes(a);
-    cudaError_t e = ensure_smem(stencil_ldg_kernel<T, TW, TH, RPT, VEC>, smem);
-    if (e != cudaSuccess) return e;
-    dim3 block(TW / VEC, TH / RPT);
-    dim3 grid((a.nx + TW - 1) / TW, (a.rows + TH - 1) / TH);
-    stencil_ldg_kernel<T, TW, TH, RPT, VEC><<<grid, block, smem, s>>>(a);
-    return cudaGetLastError();
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time libcuda dependency).
@@ -122,13 +84,62 @@ inline int sm_count() {
 // Resident threads per SM of the persistent FP32 grid (see launch_tma_mode).
 constexpr int kF32ThreadsPerSM = 768;
 
+// CTAs of a persistent launch: those that fit, at most one per tile, under the test cap.
+inline int persistent_grid(int tiles_total, int per_sm) {
+    const int grid = std::min(tiles_total, per_sm * sm_count());
+    const int cap = persistent_grid_cap();
+    return cap > 0 ? std::min(grid, cap) : grid;
+}
+
+// Launch with programmatic stream serialization: the kernel may start before the previous kernel of the stream has
+// ended and waits for it itself (launch_wait). Each CTA allows that when it starts its last tile: 256^2, twelve FP64
+// operators in stream order, 99 us when allowed from the start, 55 us so (116 us without, and with the former set-up
+// and tiles); 4096^2 FP32 in four tiles: 352, 324 and 343 us.
+template <typename... P, typename... A>
+cudaError_t launch_overlapped(void (*kern)(P...), int grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// cp.async path, for every geometry whose window fits shared memory: as many ring stages as leave two CTAs per SM,
+// at least one.
+template <typename T, int TW, int TH, int RPT, int VEC, int MODE>
+cudaError_t launch_async_mode(const StencilArgs& a, cudaStream_t s) {
+    TileGeom<T, TW, TH> g(a);
+    auto kern = stencil_async_kernel<T, TW, TH, RPT, VEC, MODE>;
+    const size_t stage = async_stage_bytes<T>(g.SR, g.SW);
+    const size_t limit = smem_optin_limit();
+    int stages = kAsyncStages;
+    while (stages > 1 && 2 * (stages * stage + g.coef_bytes(a)) > limit) --stages;
+    const size_t smem = stages * stage + g.coef_bytes(a) + 16;
+    cudaError_t e = ensure_smem(kern, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (TW / VEC) * (TH / RPT), smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const int tiles_x = (a.nx + TW - 1) / TW;
+    const int tiles_total = tiles_x * ((a.rows + TH - 1) / TH);
+    return launch_overlapped(kern, persistent_grid(tiles_total, per_sm), dim3(TW / VEC, TH / RPT), smem, s, a, tiles_x,
+                             tiles_total, stages);
+}
+
 // TMA path: returns cudaErrorNotSupported (without launching) when the geometry does not allow it.
 template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP>
 cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     TileGeom<T, TW, TH> g(a);
-    // One box per window: at most 256 columns and 256 rows; rows and columns tile exactly; rows
-    // 16-byte aligned (global address and stride rules of cuTensorMapEncodeTiled).
-    if (!a.vec_ok || a.nx % TW != 0 || a.rows % TH != 0 || g.SW > 256 || g.SR > 256) return cudaErrorNotSupported;
+    // One box per window: at most 256 columns and 256 rows; rows 16-byte aligned (global address and stride
+    // rules of cuTensorMapEncodeTiled).
+    if (!a.vec_ok || g.SW > 256 || g.SR > 256) return cudaErrorNotSupported;
     TmaMaps maps;
     memset(&maps, 0, sizeof(maps));
     if (!encode_rows_map<T>(&maps.win, a.in, a.nx, a.rows, g.SW, g.SR)) return cudaErrorNotSupported;
@@ -138,8 +149,7 @@ cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     if (wl_bytes && !encode_rows_map<T>(&maps.wrap_l, a.in, a.nx, a.rows, g.LP, g.SR)) return cudaErrorNotSupported;
     if (wr_bytes && !encode_rows_map<T>(&maps.wrap_r, a.in, a.nx, a.rows, g.RP, g.SR)) return cudaErrorNotSupported;
     const size_t stage_bytes = round_up_int((int)((size_t)g.SR * g.SW * sizeof(T)), 128);
-    const size_t smem = S * (stage_bytes + wl_bytes + wr_bytes) + round_up_int(a.ncoef * (int)sizeof(T), 16) +
-                        round_up_int(a.ncoef * (int)sizeof(int), 16) + round_up_int(a.ncoef * (int)sizeof(T), 16) +
+    const size_t smem = S * (stage_bytes + wl_bytes + wr_bytes) + g.coef_bytes(a) +
                         256;   // 128 bytes of alignment slack for the ring base + tail padding
     auto kern = stencil_tma_kernel<T, TW, TH, RPT, VEC, S, MODE, WRAP>;
     cudaError_t e = ensure_smem(kern, smem);
@@ -152,14 +162,10 @@ cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     // capped at 768 threads per SM, 624 at 512. The FP64 launches, bound by the FP64 pipe, keep every
     // CTA that fits (the 768 cap cost them 0.3%).
     if (sizeof(T) == 4) per_sm = std::min(per_sm, std::max(1, kF32ThreadsPerSM / ((TW / VEC) * (TH / RPT))));
-    const int tiles_x = a.nx / TW;
-    const int tiles_total = tiles_x * (a.rows / TH);
-    int grid = std::min(tiles_total, per_sm * sm_count());
-    const int cap = persistent_grid_cap();
-    if (cap > 0) grid = std::min(grid, cap);
-    dim3 block(TW / VEC, TH / RPT);
-    kern<<<grid, block, smem, s>>>(maps, a, tiles_x, tiles_total);
-    return cudaGetLastError();
+    const int tiles_x = (a.nx + TW - 1) / TW;
+    const int tiles_total = tiles_x * ((a.rows + TH - 1) / TH);
+    return launch_overlapped(kern, persistent_grid(tiles_total, per_sm), dim3(TW / VEC, TH / RPT), smem, s, maps, a,
+                             tiles_x, tiles_total);
 }
 
 // The instantiation with or without the wrap-around boxes; the Y shapes have no columns to wrap.
@@ -173,11 +179,15 @@ cudaError_t launch_tma_wrap(const StencilArgs& a, cudaStream_t s, bool wrap) {
     }
 }
 
+// The kernel mode of a launch.
+inline int launch_mode(const StencilArgs& a) {
+    return (variant_is_fun(a.variant) && !a.pre) ? (int)MODE_FUN : shape_mode(a.H, a.L, a.V, a.T);
+}
+
 template <typename T, int TW, int TH, int RPT, int VEC, int S>
 cudaError_t launch_tma(const StencilArgs& a, cudaStream_t s) {
-    const int mode = (variant_is_fun(a.variant) && !a.pre) ? (int)MODE_FUN : shape_mode(a.H, a.L, a.V, a.T);
     const bool wrap = a.wrap_x && (a.L > 0 || a.R > 0);
-    switch (mode) {
+    switch (launch_mode(a)) {
     case MODE_FUN: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, MODE_FUN>(a, s, wrap);
     case 2: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, 2>(a, s, wrap);
     case 3: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, 3>(a, s, wrap);
@@ -188,6 +198,22 @@ cudaError_t launch_tma(const StencilArgs& a, cudaStream_t s) {
     case 8: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, 8>(a, s, wrap);
     case 9: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, 9>(a, s, wrap);
     default: return launch_tma_wrap<T, TW, TH, RPT, VEC, S, MODE_LIST>(a, s, wrap);
+    }
+}
+
+template <typename T, int TW, int TH, int RPT, int VEC>
+cudaError_t launch_async(const StencilArgs& a, cudaStream_t s) {
+    switch (launch_mode(a)) {
+    case MODE_FUN: return launch_async_mode<T, TW, TH, RPT, VEC, MODE_FUN>(a, s);
+    case 2: return launch_async_mode<T, TW, TH, RPT, VEC, 2>(a, s);
+    case 3: return launch_async_mode<T, TW, TH, RPT, VEC, 3>(a, s);
+    case 4: return launch_async_mode<T, TW, TH, RPT, VEC, 4>(a, s);
+    case 5: return launch_async_mode<T, TW, TH, RPT, VEC, 5>(a, s);
+    case 6: return launch_async_mode<T, TW, TH, RPT, VEC, 6>(a, s);
+    case 7: return launch_async_mode<T, TW, TH, RPT, VEC, 7>(a, s);
+    case 8: return launch_async_mode<T, TW, TH, RPT, VEC, 8>(a, s);
+    case 9: return launch_async_mode<T, TW, TH, RPT, VEC, 9>(a, s);
+    default: return launch_async_mode<T, TW, TH, RPT, VEC, MODE_LIST>(a, s);
     }
 }
 

@@ -5,7 +5,8 @@
 // box of SW = LP + TW + RP columns by SR = T + TH + B rows starting at (x0 - LP, y0 - T), landing at a
 // 128-byte aligned stage. Completion is signalled on the stage's mbarrier (complete_tx); the next
 // tiles' copies run while the current tile computes. Rows and columns outside the launch arrive
-// zero-filled. Periodic variants add wrap-around boxes on the first and last tile column: the LP
+// zero-filled; the last tile column and row may be partial. Periodic variants add wrap-around boxes on the first
+// and last tile columns: the LP
 // columns left of x = 0 come from x = nx - LP, the RP columns right of nx from x = 0, each into a
 // side area of the stage on the same mbarrier, from where the edge tile copies them into place.
 // Edge tiles of the first and last tile row fetch their halo rows through the halo pointers with
@@ -79,7 +80,7 @@ __device__ __forceinline__ void issue_window(const StencilArgs& a, const TmaMaps
                                              int wr_elems, uint64_t* bar, int x0, int y0,
                                              const TileGeom<T, TW, TH>& g) {
     const bool left = wl_elems > 0 && x0 == 0;
-    const bool right = wr_elems > 0 && x0 + TW == a.nx;
+    const bool right = wr_elems > 0 && x0 + TW + a.R > a.nx;   // the last column, and the one before a narrow last
     uint32_t bytes = (uint32_t)(g.SR * g.SW * sizeof(T));
     if (left) bytes += (uint32_t)(g.SR * g.LP * sizeof(T));
     if (right) bytes += (uint32_t)(g.SR * g.RP * sizeof(T));
@@ -117,11 +118,12 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
         }
     }
     if (cols_fix) {
-        // wrapped halo columns of the rows inside the launch, from the side areas: column k < LP of
-        // row r is side[r * LP + k] (x = nx - LP + k), column LP + TW + k is side_r[r * RP + k] (x = k);
-        // the boxes zero-fill x outside [0, nx) as a too-narrow field needs
-        const bool left = x0 == 0, right = x0 + TW == a.nx;
+        // wrapped halo columns of the rows inside the launch, from the side areas: column k < LP of row r is
+        // side[r * LP + k] (x = nx - LP + k), the column of x = nx + k is side_r[r * RP + k] (x = k); the boxes
+        // zero-fill x outside [0, nx) as a too-narrow field needs
+        const bool left = x0 == 0, right = x0 + TW + a.R > a.nx;
         const T* side_r = side + wl_elems;
+        const int c_end = g.LP + a.nx - x0;   // window column of x = nx
         const int ncols = g.LP + g.RP;
         const int total = g.SR * ncols;
         for (int e = tid; e < total; e += NT) {
@@ -134,21 +136,14 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
                 if (!in_bounds((long long)r * g.SW + k, 0, (long long)g.SR * g.SW)) continue;
                 tile[r * g.SW + k] = side[r * g.LP + k];
             } else {
-                if (!right) continue;
                 const int kk = k - g.LP;
-                if (!in_bounds((long long)r * g.SW + g.LP + TW + kk, 0, (long long)g.SR * g.SW)) continue;
-                tile[r * g.SW + g.LP + TW + kk] = side_r[r * g.RP + kk];
+                if (!right || c_end + kk >= g.SW) continue;
+                if (!in_bounds((long long)r * g.SW + c_end + kk, 0, (long long)g.SR * g.SW)) continue;
+                tile[r * g.SW + c_end + kk] = side_r[r * g.RP + kk];
             }
         }
     }
 }
-
-// MODE: MODE_LIST (weights, generic window), MODE_FUN (device function), or a compile-time shape.
-// FP64 shape kernels fall back to the list when a weight is zero (FP64 FMAs are the bottleneck on
-// GB300; dropping exact zeros is bit-neutral for finite inputs).
-// Resident CTAs the register allocation must allow: 768 threads per SM (512 for the device-function
-// mode, whose indirect calls need more registers).
-constexpr int min_blocks_for(int threads, bool fun) { return (fun ? 512 : 768) / threads > 0 ? (fun ? 512 : 768) / threads : 1; }
 
 // WRAP: the launch is periodic in x with a left or right halo (wrap-around boxes and side areas); the
 // other launches run an instantiation without them, which keeps their register allocation.
@@ -177,9 +172,8 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
     T* sides = reinterpret_cast<T*>(smem + S * stage_bytes);
     unsigned char* after = smem + S * (stage_bytes + wl_bytes + wr_bytes);
     T* coef_s = reinterpret_cast<T*>(after);
-    int* list_off = reinterpret_cast<int*>(after + round_up_int(a.ncoef * (int)sizeof(T), 16));
-    T* list_w = reinterpret_cast<T*>(reinterpret_cast<unsigned char*>(list_off) +
-                                     round_up_int(a.ncoef * (int)sizeof(int), 16));
+    int* list_off = reinterpret_cast<int*>(after + g.list_off(a));
+    T* list_w = reinterpret_cast<T*>(after + g.listw_off(a));
     const int tid = threadIdx.x + threadIdx.y * NTX;
     constexpr bool is_fun = (MODE == MODE_FUN);
     const Zeros<T> zeros;
@@ -187,6 +181,9 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
     if (tid == 0) {
         for (int s = 0; s < S; ++s) mbar_init(&full[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    launch_wait();
+    if (tid == 0) {
         for (int k = 0; k < S; ++k) {
             const int t = blockIdx.x + k * gridDim.x;
             if (t >= tiles_total) break;
@@ -196,11 +193,12 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
                                     txi * TW, tyi * TH, g);
         }
     }
-    const int nlist = stage_coefficients<T, NT>(a, coef_s, list_off, list_w, g.SW, tid, is_fun);  // syncs
+    const int nlist = stage_coefficients<T, NT>(a, coef_s, list_off, list_w, g.SW, tid, is_fun, MODE >= MODE_FIRST_SHAPE);  // syncs
 
     for (int it = 0;; ++it) {
         const int t = blockIdx.x + it * gridDim.x;
         if (t >= tiles_total) break;
+        if (t + gridDim.x >= tiles_total) launch_dependents();   // the CTA's last tile
         const int s = it % S;
         const uint32_t parity = (uint32_t)((it / S) & 1);
         T* tile = ring + (size_t)s * stage_bytes / sizeof(T);
@@ -211,8 +209,8 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
         const bool ok = mbar_wait(&full[s], parity);
         const int tyi = t / tiles_x, txi = t - tyi * tiles_x;
         const int x0 = txi * TW, y0 = tyi * TH;
-        const bool rows_fix = (y0 == 0 && a.T > 0 && a.has_top) || (y0 + TH == a.rows && a.B > 0 && a.has_bot);
-        const bool cols_fix = WRAP && (x0 == 0 || x0 + TW == a.nx);
+        const bool rows_fix = (y0 == 0 && a.T > 0 && a.has_top) || (y0 + TH + a.B > a.rows && a.B > 0 && a.has_bot);
+        const bool cols_fix = WRAP && (x0 == 0 || x0 + TW + a.R > a.nx);
         if (rows_fix || cols_fix) {
             edge_fixup<T, TW, TH, NT>(a, tile, side, wl_elems, g, x0, y0, tid, rows_fix, cols_fix);
             __syncthreads();
@@ -222,20 +220,8 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
             __syncthreads();
         }
         const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
-        if (ok) {
-            if constexpr (MODE >= MODE_FIRST_SHAPE) {
-                using SH = typename ShapeOf<MODE>::type;
-                if (sizeof(T) == 4 || nlist == SH::H * SH::V)
-                    compute_window_store<T, TW, TH, RPT, VEC, SH>(a, tile, coef_s, g, x0, y0, threadIdx.x,
-                                                                  threadIdx.y, all_write, zeros);
-                else
-                    compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0,
-                                                           threadIdx.x, threadIdx.y, false, all_write, zeros);
-            } else {
-                compute_and_store<T, TW, TH, RPT, VEC>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0,
-                                                       threadIdx.x, threadIdx.y, is_fun, all_write, zeros);
-            }
-        }
+        if (ok)
+            compute_tile<T, TW, TH, RPT, VEC, MODE>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
         fence_proxy_async_smem();
         // every thread is done with stage s; a copy that never completed ends the CTA here: record it,
         // wait (bounded) for the copies this CTA still has in flight, and leave
