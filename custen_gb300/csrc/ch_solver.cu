@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
     const double m_four_d = factors[1], m_two_thirds_d = factors[2];
     const Arith<T> ar;
     const Arith<double> ar_d;
+    launch_wait();
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
     const Arith<T> ar;
+    launch_wait();
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -216,6 +218,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __rest
     const volatile double* factors = g_rhs_factors;
     const T m_four = (T)factors[1], m_two_thirds = (T)factors[2];
     const Arith<T> ar;
+    launch_wait();
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
         const GridDev gd = grids[item.grid];
@@ -306,6 +309,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
     const volatile double* factors = g_rhs_factors;
     const double m_four = factors[1], m_two_thirds = factors[2];
     const Arith<double> ar;
+    launch_wait();
     int it_cur = blockIdx.x;
     if (it_cur < n_items) rhs2_issue<NW>(rhs2_smem, grids[items[it_cur].grid], items[it_cur], parity, tid);
     cp_async_commit();
@@ -603,6 +607,7 @@ __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev*
     const GridDev gd = grids[item.grid];
     const CUtensorMap* map = maps + 2 * item.grid;
     auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base<1024>(sweep_smem));
+    launch_wait();
     if (warp == 0) xsweep_chain<1>(gd, item.block, lane, stage, bars[0], ex[0], ex[1]);
     else if (warp == 1) xsweep_chain<-1>(gd, item.block, lane, stage + kStages, bars[1], ex[1], ex[0]);
     else if (lane == 0) {
@@ -713,6 +718,7 @@ __global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev*
     const GridDev gd = grids[item.grid];
     const CUtensorMap* map = maps + 2 * item.grid + 1;
     auto* stage = reinterpret_cast<double(*)[kChunk][BLK]>(ring_base<128>(sweep_smem));
+    launch_wait();
     auto* amp_b = amp + (CLOSE ? kStages : 2);
     auto *ex_a = reinterpret_cast<double(*)[BLK]>(amp), *ex_b = reinterpret_cast<double(*)[BLK]>(amp_b);
     if (warp == 0) ysweep_chain<1, CLOSE>(gd, item.block, lane, stage, amp, bars[0], ex_a, ex_b);
@@ -730,6 +736,7 @@ __global__ void __launch_bounds__(256, 6) ch_xclose_kernel(const GridDev* __rest
                                                         const Item* __restrict__ items) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    launch_wait();
     if (gd.general) return;
     const int n = gd.n;
     const int bpr = n / BLK;
@@ -760,6 +767,7 @@ __global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __rest
                                                         const Item* __restrict__ items, int parity) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    launch_wait();
     if (gd.general) return;   // its y sweep has updated the field
     const int n = gd.n;
     const int bpr = n / BLK;
@@ -820,6 +828,7 @@ __global__ void __launch_bounds__(BLK) ch_xsolve_general_kernel(const GridDev* _
     {
         const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
+        launch_wait();
         const int n = gd.n, m = n - 2;
         const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
@@ -948,6 +957,7 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_general_kernel(const GridDev* _
     {
         const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
+        launch_wait();
         const int n = gd.n, m = n - 2;
         const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
@@ -1099,6 +1109,7 @@ __global__ void __launch_bounds__(256) ch_xcorr_general_kernel(const GridDev* __
                                                        const Item* __restrict__ items) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    launch_wait();
     if (!gd.general) return;
     const int n = gd.n, m = n - 2;
     const int bpr = n / BLK;
@@ -1120,6 +1131,7 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
                                                         const Item* __restrict__ items, int parity) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
+    launch_wait();
     if (!gd.general) return;
     const int n = gd.n, m = n - 2;
     const int bpr = n / BLK;
@@ -1148,6 +1160,7 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_split_general_kernel(const Grid
     {
         const Item item = items[blockIdx.x];
         const GridDev gd = grids[item.grid];
+        launch_wait();
         const int n = gd.n, m = n - 2;
         const double* tab = gd.tab + kTabParams;
         const double* ds = tab;
@@ -1294,8 +1307,7 @@ static cudaError_t launch_rhs2_pipe(int grid, const GridDev* g, const Item* it, 
         if (e != cudaSuccess) return e;
         ready[dev].store(1, std::memory_order_release);
     }
-    ch_rhs2_pipe_kernel<NW><<<grid, NW * BLK, kRhs2PipeBytes, s>>>(g, it, n, parity);
-    return cudaGetLastError();
+    return launch_overlapped(ch_rhs2_pipe_kernel<NW>, grid, dim3(NW * BLK), kRhs2PipeBytes, s, g, it, n, parity);
 }
 
 template <typename T, int NW>
@@ -1303,16 +1315,13 @@ static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, in
     // persistent grids over the work list
     const int n = w.n_blocks, grid = std::max(1, std::min(n, sms * 32 / NW));
     if (!c.rhs_split) {
-        ch_rhs_kernel<T, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
-        return cudaGetLastError();
+        return launch_overlapped(ch_rhs_kernel<T, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
     }
-    ch_h_kernel<T, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(ch_h_kernel<T, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
     if (e != cudaSuccess) return e;
     if (c.rhs_split == 2)   // four CTAs per SM fit the double buffer
         return launch_rhs2_pipe<NW>(std::max(1, std::min(n, sms * 4)), w.grids, w.blocks, n, parity, s);
-    ch_rhs2_kernel<double, NW><<<grid, NW * BLK, 0, s>>>(w.grids, w.blocks, n, parity);
-    return cudaGetLastError();
+    return launch_overlapped(ch_rhs2_kernel<double, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
 }
 
 template <typename T>
@@ -1329,34 +1338,30 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
     cudaError_t e = rhs_fp32 ? launch_rhs<float>(c, w, parity, sms, s) : launch_rhs<double>(c, w, parity, sms, s);
     if (e != cudaSuccess) return e;
     const int n = w.n_lines - w.n_general;
+    const dim3 sweep(kSweepThreads), line(BLK), block(256);
+    auto then = [&](auto kern, int grid, dim3 threads, size_t smem, auto... args) {
+        if (e == cudaSuccess) e = launch_overlapped(kern, grid, threads, smem, s, args...);
+    };
     if (n > 0) {   // one CTA (two chains) per 32 lines, largest grids first
-        ch_xsweep_kernel<<<n, kSweepThreads, kXSweepBytes, s>>>(w.grids, w.lines, w.maps);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        then(ch_xsweep_kernel, n, sweep, kXSweepBytes, w.grids, w.lines, w.maps);
         if (close_apart(c, w, sms)) {
-            ch_xclose_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_ysweep_kernel<false><<<n, kSweepThreads, kYSweepBytes, s>>>(w.grids, w.lines, w.maps);
+            then(ch_xclose_kernel, w.n_blocks, block, 0, w.grids, w.blocks);
+            then(ch_ysweep_kernel<false>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps);
         } else {
-            ch_ysweep_kernel<true><<<n, kSweepThreads, kYSweepBytes, s>>>(w.grids, w.lines, w.maps);
+            then(ch_ysweep_kernel<true>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps);
         }
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        ch_update_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks, parity);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        then(ch_update_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
     }
     if (w.n_general > 0) {
         const Item* lines = w.lines + n;
-        ch_xsolve_general_kernel<16><<<w.n_general, BLK, 0, s>>>(w.grids, lines);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        then(ch_xsolve_general_kernel<16>, w.n_general, line, 0, w.grids, lines);
         if (few_chains(w.n_general, sms)) {
-            ch_xcorr_general_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_ysolve_split_general_kernel<8><<<w.n_general, BLK, 0, s>>>(w.grids, lines);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            ch_update_general_kernel<<<w.n_blocks, 256, 0, s>>>(w.grids, w.blocks, parity);
+            then(ch_xcorr_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks);
+            then(ch_ysolve_split_general_kernel<8>, w.n_general, line, 0, w.grids, lines);
+            then(ch_update_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
         } else {
-            ch_ysolve_general_kernel<8><<<w.n_general, BLK, 0, s>>>(w.grids, lines, parity);
+            then(ch_ysolve_general_kernel<8>, w.n_general, line, 0, w.grids, lines, parity);
         }
-        e = cudaGetLastError();
     }
     return e;
 }
