@@ -16,12 +16,14 @@ constexpr int BLK = 32;   // rows / columns per work item; n must be a multiple 
 struct GridDev {
     double* buf[2];       // the two field buffers: cCurr = buf[parity], cOld = buf[parity ^ 1]
     double* tmp;          // n x n work field (rhs, then the line solutions)
-    double* ends;         // 8 n values: closure amplitudes of every row (4 n), then of every column (4 n); may lie
-                          // in hbuf, which the sweeps do not read
+    double* ends;         // 8 n cuts values: closure amplitudes of the rows (four per row, segment by segment), then
+                          // of the columns; may lie in hbuf, which the sweeps do not read
     double* hbuf;         // n x n h of the two-pass right-hand side (null in the allocation-free step)
     const double* tab;    // solver table for n (layout below)
     int n;
     int general;          // 1: general sweeps (banded factors) instead of the factored ones
+    int cuts;             // segments per line, 1 or 2 (line_cuts)
+    int pad;
 };
 
 // Table layout for one n, all double. First kTabParams parameters:
@@ -33,10 +35,11 @@ enum : int {
     TAB_KAPPA = 4,   // 1 / G^2: the two line operators are G P(z) P(1/z)
     TAB_REACH = 5,   // entries of f1, f2 that are not negligible (the bits of an integer)
     TAB_MID = 6,     // 2 x 4: the other chain's two values next to the middle from (own, own, other, other) ends
-    TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the chain's outer end
+    TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the outer end of the neighbouring segment
+    TAB_CLOSE2 = 18, // 2 x 2: with two segments, from those of the segment itself, once around the ring
     kTabParams = 32
 };
-// then f1[n], f2[n] (homogeneous solutions), or for a general grid (m = n - 2) the banded factors
+// then f1[n], f2[n] (homogeneous solutions, n / cuts entries used), or for a general grid (m = n - 2) the banded factors
 //   [0, m) ds  [m, 2m) dl  [2m, 3m) rd = 1/diag  [3m, 4m) du  [4m, 5m) dw   (zero-padded: ds[0] = ds[1] = dl[0]
 //   = 0, du[m-1] = 0, dw[m-2] = dw[m-1] = 0)  [5m, 6m) inv1  [6m, 7m) inv2   border columns of the cyclic
 //   correction  [7m, 7m+4) omega  [7m+4, 7m+8) a, b, d, e
@@ -45,6 +48,7 @@ __host__ __device__ inline int tab_size(int n) { return kTabParams + 7 * (n - 2)
 struct Item {
     int grid;
     int block;   // right-hand side and update: 32 x 32 block index (row-major over the grid); sweeps: row / column block
+                 // times cuts, plus the segment (segments of a block are neighbours in the list)
 };
 
 // Sum of `count` values into out->sum (zeroed before the first call; one sum at a time on a scratch).
@@ -76,7 +80,8 @@ struct ChWork {
     const Item* blocks;
     const Item* lines;
     const CUtensorMap* maps;   // two per grid (sweep_maps); not read for general grids
-    int n_blocks, n_lines, n_general;   // n_lines counts the line blocks of all grids, n_general the general ones'
+    unsigned int* arrived;     // one per line block entry, zero between sweeps
+    int n_blocks, n_lines, n_general;   // n_lines counts the line entries of all grids, n_general the general ones'
 };
 int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms);
 
@@ -85,6 +90,9 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
 
 // Whether an n x n grid takes the general sweeps (GridDev::general).
 bool line_is_general(int n, double lx, double gamma, double dt_factor, bool rhs_fp32);
+
+// Segments per line of a grid.
+int line_cuts(int n, bool general);
 
 // Tensor maps of an n x n work field for the sweeps (two); false when they cannot be encoded.
 bool sweep_maps(CUtensorMap maps[2], double* tmp, int n);

@@ -92,9 +92,10 @@ struct Server {
     std::map<std::string, TableRef> tables;
     GridDev* grids_d = nullptr;
     CUtensorMap* maps_d = nullptr;
+    unsigned int* arrived_d = nullptr;   // of the sweeps, one per line entry
     Item* items_rhs_d = nullptr;
     Item* items_rows_d = nullptr;
-    size_t cap_grids = 0, cap_maps = 0, cap_rhs = 0, cap_rows = 0;
+    size_t cap_grids = 0, cap_maps = 0, cap_arrived = 0, cap_rhs = 0, cap_rows = 0;
     int n_rhs = 0, n_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
     MassScratch* mass_d = nullptr;
     int sms = 0;
@@ -150,7 +151,7 @@ static int rebuild(Server* S) {
         const int bpr = r.n / BLK;
         for (int b = 0; b < bpr * bpr; ++b) rhs.push_back({(int)k, b});
         if (!r.g.general)
-            for (int b = 0; b < bpr; ++b) rows.push_back({(int)k, b});
+            for (int b = 0; b < bpr * r.g.cuts; ++b) rows.push_back({(int)k, b});
     }
     S->n_general = 0;
     for (size_t k = 0; k < grids.size(); ++k)
@@ -161,6 +162,8 @@ static int rebuild(Server* S) {
     if ((st = grow((void**)&S->maps_d, &S->cap_maps, maps.size(), sizeof(CUtensorMap), S->stream))) return st;
     if ((st = grow((void**)&S->items_rhs_d, &S->cap_rhs, rhs.size(), sizeof(Item), S->stream))) return st;
     if ((st = grow((void**)&S->items_rows_d, &S->cap_rows, rows.size(), sizeof(Item), S->stream))) return st;
+    if ((st = grow((void**)&S->arrived_d, &S->cap_arrived, rows.size(), sizeof(unsigned int), S->stream))) return st;
+    SRV_TRY(cudaMemsetAsync(S->arrived_d, 0, rows.size() * sizeof(unsigned int), S->stream), "Clearing the arrival counts");
     // pageable copies: the host vectors may be released as soon as the calls return
     SRV_TRY(cudaMemcpyAsync(S->grids_d, grids.data(), grids.size() * sizeof(GridDev), cudaMemcpyHostToDevice,
                             S->stream), "Uploading grid descriptors");
@@ -261,6 +264,7 @@ static int admit(Server* S, int id, double now) {
     r.g.tab = t.ptr;
     r.g.n = r.n;
     r.g.general = general;
+    r.g.cuts = line_cuts(r.n, general);
     r.mean0 = m / ((double)r.n * r.n);
     r.bytes = grid_bytes(r.n);
     S->used += (double)r.bytes;
@@ -349,7 +353,7 @@ static int drop(Server* S, int id, const std::string& why, double now) {
 
 static int enqueue_steps(Server* S, int k) {
     const ChConfig cfg = ch_config(kChBatchDefault);
-    const ChWork w{S->grids_d, S->items_rhs_d, S->items_rows_d, S->maps_d, S->n_rhs, S->n_rows, S->n_general};
+    const ChWork w{S->grids_d, S->items_rhs_d, S->items_rows_d, S->maps_d, S->arrived_d, S->n_rhs, S->n_rows, S->n_general};
     for (int s = 0; s < k; ++s) {
         SRV_TRY(launch_ch_step(cfg, S->rhs_fp32 != 0, w, S->parity, S->sms, S->stream), "Launching a step");
         S->launches += ch_launches_per_step(cfg, w, S->sms);
@@ -643,6 +647,7 @@ int custen_ch_server_destroy(void* h) {
         if (t.second.ptr) cudaFreeAsync(t.second.ptr, S->stream);
     if (S->grids_d) cudaFreeAsync(S->grids_d, S->stream);
     if (S->maps_d) cudaFreeAsync(S->maps_d, S->stream);
+    if (S->arrived_d) cudaFreeAsync(S->arrived_d, S->stream);
     if (S->items_rhs_d) cudaFreeAsync(S->items_rhs_d, S->stream);
     if (S->items_rows_d) cudaFreeAsync(S->items_rows_d, S->stream);
     cudaFreeAsync(S->mass_d, S->stream);

@@ -371,10 +371,16 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 // is half as long. The arithmetic is a function of n, lx, gamma and dt alone, so a grid's result does not depend
 // on its batch.
 //
+// Short and very long lines are cut into two segments, four chains (line_cuts): each segment is
+// solved as above, zero beyond its ends, and the closure of a segment's end sums the other segment's tail and, once
+// around the ring, its own: (1 - M^n)^-1 applied to the neighbour's end values (TAB_CLOSE) and to M^(n/2) of its own
+// (TAB_CLOSE2). A segment is a CTA; the one that finishes last forms the amplitudes of both. The closure then reaches
+// every point of most lines, up to two multiply-adds a sweep more, for chains of half the length.
+//
 // A warp's FP64 instruction holds its sub-partition's FP64 pipe for 64 cycles however few lanes it has, so with
 // fewer chains than FP64 sub-partitions (4 per SM) a step takes the chain's instruction count: n / 2 elements
 // of 4 instructions per sweep. Measured, us per step (before: banded factors, one warp per 32 lines): one grid of 256^2
-// 65 (159), 512^2 118 (298), 1024^2 249 (601), 2048^2 555 (1331); 96 grids of 64^2 .. 1024^2 1475 (1973).
+// 46 (159), 512^2 75 (298), 1024^2 242 (601), 2048^2 388 (1331); 96 grids of 64^2 .. 1024^2 1488 (1973).
 
 // Chunks of kChunk elements of a warp's 32 lines move between the work field and a shared-memory ring of kStages
 // stages by the tensor memory accelerator, one copy per chunk each way, issued by a copy warp per chain (two chain
@@ -516,30 +522,73 @@ __device__ __forceinline__ void recur(double (&w)[kChunk], double np1, double np
 // x sweep: DIR = 1 is chain A (columns upwards), -1 chain B. A stage holds 32 rows of 128 bytes in the 128-byte
 // swizzle (the 16-byte unit u of row r lies at u ^ (r & 7)), in which a lane per row reads and writes 16 bytes at a
 // time without bank conflicts.
+struct Segment {
+    int block, seg, lo, len;   // line block, segment of the line, its first element and length
+    __device__ __forceinline__ Segment(const GridDev& gd, const Item& item)
+        : block(gd.cuts == 2 ? item.block >> 1 : item.block), seg(gd.cuts == 2 ? item.block & 1 : 0),
+          lo(gd.cuts == 2 && seg ? gd.n / 2 : 0), len(gd.cuts == 2 ? gd.n / 2 : gd.n) {}
+    __device__ __forceinline__ int chunks() const { return len / 2 / kChunk; }
+};
 template <int DIR>
-__device__ __forceinline__ int chunk_origin(int n, int c) { return DIR > 0 ? c * kChunk : n - (c + 1) * kChunk; }
+__device__ __forceinline__ int chunk_origin(const Segment& sg, int c) {
+    return DIR > 0 ? sg.lo + c * kChunk : sg.lo + sg.len - (c + 1) * kChunk;
+}
+
+// The closure amplitudes of a chain's end for its 32 lines: four per line at ends[4 (seg n + line)], alpha1, alpha2
+// (from the left) by chain B, beta1, beta2 (from the right) by chain A. With one segment they follow from the
+// chain's own end values; with two, the values themselves are left there and the CTA that arrives last replaces
+// those of both segments.
+template <int DIR>
+__device__ __forceinline__ void close_segment(const GridDev& gd, const Segment& sg, double* ends, int line, int lane, double v1,
+                                              double v2, unsigned int* arrived, int* flag) {
+    const double* cl = gd.tab + TAB_CLOSE;
+    const int n = gd.n;
+    double2* mine = reinterpret_cast<double2*>(ends + 4 * (sg.seg * n + line) + (DIR > 0 ? 2 : 0));
+    if (!in_bounds(4 * (sg.seg * n + line) + 3, 0, 4 * n * gd.cuts)) return;
+    if (gd.cuts == 1) {
+        *mine = make_double2(fma(cl[0], v1, cl[1] * v2), fma(cl[2], v1, cl[3] * v2));
+        return;
+    }
+    *mine = make_double2(v1, v2);
+    __threadfence();
+    pair_barrier();
+    if (DIR > 0 && lane == 0) *flag = (int)atomicAdd(arrived, 1u);
+    pair_barrier();
+    if (*flag == 0) return;   // the other segment's CTA has yet to arrive
+    if (DIR > 0 && lane == 0) *arrived = 0;   // for the next sweep
+    __threadfence();
+    double2* theirs = reinterpret_cast<double2*>(ends + 4 * ((sg.seg ^ 1) * n + line) + (DIR > 0 ? 2 : 0));
+    const double2 o = __ldcg(theirs);
+    const double* c2 = gd.tab + TAB_CLOSE2;
+    auto amplitude = [&](double a1, double a2, double b1, double b2) {   // neighbour a, itself b
+        return make_double2(fma(cl[0], a1, fma(cl[1], a2, fma(c2[0], b1, c2[1] * b2))),
+                            fma(cl[2], a1, fma(cl[3], a2, fma(c2[2], b1, c2[3] * b2))));
+    };
+    *mine = amplitude(o.x, o.y, v1, v2);
+    *theirs = amplitude(v1, v2, o.x, o.y);
+}
 
 template <int DIR>
-__device__ __forceinline__ void xsweep_copies(const GridDev& gd, const CUtensorMap* map, int block,
+__device__ __forceinline__ void xsweep_copies(const GridDev& gd, const CUtensorMap* map, const Segment& sg,
                                               double (*stage)[BLK][kChunk], ChainBars& bars) {
-    const int n = gd.n;
+    const int n = gd.n, block = sg.block;
     auto load = [&](int c, int st, auto) {
         mbar_arrive_expect_tx(&bars.full[st], BLK * kChunk * sizeof(double));
-        tma_load_2d(&stage[st][0][0], map, chunk_origin<DIR>(n, c), block * BLK, &bars.full[st]);
+        tma_load_2d(&stage[st][0][0], map, chunk_origin<DIR>(sg, c), block * BLK, &bars.full[st]);
     };
     auto store = [&](int c, int st) {
-        const int x = chunk_origin<DIR>(n, c);
+        const int x = chunk_origin<DIR>(sg, c);
         if (!in_bounds(x, 0, n - kChunk + 1) || !in_bounds(block * BLK, 0, n - BLK + 1)) return;
         tma_store_2d(map, x, block * BLK, &stage[st][0][0]);
         bulk_commit();
     };
-    run_copies(n / 2 / kChunk, bars, load, store);
+    run_copies(sg.chunks(), bars, load, store);
 }
 
 template <int DIR>
-__device__ __forceinline__ void xsweep_chain(const GridDev& gd, int block, int lane, double (*stage)[BLK][kChunk],
-                                             ChainBars& bars, double (*own)[BLK], double (*other)[BLK]) {
-    const int n = gd.n;
+__device__ __forceinline__ void xsweep_chain(const GridDev& gd, const Segment& sg, int lane, double (*stage)[BLK][kChunk],
+                                             ChainBars& bars, double (*own)[BLK], double (*other)[BLK],
+                                             unsigned int* arrived, int* flag) {
     const double np1 = gd.tab[TAB_NP1], np2 = gd.tab[TAB_NP2];
     const int swz = lane & 7;
     auto solve = [&](int st, double& a1, double& a2, auto forward) {
@@ -559,13 +608,8 @@ __device__ __forceinline__ void xsweep_chain(const GridDev& gd, int block, int l
                 up ? make_double2(w[2 * k], w[2 * k + 1]) : make_double2(w[2 * k + 1], w[2 * k]);
     };
     double v1, v2;
-    run_chain(n / 2 / kChunk, bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
-    const double* cl = gd.tab + TAB_CLOSE;
-    const int y = block * BLK + lane;
-    if (in_bounds(4 * y + 3, 0, 4 * n)) {
-        gd.ends[4 * y + (DIR > 0 ? 2 : 0)] = fma(cl[0], v1, cl[1] * v2);
-        gd.ends[4 * y + (DIR > 0 ? 3 : 1)] = fma(cl[2], v1, cl[3] * v2);
-    }
+    run_chain(sg.chunks(), bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
+    close_segment<DIR>(gd, sg, gd.ends, sg.block * BLK + lane, lane, v1, v2, arrived, flag);
 }
 
 __device__ __forceinline__ void init_ring(ChainBars (&bars)[2]) {
@@ -597,9 +641,10 @@ constexpr int kSweepThreads = 4 * BLK;   // warps: chain A, chain B, the copies 
 
 __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev* __restrict__ grids,
                                                                   const Item* __restrict__ items,
-                                                                  const CUtensorMap* maps) {
+                                                                  const CUtensorMap* maps, unsigned int* arrived) {
     extern __shared__ __align__(16) unsigned char sweep_smem[];
     __shared__ double ex[2][2][BLK];
+    __shared__ int flag;
     __shared__ __align__(8) ChainBars bars[2];
     init_ring(bars);
     const int lane = threadIdx.x & (BLK - 1), warp = threadIdx.x / BLK;
@@ -608,12 +653,14 @@ __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev*
     const CUtensorMap* map = maps + 2 * item.grid;
     auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base<1024>(sweep_smem));
     launch_wait();
-    if (warp == 0) xsweep_chain<1>(gd, item.block, lane, stage, bars[0], ex[0], ex[1]);
-    else if (warp == 1) xsweep_chain<-1>(gd, item.block, lane, stage + kStages, bars[1], ex[1], ex[0]);
+    const Segment sg(gd, item);
+    arrived += blockIdx.x - sg.seg;   // of the line block
+    if (warp == 0) xsweep_chain<1>(gd, sg, lane, stage, bars[0], ex[0], ex[1], arrived, &flag);
+    else if (warp == 1) xsweep_chain<-1>(gd, sg, lane, stage + kStages, bars[1], ex[1], ex[0], arrived, &flag);
     else if (lane == 0) {
         acquire_map(map);
-        if (warp == 2) xsweep_copies<1>(gd, map, item.block, stage, bars[0]);
-        else xsweep_copies<-1>(gd, map, item.block, stage + kStages, bars[1]);
+        if (warp == 2) xsweep_copies<1>(gd, map, sg, stage, bars[0]);
+        else xsweep_copies<-1>(gd, map, sg, stage + kStages, bars[1]);
     }
 }
 
@@ -635,49 +682,55 @@ __device__ __forceinline__ void close_end(bool within, double (&v)[N], double f1
     }
 }
 
+// Where the 32 elements from i0 lie in their segment of a line, and whether within reach of either end.
 struct CloseEnds {
-    bool left, right;   // whether the block's columns lie within reach of either end
-    __device__ __forceinline__ CloseEnds(const GridDev& gd, int block) {
+    int seg, at, len;   // segment, position in it, its length
+    bool left, right;
+    __device__ __forceinline__ CloseEnds(const GridDev& gd, int i0) {
         const int reach = reach_of(gd);
-        left = block * BLK < reach;
-        right = (block + 1) * BLK > gd.n - reach;
+        len = gd.cuts == 2 ? gd.n / 2 : gd.n;
+        seg = i0 >= len;
+        at = i0 - seg * len;
+        left = at < reach;
+        right = at + BLK > len - reach;
     }
 };
 
 template <int DIR, bool CLOSE>
-__device__ __forceinline__ void ysweep_copies(const GridDev& gd, const CUtensorMap* map, int block,
+__device__ __forceinline__ void ysweep_copies(const GridDev& gd, const CUtensorMap* map, const Segment& sg,
                                               double (*stage)[kChunk][BLK], double (*amp)[kChunk][4], ChainBars& bars) {
-    const int n = gd.n;
-    const CloseEnds ends(gd, block);
+    const int n = gd.n, block = sg.block;
+    const CloseEnds ends(gd, block * BLK);
     auto load = [&](int c, int st, auto forward) {
-        const int y = chunk_origin<DIR>(n, c);
+        const int y = chunk_origin<DIR>(sg, c);
         const bool amps = CLOSE && decltype(forward)::value && (ends.left || ends.right);
         mbar_arrive_expect_tx(&bars.full[st], kChunk * BLK * sizeof(double) + (amps ? kChunk * 4 * sizeof(double) : 0));
         tma_load_2d(&stage[st][0][0], map, block * BLK, y, &bars.full[st]);
-        if (amps) bulk_load(&amp[st][0][0], gd.ends + 4 * y, kChunk * 4 * sizeof(double), &bars.full[st]);
+        if (amps) bulk_load(&amp[st][0][0], gd.ends + 4 * (ends.seg * n + y), kChunk * 4 * sizeof(double), &bars.full[st]);
     };
     auto store = [&](int c, int st) {
-        const int y = chunk_origin<DIR>(n, c);
+        const int y = chunk_origin<DIR>(sg, c);
         if (!in_bounds(y, 0, n - kChunk + 1) || !in_bounds(block * BLK, 0, n - BLK + 1)) return;
         tma_store_2d(map, block * BLK, y, &stage[st][0][0]);
         bulk_commit();
     };
-    run_copies(n / 2 / kChunk, bars, load, store);
+    run_copies(sg.chunks(), bars, load, store);
 }
 
 template <int DIR, bool CLOSE>
-__device__ __forceinline__ void ysweep_chain(const GridDev& gd, int block, int lane, double (*stage)[kChunk][BLK],
+__device__ __forceinline__ void ysweep_chain(const GridDev& gd, const Segment& sg, int lane, double (*stage)[kChunk][BLK],
                                              double (*amp)[kChunk][4], ChainBars& bars, double (*own)[BLK],
-                                             double (*other)[BLK]) {
-    const int n = gd.n;
+                                             double (*other)[BLK], unsigned int* arrived, int* flag) {
+    const int n = gd.n, block = sg.block;
     const double np1 = gd.tab[TAB_NP1], np2 = gd.tab[TAB_NP2];
     const int x = block * BLK + lane;
     double l1 = 0.0, l2 = 0.0, r1 = 0.0, r2 = 0.0;
-    const CloseEnds ends_of(gd, block);
-    const bool left = ends_of.left, right = ends_of.right;   // uniform over the warp
+    const CloseEnds in(gd, block * BLK);
+    const bool left = in.left, right = in.right;   // uniform over the warp
     if (CLOSE) {
         const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
-        l1 = f1[x]; l2 = f2[x]; r1 = f1[n - 1 - x]; r2 = f2[n - 1 - x];
+        const int i = in.at + lane, j = in.len - 1 - i;
+        l1 = f1[i]; l2 = f2[i]; r1 = f1[j]; r2 = f2[j];
     }
     auto solve = [&](int st, double& a1, double& a2, auto forward) {
         constexpr bool up = (DIR > 0) == decltype(forward)::value;
@@ -694,20 +747,16 @@ __device__ __forceinline__ void ysweep_chain(const GridDev& gd, int block, int l
         for (int k = 0; k < kChunk; ++k) stage[st][up ? k : kChunk - 1 - k][lane] = w[k];
     };
     double v1, v2;
-    run_chain(n / 2 / kChunk, bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
-    const double* cl = gd.tab + TAB_CLOSE;
-    double* ends = gd.ends + 4 * n;
-    if (in_bounds(4 * x + 3, 0, 4 * n)) {
-        ends[4 * x + (DIR > 0 ? 2 : 0)] = fma(cl[0], v1, cl[1] * v2);
-        ends[4 * x + (DIR > 0 ? 3 : 1)] = fma(cl[2], v1, cl[3] * v2);
-    }
+    run_chain(sg.chunks(), bars, own, other, lane, gd.tab + TAB_MID, v1, v2, solve);
+    close_segment<DIR>(gd, sg, gd.ends + 4 * n * gd.cuts, x, lane, v1, v2, arrived, flag);
 }
 
 template <bool CLOSE>
 __global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev* __restrict__ grids,
                                                                   const Item* __restrict__ items,
-                                                                  const CUtensorMap* maps) {
+                                                                  const CUtensorMap* maps, unsigned int* arrived) {
     extern __shared__ __align__(16) unsigned char sweep_smem[];
+    __shared__ int flag;
     // A chain leaves its end values for the other in its own amplitude area, which the backward pass does not use:
     // 37 KB per CTA, so six fit an SM.
     __shared__ __align__(16) double amp[CLOSE ? 2 * kStages : 4][kChunk][4];
@@ -721,12 +770,15 @@ __global__ void __launch_bounds__(kSweepThreads) ch_ysweep_kernel(const GridDev*
     launch_wait();
     auto* amp_b = amp + (CLOSE ? kStages : 2);
     auto *ex_a = reinterpret_cast<double(*)[BLK]>(amp), *ex_b = reinterpret_cast<double(*)[BLK]>(amp_b);
-    if (warp == 0) ysweep_chain<1, CLOSE>(gd, item.block, lane, stage, amp, bars[0], ex_a, ex_b);
-    else if (warp == 1) ysweep_chain<-1, CLOSE>(gd, item.block, lane, stage + kStages, amp_b, bars[1], ex_b, ex_a);
+    const Segment sg(gd, item);
+    arrived += blockIdx.x - sg.seg;
+    if (warp == 0) ysweep_chain<1, CLOSE>(gd, sg, lane, stage, amp, bars[0], ex_a, ex_b, arrived, &flag);
+    else if (warp == 1)
+        ysweep_chain<-1, CLOSE>(gd, sg, lane, stage + kStages, amp_b, bars[1], ex_b, ex_a, arrived, &flag);
     else if (lane == 0) {
         acquire_map(map);
-        if (warp == 2) ysweep_copies<1, CLOSE>(gd, map, item.block, stage, amp, bars[0]);
-        else ysweep_copies<-1, CLOSE>(gd, map, item.block, stage + kStages, amp_b, bars[1]);
+        if (warp == 2) ysweep_copies<1, CLOSE>(gd, map, sg, stage, amp, bars[0]);
+        else ysweep_copies<-1, CLOSE>(gd, map, sg, stage + kStages, amp_b, bars[1]);
     }
 }
 
@@ -741,17 +793,17 @@ __global__ void __launch_bounds__(256, 6) ch_xclose_kernel(const GridDev* __rest
     const int n = gd.n;
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-    const int reach = reach_of(gd);
-    const bool left = x0 < reach, right = x0 + BLK > n - reach;
+    const CloseEnds in(gd, x0);
+    const bool left = in.left, right = in.right;
     if (!left && !right) return;
-    const int x = x0 + (threadIdx.x & (BLK - 1));
+    const int lane = threadIdx.x & (BLK - 1), x = x0 + lane, i = in.at + lane, j = in.len - 1 - i;
     const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
-    const double l1 = f1[x], l2 = f2[x], r1 = f1[n - 1 - x], r2 = f2[n - 1 - x];
+    const double l1 = f1[i], l2 = f2[i], r1 = f1[j], r2 = f2[j];
     const int r0 = threadIdx.x / BLK;
     double v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = gd.tmp[(size_t)(y0 + r0 + 8 * k) * n + x];
-    auto e = [&](int k) { return reinterpret_cast<const double2*>(gd.ends + 4 * (y0 + r0 + 8 * k)); };
+    auto e = [&](int k) { return reinterpret_cast<const double2*>(gd.ends + 4 * (in.seg * n + y0 + r0 + 8 * k)); };
     close_end(left, v, l1, l2, [&](int k) { return e(k)[0]; });
     close_end(right, v, r1, r2, [&](int k) { return e(k)[1]; });
 #pragma unroll
@@ -773,9 +825,8 @@ __global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __rest
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     const int x = x0 + (threadIdx.x & (BLK - 1));
-    const int reach = reach_of(gd);
+    const CloseEnds in(gd, y0);
     const double *f1 = gd.tab + kTabParams, *f2 = f1 + n;
-    const bool top = y0 < reach, bottom = y0 + BLK > n - reach;
     const double two = ((const volatile double*)g_rhs_factors)[0];
     const double kappa = gd.tab[TAB_KAPPA];
     const double* cur = parity ? gd.buf[1] : gd.buf[0];
@@ -789,17 +840,17 @@ __global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __rest
         cv[k] = cur[q];
         ov[k] = old[q];
     }
-    const double2* e = reinterpret_cast<const double2*>(gd.ends + 4 * n + 4 * x);
-    if (top) {
+    const double2* e = reinterpret_cast<const double2*>(gd.ends + 4 * n * gd.cuts + 4 * (in.seg * n + x));
+    if (in.left) {
         const double2 a = e[0];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = fma(f1[y0 + r0 + 8 * k], a.x, fma(f2[y0 + r0 + 8 * k], a.y, v[k]));
+        for (int k = 0; k < 4; ++k) v[k] = fma(f1[in.at + r0 + 8 * k], a.x, fma(f2[in.at + r0 + 8 * k], a.y, v[k]));
     }
-    if (bottom) {
+    if (in.right) {
         const double2 a = e[1];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int i = n - 1 - (y0 + r0 + 8 * k);
+            const int i = in.len - 1 - (in.at + r0 + 8 * k);
             v[k] = fma(f1[i], a.x, fma(f2[i], a.y, v[k]));
         }
     }
@@ -1343,12 +1394,12 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
         if (e == cudaSuccess) e = launch_overlapped(kern, grid, threads, smem, s, args...);
     };
     if (n > 0) {   // one CTA (two chains) per 32 lines, largest grids first
-        then(ch_xsweep_kernel, n, sweep, kXSweepBytes, w.grids, w.lines, w.maps);
+        then(ch_xsweep_kernel, n, sweep, kXSweepBytes, w.grids, w.lines, w.maps, w.arrived);
         if (close_apart(c, w, sms)) {
             then(ch_xclose_kernel, w.n_blocks, block, 0, w.grids, w.blocks);
-            then(ch_ysweep_kernel<false>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps);
+            then(ch_ysweep_kernel<false>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps, w.arrived);
         } else {
-            then(ch_ysweep_kernel<true>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps);
+            then(ch_ysweep_kernel<true>, n, sweep, kYSweepBytes, w.grids, w.lines, w.maps, w.arrived);
         }
         then(ch_update_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
     }
@@ -1438,6 +1489,17 @@ static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
     return 2.0 * dt * D * gamma / (3.0 * (dx * dx * dx * dx));
 }
 
+// Two segments halve a chain, which is the time of a sweep when few lines are resident, and add up to two
+// multiply-adds per point and sweep where the closure's reach is long against half a line, which is the time when
+// many are. Measured (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
+// 384^2 152 / 123, 96 grids of 64^2 .. 1024^2 with those up to 512^2 cut 1466 / 1488; one grid of 1024^2 242 / 161, but the
+// 96 grids 1488 / 1570 with the 1024^2 ones cut as well; 2048^2: one grid 547 / 388, four 1092 / 1039, eight 1909 / 2054.
+// Grids of 1024^2 come in the large batches, larger ones do not, so those between the two sizes keep one segment.
+constexpr int kCutUpTo = 512, kCutAbove = 1024;
+int line_cuts(int n, bool general) {
+    return !general && n % 64 == 0 && (n <= kCutUpTo || n > kCutAbove) ? 2 : 1;
+}
+
 bool line_is_general(int n, double lx, double gamma, double dt_factor, bool rhs_fp32) {
     return rhs_fp32 || !(sigma_lin(n, lx, gamma, dt_factor) >= 0.0);
 }
@@ -1457,6 +1519,7 @@ static void line_factor(double s, double* p1, double* p2) {
 
 // The factored sweeps' part of the table: parameters and homogeneous solutions (see K2 / K3).
 static void fill_line_table(double* t, int n, double s) {
+    const int cuts = line_cuts(n, false), len = n / cuts;
     double p1d, p2d;
     line_factor(s, &p1d, &p2d);
     const long double p1 = p1d, p2 = p2d;
@@ -1489,26 +1552,32 @@ static void fill_line_table(double* t, int n, double s) {
     // f1, f2: P f = 0 from (f[-1], f[-2]) = (1, 0) and (0, 1)
     double *f1 = t + kTabParams, *f2 = f1 + n;
     long double a1 = 1.0L, a2 = 0.0L, b1 = 0.0L, b2 = 1.0L, peak = 1.0L;
+    long double h1 = 1.0L, h2 = 0.0L, g1 = 0.0L, g2 = 1.0L;   // at the end of a segment
     for (int i = 0; i < n; ++i) {
         const long double a = -p1 * a1 - p2 * a2, b = -p1 * b1 - p2 * b2;
         a2 = a1;
         a1 = a;
         b2 = b1;
         b1 = b;
+        if (i >= len) continue;
         f1[i] = (double)a;
         f2[i] = (double)b;
         peak = std::max(peak, std::max(fabsl(a), fabsl(b)));
+        h1 = a1; h2 = a2; g1 = b1; g2 = b2;
     }
-    int reach = n;
+    int reach = len;
     while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp((double)peak, -62)) --reach;
     const long long reach_bits = reach;   // as bits: a conversion on the device would take the FP64 pipe
     memcpy(&t[TAB_REACH], &reach_bits, sizeof(reach_bits));
     // (1 - M^n)^-1, M^n = [f1[n-1] f2[n-1]; f1[n-2] f2[n-2]]
     const long double c00 = 1.0L - a1, c01 = -b1, c10 = -a2, c11 = 1.0L - b2, det = c00 * c11 - c01 * c10;
-    t[TAB_CLOSE] = (double)(c11 / det);
-    t[TAB_CLOSE + 1] = (double)(-c01 / det);
-    t[TAB_CLOSE + 2] = (double)(-c10 / det);
-    t[TAB_CLOSE + 3] = (double)(c00 / det);
+    const long double inv[4] = {c11 / det, -c01 / det, -c10 / det, c00 / det};
+    const long double step[4] = {h1, g1, h2, g2};   // M^(n / cuts)
+    for (int r = 0; r < 2; ++r)
+        for (int c = 0; c < 2; ++c) {
+            t[TAB_CLOSE + 2 * r + c] = (double)inv[2 * r + c];
+            t[TAB_CLOSE2 + 2 * r + c] = (double)(inv[2 * r] * step[c] + inv[2 * r + 1] * step[2 + c]);
+        }
 }
 
 // Solver table for an n x n grid (layout in ch_internal.cuh), written into t (tab_size(n) doubles) with `work`
@@ -1622,6 +1691,7 @@ struct Batch {
     Item* items_rhs = nullptr;
     Item* items_rows = nullptr;   // K2 and K3 share the per-grid block lists (row / column blocks)
     int n_items_rhs = 0, n_items_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
+    unsigned int* arrived = nullptr;   // of the sweeps, one per line entry
     MassScratch* mass_d = nullptr;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -1634,7 +1704,7 @@ struct Batch {
 static ChConfig batch_config(const Batch* b) { return ch_config(b->cfg >= 0 ? b->cfg : kChBatchDefault); }
 
 static ChWork batch_work(const Batch* b) {
-    return ChWork{b->grids_d, b->items_rhs, b->items_rows, b->maps_d, b->n_items_rhs, b->n_items_rows, b->n_general};
+    return ChWork{b->grids_d, b->items_rhs, b->items_rows, b->maps_d, b->arrived, b->n_items_rhs, b->n_items_rows, b->n_general};
 }
 
 static thread_local std::string g_ch_err;
@@ -1683,23 +1753,24 @@ static int capture_pairs(Batch* b) {
 // that owns every device allocation through its own budgeted pool, or a latency-critical loop that
 // must never enter cudaMalloc / cudaFree (they synchronise the device). For them one step of one
 // grid runs with all of its work buffers in this file-scope array: the right-hand side / x-sweep
-// field, the closure amplitudes, the solver table, the descriptor, the work lists
-// and the tensor maps.
+// field, the closure amplitudes, the solver table, the descriptor, the work lists,
+// the tensor maps and the sweeps' arrival counts.
 // Maximum grid: kNoAllocMaxN x kNoAllocMaxN. Every GPU that loads the library holds the array
-// (about 544 KiB) until the process exits.
+// (about 560 KiB) until the process exits.
 constexpr int kNoAllocMaxN = 256;
 constexpr size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr size_t kNoAllocTmpOff = 0;
 constexpr size_t kNoAllocEndsOff = align256(kNoAllocTmpOff + sizeof(double) * kNoAllocMaxN * kNoAllocMaxN);
-constexpr size_t kNoAllocTabOff = align256(kNoAllocEndsOff + sizeof(double) * 8 * kNoAllocMaxN);
+constexpr size_t kNoAllocTabOff = align256(kNoAllocEndsOff + sizeof(double) * 16 * kNoAllocMaxN);
 constexpr int kNoAllocTabLen = kTabParams + 7 * (kNoAllocMaxN - 2) + 8;
 constexpr size_t kNoAllocGridOff = align256(kNoAllocTabOff + sizeof(double) * kNoAllocTabLen);
 constexpr int kNoAllocBlocks = (kNoAllocMaxN / BLK) * (kNoAllocMaxN / BLK);
-constexpr int kNoAllocRows = kNoAllocMaxN / BLK;
+constexpr int kNoAllocRows = 2 * kNoAllocMaxN / BLK;   // two segments per line block
 constexpr size_t kNoAllocRhsOff = align256(kNoAllocGridOff + sizeof(GridDev));
 constexpr size_t kNoAllocRowsOff = align256(kNoAllocRhsOff + sizeof(Item) * kNoAllocBlocks);
 constexpr size_t kNoAllocMapsOff = align256(kNoAllocRowsOff + sizeof(Item) * kNoAllocRows);
-constexpr size_t kNoAllocBytes = align256(kNoAllocMapsOff + 2 * sizeof(CUtensorMap));
+constexpr size_t kNoAllocArrivedOff = align256(kNoAllocMapsOff + 2 * sizeof(CUtensorMap));   // zero between calls
+constexpr size_t kNoAllocBytes = align256(kNoAllocArrivedOff + kNoAllocRows * sizeof(unsigned int));
 
 static __device__ __align__(256) unsigned char g_ch_noalloc_scratch[kNoAllocBytes];
 
@@ -1770,6 +1841,7 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
         g.tab = tab;
         g.n = ns;
         g.general = general;
+        g.cuts = line_cuts(ns, general);
         b->grids_h[s] = g;
     }
     // work lists, largest grids first
@@ -1781,7 +1853,7 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
         const int bpr = n[s] / BLK;
         for (int k = 0; k < bpr * bpr; ++k) rhs.push_back({s, k});
         if (!b->grids_h[s].general)
-            for (int k = 0; k < bpr; ++k) rows.push_back({s, k});
+            for (int k = 0; k < bpr * b->grids_h[s].cuts; ++k) rows.push_back({s, k});
     }
     for (int s : order)
         if (b->grids_h[s].general)
@@ -1795,6 +1867,8 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     if (e == cudaSuccess) e = cudaMalloc(&b->items_rows, rows.size() * sizeof(Item));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->items_rows, rows.data(), rows.size() * sizeof(Item), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&b->arrived, rows.size() * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(b->arrived, 0, rows.size() * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMalloc(&b->mass_d, sizeof(MassScratch));
     if (e == cudaSuccess) e = cudaMemset(b->mass_d, 0, sizeof(MassScratch));
     std::vector<CUtensorMap> maps(2 * (size_t)nsims);
@@ -1971,7 +2045,9 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
     const int bpr = n / BLK;
     Item rhs[kNoAllocBlocks], rows[kNoAllocRows];
     for (int k = 0; k < bpr * bpr; ++k) rhs[k] = Item{0, k};
-    for (int k = 0; k < bpr; ++k) rows[k] = Item{0, k};
+    g.cuts = line_cuts(n, g.general != 0);
+    const int n_lines = bpr * g.cuts;
+    for (int k = 0; k < n_lines; ++k) rows[k] = Item{0, k};
 
     const size_t bytes = (size_t)n * n * sizeof(double);
     // the update is written over the "old" buffer: start it from c_old
@@ -1982,7 +2058,7 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
            "Uploading the grid descriptor");
     CH_TRY(cudaMemcpyAsync(base + kNoAllocRhsOff, rhs, sizeof(Item) * bpr * bpr, cudaMemcpyHostToDevice, s),
            "Uploading the work list");
-    CH_TRY(cudaMemcpyAsync(base + kNoAllocRowsOff, rows, sizeof(Item) * bpr, cudaMemcpyHostToDevice, s),
+    CH_TRY(cudaMemcpyAsync(base + kNoAllocRowsOff, rows, sizeof(Item) * n_lines, cudaMemcpyHostToDevice, s),
            "Uploading the work list");
     const GridDev* gd = reinterpret_cast<const GridDev*>(base + kNoAllocGridOff);
     const Item* it_rhs = reinterpret_cast<const Item*>(base + kNoAllocRhsOff);
@@ -1996,7 +2072,8 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
                "Uploading the tensor maps");
     }
     const ChWork w{gd, it_rhs, it_rows, reinterpret_cast<const CUtensorMap*>(base + kNoAllocMapsOff),
-                   bpr * bpr, bpr, g.general ? bpr : 0};
+                   reinterpret_cast<unsigned int*>(base + kNoAllocArrivedOff), bpr * bpr, n_lines,
+                   g.general ? n_lines : 0};
     CH_TRY(launch_ch_step(ch_config(kChOneGrid), false, w, 0, sms, s), "Launching the step");
     return 0;
 }
@@ -2114,6 +2191,7 @@ int custen_ch_batch_destroy(void* h) {
     cudaFree(b->items_rhs);
     cudaFree(b->items_rows);
     cudaFree(b->mass_d);
+    cudaFree(b->arrived);
     if (b->own_stream) cudaStreamDestroy(b->stream);
     delete b;
     return 0;

@@ -299,7 +299,7 @@ int custen_ch_server_destroy(void* server);
 /* One Cahn-Hilliard step of one n x n grid that allocates nothing: for callers that cannot allocate
  * device memory (a plug-in inside an application that owns all device memory, or a loop that must
  * never enter cudaMalloc / cudaFree, which synchronise the device). Its work buffers live in a
- * library-owned static device array sized for n <= 256 (about 544 KiB, held by every GPU that loads
+ * library-owned static device array sized for n <= 256 (about 560 KiB, held by every GPU that loads
  * the library until exit); larger n is rejected with status 2. c_old and c_cur are the previous two
  * fields, c_new receives the next (it may be the c_old buffer, not the c_cur buffer); all three are
  * device-accessible n*n doubles. The first call on a device looks up the array's device address, so

@@ -1,5 +1,5 @@
 """The Cahn-Hilliard line solves at the sizes where their schedule changes (fewer, as many and more chunks per
-chain than ring stages) and over parameters that change the reach of the periodic closure: against a Fourier
+chain than ring stages; one and two segments per line) and over parameters that change the reach of the periodic closure: against a Fourier
 solution of the same scheme, which shares nothing with the factored sweeps (GPU)."""
 import math
 
@@ -33,7 +33,7 @@ def fourier_steps(c, steps, lx, gamma, dt_factor):
 
 
 @pytest.mark.parametrize("config", [8, 20, 21])
-@pytest.mark.parametrize("n", [64, 96, 128, 160, 192, 288, 544])
+@pytest.mark.parametrize("n", [64, 96, 128, 160, 192, 288, 512, 544, 576, 1088])
 def test_sizes(gpu, n, config):
     c0 = np.random.default_rng(n).uniform(-0.1, 0.1, (n, n))
     b = cs.CahnHilliardBatch([n])
