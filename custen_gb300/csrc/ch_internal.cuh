@@ -36,10 +36,10 @@ enum : int {
     TAB_REACH = 5,   // entries of f1, f2 that are not negligible (the bits of an integer)
     TAB_MID = 6,     // 2 x 4: the other chain's two values next to the middle from (own, own, other, other) ends
     TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the outer end of the neighbouring segment
-    TAB_CLOSE2 = 18, // 2 x 2: with two segments, from those of the segment itself, once around the ring
+    TAB_CLOSE2 = 18, // 2 x 2 for each of two segments: from those of the segment itself, once around the ring
     kTabParams = 32
 };
-// then f1[n], f2[n] (homogeneous solutions, n / cuts entries used), or for a general grid (m = n - 2) the banded factors
+// then f1[n], f2[n] (homogeneous solutions, as many entries used as the first segment has), or for a general grid (m = n - 2) the banded factors
 //   [0, m) ds  [m, 2m) dl  [2m, 3m) rd = 1/diag  [3m, 4m) du  [4m, 5m) dw   (zero-padded: ds[0] = ds[1] = dl[0]
 //   = 0, du[m-1] = 0, dw[m-2] = dw[m-1] = 0)  [5m, 6m) inv1  [6m, 7m) inv2   border columns of the cyclic
 //   correction  [7m, 7m+4) omega  [7m+4, 7m+8) a, b, d, e
@@ -82,6 +82,7 @@ struct ChWork {
     const CUtensorMap* maps;   // two per grid (sweep_maps); not read for general grids
     unsigned int* arrived;     // one per line block entry, zero between sweeps
     int n_blocks, n_lines, n_general;   // n_lines counts the line entries of all grids, n_general the general ones'
+    int n_whole;                        // entries that are whole lines (one segment)
 };
 int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms);
 
@@ -91,8 +92,9 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
 // Whether an n x n grid takes the general sweeps (GridDev::general).
 bool line_is_general(int n, double lx, double gamma, double dt_factor, bool rhs_fp32);
 
-// Segments per line of a grid.
+// Segments per line of a grid, and the length of the first: whole blocks, at least half of the line.
 int line_cuts(int n, bool general);
+__host__ __device__ inline int first_segment(int n, int cuts) { return cuts == 2 ? (n / BLK + 1) / 2 * BLK : n; }
 
 // Tensor maps of an n x n work field for the sweeps (two); false when they cannot be encoded.
 bool sweep_maps(CUtensorMap maps[2], double* tmp, int n);

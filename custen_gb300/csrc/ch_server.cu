@@ -96,7 +96,7 @@ struct Server {
     Item* items_rhs_d = nullptr;
     Item* items_rows_d = nullptr;
     size_t cap_grids = 0, cap_maps = 0, cap_arrived = 0, cap_rhs = 0, cap_rows = 0;
-    int n_rhs = 0, n_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
+    int n_rhs = 0, n_rows = 0, n_general = 0, n_whole = 0;   // as in ChWork; line entries of general grids are the last
     MassScratch* mass_d = nullptr;
     int sms = 0;
     // statistics of the last run
@@ -144,6 +144,7 @@ static int rebuild(Server* S) {
     std::vector<GridDev> grids;
     std::vector<CUtensorMap> maps;
     std::vector<Item> rhs, rows;
+    S->n_whole = 0;
     for (size_t k = 0; k < order.size(); ++k) {
         const Request& r = S->reqs[order[k]];
         grids.push_back(r.g);
@@ -151,7 +152,10 @@ static int rebuild(Server* S) {
         const int bpr = r.n / BLK;
         for (int b = 0; b < bpr * bpr; ++b) rhs.push_back({(int)k, b});
         if (!r.g.general)
-            for (int b = 0; b < bpr * r.g.cuts; ++b) rows.push_back({(int)k, b});
+            for (int b = 0; b < bpr * r.g.cuts; ++b) {
+                rows.push_back({(int)k, b});
+                S->n_whole += r.g.cuts == 1;
+            }
     }
     S->n_general = 0;
     for (size_t k = 0; k < grids.size(); ++k)
@@ -353,7 +357,7 @@ static int drop(Server* S, int id, const std::string& why, double now) {
 
 static int enqueue_steps(Server* S, int k) {
     const ChConfig cfg = ch_config(kChBatchDefault);
-    const ChWork w{S->grids_d, S->items_rhs_d, S->items_rows_d, S->maps_d, S->arrived_d, S->n_rhs, S->n_rows, S->n_general};
+    const ChWork w{S->grids_d, S->items_rhs_d, S->items_rows_d, S->maps_d, S->arrived_d, S->n_rhs, S->n_rows, S->n_general, S->n_whole};
     for (int s = 0; s < k; ++s) {
         SRV_TRY(launch_ch_step(cfg, S->rhs_fp32 != 0, w, S->parity, S->sms, S->stream), "Launching a step");
         S->launches += ch_launches_per_step(cfg, w, S->sms);

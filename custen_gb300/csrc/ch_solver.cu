@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 //
 // Short and very long lines are cut into two segments, four chains (line_cuts): each segment is
 // solved as above, zero beyond its ends, and the closure of a segment's end sums the other segment's tail and, once
-// around the ring, its own: (1 - M^n)^-1 applied to the neighbour's end values (TAB_CLOSE) and to M^(n/2) of its own
-// (TAB_CLOSE2). A segment is a CTA; the one that finishes last forms the amplitudes of both. The closure then reaches
+// around the ring, its own: (1 - M^n)^-1 applied to the neighbour's end values (TAB_CLOSE) and to its own carried
+// through the neighbour, M to its length (TAB_CLOSE2). A segment is a CTA; the one that finishes last forms the amplitudes of both. The closure then reaches
 // every point of most lines, up to two multiply-adds a sweep more, for chains of half the length.
 //
 // A warp's FP64 instruction holds its sub-partition's FP64 pipe for 64 cycles however few lanes it has, so with
@@ -526,7 +526,8 @@ struct Segment {
     int block, seg, lo, len;   // line block, segment of the line, its first element and length
     __device__ __forceinline__ Segment(const GridDev& gd, const Item& item)
         : block(gd.cuts == 2 ? item.block >> 1 : item.block), seg(gd.cuts == 2 ? item.block & 1 : 0),
-          lo(gd.cuts == 2 && seg ? gd.n / 2 : 0), len(gd.cuts == 2 ? gd.n / 2 : gd.n) {}
+          lo(seg ? first_segment(gd.n, gd.cuts) : 0),
+          len(seg ? gd.n - first_segment(gd.n, gd.cuts) : first_segment(gd.n, gd.cuts)) {}
     __device__ __forceinline__ int chunks() const { return len / 2 / kChunk; }
 };
 template <int DIR>
@@ -559,13 +560,13 @@ __device__ __forceinline__ void close_segment(const GridDev& gd, const Segment& 
     __threadfence();
     double2* theirs = reinterpret_cast<double2*>(ends + 4 * ((sg.seg ^ 1) * n + line) + (DIR > 0 ? 2 : 0));
     const double2 o = __ldcg(theirs);
-    const double* c2 = gd.tab + TAB_CLOSE2;
-    auto amplitude = [&](double a1, double a2, double b1, double b2) {   // neighbour a, itself b
+    auto amplitude = [&](int seg, double a1, double a2, double b1, double b2) {   // neighbour a, itself b
+        const double* c2 = gd.tab + TAB_CLOSE2 + 4 * seg;
         return make_double2(fma(cl[0], a1, fma(cl[1], a2, fma(c2[0], b1, c2[1] * b2))),
                             fma(cl[2], a1, fma(cl[3], a2, fma(c2[2], b1, c2[3] * b2))));
     };
-    *mine = amplitude(o.x, o.y, v1, v2);
-    *theirs = amplitude(v1, v2, o.x, o.y);
+    *mine = amplitude(sg.seg, o.x, o.y, v1, v2);
+    *theirs = amplitude(sg.seg ^ 1, v1, v2, o.x, o.y);
 }
 
 template <int DIR>
@@ -688,9 +689,10 @@ struct CloseEnds {
     bool left, right;
     __device__ __forceinline__ CloseEnds(const GridDev& gd, int i0) {
         const int reach = reach_of(gd);
-        len = gd.cuts == 2 ? gd.n / 2 : gd.n;
-        seg = i0 >= len;
-        at = i0 - seg * len;
+        const int first = first_segment(gd.n, gd.cuts);
+        seg = i0 >= first;
+        at = seg ? i0 - first : i0;
+        len = seg ? gd.n - first : first;
         left = at < reach;
         right = at + BLK > len - reach;
     }
@@ -1318,11 +1320,14 @@ __global__ void __launch_bounds__(BLK) ch_ysolve_split_general_kernel(const Grid
     }
 }
 
-// Whether the element-wise parts of a sweep run as kernels of their own: with fewer chains than FP64 sub-partitions
-// (4 per SM) a sweep takes as long as one chain, so they are taken out of it.
+// Whether the element-wise parts of a sweep run as kernels of their own. With fewer chains than FP64 sub-partitions (4
+// per SM) a sweep takes as long as one chain, so they are taken out of it; for lines in two segments, which the
+// closure reaches everywhere, that is no slower with many chains either. Measured (us per step, x closure in the y
+// sweep / apart): 24 grids of 96^2 .. 384^2 (672 chains) 131 / 125, of 512^2 (1536) 418 / 412; 8 grids of 1024^2 (512
+// chains) 551 / 569, 24 (1536) 1448 / 1519; one of 1024^2 (64) 294 / 242.
 static bool few_chains(int chains, int sms) { return chains < 4 * sms; }
 static bool close_apart(const ChConfig& c, const ChWork& w, int sms) {
-    return c.close == 2 || (c.close == 0 && few_chains(2 * (w.n_lines - w.n_general), sms));
+    return c.close == 2 || (c.close == 0 && (w.n_whole == 0 || 2 * (w.n_lines - w.n_general) < 3 * sms));
 }
 
 int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms) {
@@ -1497,7 +1502,7 @@ static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
 // Grids of 1024^2 come in the large batches, larger ones do not, so those between the two sizes keep one segment.
 constexpr int kCutUpTo = 512, kCutAbove = 1024;
 int line_cuts(int n, bool general) {
-    return !general && n % 64 == 0 && (n <= kCutUpTo || n > kCutAbove) ? 2 : 1;
+    return !general && (n <= kCutUpTo || n > kCutAbove) ? 2 : 1;
 }
 
 bool line_is_general(int n, double lx, double gamma, double dt_factor, bool rhs_fp32) {
@@ -1519,7 +1524,7 @@ static void line_factor(double s, double* p1, double* p2) {
 
 // The factored sweeps' part of the table: parameters and homogeneous solutions (see K2 / K3).
 static void fill_line_table(double* t, int n, double s) {
-    const int cuts = line_cuts(n, false), len = n / cuts;
+    const int cuts = line_cuts(n, false), len = first_segment(n, cuts), other = n - len;   // len >= other
     double p1d, p2d;
     line_factor(s, &p1d, &p2d);
     const long double p1 = p1d, p2 = p2d;
@@ -1552,7 +1557,7 @@ static void fill_line_table(double* t, int n, double s) {
     // f1, f2: P f = 0 from (f[-1], f[-2]) = (1, 0) and (0, 1)
     double *f1 = t + kTabParams, *f2 = f1 + n;
     long double a1 = 1.0L, a2 = 0.0L, b1 = 0.0L, b2 = 1.0L, peak = 1.0L;
-    long double h1 = 1.0L, h2 = 0.0L, g1 = 0.0L, g2 = 1.0L;   // at the end of a segment
+    long double step[2][4] = {};   // per segment
     for (int i = 0; i < n; ++i) {
         const long double a = -p1 * a1 - p2 * a2, b = -p1 * b1 - p2 * b2;
         a2 = a1;
@@ -1563,7 +1568,10 @@ static void fill_line_table(double* t, int n, double s) {
         f1[i] = (double)a;
         f2[i] = (double)b;
         peak = std::max(peak, std::max(fabsl(a), fabsl(b)));
-        h1 = a1; h2 = a2; g1 = b1; g2 = b2;
+        for (int k = 0; k < 2; ++k)
+            if (i == (k ? len : other) - 1) {   // M^len, M^other: the way through the other segment
+                step[k][0] = a1; step[k][1] = b1; step[k][2] = a2; step[k][3] = b2;
+            }
     }
     int reach = len;
     while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp((double)peak, -62)) --reach;
@@ -1572,11 +1580,11 @@ static void fill_line_table(double* t, int n, double s) {
     // (1 - M^n)^-1, M^n = [f1[n-1] f2[n-1]; f1[n-2] f2[n-2]]
     const long double c00 = 1.0L - a1, c01 = -b1, c10 = -a2, c11 = 1.0L - b2, det = c00 * c11 - c01 * c10;
     const long double inv[4] = {c11 / det, -c01 / det, -c10 / det, c00 / det};
-    const long double step[4] = {h1, g1, h2, g2};   // M^(n / cuts)
     for (int r = 0; r < 2; ++r)
         for (int c = 0; c < 2; ++c) {
             t[TAB_CLOSE + 2 * r + c] = (double)inv[2 * r + c];
-            t[TAB_CLOSE2 + 2 * r + c] = (double)(inv[2 * r] * step[c] + inv[2 * r + 1] * step[2 + c]);
+            for (int k = 0; k < 2; ++k)
+                t[TAB_CLOSE2 + 4 * k + 2 * r + c] = (double)(inv[2 * r] * step[k][c] + inv[2 * r + 1] * step[k][2 + c]);
         }
 }
 
@@ -1690,7 +1698,7 @@ struct Batch {
     CUtensorMap* maps_d = nullptr;   // two per grid (sweep_maps)
     Item* items_rhs = nullptr;
     Item* items_rows = nullptr;   // K2 and K3 share the per-grid block lists (row / column blocks)
-    int n_items_rhs = 0, n_items_rows = 0, n_general = 0;   // n_general: line blocks of general grids, the last
+    int n_items_rhs = 0, n_items_rows = 0, n_general = 0, n_whole = 0;   // as in ChWork; those of general grids are the last
     unsigned int* arrived = nullptr;   // of the sweeps, one per line entry
     MassScratch* mass_d = nullptr;
     cudaStream_t stream = nullptr;
@@ -1704,7 +1712,7 @@ struct Batch {
 static ChConfig batch_config(const Batch* b) { return ch_config(b->cfg >= 0 ? b->cfg : kChBatchDefault); }
 
 static ChWork batch_work(const Batch* b) {
-    return ChWork{b->grids_d, b->items_rhs, b->items_rows, b->maps_d, b->arrived, b->n_items_rhs, b->n_items_rows, b->n_general};
+    return ChWork{b->grids_d, b->items_rhs, b->items_rows, b->maps_d, b->arrived, b->n_items_rhs, b->n_items_rows, b->n_general, b->n_whole};
 }
 
 static thread_local std::string g_ch_err;
@@ -1853,7 +1861,10 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
         const int bpr = n[s] / BLK;
         for (int k = 0; k < bpr * bpr; ++k) rhs.push_back({s, k});
         if (!b->grids_h[s].general)
-            for (int k = 0; k < bpr * b->grids_h[s].cuts; ++k) rows.push_back({s, k});
+            for (int k = 0; k < bpr * b->grids_h[s].cuts; ++k) {
+                rows.push_back({s, k});
+                b->n_whole += b->grids_h[s].cuts == 1;
+            }
     }
     for (int s : order)
         if (b->grids_h[s].general)
@@ -2073,7 +2084,7 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
     }
     const ChWork w{gd, it_rhs, it_rows, reinterpret_cast<const CUtensorMap*>(base + kNoAllocMapsOff),
                    reinterpret_cast<unsigned int*>(base + kNoAllocArrivedOff), bpr * bpr, n_lines,
-                   g.general ? n_lines : 0};
+                   g.general ? n_lines : 0, g.cuts == 1 ? n_lines : 0};
     CH_TRY(launch_ch_step(ch_config(kChOneGrid), false, w, 0, sms, s), "Launching the step");
     return 0;
 }
