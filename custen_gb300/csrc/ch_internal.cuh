@@ -37,6 +37,8 @@ enum : int {
     TAB_MID = 6,     // 2 x 4: the other chain's two values next to the middle from (own, own, other, other) ends
     TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the outer end of the neighbouring segment
     TAB_CLOSE2 = 18, // 2 x 2 for each of two segments: from those of the segment itself, once around the ring
+    TAB_BAND_LO = 26,   // general grids: first and end chunk of 16 entries in which the factors are constant (the bits of
+    TAB_BAND_HI = 27,   // integers)
     kTabParams = 32
 };
 // then f1[n], f2[n] (homogeneous solutions, as many entries used as the first segment has), or for a general grid (m = n - 2) the banded factors
@@ -79,7 +81,7 @@ struct ChWork {
     const GridDev* grids;
     const Item* blocks;
     const Item* lines;
-    const CUtensorMap* maps;   // two per grid (sweep_maps); not read for general grids
+    const CUtensorMap* maps;   // two per grid (sweep_maps)
     unsigned int* arrived;     // one per line block entry, zero between sweeps
     int n_blocks, n_lines, n_general;   // n_lines counts the line entries of all grids, n_general the general ones'
     int n_whole;                        // entries that are whole lines (one segment)

@@ -67,7 +67,7 @@ struct Request {
     std::vector<double> result;
     size_t bytes = 0;
     GridDev g{};
-    CUtensorMap maps[2];             // of g.tmp, unless g.general
+    CUtensorMap maps[2];             // of g.tmp
     std::string table_key;
 };
 
@@ -222,7 +222,7 @@ static int admit(Server* S, int id, double now) {
     const size_t f = (size_t)r.n * r.n * sizeof(double);
     double* p[4] = {nullptr, nullptr, nullptr, nullptr};   // cCurr, cOld, tmp, h
     for (int k = 0; k < 4 && e == cudaSuccess; ++k) step(alloc(&p[k], f), "Allocating a grid");
-    if (e == cudaSuccess && !general && !sweep_maps(r.maps, p[2], r.n)) step(cudaErrorNotSupported, "Encoding tensor maps");
+    if (e == cudaSuccess && !sweep_maps(r.maps, p[2], r.n)) step(cudaErrorNotSupported, "Encoding tensor maps");
     double m = 0.0;
     if (e == cudaSuccess) {
         if (!r.c0.empty()) {

@@ -668,7 +668,8 @@ __global__ void __launch_bounds__(kSweepThreads) ch_xsweep_kernel(const GridDev*
 // y sweep: DIR = 1 is chain A (rows upwards). CLOSE: the x sweep's closure is added to the right-hand side as a
 // chunk is read, in the columns within reach of either end, by the rows' amplitudes (copied with the chunk).
 // Without it ch_xclose_kernel has added it, with the same operations.
-__device__ __forceinline__ int reach_of(const GridDev& gd) { return (int)__double_as_longlong(gd.tab[TAB_REACH]); }
+__device__ __forceinline__ int tab_int(const GridDev& gd, int k) { return (int)__double_as_longlong(gd.tab[k]); }
+__device__ __forceinline__ int reach_of(const GridDev& gd) { return tab_int(gd, TAB_REACH); }
 
 // The closure of one end over N values, or of none: branches around whole loops, since the compiler turns a
 // condition at each value into both ends' multiply-adds and selections.
@@ -869,293 +870,273 @@ __global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __rest
 //   - a negative sigma_lin (a negative gamma or time step): the symbol may vanish and has no real causal factor;
 //   - the precision variant: it rounds the fields to FP32 every step, which turns any other last bit of a solve into
 //     a difference of FP32 rounding size (2e-7 after 40 steps), so its results are tied to these operations.
-// One warp per 32 lines; table entries are held in registers, field values come through cp.async.
+// One chain per 32 lines (the whole line), with the ring and the copy warp of the factored sweeps; the table entries
+// of a chunk arrive with it, and in the part of the line where the factors have converged to the last bit they stay
+// in registers. 24 grids of 96^2 .. 384^2, FP32 stencils: 206 us per step (263 with cp.async double buffers and the
+// table entries read per chunk into registers); 96 grids of 64^2 .. 1024^2: 1378 (1571).
 // ------------------------------------------------------------------------------------------------
-// x sweep (lane = row) over XC-column chunks.
-template <int XC>
-__global__ void __launch_bounds__(BLK) ch_xsolve_general_kernel(const GridDev* __restrict__ grids,
-                                                                const Item* __restrict__ items) {
-    constexpr int RPI = BLK / XC;
-    __shared__ double blk[2][BLK][XC + 1];
-    const int lane = threadIdx.x;
-    {
-        const Item item = items[blockIdx.x];
-        const GridDev gd = grids[item.grid];
-        launch_wait();
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab + kTabParams;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        double* rows = gd.tmp + (size_t)item.block * BLK * n;
-        const int nchunk = n / XC;
-        const int lr = lane / XC, lc = lane % XC;
-        const size_t step = (size_t)RPI * n;
-        auto issue = [&](int c, int b) {
-            const double* src = rows + (size_t)lr * n + c * XC + lc;
-#pragma unroll 4
-            for (int j = 0; j < XC; ++j, src += step) cp_async8(&blk[b][j * RPI + lr][lc], src);
-            cp_async_commit();
-        };
-        auto write_back = [&](int c, int b) {
-            double* dst = rows + (size_t)lr * n + c * XC + lc;
-#pragma unroll 4
-            for (int j = 0; j < XC; ++j, dst += step)
-                if (in_bounds(dst - gd.tmp, 0, (long long)n * n)) *dst = blk[b][j * RPI + lr][lc];
-        };
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        issue(0, 0);
-        for (int c = 0; c < nchunk; ++c) {
-            const int b = c & 1, cx = c * XC;
-            double ts[XC], tl[XC], tr[XC];
+struct BandChunk {
+    double ds[kChunk], dl[kChunk], rd[kChunk], du[kChunk], dw[kChunk];
+};
+constexpr uint32_t kBandBytes = sizeof(BandChunk);
+
+// The table's arrays (ch_internal.cuh) and the chunks in which they are constant.
+struct BandTable {
+    const double* t;
+    int m, const_lo, const_hi;
+    __device__ __forceinline__ explicit BandTable(const GridDev& gd)
+        : t(gd.tab + kTabParams), m(gd.n - 2), const_lo(tab_int(gd, TAB_BAND_LO)), const_hi(tab_int(gd, TAB_BAND_HI)) {}
+    __device__ __forceinline__ void load(BandChunk& to, int c, uint64_t* bar) const {
+        bulk_load(to.ds, t + c * kChunk, kChunk * sizeof(double), bar);
+        bulk_load(to.dl, t + m + c * kChunk, kChunk * sizeof(double), bar);
+        bulk_load(to.rd, t + 2 * m + c * kChunk, kChunk * sizeof(double), bar);
+        bulk_load(to.du, t + 3 * m + c * kChunk, kChunk * sizeof(double), bar);
+        bulk_load(to.dw, t + 4 * m + c * kChunk, kChunk * sizeof(double), bar);
+    }
+};
+
+// The chain of 32 lines of n elements: get(stage, w, pass) and put(stage, w) move a chunk between its stage and
+// registers, ascending. x2, x1: the last two unknowns.
+template <class Get, class Put>
+__device__ __forceinline__ void run_band(const GridDev& gd, const BandTable& bt, ChainBars& bars, const BandChunk* band,
+                                         int lane, double& x2, double& x1, Get get, Put put) {
+    const int nchunk = gd.n / kChunk;
+    RingWait full;
+    auto solved = [&](int st) {
+        __syncwarp();   // every lane's writes
+        if (lane == 0) mbar_arrive(&bars.done[st]);
+    };
+    const double* tc = bt.t + min(bt.const_lo, nchunk - 1) * kChunk;
+    const double cs = tc[0], cl = tc[bt.m], cr = tc[2 * bt.m], cu = tc[3 * bt.m], cw = tc[4 * bt.m];
+    double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
+    for (int c = 0; c < nchunk; ++c) {   // forward elimination
+        const int st = c % kStages;
+        full(bars.full, st);
+        double w[kChunk];
+        get(st, w, Forward{});
+        if (c >= bt.const_lo && c < bt.const_hi) {
 #pragma unroll
-            for (int k = 0; k < XC; ++k) {
-                const bool in = cx + k < m;
-                ts[k] = in ? __ldg(ds + cx + k) : 0.0;
-                tl[k] = in ? __ldg(dl + cx + k) : 0.0;
-                tr[k] = in ? __ldg(rd + cx + k) : 0.0;
+            for (int k = 0; k < kChunk; ++k) {
+                double t = fma(-cs, b2, w[k]);
+                t = fma(-cl, b1, t);
+                t *= cr;
+                b2 = b1;
+                b1 = t;
+                w[k] = t;
             }
-            if (c + 1 < nchunk) {
-                issue(c + 1, b ^ 1);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncwarp();
+        } else {
+            const BandChunk& q = band[st];
+            const bool last = c == nchunk - 1;
 #pragma unroll
-            for (int k = 0; k < XC; ++k) {
-                const int i = cx + k;
-                const double x = blk[b][lane][k];
-                if (i < m) {
-                    double t = fma(-ts[k], b2, x);
-                    t = fma(-tl[k], b1, t);
-                    t *= tr[k];
-                    b2 = b1;
-                    b1 = t;
-                    blk[b][lane][k] = t;
-                } else if (i == m) {
-                    r2 = x;
-                } else {
-                    r1 = x;
-                }
+            for (int k = 0; k < kChunk; ++k) {
+                if (k >= kChunk - 2 && last) break;   // the two unknowns outside the band
+                double t = fma(-q.ds[k], b2, w[k]);
+                t = fma(-q.dl[k], b1, t);
+                t *= q.rd[k];
+                b2 = b1;
+                b1 = t;
+                w[k] = t;
             }
-            __syncwarp();
-            write_back(c, b);
-            __syncwarp();
+            if (last) {
+                r2 = w[kChunk - 2];
+                r1 = w[kChunk - 1];
+            }
         }
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        issue(nchunk - 1, 0);
-        for (int j = 0; j < nchunk; ++j) {
-            const int c = nchunk - 1 - j, b = j & 1, cx = c * XC;
-            double tu[XC], tw[XC];
+        put(st, w);
+        if (c < nchunk - kStages) solved(st);
+    }
+    double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
+    for (int c = nchunk - 1; c >= 0; --c) {   // backward substitution
+        const int st = c % kStages;
+        if (c < nchunk - kStages) full(bars.full, st);
+        double w[kChunk];
+        get(st, w, Backward{});
+        if (c >= bt.const_lo && c < bt.const_hi) {
 #pragma unroll
-            for (int k = 0; k < XC; ++k) {
-                const bool in = cx + k < m;
-                tu[k] = in ? __ldg(du + cx + k) : 0.0;
-                tw[k] = in ? __ldg(dw + cx + k) : 0.0;
+            for (int k = kChunk - 1; k >= 0; --k) {
+                double y = fma(-cu, f1, w[k]);
+                y = fma(-cw, f2, y);
+                f2 = f1;
+                f1 = y;
+                w[k] = y;
             }
-            if (c > 0) {
-                issue(c - 1, b ^ 1);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncwarp();
+        } else {
+            const BandChunk& q = band[st];
+            const bool last = c == nchunk - 1;
 #pragma unroll
-            for (int k = XC - 1; k >= 0; --k) {
-                const int i = cx + k;
-                if (i < m) {
-                    double y = fma(-tu[k], f1, blk[b][lane][k]);
-                    y = fma(-tw[k], f2, y);
-                    f2 = f1;
-                    f1 = y;
-                    blk[b][lane][k] = y;
-                    if (i == 0) y0v = y;
-                    if (i == 1) y1v = y;
-                    if (i == m - 2) ym2 = y;
-                    if (i == m - 1) ym1 = y;
-                }
+            for (int k = kChunk - 1; k >= 0; --k) {
+                if (k >= kChunk - 2 && last) continue;
+                double y = fma(-q.du[k], f1, w[k]);
+                y = fma(-q.dw[k], f2, y);
+                f2 = f1;
+                f1 = y;
+                w[k] = y;
             }
-            __syncwarp();
-            write_back(c, b);
-            __syncwarp();
+            if (last) {
+                ym2 = w[kChunk - 4];
+                ym1 = w[kChunk - 3];
+            }
         }
-        const double* om = tab + 7 * m;
-        const double a = om[4], bq = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + bq * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        double* row = rows + (size_t)lane * n;
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
+        if (c == 0) {
+            y0v = w[0];
+            y1v = w[1];
+        }
+        put(st, w);
+        solved(st);
+    }
+    // the last two unknowns through the 2 x 2 Schur complement (BatchHyper.cu:195-227)
+    const double* om = bt.t + 7 * bt.m;
+    const double a = om[4], b = om[5], d = om[6], e = om[7];
+    const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
+    const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
+    x2 = om[0] * nx2 + om[1] * nx1;
+    x1 = om[2] * nx2 + om[3] * nx1;
+    if (lane == 0) full.report();
+}
+
+constexpr int kBandThreads = 2 * BLK;   // warps: the chain, its copies
+constexpr size_t kBandRingBytes = kStages * kStageWords * sizeof(double);
+constexpr size_t kXBandBytes = kBandRingBytes + 1024, kYBandBytes = kBandRingBytes + 128;   // dynamic shared memory
+
+__device__ __forceinline__ void init_bars(ChainBars& bars) {
+    if (threadIdx.x == 0) {
+        for (int st = 0; st < kStages; ++st) {
+            mbar_init(&bars.full[st], 1);
+            mbar_init(&bars.done[st], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
+
+// x sweep (lane = row); leaves the banded solution and the two border values of every row, which the ends buffer
+// keeps as well.
+__global__ void __launch_bounds__(kBandThreads) ch_xband_kernel(const GridDev* __restrict__ grids,
+                                                                const Item* __restrict__ items, const CUtensorMap* maps) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    __shared__ __align__(16) BandChunk band[kStages];
+    __shared__ __align__(8) ChainBars bars;
+    init_bars(bars);
+    const int lane = threadIdx.x & (BLK - 1);
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    const CUtensorMap* map = maps + 2 * item.grid;
+    const BandTable bt(gd);
+    const int n = gd.n, y0 = item.block * BLK;
+    auto* stage = reinterpret_cast<double(*)[BLK][kChunk]>(ring_base<1024>(sweep_smem));
+    launch_wait();
+    if (threadIdx.x >= BLK) {
+        if (lane == 0) {
+            acquire_map(map);
+            auto load = [&](int c, int st, auto) {
+                mbar_arrive_expect_tx(&bars.full[st], BLK * kChunk * sizeof(double) + kBandBytes);
+                tma_load_2d(&stage[st][0][0], map, c * kChunk, y0, &bars.full[st]);
+                bt.load(band[st], c, &bars.full[st]);
+            };
+            auto store = [&](int c, int st) {
+                if (!in_bounds(c * kChunk, 0, n - kChunk + 1) || !in_bounds(y0, 0, n - BLK + 1)) return;
+                tma_store_2d(map, c * kChunk, y0, &stage[st][0][0]);
+                bulk_commit();
+            };
+            run_copies(n / kChunk, bars, load, store);
+            asm volatile("fence.proxy.async;" ::: "memory");   // the chain's stores below follow the copies'
+        }
+        __syncwarp();
+        pair_barrier();
+        return;
+    }
+    const int swz = lane & 7;
+    auto get = [&](int st, double (&w)[kChunk], auto) {
+        const double2* p = reinterpret_cast<const double2*>(&stage[st][lane][0]);
+#pragma unroll
+        for (int k = 0; k < kChunk / 2; ++k) {
+            const double2 q = p[k ^ swz];
+            w[2 * k] = q.x;
+            w[2 * k + 1] = q.y;
+        }
+    };
+    auto put = [&](int st, const double (&w)[kChunk]) {
+        double2* p = reinterpret_cast<double2*>(&stage[st][lane][0]);
+#pragma unroll
+        for (int k = 0; k < kChunk / 2; ++k) p[k ^ swz] = make_double2(w[2 * k], w[2 * k + 1]);
+    };
+    double x2, x1;
+    run_band(gd, bt, bars, band, lane, x2, x1, get, put);
+    pair_barrier();   // the last chunk has been copied out with the border values' right-hand sides
+    const int y = y0 + lane;
+    double* row = gd.tmp + (size_t)y * n;
+    if (in_bounds(2 * y + 1, 0, 2 * n)) {
         row[n - 2] = x2;
         row[n - 1] = x1;
-        const int gy = item.block * BLK + lane;
-        if (in_bounds(2 * gy + 1, 0, 2 * n)) {
-            gd.ends[2 * gy] = x2;
-            gd.ends[2 * gy + 1] = x1;
-        }
+        gd.ends[2 * y] = x2;
+        gd.ends[2 * y + 1] = x1;
     }
 }
 
-// y sweep (lane = column) over CH-row chunks, with the x sweep's rank-2 correction on read and the update.
-template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_general_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items, int parity) {
-    __shared__ double vb[2][CH][BLK];
-    constexpr int UD = 8;
-    const int lane = threadIdx.x;
-    const double two = ((const volatile double*)g_rhs_factors)[0];
-    {
-        const Item item = items[blockIdx.x];
-        const GridDev gd = grids[item.grid];
-        launch_wait();
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab + kTabParams;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        const double* inv1 = tab + 5 * m;
-        const double* inv2 = tab + 6 * m;
-        const int x = item.block * BLK + lane;
-        double* t = gd.tmp;
-        const double* ends = gd.ends;
-        const bool corr = x < m;
-        const double cx1 = corr ? inv1[x] : 0.0;
-        const double cx2 = corr ? inv2[x] : 0.0;
-        const int nb = n / CH;
-        auto issue = [&](int bb, int b, bool below_m) {
-            const int yb = bb * CH;
-            const double* src = t + (size_t)yb * n + x;
-#pragma unroll 4
-            for (int k = 0; k < CH; ++k, src += n)
-                if (!below_m || yb + k < m) cp_async8(&vb[b][k][lane], src);
-            cp_async_commit();
-        };
-        // forward elimination along y
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        issue(0, 0, false);
-        for (int bb = 0; bb < nb; ++bb) {
-            const int b = bb & 1, yb = bb * CH;
-            double ts[CH], tl[CH], tr[CH], te2[CH], te1[CH];
+// y sweep (lane = column); leaves the banded solution and, at ends + 2 n, the two border values of every column.
+// CLOSE: with the x sweep's rank-2 correction of the columns x < n - 2 as rows are read (BatchHyper.cu:233-259), by
+// the rows' border values, copied with the chunk; without it ch_xcorr_general_kernel has applied it.
+template <bool CLOSE>
+__global__ void __launch_bounds__(kBandThreads) ch_yband_kernel(const GridDev* __restrict__ grids,
+                                                                const Item* __restrict__ items, const CUtensorMap* maps) {
+    extern __shared__ __align__(16) unsigned char sweep_smem[];
+    __shared__ __align__(16) BandChunk band[kStages];
+    __shared__ __align__(16) double amp[CLOSE ? kStages : 1][kChunk][2];
+    __shared__ __align__(8) ChainBars bars;
+    init_bars(bars);
+    const int lane = threadIdx.x & (BLK - 1);
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    const CUtensorMap* map = maps + 2 * item.grid + 1;
+    const BandTable bt(gd);
+    const int n = gd.n, x0 = item.block * BLK, x = x0 + lane;
+    auto* stage = reinterpret_cast<double(*)[kChunk][BLK]>(ring_base<128>(sweep_smem));
+    launch_wait();
+    if (threadIdx.x >= BLK) {
+        if (lane == 0) {
+            acquire_map(map);
+            auto load = [&](int c, int st, auto forward) {
+                const uint32_t amps = CLOSE && decltype(forward)::value ? 2 * kChunk * sizeof(double) : 0;
+                mbar_arrive_expect_tx(&bars.full[st], BLK * kChunk * sizeof(double) + kBandBytes + amps);
+                tma_load_2d(&stage[st][0][0], map, x0, c * kChunk, &bars.full[st]);
+                bt.load(band[st], c, &bars.full[st]);
+                if (amps) bulk_load(&amp[st][0][0], gd.ends + 2 * c * kChunk, amps, &bars.full[st]);
+            };
+            auto store = [&](int c, int st) {
+                if (!in_bounds(c * kChunk, 0, n - kChunk + 1) || !in_bounds(x0, 0, n - BLK + 1)) return;
+                tma_store_2d(map, x0, c * kChunk, &stage[st][0][0]);
+                bulk_commit();
+            };
+            run_copies(n / kChunk, bars, load, store);
+        }
+        return;
+    }
+    const bool corr = CLOSE && x < bt.m;
+    const double cx1 = corr ? bt.t[5 * bt.m + x] : 0.0, cx2 = corr ? bt.t[6 * bt.m + x] : 0.0;
+    auto get = [&](int st, double (&w)[kChunk], auto forward) {
 #pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const bool in = yb + k < m;
-                ts[k] = in ? __ldg(ds + yb + k) : 0.0;
-                tl[k] = in ? __ldg(dl + yb + k) : 0.0;
-                tr[k] = in ? __ldg(rd + yb + k) : 0.0;
-                te2[k] = ends[2 * (yb + k)];
-                te1[k] = ends[2 * (yb + k) + 1];
-            }
-            if (bb + 1 < nb) {
-                issue(bb + 1, b ^ 1, false);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
+        for (int k = 0; k < kChunk; ++k) w[k] = stage[st][k][lane];
+        if (CLOSE && decltype(forward)::value) {
 #pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int y = yb + k;
-                const double c2 = te2[k], c1 = te1[k];
-                const double a_s = ts[k], a_l = tl[k];
-                const double a_r = tr[k];
-                const double vk = vb[b][k][lane];
-                const double val = corr ? fma(-cx1, c2, fma(-cx2, c1, vk)) : vk;
-                if (y < m) {
-                    double w = fma(-a_s, b2, val);
-                    w = fma(-a_l, b1, w);
-                    w *= a_r;
-                    b2 = b1;
-                    b1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                } else if (y == m) {
-                    r2 = val;
-                } else {
-                    r1 = val;
-                }
+            for (int k = 0; k < kChunk; ++k) {
+                const double2 e = *reinterpret_cast<const double2*>(amp[st][k]);
+                const double v = fma(-cx1, e.x, fma(-cx2, e.y, w[k]));
+                w[k] = corr ? v : w[k];
             }
         }
-        // backward substitution (rows below m only; the lane re-reads what it stored above)
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        issue(nb - 1, 0, true);
-        for (int j = 0; j < nb; ++j) {
-            const int bb = nb - 1 - j, b = j & 1, yb = bb * CH;
-            double tu[CH], tw[CH];
+    };
+    auto put = [&](int st, const double (&w)[kChunk]) {
 #pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const bool in = yb + k < m;
-                tu[k] = in ? __ldg(du + yb + k) : 0.0;
-                tw[k] = in ? __ldg(dw + yb + k) : 0.0;
-            }
-            if (bb > 0) {
-                issue(bb - 1, b ^ 1, true);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-#pragma unroll
-            for (int k = CH - 1; k >= 0; --k) {
-                const int y = yb + k;
-                const double a_u = tu[k], a_w = tw[k];
-                if (y < m) {
-                    double w = fma(-a_u, f1, vb[b][k][lane]);
-                    w = fma(-a_w, f2, w);
-                    f2 = f1;
-                    f1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                    if (y == m - 1) ym1 = w;
-                    if (y == m - 2) ym2 = w;
-                    if (y == 1) y1v = w;
-                    if (y == 0) y0v = w;
-                }
-            }
-        }
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        // cNew = cBar + delta over cOld (cuPentCahnADI.cu:58-69, 89-100)
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        double* old = parity ? gd.buf[0] : gd.buf[1];
-        for (int yb = 0; yb < n; yb += UD) {
-            double i1[UD], i2[UD];
-#pragma unroll
-            for (int k = 0; k < UD; ++k) {
-                const bool in = yb + k < m;
-                i1[k] = in ? __ldg(inv1 + yb + k) : 0.0;
-                i2[k] = in ? __ldg(inv2 + yb + k) : 0.0;
-            }
-            double v[UD], cv[UD], ov[UD];
-#pragma unroll
-            for (int k = 0; k < UD; ++k) {
-                const size_t q = (size_t)(yb + k) * n + x;
-                v[k] = (yb + k < m) ? t[q] : 0.0;
-                cv[k] = cur[q];
-                ov[k] = old[q];
-            }
-#pragma unroll
-            for (int k = 0; k < UD; ++k) {
-                const int y = yb + k;
-                const double a1 = i1[k], a2 = i2[k];
-                double dlt;
-                if (y < m) dlt = fma(-a1, x2, fma(-a2, x1, v[k]));
-                else dlt = (y == m) ? x2 : x1;
-                const double cbar = fma(two, cv[k], -ov[k]);
-                if (in_bounds((long long)y * n + x, 0, (long long)n * n)) old[(size_t)y * n + x] = cbar + dlt;
-            }
-        }
+        for (int k = 0; k < kChunk; ++k) stage[st][k][lane] = w[k];
+    };
+    double x2, x1;
+    run_band(gd, bt, bars, band, lane, x2, x1, get, put);
+    if (in_bounds(2 * n + 2 * x + 1, 0, 4 * n)) {
+        gd.ends[2 * n + 2 * x] = x2;
+        gd.ends[2 * n + 2 * x + 1] = x1;
     }
 }
 
-// The y sweep in three, for batches too small to fill the GPU with line warps: ch_xcorr_general_kernel applies the
-// x sweep's rank-2 correction to the work field, ch_ysolve_split_general_kernel runs the recurrences alone and
-// leaves each column's two cyclic unknowns in GridDev::ends, ch_update_general_kernel forms cNew = cBar + delta.
-// Same expressions, same bits.
 // One 32 x 32 block of a grid per CTA (the right-hand side's work list): t[y][x] -= inv1[x] x2(y) +
 // inv2[x] x1(y) for the columns x < n - 2 of the block's rows, as fma(-inv1, x2, fma(-inv2, x1, t)).
 __global__ void __launch_bounds__(256) ch_xcorr_general_kernel(const GridDev* __restrict__ grids,
@@ -1191,7 +1172,7 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     const int x = x0 + (threadIdx.x & (BLK - 1));
     const double two = ((const volatile double*)g_rhs_factors)[0];
-    const double x2 = gd.ends[2 * x], x1 = gd.ends[2 * x + 1];
+    const double x2 = gd.ends[2 * n + 2 * x], x1 = gd.ends[2 * n + 2 * x + 1];
     const double* cur = parity ? gd.buf[1] : gd.buf[0];
     double* old = parity ? gd.buf[0] : gd.buf[1];
     for (int r = threadIdx.x / BLK; r < BLK; r += blockDim.x / BLK) {
@@ -1202,121 +1183,6 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
         else dlt = (y == m) ? x2 : x1;
         const double cbar = fma(two, cur[q], -old[q]);
         if (in_bounds(q, 0, (long long)n * n)) old[q] = cbar + dlt;
-    }
-}
-
-template <int CH>
-__global__ void __launch_bounds__(BLK) ch_ysolve_split_general_kernel(const GridDev* __restrict__ grids,
-                                                             const Item* __restrict__ items) {
-    __shared__ double vb[2][CH][BLK];
-    const int lane = threadIdx.x;
-    {
-        const Item item = items[blockIdx.x];
-        const GridDev gd = grids[item.grid];
-        launch_wait();
-        const int n = gd.n, m = n - 2;
-        const double* tab = gd.tab + kTabParams;
-        const double* ds = tab;
-        const double* dl = tab + m;
-        const double* rd = tab + 2 * m;
-        const double* du = tab + 3 * m;
-        const double* dw = tab + 4 * m;
-        const int x = item.block * BLK + lane;
-        double* t = gd.tmp;
-        const int nb = n / CH;
-        auto issue = [&](int bb, int b, bool below_m) {
-            const int yb = bb * CH;
-            const double* src = t + (size_t)yb * n + x;
-#pragma unroll 4
-            for (int k = 0; k < CH; ++k, src += n)
-                if (!below_m || yb + k < m) cp_async8(&vb[b][k][lane], src);
-            cp_async_commit();
-        };
-        // forward elimination along y
-        double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
-        issue(0, 0, false);
-        for (int bb = 0; bb < nb; ++bb) {
-            const int b = bb & 1, yb = bb * CH;
-            double ts[CH], tl[CH], tr[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const bool in = yb + k < m;
-                ts[k] = in ? __ldg(ds + yb + k) : 0.0;
-                tl[k] = in ? __ldg(dl + yb + k) : 0.0;
-                tr[k] = in ? __ldg(rd + yb + k) : 0.0;
-            }
-            if (bb + 1 < nb) {
-                issue(bb + 1, b ^ 1, false);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const int y = yb + k;
-                const double a_s = ts[k], a_l = tl[k];
-                const double a_r = tr[k];
-                const double vk = vb[b][k][lane];
-                const double val = vk;   // corrected by ch_xcorr_general_kernel
-                if (y < m) {
-                    double w = fma(-a_s, b2, val);
-                    w = fma(-a_l, b1, w);
-                    w *= a_r;
-                    b2 = b1;
-                    b1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                } else if (y == m) {
-                    r2 = val;
-                } else {
-                    r1 = val;
-                }
-            }
-        }
-        // backward substitution (rows below m only; the lane re-reads what it stored above)
-        double f1 = 0.0, f2 = 0.0, y0v = 0.0, y1v = 0.0, ym2 = 0.0, ym1 = 0.0;
-        issue(nb - 1, 0, true);
-        for (int j = 0; j < nb; ++j) {
-            const int bb = nb - 1 - j, b = j & 1, yb = bb * CH;
-            double tu[CH], tw[CH];
-#pragma unroll
-            for (int k = 0; k < CH; ++k) {
-                const bool in = yb + k < m;
-                tu[k] = in ? __ldg(du + yb + k) : 0.0;
-                tw[k] = in ? __ldg(dw + yb + k) : 0.0;
-            }
-            if (bb > 0) {
-                issue(bb - 1, b ^ 1, true);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-#pragma unroll
-            for (int k = CH - 1; k >= 0; --k) {
-                const int y = yb + k;
-                const double a_u = tu[k], a_w = tw[k];
-                if (y < m) {
-                    double w = fma(-a_u, f1, vb[b][k][lane]);
-                    w = fma(-a_w, f2, w);
-                    f2 = f1;
-                    f1 = w;
-                    if (in_bounds((long long)y * n + x, 0, (long long)n * n)) t[(size_t)y * n + x] = w;
-                    if (y == m - 1) ym1 = w;
-                    if (y == m - 2) ym2 = w;
-                    if (y == 1) y1v = w;
-                    if (y == 0) y0v = w;
-                }
-            }
-        }
-        const double* om = tab + 7 * m;
-        const double a = om[4], b = om[5], d = om[6], e = om[7];
-        const double nx2 = r2 - (e * y0v + a * ym2 + b * ym1);
-        const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
-        const double x2 = om[0] * nx2 + om[1] * nx1;
-        const double x1 = om[2] * nx2 + om[3] * nx1;
-        // the column's two cyclic unknowns, for ch_update_general_kernel (the x sweep's row ends were consumed
-        // by ch_xcorr_general_kernel, so their buffer is free)
-        gd.ends[2 * x] = x2;
-        gd.ends[2 * x + 1] = x1;
     }
 }
 
@@ -1332,7 +1198,7 @@ static bool close_apart(const ChConfig& c, const ChWork& w, int sms) {
 
 int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms) {
     return (c.rhs_split ? 2 : 1) + (w.n_lines > w.n_general ? 3 + close_apart(c, w, sms) : 0) +
-           (w.n_general > 0 ? (few_chains(w.n_general, sms) ? 4 : 2) : 0);
+           (w.n_general > 0 ? 3 + few_chains(w.n_general, sms) : 0);
 }
 
 ChConfig ch_config(int index) {
@@ -1394,7 +1260,7 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
     cudaError_t e = rhs_fp32 ? launch_rhs<float>(c, w, parity, sms, s) : launch_rhs<double>(c, w, parity, sms, s);
     if (e != cudaSuccess) return e;
     const int n = w.n_lines - w.n_general;
-    const dim3 sweep(kSweepThreads), line(BLK), block(256);
+    const dim3 sweep(kSweepThreads), line(kBandThreads), block(256);
     auto then = [&](auto kern, int grid, dim3 threads, size_t smem, auto... args) {
         if (e == cudaSuccess) e = launch_overlapped(kern, grid, threads, smem, s, args...);
     };
@@ -1410,14 +1276,14 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
     }
     if (w.n_general > 0) {
         const Item* lines = w.lines + n;
-        then(ch_xsolve_general_kernel<16>, w.n_general, line, 0, w.grids, lines);
+        then(ch_xband_kernel, w.n_general, line, kXBandBytes, w.grids, lines, w.maps);
         if (few_chains(w.n_general, sms)) {
             then(ch_xcorr_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks);
-            then(ch_ysolve_split_general_kernel<8>, w.n_general, line, 0, w.grids, lines);
-            then(ch_update_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
+            then(ch_yband_kernel<false>, w.n_general, line, kYBandBytes, w.grids, lines, w.maps);
         } else {
-            then(ch_ysolve_general_kernel<8>, w.n_general, line, 0, w.grids, lines, parity);
+            then(ch_yband_kernel<true>, w.n_general, line, kYBandBytes, w.grids, lines, w.maps);
         }
+        then(ch_update_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
     }
     return e;
 }
@@ -1601,6 +1467,7 @@ static void fill_table(double* t, double* work, int n, double lx, double gamma, 
         fill_line_table(t, n, sl);
         return;
     }
+    double* params = t;
     t += kTabParams;
     const double a = sl, b = -4 * sl, c = 1 + 6 * sl, d = -4 * sl, e = sl;
     double *ds = work, *dl = work + m, *dg = work + 2 * m, *du = work + 3 * m, *dw = work + 4 * m;
@@ -1652,6 +1519,19 @@ static void fill_table(double* t, double* work, int n, double lx, double gamma, 
         t[5 * m + i] = inv1[i];
         t[6 * m + i] = inv2[i];
     }
+    // the chunks, short of the last, whose entries are all those of their neighbours to the last bit
+    const int nchunk = n / kChunk;
+    int lo = nchunk - 1;
+    auto same = [&](int i, int j) {
+        for (int k = 0; k < 5; ++k)
+            if (memcmp(&t[k * m + i], &t[k * m + j], sizeof(double)) != 0) return false;
+        return true;
+    };
+    for (int i = (nchunk - 1) * kChunk - 1; i >= 0 && same(i, (nchunk - 1) * kChunk - 1); --i)
+        if (i % kChunk == 0) lo = i / kChunk;
+    const long long band[2] = {lo, nchunk - 1};
+    memcpy(params + TAB_BAND_LO, &band[0], sizeof(double));
+    memcpy(params + TAB_BAND_HI, &band[1], sizeof(double));
     double* om = &t[7 * m];
     om[0] = y22 * det;
     om[1] = -y12 * det;
@@ -1884,7 +1764,7 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
     if (e == cudaSuccess) e = cudaMemset(b->mass_d, 0, sizeof(MassScratch));
     std::vector<CUtensorMap> maps(2 * (size_t)nsims);
     for (int s = 0; s < nsims && e == cudaSuccess; ++s)
-        if (!b->grids_h[s].general && !sweep_maps(&maps[2 * s], b->grids_h[s].tmp, n[s])) e = cudaErrorNotSupported;
+        if (!sweep_maps(&maps[2 * s], b->grids_h[s].tmp, n[s])) e = cudaErrorNotSupported;
     if (e == cudaSuccess) e = cudaMalloc(&b->maps_d, maps.size() * sizeof(CUtensorMap));
     if (e == cudaSuccess)
         e = cudaMemcpy(b->maps_d, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
@@ -2077,11 +1957,9 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     CUtensorMap maps[2];
-    if (!g.general) {
-        if (!sweep_maps(maps, g.tmp, n)) return ch_fail(cudaErrorNotSupported, "Encoding the tensor maps");
-        CH_TRY(cudaMemcpyAsync(base + kNoAllocMapsOff, maps, sizeof(maps), cudaMemcpyHostToDevice, s),
-               "Uploading the tensor maps");
-    }
+    if (!sweep_maps(maps, g.tmp, n)) return ch_fail(cudaErrorNotSupported, "Encoding the tensor maps");
+    CH_TRY(cudaMemcpyAsync(base + kNoAllocMapsOff, maps, sizeof(maps), cudaMemcpyHostToDevice, s),
+           "Uploading the tensor maps");
     const ChWork w{gd, it_rhs, it_rows, reinterpret_cast<const CUtensorMap*>(base + kNoAllocMapsOff),
                    reinterpret_cast<unsigned int*>(base + kNoAllocArrivedOff), bpr * bpr, n_lines,
                    g.general ? n_lines : 0, g.cuts == 1 ? n_lines : 0};

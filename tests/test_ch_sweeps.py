@@ -51,7 +51,8 @@ def test_sizes(gpu, n, config):
 # and negative values, which take the general sweeps
 @pytest.mark.parametrize("n,lx,gamma,dt_factor", [(128, 2 * np.pi, 0.0, 0.1), (128, 60.0, 0.01, 0.1),
                                                   (96, 2 * np.pi, 1e-5, 0.1), (128, 1.0, 0.01, 0.1),
-                                                  (64, 0.3, 0.01, 0.1), (128, 2 * np.pi, -1e-4, 0.05),
+                                                  (64, 0.3, 0.01, 0.1), (128, 2 * np.pi, -1e-4, 0.05), (384, 2 * np.pi, -4e-6, 0.05),
+                                                  (1056, 2 * np.pi, -1e-7, 0.1),
                                                   (64, 2 * np.pi, -0.002, 0.05)])
 def test_parameters(gpu, n, lx, gamma, dt_factor):
     c0 = np.random.default_rng(3).uniform(-0.1, 0.1, (n, n))
