@@ -187,11 +187,12 @@ int tune(const StencilArgs& a, int dtype, cudaStream_t s, int reps, std::vector<
 // in us, configurations 0 (64 x 32 points in FP64, 128 x 32 in FP32), 1 (half as wide) and 5 (32 x 16, 64 x 16):
 //   FP64  256^2 92 / 78 / 60   1024^2 209 / 194 / 192   1536^2 364 / 355 / 361   3072^2 1266 / 1258 / 1273
 //         4096^2 2144 / 2165 / 2204   8192^2 8207 / 8298 / -
-//   FP32  256^2 65 / 63 / 51   1536^2 99 / 94 / 93   2048^2 127 / 126 / 132   4096^2 316 / 319 / 366
+//   FP32  256^2 65 / 63 / 51   1536^2 83 / 81 / 74   2048^2 120 / 113 / 118   3000^2 228 / 176 / 187
+//         4096^2 314 / 306 / 359   6000^2 624 / 641 / 684
 static int default_config(const StencilArgs& a, int dtype) {
     const double points = (double)a.nx * a.rows;
     if (dtype == DT_F64) return points < 1.5e6 ? 5 : (points < 1.2e7 ? 1 : 0);
-    return points < 3e6 ? 5 : (points < 6e6 ? 1 : 0);
+    return points < 3e6 ? 5 : (points < 2e7 ? 1 : 0);
 }
 
 // The configuration for a device-resident launch: from the cache, from tuning (modes 1, 2 or force),

@@ -81,8 +81,12 @@ inline int sm_count() {
     return v;
 }
 
-// Resident threads per SM of the persistent FP32 grid (see launch_tma_mode).
-constexpr int kF32ThreadsPerSM = 768;
+// Resident threads per SM of the persistent FP32 grid. These launches are bound by HBM or L2. Beyond about 2e7 points
+// (input and output exceed L2) more resident CTAs, each keeping S windows in flight, make them slower: over the twelve
+// operators at 16384^2, 650 Gpts/s with every CTA that fits, 730 capped at 768 threads per SM, 624 at 512. Below, a
+// few more keep the SMs busier (768 / 1024 / 1536 threads, us): 1024^2 60 / 52 / 52, 2048^2 118 / 113 / 113, 4096^2
+// 318 / 306 / 306.
+inline int f32_threads_per_sm(const StencilArgs& a) { return (double)a.nx * a.rows < 2e7 ? 1024 : 768; }
 
 // CTAs of a persistent launch: those that fit, at most one per tile, under the test cap.
 inline int persistent_grid(int tiles_total, int per_sm) {
@@ -157,11 +161,8 @@ cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, (TW / VEC) * (TH / RPT), smem);
     if (e != cudaSuccess || per_sm < 1) return cudaErrorNotSupported;
-    // FP32 launches are bound by HBM, and more resident CTAs (each keeping S windows in flight) made
-    // them slower: over the twelve operators at 16384^2, 650 Gpts/s with every CTA that fits, 730
-    // capped at 768 threads per SM, 624 at 512. The FP64 launches, bound by the FP64 pipe, keep every
-    // CTA that fits (the 768 cap cost them 0.3%).
-    if (sizeof(T) == 4) per_sm = std::min(per_sm, std::max(1, kF32ThreadsPerSM / ((TW / VEC) * (TH / RPT))));
+    // The FP64 launches, bound by the FP64 pipe, keep every CTA that fits (a 768 cap cost them 0.3%).
+    if (sizeof(T) == 4) per_sm = std::min(per_sm, std::max(1, f32_threads_per_sm(a) / ((TW / VEC) * (TH / RPT))));
     const int tiles_x = (a.nx + TW - 1) / TW;
     const int tiles_total = tiles_x * ((a.rows + TH - 1) / TH);
     return launch_overlapped(kern, persistent_grid(tiles_total, per_sm), dim3(TW / VEC, TH / RPT), smem, s, maps, a,

@@ -65,7 +65,7 @@ def test_many_tiles_per_cta(gpu, variant, geom, fun):
 
 @pytest.mark.parametrize("nx,ny,dtype,config", [(1250, 1199, np.float64, 5), (1250, 1200, np.float64, 1),
                                                 (4000, 3000, np.float64, 0), (2000, 1499, np.float32, 5),
-                                                (2000, 1500, np.float32, 1), (2000, 3000, np.float32, 0)])
+                                                (2000, 1500, np.float32, 1), (5000, 4000, np.float32, 0)])
 def test_default_configuration_by_size(gpu, nx, ny, dtype, config, tmp_path):
     from custen_gb300.buffers import DeviceBuffer
     cs.set_tune_cache(tmp_path / "none.json")
