@@ -163,7 +163,7 @@ template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restrict__ grids,
                                                         const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T cb[34][35];
-    __shared__ T gg[32][33];   // sigma_nl * (c^3 - c)
+    __shared__ T cc[32][33];
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const volatile double* factors = g_rhs_factors;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
             const double ov = old[(size_t)gy * n + gx];
             const T c32 = (T)cv, o32 = (T)ov;
             cb[r][c] = fma(two, c32, -o32);
-            if (r >= 1 && r < 33 && c >= 1 && c < 33) gg[r - 1][c - 1] = scaled_cube_minus(ar, s_nl, c32);
+            if (r >= 1 && r < 33 && c >= 1 && c < 33) cc[r - 1][c - 1] = c32;
         }
         __syncthreads();
 #pragma unroll 4
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
             const int r = e / 32, c = e - r * 32;
             const T lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
             const long long q = (long long)(y0 + r) * n + x0 + c;
-            if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)fma(-s_lin, lap, gg[r][c]);
+            if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)fma(-s_lin, lap, scaled_cube_minus(ar, s_nl, cc[r][c]));
         }
         __syncthreads();
     }
@@ -818,7 +818,7 @@ __global__ void __launch_bounds__(256, 6) ch_xclose_kernel(const GridDev* __rest
 
 // K4: cNew = cBar + delta written over cOld (cuPentCahnADI.cu:58-69, 89-100), one 32 x 32 block per CTA: delta is
 // kappa times the y solution with its closure, for the rows within reach of either end.
-__global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __restrict__ grids,
+__global__ void __launch_bounds__(256, 4) ch_update_kernel(const GridDev* __restrict__ grids,
                                                         const Item* __restrict__ items, int parity) {
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
@@ -845,11 +845,14 @@ __global__ void __launch_bounds__(256, 6) ch_update_kernel(const GridDev* __rest
     }
     const double2* e = reinterpret_cast<const double2*>(gd.ends + 4 * n * gd.cuts + 4 * (in.seg * n + x));
     if (in.left) {
+        __syncwarp();   // keeps the branch: predicated-off multiply-adds take the FP64 pipe (4.9 -> 3.9 per point and 219 -> 169 us at
+        // 24 grids of 1024^2)
         const double2 a = e[0];
 #pragma unroll
         for (int k = 0; k < 4; ++k) v[k] = fma(f1[in.at + r0 + 8 * k], a.x, fma(f2[in.at + r0 + 8 * k], a.y, v[k]));
     }
     if (in.right) {
+        __syncwarp();
         const double2 a = e[1];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
