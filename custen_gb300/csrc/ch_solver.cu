@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 //   - close the ring: the periodic solution is v summed over all its translates by n. To the right of the line v
 //     decays as the homogeneous solutions of P, so the translates from the left add alpha1 f1(i) + alpha2 f2(i) with
 //     (alpha1, alpha2) = (1 - M^n)^-1 (v[n-1], v[n-2]) (TAB_CLOSE; M the one-step matrix), and the mirrored sum at
-//     the other end adds beta1 f1(n-1-i) + beta2 f2(n-1-i). f1 and f2 fall off; beyond TAB_REACH entries (2^-62 of
+//     the other end adds beta1 f1(n-1-i) + beta2 f2(n-1-i). f1 and f2 fall off; beyond TAB_REACH entries (2^-56 of
 //     their peak) they are left out.
 // The x sweep's closure is applied where the y sweep reads, the y sweep's in the update. Per point that is 8
 // multiply-adds for the recurrences and 2 for each end within reach, against 10 and 4, and a line's dependent chain
@@ -1391,6 +1391,19 @@ static void line_factor(double s, double* p1, double* p2) {
     *p2 = (double)std::norm(z);
 }
 
+// -(p1 a + p2 b) of pairs of doubles a, b (their low parts to first order): the homogeneous solutions' recurrence, whose
+// n steps in long double are software on the host of a GB300 (0.25 us each).
+struct Pair {
+    double hi, lo;
+};
+static Pair next_term(double p1, Pair a, double p2, Pair b) {
+    const double u = -p1 * a.hi, eu = std::fma(-p1, a.hi, -u) - p1 * a.lo;
+    const double v = -p2 * b.hi, ev = std::fma(-p2, b.hi, -v) - p2 * b.lo;
+    const double s = u + v, bb = s - u, es = (u - (s - bb)) + (v - bb);   // two-sum
+    const double lo = es + (eu + ev), hi = s + lo;
+    return {hi, lo - (hi - s)};
+}
+
 // The factored sweeps' part of the table: parameters and homogeneous solutions (see K2 / K3).
 static void fill_line_table(double* t, int n, double s) {
     const int cuts = line_cuts(n, false), len = first_segment(n, cuts), other = n - len;   // len >= other
@@ -1425,29 +1438,34 @@ static void fill_line_table(double* t, int n, double s) {
     }
     // f1, f2: P f = 0 from (f[-1], f[-2]) = (1, 0) and (0, 1)
     double *f1 = t + kTabParams, *f2 = f1 + n;
-    long double a1 = 1.0L, a2 = 0.0L, b1 = 0.0L, b2 = 1.0L, peak = 1.0L;
+    Pair a1{1.0, 0.0}, a2{0.0, 0.0}, b1{0.0, 0.0}, b2{1.0, 0.0};
+    double peak = 1.0;
     long double step[2][4] = {};   // per segment
+    auto power = [&](long double* to) {   // M^i from the last two terms
+        const Pair from[4] = {a1, b1, a2, b2};
+        for (int k = 0; k < 4; ++k) to[k] = (long double)from[k].hi + from[k].lo;
+    };
     for (int i = 0; i < n; ++i) {
-        const long double a = -p1 * a1 - p2 * a2, b = -p1 * b1 - p2 * b2;
+        const Pair a = next_term(p1d, a1, p2d, a2), b = next_term(p1d, b1, p2d, b2);
         a2 = a1;
         a1 = a;
         b2 = b1;
         b1 = b;
         if (i >= len) continue;
-        f1[i] = (double)a;
-        f2[i] = (double)b;
-        peak = std::max(peak, std::max(fabsl(a), fabsl(b)));
+        f1[i] = a.hi;
+        f2[i] = b.hi;
+        peak = std::max(peak, std::max(std::fabs(a.hi), std::fabs(b.hi)));
         for (int k = 0; k < 2; ++k)
-            if (i == (k ? len : other) - 1) {   // M^len, M^other: the way through the other segment
-                step[k][0] = a1; step[k][1] = b1; step[k][2] = a2; step[k][3] = b2;
-            }
+            if (i == (k ? len : other) - 1) power(step[k]);   // M^len, M^other: the way through the other segment
     }
     int reach = len;
-    while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp((double)peak, -62)) --reach;
+    while (reach > 0 && std::max(fabs(f1[reach - 1]), fabs(f2[reach - 1])) <= ldexp(peak, -56)) --reach;
     const long long reach_bits = reach;   // as bits: a conversion on the device would take the FP64 pipe
     memcpy(&t[TAB_REACH], &reach_bits, sizeof(reach_bits));
     // (1 - M^n)^-1, M^n = [f1[n-1] f2[n-1]; f1[n-2] f2[n-2]]
-    const long double c00 = 1.0L - a1, c01 = -b1, c10 = -a2, c11 = 1.0L - b2, det = c00 * c11 - c01 * c10;
+    long double mn[4];
+    power(mn);
+    const long double c00 = 1.0L - mn[0], c01 = -mn[1], c10 = -mn[2], c11 = 1.0L - mn[3], det = c00 * c11 - c01 * c10;
     const long double inv[4] = {c11 / det, -c01 / det, -c10 / det, c00 / det};
     for (int r = 0; r < 2; ++r)
         for (int c = 0; c < 2; ++c) {
