@@ -607,9 +607,9 @@ def run_gpu(args, world, rank, local):
             "bound": "fp64", "algorithmic_bytes_per_point_step": 56,
             "achieved_gbs": round(56.0 * ch_batched["fp64"]["gpt_steps_per_s"], 1), "hbm_peak_gbs": hbm_peak,
             "hbm_frac": round(56.0 * ch_batched["fp64"]["gpt_steps_per_s"] / hbm_peak, 4),
-            "fp64_ops_per_point_step": 29,
-            "fp64_frac": round(29e9 * ch_batched["fp64"]["gpt_steps_per_s"] / fp64_rate, 3),
-            "note": "FP64-pipe bound: about 29 FP64 operations per point and step (right-hand side 15.2, x sweep "
+            "fp64_ops_per_point_step": 26,
+            "fp64_frac": round(26e9 * ch_batched["fp64"]["gpt_steps_per_s"] / fp64_rate, 3),
+            "note": "FP64-pipe bound: about 26 FP64 operations per point and step (right-hand side 12.7, x sweep "
                     "4, y sweep 5.7, update 3.7) against 56 compulsory bytes"}
         del pts_b
         if rank == 0 and not args.skip_cpu:

@@ -32,13 +32,16 @@ enum : int {
     TAB_SNL = 1,     // sigma_nl, weight of the explicit Laplacian of c^3 - c
     TAB_NP1 = 2,     // -p1, -p2 of the causal factor P(z) = 1 + p1 / z + p2 / z^2 of the line operator
     TAB_NP2 = 3,
-    TAB_KAPPA = 4,   // 1 / G^2: the two line operators are G P(z) P(1/z)
+    TAB_KAPPA = 4,   // (2/3) / G^2: the two line operators are G P(z) P(1/z), the right-hand side is in units of 2/3
     TAB_REACH = 5,   // entries of f1, f2 that are not negligible (the bits of an integer)
     TAB_MID = 6,     // 2 x 4: the other chain's two values next to the middle from (own, own, other, other) ends
     TAB_CLOSE = 14,  // 2 x 2: closure amplitudes from the two values at the outer end of the neighbouring segment
     TAB_CLOSE2 = 18, // 2 x 2 for each of two segments: from those of the segment itself, once around the ring
     TAB_BAND_LO = 26,   // general grids: first and end chunk of 16 entries in which the factors are constant (the bits of
     TAB_BAND_HI = 27,   // integers)
+    TAB_RATIO = 28,  // sigma_lin / sigma_nl and 3/2 sigma_nl: the FP64 right-hand side's units (h in sigma_nl, the sum in 2/3)
+    TAB_LAP = 29,
+    TAB_OUT = 30,    // general grids: the unit of the right-hand side, 2/3 in FP64 and 1 over FP32 stencils
     kTabParams = 32
 };
 // then f1[n], f2[n] (homogeneous solutions, as many entries used as the first segment has), or for a general grid (m = n - 2) the banded factors
@@ -102,7 +105,7 @@ __host__ __device__ inline int first_segment(int n, int cuts) { return cuts == 2
 bool sweep_maps(CUtensorMap maps[2], double* tmp, int n);
 
 // Solver table of an n x n grid (tab_size(n) doubles) built on the host.
-std::vector<double> build_table(int n, double lx, double gamma, double dt_factor, bool general);
+std::vector<double> build_table(int n, double lx, double gamma, double dt_factor, bool general, bool rhs_fp32);
 
 }  // namespace ch
 }  // namespace custen

@@ -210,7 +210,7 @@ static int admit(Server* S, int id, double now) {
     };
     bool new_table = false;
     if (!t.ptr) {
-        std::vector<double> h = build_table(r.n, r.lx, S->gamma, S->dt_factor, general);
+        std::vector<double> h = build_table(r.n, r.lx, S->gamma, S->dt_factor, general, S->rhs_fp32 != 0);
         t.bytes = h.size() * sizeof(double);
         step(alloc(&t.ptr, t.bytes), "Allocating a solver table");
         if (e == cudaSuccess) {

@@ -8,7 +8,7 @@
 //   cNew = cBar + delta;  cOld <- cCurr;  cCurr <- cNew
 //
 // GB300 shape: FP64 FMAs (about 2 per clock per SM) bound this solver, not HBM, so the kernels
-// minimise FP64 operations (about 27 per point and step, against about 100 in the reference: the two
+// minimise FP64 operations (about 26 per point and step, against about 100 in the reference: the two
 // explicit stencils as two 5-point Laplacians, cBar and c^3 - c computed once per point, the line operators
 // factored with constant coefficients) and keep every SM sub-partition busy:
 //   K1 ch_rhs_kernel / ch_h_kernel + ch_rhs2_kernel -- right-hand side, 32 x 32 blocks, lane = column, all points
@@ -51,7 +51,7 @@ namespace ch {
 // (cuPentCahnADI.cu:463-467, 509-513). The biharmonic is the 5-point Laplacian applied twice, so
 //   Lin(cBar) + Nl(g) = Lap(h),   h = sigma_nl * g - sigma_lin * Lap(cBar),
 // with Lap the unit-weight 5-point Laplacian (N + S + W + E - 4 C). The kernel evaluates that form:
-// about 16 FP64 operations per point instead of 24 for the two stencils taken separately. The sums are
+// about 14 FP64 operations per point instead of 24 for the two stencils taken separately. The sums are
 // the same mathematically; their rounding differs from the reference's weight-by-weight chain at the
 // level of one rounding per term, far inside the solver's 1e-10 parity bar.
 // NW warps per CTA share one 32 x 32 work item: shared memory limits residency to a few CTAs per SM, so
@@ -74,28 +74,66 @@ struct Arith {
 template <>
 struct Arith<double> : f64::F64 {};
 
-// c^3 - c, times s; the five-point Laplacian N + S + W + E - 4 C
-template <typename T>
-__device__ __forceinline__ T scaled_cube_minus(const Arith<T>& ar, T s, T c) {
-    return ar.mul(s, fma(ar.mul(c, c), c, -c));
-}
+// The five-point Laplacian N + S + W + E - 4 C. The FP64 one adds N + E and W + S first: with d(r, c) = v(r, c) +
+// v(r + 1, c + 1) these are d of the point above and d of the point to the left, so the kernels of the two-pass form
+// add d once per point (diagonal_sums) and take two additions where the points apart take three.
 template <typename T>
 __device__ __forceinline__ T laplacian(const Arith<T>& ar, T m_four, T c, T n, T s, T w, T e) {
-    return fma(m_four, c, ar.add(ar.add(n, s), ar.add(w, e)));
+    if constexpr (std::is_same<T, double>::value) return fma(m_four, c, ar.add(ar.add(n, e), ar.add(w, s)));
+    else return fma(m_four, c, ar.add(ar.add(n, s), ar.add(w, e)));
 }
+// d over a 32 x 32 block with its halo: 1089 sums for 1024 points. The caller synchronises before and after.
+template <int NT>
+__device__ __forceinline__ void diagonal_sums(const Arith<double>& ar, const double* v, double (&d)[33][33], int tid) {
+#pragma unroll
+    for (int e = tid; e < 33 * 33; e += NT) {
+        const int r = e / 33, c = e - r * 33;
+        d[r][c] = ar.add(v[r * 35 + c], v[(r + 1) * 35 + c + 1]);
+    }
+}
+
+// h from c and Lap(cBar), in units of sigma_nl in FP64 (one operation less): c (c^2 - 1) - ratio Lap(cBar), ratio =
+// sigma_lin / sigma_nl, with a = ratio; in FP32 sigma_nl (c^3 - c) - sigma_lin Lap(cBar), with a, b = sigma_lin,
+// sigma_nl.
+template <typename T>
+struct HValue {
+    T a, b;
+    __device__ __forceinline__ explicit HValue(const double* tab) {
+        constexpr bool d = std::is_same<T, double>::value;
+        a = (T)tab[d ? TAB_RATIO : TAB_SLIN];
+        b = (T)tab[TAB_SNL];
+    }
+    __device__ __forceinline__ T operator()(const Arith<T>& ar, T c, T lap) const {
+        if constexpr (std::is_same<T, double>::value) return fma(c, fma(c, c, -ar.one), ar.mul(-a, lap));
+        else return fma(-a, lap, ar.mul(b, fma(ar.mul(c, c), c, -c)));
+    }
+};
+
+// The right-hand side (findRHS, cuPentCahnADI.cu:72-86) from Lap(h) and cCurr - cOld: over FP64 h in units of 2/3,
+// (3/2) sigma_nl Lap(h) - (cCurr - cOld), which the update takes back (TAB_KAPPA, TAB_OUT); over FP32 h as it stands.
+template <typename T>
+struct RhsValue {
+    double k;
+    __device__ __forceinline__ explicit RhsValue(const double* tab) {
+        k = std::is_same<T, double>::value ? tab[TAB_LAP] : ((const volatile double*)g_rhs_factors)[2];
+    }
+    __device__ __forceinline__ double operator()(double lap, double dco) const {
+        return std::is_same<T, double>::value ? fma(k, lap, -dco) : fma(k, dco, lap);
+    }
+};
 
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restrict__ grids,
                                                           const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T cb[36][37];        // cBar over the block and a 2-point halo
-    __shared__ T hh[34][35];        // sigma_nl * (c^3 - c), then h, over the block and a 1-point halo
+    __shared__ T hh[34][35];        // c, then h, over the block and a 1-point halo
     __shared__ double dco[32][33];  // cCurr - cOld at the block's points (FP64 in both variants)
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
-    const double m_four_d = factors[1], m_two_thirds_d = factors[2];
+    const double m_four_d = factors[1];
     const Arith<T> ar;
     const Arith<double> ar_d;
     launch_wait();
@@ -109,8 +147,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
         const double* tab = gd.tab;
         const int bpr = n / BLK;
         const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const T s_lin = (T)tab[TAB_SLIN];
-        const T s_nl = (T)tab[TAB_SNL];
+        const HValue<T> h(tab);
         // stage the 36 x 36 window (periodic wrap)
 #pragma unroll 4
         for (int e = tid; e < 36 * 36; e += NT) {
@@ -122,22 +159,23 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
             const double ov = old[(size_t)gy * n + gx];
             const T c32 = (T)cv, o32 = (T)ov;
             cb[r][c] = fma(two, c32, -o32);
-            if (r >= 1 && r < 35 && c >= 1 && c < 35) hh[r - 1][c - 1] = scaled_cube_minus(ar, s_nl, c32);
+            if (r >= 1 && r < 35 && c >= 1 && c < 35) hh[r - 1][c - 1] = c32;
             if (r >= 2 && r < 34 && c >= 2 && c < 34) dco[r - 2][c - 2] = ar_d.sub(cv, ov);
         }
         __syncthreads();
-        // h = sigma_nl * g - sigma_lin * Lap(cBar) over the 34 x 34 block + halo
+        // h over the 34 x 34 block + halo
 #pragma unroll 4
         for (int e = tid; e < 34 * 34; e += NT) {
             const int r = e / 34, c = e - r * 34;
             const T lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
-            hh[r][c] = fma(-s_lin, lap, hh[r][c]);
+            hh[r][c] = h(ar, hh[r][c], lap);
         }
         __syncthreads();
         // rhs = Lap(h) - (2/3)(cCurr - cOld)  (findRHS, cuPentCahnADI.cu:72-86); lane = column. Summed in
         // FP64 in both variants: over FP32 values of h (the precision variant) the FP64 sums are exact, so
         // the discrete Laplacian sums to zero over the periodic grid and the mass is conserved to FP64
         // rounding, as in the FP64 variant.
+        const RhsValue<T> rhs(tab);
         const int j = lane;
         double* out = gd.tmp + (size_t)y0 * n + x0 + j;
 #pragma unroll 4
@@ -145,7 +183,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
             const double lap = laplacian(ar_d, m_four_d, (double)hh[rr + 1][j + 1], (double)hh[rr][j + 1],
                                          (double)hh[rr + 2][j + 1], (double)hh[rr + 1][j], (double)hh[rr + 1][j + 2]);
             if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
-            out[(size_t)rr * n] = fma(m_two_thirds_d, dco[rr][j], lap);
+            out[(size_t)rr * n] = rhs(lap, dco[rr][j]);
         }
         __syncthreads();
     }
@@ -154,9 +192,10 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
 // ------------------------------------------------------------------------------------------------
 // K1 in two passes (batch configurations with rhs_split): h is formed once per point and kept in the
 // grid's h buffer, so that no block recomputes its neighbours' halo values of h (K1 above forms cBar
-// on a 2-point halo and h on a 1-point halo of every block: about 16.3 FP64 operations per point;
-// the two passes take about 15.1). The expressions and their order are those of K1, so the results
-// are the same bit for bit.
+// on a 2-point halo and h on a 1-point halo of every block, 15.1 FP64 operations per point; the two passes take
+// 12.7, since they also add the Laplacians' diagonal sums once per point). The values are those of K1 bit for bit.
+// With h in units of sigma_nl and the sum in units of 2/3 as well, pass 1 takes 7.4 operations and pass 2 5.25, against 9.2 and 6:
+// h 428 -> 360 us and pass 2 296 -> 249 us at 24 grids of 1024^2; 96 grids of 64^2 .. 1024^2 1423 -> 1317 us a step.
 // ------------------------------------------------------------------------------------------------
 // Pass 1: h = sigma_nl * (c^3 - c) - sigma_lin * Lap(cBar), cBar over the block and a 1-point halo.
 template <typename T, int NW>
@@ -164,6 +203,8 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
                                                         const Item* __restrict__ items, int n_items, int parity) {
     __shared__ T cb[34][35];
     __shared__ T cc[32][33];
+    constexpr bool kFp64 = std::is_same<T, double>::value;
+    __shared__ double diag[kFp64 ? 33 : 1][33];
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const volatile double* factors = g_rhs_factors;
@@ -179,8 +220,7 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
         const double* tab = gd.tab;
         const int bpr = n / BLK;
         const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const T s_lin = (T)tab[TAB_SLIN];
-        const T s_nl = (T)tab[TAB_SNL];
+        const HValue<T> h(tab);
 #pragma unroll 4
         for (int e = tid; e < 34 * 34; e += NT) {
             const int r = e / 34, c = e - r * 34;
@@ -194,12 +234,18 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
             if (r >= 1 && r < 33 && c >= 1 && c < 33) cc[r - 1][c - 1] = c32;
         }
         __syncthreads();
+        if constexpr (kFp64) {
+            diagonal_sums<NT>(ar, &cb[0][0], diag, tid);
+            __syncthreads();
+        }
 #pragma unroll 4
         for (int e = tid; e < 32 * 32; e += NT) {
             const int r = e / 32, c = e - r * 32;
-            const T lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
+            T lap;
+            if constexpr (kFp64) lap = fma(m_four, cb[r + 1][c + 1], ar.add(diag[r][c + 1], diag[r + 1][c]));
+            else lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
             const long long q = (long long)(y0 + r) * n + x0 + c;
-            if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)fma(-s_lin, lap, scaled_cube_minus(ar, s_nl, cc[r][c]));
+            if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)h(ar, cc[r][c], lap);
         }
         __syncthreads();
     }
@@ -210,14 +256,15 @@ __global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restric
 template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __restrict__ grids,
                                                            const Item* __restrict__ items, int n_items, int parity) {
-    __shared__ T hh[34][35];
-    __shared__ T dco[32][33];
+    __shared__ double hh[34][35];
+    __shared__ double dco[32][33];
+    __shared__ double diag[33][33];
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const int lane = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
-    const T m_four = (T)factors[1], m_two_thirds = (T)factors[2];
-    const Arith<T> ar;
+    const double m_four = factors[1];
+    const Arith<double> ar;
     launch_wait();
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const Item item = items[it];
@@ -233,20 +280,22 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __rest
             int gy = y0 - 1 + r, gx = x0 - 1 + c;
             gy = gy < 0 ? gy + n : (gy >= n ? gy - n : gy);
             gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
-            hh[r][c] = (T)gd.hbuf[(size_t)gy * n + gx];
+            hh[r][c] = gd.hbuf[(size_t)gy * n + gx];
             if (r >= 1 && r < 33 && c >= 1 && c < 33) {
-                const T c32 = (T)cur[(size_t)gy * n + gx], o32 = (T)old[(size_t)gy * n + gx];
-                dco[r - 1][c - 1] = ar.sub(c32, o32);
+                dco[r - 1][c - 1] = ar.sub(cur[(size_t)gy * n + gx], old[(size_t)gy * n + gx]);
             }
         }
+        __syncthreads();
+        diagonal_sums<NT>(ar, &hh[0][0], diag, tid);
+        const RhsValue<T> rhs(gd.tab);
         __syncthreads();
         const int j = lane;
         double* out = gd.tmp + (size_t)y0 * n + x0 + j;
 #pragma unroll 4
         for (int rr = warp; rr < BLK; rr += NW) {
-            const T lap = laplacian(ar, m_four, hh[rr + 1][j + 1], hh[rr][j + 1], hh[rr + 2][j + 1], hh[rr + 1][j], hh[rr + 1][j + 2]);
+            const double lap = fma(m_four, hh[rr + 1][j + 1], ar.add(diag[rr][j + 1], diag[rr + 1][j]));
             if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
-            out[(size_t)rr * n] = (double)fma(m_two_thirds, dco[rr][j], lap);
+            out[(size_t)rr * n] = rhs(lap, dco[rr][j]);
         }
         __syncthreads();
     }
@@ -261,29 +310,19 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Pass 2, pipelined (configurations with rhs_split = 2): the same expressions as ch_rhs2_kernel<double>,
-// so the same results, with the next work item's h window and cCurr / cOld blocks copied into the other
-// half of a shared-memory double buffer (cp.async) while the current item computes. ch_rhs2_kernel waits
-// on its loads (long-scoreboard stalls about 22 warps per issue at 32 grids of 512^2, FP64 pipe 68% busy);
-// here they are in flight during the previous item's arithmetic. The buffer is dynamic shared memory:
-// kRhs2PipeWords doubles per half, so four CTAs fit an SM; with 8 warps per CTA (configuration 20, the
-// batch default) a step of the 512-grid batch takes 8.54 ms against 8.72 with ch_rhs2_kernel
-// (configuration 17); with 4 warps per CTA, 16 warps per SM hide too little and it takes 8.74.
-constexpr int kRhs2H = 34 * 35, kRhs2C = 32 * 33;
-constexpr int kRhs2PipeWords = kRhs2H + 2 * kRhs2C;
-constexpr size_t kRhs2PipeBytes = 2 * kRhs2PipeWords * sizeof(double);
+// Pass 2, pipelined (configurations with rhs_split = 2): the same values, with the next work item's h window copied
+// into the other half of a shared-memory double buffer (cp.async) while the current item computes; cCurr and cOld are
+// read into registers before the wait for the window. 96 grids of 64^2 .. 1024^2: 1317 us a step,
+// with ch_rhs2_kernel 1506 .. 1569; cCurr and cOld in the double buffer as well leave no room for the diagonal sums at four
+// CTAs per SM.
+constexpr int kRhs2H = 34 * 35;
 
 template <int NW>
-__device__ __forceinline__ void rhs2_issue(double* buf, const GridDev& gd, const Item& item, int parity, int tid) {
+__device__ __forceinline__ void rhs2_issue(double* hh, const GridDev& gd, const Item& item, int tid) {
     constexpr int NT = NW * BLK;
     const int n = gd.n;
-    const double* cur = parity ? gd.buf[1] : gd.buf[0];
-    const double* old = parity ? gd.buf[0] : gd.buf[1];
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-    double* hh = buf;
-    double* cu = buf + kRhs2H;
-    double* ol = cu + kRhs2C;
     for (int e = tid; e < 34 * 34; e += NT) {
         const int r = e / 34, c = e - r * 34;
         int gy = y0 - 1 + r, gx = x0 - 1 + c;
@@ -291,55 +330,56 @@ __device__ __forceinline__ void rhs2_issue(double* buf, const GridDev& gd, const
         gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
         cp_async8(hh + r * 35 + c, gd.hbuf + (size_t)gy * n + gx);
     }
-    for (int e = tid; e < 32 * 32; e += NT) {
-        const int r = e >> 5, c = e & 31;
-        const size_t q = (size_t)(y0 + r) * n + x0 + c;
-        cp_async8(cu + r * 33 + c, cur + q);
-        cp_async8(ol + r * 33 + c, old + q);
-    }
 }
 
-template <int NW>
+template <typename T, int NW>
 __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* __restrict__ grids,
                                                                 const Item* __restrict__ items, int n_items,
                                                                 int parity) {
-    extern __shared__ __align__(16) double rhs2_smem[];
+    __shared__ double ring[2][kRhs2H];
+    __shared__ double diag[33][33];
+    constexpr int R = BLK / NW;   // rows per warp
     const int tid = threadIdx.x;
-    const int lane = tid & (BLK - 1), warp = tid / BLK;
+    const int j = tid & (BLK - 1), warp = tid / BLK;
     const volatile double* factors = g_rhs_factors;
-    const double m_four = factors[1], m_two_thirds = factors[2];
+    const double m_four = factors[1];
     const Arith<double> ar;
     launch_wait();
     int it_cur = blockIdx.x;
-    if (it_cur < n_items) rhs2_issue<NW>(rhs2_smem, grids[items[it_cur].grid], items[it_cur], parity, tid);
+    if (it_cur < n_items) rhs2_issue<NW>(ring[0], grids[items[it_cur].grid], items[it_cur], tid);
     cp_async_commit();
     for (int k = 0;; ++k) {
         if (it_cur >= n_items) break;
-        __syncthreads();   // every thread is done with the other half of the buffer
+        __syncthreads();   // every thread is done with the other half of the buffer and with diag
         const int it_next = it_cur + gridDim.x;
-        if (it_next < n_items)
-            rhs2_issue<NW>(rhs2_smem + ((k + 1) & 1) * kRhs2PipeWords, grids[items[it_next].grid], items[it_next],
-                           parity, tid);
+        if (it_next < n_items) rhs2_issue<NW>(ring[(k + 1) & 1], grids[items[it_next].grid], items[it_next], tid);
         cp_async_commit();
-        cp_async_wait<1>();   // this thread's copies of the current item have landed
-        __syncthreads();      // and every other thread's
-        const double* hh = rhs2_smem + (k & 1) * kRhs2PipeWords;
-        const double* cu = hh + kRhs2H;
-        const double* ol = cu + kRhs2C;
         const Item item = items[it_cur];
         const GridDev gd = grids[item.grid];
         const int n = gd.n;
+        const double* cur = parity ? gd.buf[1] : gd.buf[0];
+        const double* old = parity ? gd.buf[0] : gd.buf[1];
         const int bpr = n / BLK;
         const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const int j = lane;
-        double* out = gd.tmp + (size_t)y0 * n + x0 + j;
-#pragma unroll 4
-        for (int rr = warp; rr < BLK; rr += NW) {
-            const double lap = laplacian(ar, m_four, hh[(rr + 1) * 35 + j + 1], hh[rr * 35 + j + 1], hh[(rr + 2) * 35 + j + 1],
-                                         hh[(rr + 1) * 35 + j], hh[(rr + 1) * 35 + j + 2]);
-            const double dco = ar.sub(cu[rr * 33 + j], ol[rr * 33 + j]);
-            if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
-            out[(size_t)rr * n] = fma(m_two_thirds, dco, lap);
+        const size_t at = (size_t)(y0 + warp) * n + x0 + j;
+        double cv[R], ov[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            cv[r] = cur[at + (size_t)(r * NW) * n];
+            ov[r] = old[at + (size_t)(r * NW) * n];
+        }
+        const RhsValue<T> rhs(gd.tab);
+        cp_async_wait<1>();   // this thread's copies of the current item have landed
+        __syncthreads();      // and every other thread's
+        const double* hh = ring[k & 1];
+        diagonal_sums<NW * BLK>(ar, hh, diag, tid);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int rr = warp + r * NW;
+            const double lap = fma(m_four, hh[(rr + 1) * 35 + j + 1], ar.add(diag[rr][j + 1], diag[rr + 1][j]));
+            const size_t q = at + (size_t)(r * NW) * n;
+            if (in_bounds((long long)q, 0, (long long)n * n)) gd.tmp[q] = rhs(lap, ar.sub(cv[r], ov[r]));
         }
         it_cur = it_next;
     }
@@ -1174,7 +1214,7 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     const int x = x0 + (threadIdx.x & (BLK - 1));
-    const double two = ((const volatile double*)g_rhs_factors)[0];
+    const double two = ((const volatile double*)g_rhs_factors)[0], unit = gd.tab[TAB_OUT];
     const double x2 = gd.ends[2 * n + 2 * x], x1 = gd.ends[2 * n + 2 * x + 1];
     const double* cur = parity ? gd.buf[1] : gd.buf[0];
     double* old = parity ? gd.buf[0] : gd.buf[1];
@@ -1185,7 +1225,7 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
         if (y < m) dlt = fma(-gd.tab[kTabParams + 5 * m + y], x2, fma(-gd.tab[kTabParams + 6 * m + y], x1, gd.tmp[q]));
         else dlt = (y == m) ? x2 : x1;
         const double cbar = fma(two, cur[q], -old[q]);
-        if (in_bounds(q, 0, (long long)n * n)) old[q] = cbar + dlt;
+        if (in_bounds(q, 0, (long long)n * n)) old[q] = fma(unit, dlt, cbar);
     }
 }
 
@@ -1220,21 +1260,6 @@ void config_name(const ChConfig& c, char* name, size_t len) {
 // The two passes of the split right-hand side. Pass 2 runs in FP64 in both variants: the precision variant's h
 // buffer holds FP32 values, whose FP64 Laplacian is exact, so its mass is conserved to FP64 rounding (the
 // one-pass kernel does the same). Pass 2 pipelined: dynamic shared memory beyond 48 KB, allowed once per device.
-template <int NW>
-static cudaError_t launch_rhs2_pipe(int grid, const GridDev* g, const Item* it, int n, int parity, cudaStream_t s) {
-    static std::atomic<int> ready[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    if (!ready[dev].load(std::memory_order_acquire)) {
-        cudaError_t e = cudaFuncSetAttribute(ch_rhs2_pipe_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kRhs2PipeBytes);
-        if (e != cudaSuccess) return e;
-        ready[dev].store(1, std::memory_order_release);
-    }
-    return launch_overlapped(ch_rhs2_pipe_kernel<NW>, grid, dim3(NW * BLK), kRhs2PipeBytes, s, g, it, n, parity);
-}
-
 template <typename T, int NW>
 static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, int sms, cudaStream_t s) {
     // persistent grids over the work list
@@ -1242,11 +1267,18 @@ static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, in
     if (!c.rhs_split) {
         return launch_overlapped(ch_rhs_kernel<T, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
     }
-    const cudaError_t e = launch_overlapped(ch_h_kernel<T, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
+    // 48 warps per SM in FP64: three CTAs of 8 warps are resident beside the L1 the stencil's halos use, so 32 leave a
+    // third of an SM's work to a second wave (96 grids of 64^2 .. 1024^2: 1319 us a step, 32 warps 1474; a larger
+    // shared-memory carve-out, which makes all of them resident, 1327 and 1481; a CTA per block 1309 .. 1328). Over FP32
+    // values, bound by memory, 32 warps (1330; 48 warps 1382).
+    const int per_sm = std::is_same<T, double>::value ? std::min(48 / NW, 8) : 32 / NW;
+    const int split = std::max(1, std::min(n, sms * per_sm));
+    const cudaError_t e = launch_overlapped(ch_h_kernel<T, NW>, split, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
     if (e != cudaSuccess) return e;
     if (c.rhs_split == 2)   // four CTAs per SM fit the double buffer
-        return launch_rhs2_pipe<NW>(std::max(1, std::min(n, sms * 4)), w.grids, w.blocks, n, parity, s);
-    return launch_overlapped(ch_rhs2_kernel<double, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
+        return launch_overlapped(ch_rhs2_pipe_kernel<T, NW>, std::max(1, std::min(n, sms * 4)), dim3(NW * BLK), 0, s, w.grids,
+                                 w.blocks, n, parity);
+    return launch_overlapped(ch_rhs2_kernel<T, NW>, split, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
 }
 
 template <typename T>
@@ -1413,7 +1445,7 @@ static void fill_line_table(double* t, int n, double s) {
     t[TAB_NP1] = -p1d;
     t[TAB_NP2] = -p2d;
     const long double at1 = 1.0L + p1 + p2;   // P(1): G P(1)^2 = 1, the operator on constants
-    t[TAB_KAPPA] = (double)(at1 * at1 * at1 * at1);
+    t[TAB_KAPPA] = (double)(at1 * at1 * at1 * at1 * 2.0L / 3.0L);
     // the four values around the middle (X1, X2 | Y1, Y2) from the chains' ends (a1, a2 | b1, b2)
     long double m[4][8] = {{1, 0, p1, p2, 1, 0, 0, 0},
                            {p1, 1, p2, 0, 0, 1, 0, 0},
@@ -1477,13 +1509,16 @@ static void fill_line_table(double* t, int n, double s) {
 
 // Solver table for an n x n grid (layout in ch_internal.cuh), written into t (tab_size(n) doubles) with `work`
 // (7 * (n - 2) doubles) as scratch.
-static void fill_table(double* t, double* work, int n, double lx, double gamma, double dt_factor, bool general) {
+static void fill_table(double* t, double* work, int n, double lx, double gamma, double dt_factor, bool general, bool rhs_fp32) {
     const int m = n - 2;
     const double D = 1.0, dx = lx / n, dt = dt_factor * dx;
     const double sl = sigma_lin(n, lx, gamma, dt_factor);
     for (int k = 0; k < tab_size(n); ++k) t[k] = 0.0;
     t[TAB_SLIN] = sl;
     t[TAB_SNL] = (dt / 3.0) * D * (2.0 / (dx * dx));
+    t[TAB_RATIO] = t[TAB_SNL] != 0.0 ? sl / t[TAB_SNL] : 0.0;
+    t[TAB_LAP] = 1.5 * t[TAB_SNL];
+    t[TAB_OUT] = rhs_fp32 ? 1.0 : 2.0 / 3.0;
     if (!general) {
         fill_line_table(t, n, sl);
         return;
@@ -1561,9 +1596,9 @@ static void fill_table(double* t, double* work, int n, double lx, double gamma, 
     om[4] = a; om[5] = b; om[6] = d; om[7] = e;
 }
 
-std::vector<double> build_table(int n, double lx, double gamma, double dt_factor, bool general) {
+std::vector<double> build_table(int n, double lx, double gamma, double dt_factor, bool general, bool rhs_fp32) {
     std::vector<double> t(tab_size(n)), work(7 * (n - 2));
-    fill_table(t.data(), work.data(), n, lx, gamma, dt_factor, general);
+    fill_table(t.data(), work.data(), n, lx, gamma, dt_factor, general, rhs_fp32);
     return t;
 }
 
@@ -1731,7 +1766,7 @@ int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx
         for (auto& t : b->tables)
             if (t.first == key) tab = t.second;
         if (!tab) {
-            std::vector<double> h = build_table(ns, b->lx[s], gamma, dt_factor, general);
+            std::vector<double> h = build_table(ns, b->lx[s], gamma, dt_factor, general, b->rhs_fp32 != 0);
             cudaError_t e = cudaMalloc(&tab, h.size() * sizeof(double));
             if (e != cudaSuccess) return cleanup_fail(ch_fail(e, "Allocating solver table"));
             e = cudaMemcpy(tab, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice);
@@ -1947,7 +1982,7 @@ int custen_ch_step_noalloc(const double* c_old, const double* c_cur, double* c_n
     double work[7 * (kNoAllocMaxN - 2)];
     GridDev g{};
     g.general = line_is_general(n, lx, gamma, dt_factor, false);
-    fill_table(tab, work, n, lx, gamma, dt_factor, g.general != 0);
+    fill_table(tab, work, n, lx, gamma, dt_factor, g.general != 0, false);
     g.buf[0] = const_cast<double*>(c_cur);
     g.buf[1] = c_new;
     g.tmp = reinterpret_cast<double*>(base + kNoAllocTmpOff);
