@@ -65,12 +65,11 @@ struct MassScratch {
 };
 cudaError_t launch_ch_mass(const double* f, long long count, MassScratch* out, cudaStream_t s);
 
-// Kernel configuration of a step: warps per right-hand-side CTA, one or two passes of it, and where the x sweep's
+// Kernel configuration of a step: warps per right-hand-side CTA (of pass 1), one or two passes, and where the x sweep's
 // closure is applied. Every configuration computes the same values; the batch tuner times them.
 struct ChConfig {
     int rhs_warps;   // 1, 2, 4 or 8
-    int rhs_split;   // 1: the right-hand side in two passes through GridDev::hbuf (batches only); 2: the same
-                     // with pass 2 pipelined (cp.async double buffer)
+    int warps2;      // of the right-hand side in two passes, warps per CTA of pass 2; 0: one pass (no h buffer)
     int close;       // x closure: 1 as the y sweep reads, 2 in a kernel of its own, 0 by the number of chains
 };
 constexpr int kChOneGrid = 12;        // needs no h buffer (the allocation-free step)

@@ -63,8 +63,8 @@ namespace ch {
 // so the results, are the same as with literals.
 __device__ double g_rhs_factors[3] = {2.0, -4.0, -2.0 / 3.0};
 
-// Sums and products: FP64 ones as multiply-adds (fp64_offload.cuh; h kernel 459 -> 425 us and pass 2 320 -> 296 us at
-// 24 grids of 1024^2), FP32 ones as they are.
+// Sums and products: FP64 ones as multiply-adds (fp64_offload.cuh; at first use h kernel 459 -> 425 us and pass 2 320 ->
+// 296 us at 24 grids of 1024^2), FP32 ones as they are.
 template <typename T>
 struct Arith {
     __device__ __forceinline__ T add(T a, T b) const { return a + b; }
@@ -190,117 +190,68 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs_kernel(const GridDev* __restr
 }
 
 // ------------------------------------------------------------------------------------------------
-// K1 in two passes (batch configurations with rhs_split): h is formed once per point and kept in the
-// grid's h buffer, so that no block recomputes its neighbours' halo values of h (K1 above forms cBar
-// on a 2-point halo and h on a 1-point halo of every block, 15.1 FP64 operations per point; the two passes take
-// 12.7, since they also add the Laplacians' diagonal sums once per point). The values are those of K1 bit for bit.
-// With h in units of sigma_nl and the sum in units of 2/3 as well, pass 1 takes 7.4 operations and pass 2 5.25, against 9.2 and 6:
-// h 428 -> 360 us and pass 2 296 -> 249 us at 24 grids of 1024^2; 96 grids of 64^2 .. 1024^2 1423 -> 1317 us a step.
+// K1 in two passes (configurations with warps2): h is formed once per point and kept in the grid's h buffer, so that no
+// block recomputes its neighbours' halo values of h (K1 above forms cBar on a 2-point halo and h on a 1-point halo of
+// every block, 15.1 FP64 operations per point), and the Laplacians' diagonal sums are added once per point: 7.3
+// operations in pass 1 and 5.1 in pass 2. The values are those of K1 bit for bit.
+// One CTA per block, its descriptor read before the wait for the previous kernel: 7 to 9 CTAs of 8 warps share an SM and
+// hide one another's loads and barriers. At 24 grids of 1024^2, us (share of the FP64 pipe): pass 1 312 (94%), pass 2
+// 221 (94%); before, persistent CTAs without shared sums and with h and the sum in plain units 428 (89%) and 296 (84%,
+// with a cp.async double buffer); persistent CTAs with them 363 (85%) and 248 (87%). 96 grids of 64^2 .. 1024^2 in all:
+// 1231, 1423 and 1317 us a step; over FP32 values 1294, 1379 and 1330.
 // ------------------------------------------------------------------------------------------------
 // Pass 1: h = sigma_nl * (c^3 - c) - sigma_lin * Lap(cBar), cBar over the block and a 1-point halo.
 template <typename T, int NW>
-__global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restrict__ grids,
-                                                        const Item* __restrict__ items, int n_items, int parity) {
+__global__ void __launch_bounds__(NW * BLK) ch_h_kernel(const GridDev* __restrict__ grids, const Item* __restrict__ items,
+                                                        int parity) {
+    constexpr bool kFp64 = std::is_same<T, double>::value;
     __shared__ T cb[34][35];
     __shared__ T cc[32][33];
-    constexpr bool kFp64 = std::is_same<T, double>::value;
     __shared__ double diag[kFp64 ? 33 : 1][33];
     constexpr int NT = NW * BLK;
     const int tid = threadIdx.x;
     const volatile double* factors = g_rhs_factors;
     const T two = (T)factors[0], m_four = (T)factors[1];
     const Arith<T> ar;
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    const HValue<T> h(gd.tab);
     launch_wait();
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n;
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        const double* old = parity ? gd.buf[0] : gd.buf[1];
-        const double* tab = gd.tab;
-        const int bpr = n / BLK;
-        const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const HValue<T> h(tab);
+    const int n = gd.n;
+    const double* cur = parity ? gd.buf[1] : gd.buf[0];
+    const double* old = parity ? gd.buf[0] : gd.buf[1];
+    const int bpr = n / BLK;
+    const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
 #pragma unroll 4
-        for (int e = tid; e < 34 * 34; e += NT) {
-            const int r = e / 34, c = e - r * 34;
-            int gy = y0 - 1 + r, gx = x0 - 1 + c;
-            gy = gy < 0 ? gy + n : (gy >= n ? gy - n : gy);
-            gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
-            const double cv = cur[(size_t)gy * n + gx];
-            const double ov = old[(size_t)gy * n + gx];
-            const T c32 = (T)cv, o32 = (T)ov;
-            cb[r][c] = fma(two, c32, -o32);
-            if (r >= 1 && r < 33 && c >= 1 && c < 33) cc[r - 1][c - 1] = c32;
-        }
+    for (int e = tid; e < 34 * 34; e += NT) {
+        const int r = e / 34, c = e - r * 34;
+        int gy = y0 - 1 + r, gx = x0 - 1 + c;
+        gy = gy < 0 ? gy + n : (gy >= n ? gy - n : gy);
+        gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
+        const double cv = cur[(size_t)gy * n + gx];
+        const double ov = old[(size_t)gy * n + gx];
+        const T c32 = (T)cv, o32 = (T)ov;
+        cb[r][c] = fma(two, c32, -o32);
+        if (r >= 1 && r < 33 && c >= 1 && c < 33) cc[r - 1][c - 1] = c32;
+    }
+    __syncthreads();
+    if constexpr (kFp64) {
+        diagonal_sums<NT>(ar, &cb[0][0], diag, tid);
         __syncthreads();
-        if constexpr (kFp64) {
-            diagonal_sums<NT>(ar, &cb[0][0], diag, tid);
-            __syncthreads();
-        }
+    }
 #pragma unroll 4
-        for (int e = tid; e < 32 * 32; e += NT) {
-            const int r = e / 32, c = e - r * 32;
-            T lap;
-            if constexpr (kFp64) lap = fma(m_four, cb[r + 1][c + 1], ar.add(diag[r][c + 1], diag[r + 1][c]));
-            else lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
-            const long long q = (long long)(y0 + r) * n + x0 + c;
-            if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)h(ar, cc[r][c], lap);
-        }
-        __syncthreads();
+    for (int e = tid; e < 32 * 32; e += NT) {
+        const int r = e / 32, c = e - r * 32;
+        T lap;
+        if constexpr (kFp64) lap = fma(m_four, cb[r + 1][c + 1], ar.add(diag[r][c + 1], diag[r + 1][c]));
+        else lap = laplacian(ar, m_four, cb[r + 1][c + 1], cb[r][c + 1], cb[r + 2][c + 1], cb[r + 1][c], cb[r + 1][c + 2]);
+        const long long q = (long long)(y0 + r) * n + x0 + c;
+        if (in_bounds(q, 0, (long long)n * n)) gd.hbuf[q] = (double)h(ar, cc[r][c], lap);
     }
 }
 
 // Pass 2: rhs = Lap(h) - (2/3)(cCurr - cOld) (findRHS, cuPentCahnADI.cu:72-86), h over the block and a
 // 1-point halo from the h buffer.
-template <typename T, int NW>
-__global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __restrict__ grids,
-                                                           const Item* __restrict__ items, int n_items, int parity) {
-    __shared__ double hh[34][35];
-    __shared__ double dco[32][33];
-    __shared__ double diag[33][33];
-    constexpr int NT = NW * BLK;
-    const int tid = threadIdx.x;
-    const int lane = tid & (BLK - 1), warp = tid / BLK;
-    const volatile double* factors = g_rhs_factors;
-    const double m_four = factors[1];
-    const Arith<double> ar;
-    launch_wait();
-    for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const Item item = items[it];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n;
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        const double* old = parity ? gd.buf[0] : gd.buf[1];
-        const int bpr = n / BLK;
-        const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-#pragma unroll 4
-        for (int e = tid; e < 34 * 34; e += NT) {
-            const int r = e / 34, c = e - r * 34;
-            int gy = y0 - 1 + r, gx = x0 - 1 + c;
-            gy = gy < 0 ? gy + n : (gy >= n ? gy - n : gy);
-            gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
-            hh[r][c] = gd.hbuf[(size_t)gy * n + gx];
-            if (r >= 1 && r < 33 && c >= 1 && c < 33) {
-                dco[r - 1][c - 1] = ar.sub(cur[(size_t)gy * n + gx], old[(size_t)gy * n + gx]);
-            }
-        }
-        __syncthreads();
-        diagonal_sums<NT>(ar, &hh[0][0], diag, tid);
-        const RhsValue<T> rhs(gd.tab);
-        __syncthreads();
-        const int j = lane;
-        double* out = gd.tmp + (size_t)y0 * n + x0 + j;
-#pragma unroll 4
-        for (int rr = warp; rr < BLK; rr += NW) {
-            const double lap = fma(m_four, hh[rr + 1][j + 1], ar.add(diag[rr][j + 1], diag[rr + 1][j]));
-            if (!in_bounds((long long)(y0 + rr) * n + x0 + j, 0, (long long)n * n)) continue;
-            out[(size_t)rr * n] = rhs(lap, dco[rr][j]);
-        }
-        __syncthreads();
-    }
-}
-
 // cp.async helpers (8-byte copies into shared memory, grouped, waited on by group count)
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -310,17 +261,23 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Pass 2, pipelined (configurations with rhs_split = 2): the same values, with the next work item's h window copied
-// into the other half of a shared-memory double buffer (cp.async) while the current item computes; cCurr and cOld are
-// read into registers before the wait for the window. 96 grids of 64^2 .. 1024^2: 1317 us a step,
-// with ch_rhs2_kernel 1506 .. 1569; cCurr and cOld in the double buffer as well leave no room for the diagonal sums at four
-// CTAs per SM.
-constexpr int kRhs2H = 34 * 35;
-
-template <int NW>
-__device__ __forceinline__ void rhs2_issue(double* hh, const GridDev& gd, const Item& item, int tid) {
-    constexpr int NT = NW * BLK;
+template <typename T, int NW>
+__global__ void __launch_bounds__(NW * BLK) ch_rhs2_kernel(const GridDev* __restrict__ grids,
+                                                           const Item* __restrict__ items, int parity) {
+    __shared__ double hh[34 * 35];
+    __shared__ double diag[33][33];
+    constexpr int NT = NW * BLK, R = BLK / NW;   // rows per warp
+    const int tid = threadIdx.x;
+    const int j = tid & (BLK - 1), warp = tid / BLK;
+    const volatile double* factors = g_rhs_factors;
+    const double m_four = factors[1];
+    const Arith<double> ar;
+    const Item item = items[blockIdx.x];
+    const GridDev gd = grids[item.grid];
+    launch_wait();
     const int n = gd.n;
+    const double* cur = parity ? gd.buf[1] : gd.buf[0];
+    const double* old = parity ? gd.buf[0] : gd.buf[1];
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
     for (int e = tid; e < 34 * 34; e += NT) {
@@ -330,60 +287,26 @@ __device__ __forceinline__ void rhs2_issue(double* hh, const GridDev& gd, const 
         gx = gx < 0 ? gx + n : (gx >= n ? gx - n : gx);
         cp_async8(hh + r * 35 + c, gd.hbuf + (size_t)gy * n + gx);
     }
-}
-
-template <typename T, int NW>
-__global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* __restrict__ grids,
-                                                                const Item* __restrict__ items, int n_items,
-                                                                int parity) {
-    __shared__ double ring[2][kRhs2H];
-    __shared__ double diag[33][33];
-    constexpr int R = BLK / NW;   // rows per warp
-    const int tid = threadIdx.x;
-    const int j = tid & (BLK - 1), warp = tid / BLK;
-    const volatile double* factors = g_rhs_factors;
-    const double m_four = factors[1];
-    const Arith<double> ar;
-    launch_wait();
-    int it_cur = blockIdx.x;
-    if (it_cur < n_items) rhs2_issue<NW>(ring[0], grids[items[it_cur].grid], items[it_cur], tid);
     cp_async_commit();
-    for (int k = 0;; ++k) {
-        if (it_cur >= n_items) break;
-        __syncthreads();   // every thread is done with the other half of the buffer and with diag
-        const int it_next = it_cur + gridDim.x;
-        if (it_next < n_items) rhs2_issue<NW>(ring[(k + 1) & 1], grids[items[it_next].grid], items[it_next], tid);
-        cp_async_commit();
-        const Item item = items[it_cur];
-        const GridDev gd = grids[item.grid];
-        const int n = gd.n;
-        const double* cur = parity ? gd.buf[1] : gd.buf[0];
-        const double* old = parity ? gd.buf[0] : gd.buf[1];
-        const int bpr = n / BLK;
-        const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
-        const size_t at = (size_t)(y0 + warp) * n + x0 + j;
-        double cv[R], ov[R];
+    const size_t at = (size_t)(y0 + warp) * n + x0 + j;
+    double cv[R], ov[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            cv[r] = cur[at + (size_t)(r * NW) * n];
-            ov[r] = old[at + (size_t)(r * NW) * n];
-        }
-        const RhsValue<T> rhs(gd.tab);
-        cp_async_wait<1>();   // this thread's copies of the current item have landed
-        __syncthreads();      // and every other thread's
-        const double* hh = ring[k & 1];
-        diagonal_sums<NW * BLK>(ar, hh, diag, tid);
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int rr = warp + r * NW;
-            const double lap = fma(m_four, hh[(rr + 1) * 35 + j + 1], ar.add(diag[rr][j + 1], diag[rr + 1][j]));
-            const size_t q = at + (size_t)(r * NW) * n;
-            if (in_bounds((long long)q, 0, (long long)n * n)) gd.tmp[q] = rhs(lap, ar.sub(cv[r], ov[r]));
-        }
-        it_cur = it_next;
+    for (int r = 0; r < R; ++r) {
+        cv[r] = cur[at + (size_t)(r * NW) * n];
+        ov[r] = old[at + (size_t)(r * NW) * n];
     }
+    const RhsValue<T> rhs(gd.tab);
     cp_async_wait<0>();
+    __syncthreads();
+    diagonal_sums<NT>(ar, hh, diag, tid);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int rr = warp + r * NW;
+        const double lap = fma(m_four, hh[(rr + 1) * 35 + j + 1], ar.add(diag[rr][j + 1], diag[rr + 1][j]));
+        const size_t q = at + (size_t)(r * NW) * n;
+        if (in_bounds((long long)q, 0, (long long)n * n)) gd.tmp[q] = rhs(lap, ar.sub(cv[r], ov[r]));
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -419,8 +342,9 @@ __global__ void __launch_bounds__(NW * BLK) ch_rhs2_pipe_kernel(const GridDev* _
 //
 // A warp's FP64 instruction holds its sub-partition's FP64 pipe for 64 cycles however few lanes it has, so with
 // fewer chains than FP64 sub-partitions (4 per SM) a step takes the chain's instruction count: n / 2 elements
-// of 4 instructions per sweep. Measured, us per step (before: banded factors, one warp per 32 lines): one grid of 256^2
-// 46 (159), 512^2 75 (298), 1024^2 242 (601), 2048^2 388 (1331); 96 grids of 64^2 .. 1024^2 1488 (1973).
+// of 4 instructions per sweep. Measured, us per step (before: banded factors, one warp per 32 lines, and the former
+// right-hand side): one grid of 256^2 45 (159), 512^2 73 (298), 1024^2 231 (601), 2048^2 353 (1331); 96 grids of 64^2 ..
+// 1024^2 1231 (1973).
 
 // Chunks of kChunk elements of a warp's 32 lines move between the work field and a shared-memory ring of kStages
 // stages by the tensor memory accelerator, one copy per chunk each way, issued by a copy warp per chain (two chain
@@ -915,8 +839,9 @@ __global__ void __launch_bounds__(256, 4) ch_update_kernel(const GridDev* __rest
 //     a difference of FP32 rounding size (2e-7 after 40 steps), so its results are tied to these operations.
 // One chain per 32 lines (the whole line), with the ring and the copy warp of the factored sweeps; the table entries
 // of a chunk arrive with it, and in the part of the line where the factors have converged to the last bit they stay
-// in registers. 24 grids of 96^2 .. 384^2, FP32 stencils: 206 us per step (263 with cp.async double buffers and the
-// table entries read per chunk into registers); 96 grids of 64^2 .. 1024^2: 1378 (1571).
+// in registers. 24 grids of 96^2 .. 384^2, FP32 stencils: 204 us per step (263 with cp.async double buffers and the
+// table entries read per chunk into registers); 96 grids of 64^2 .. 1024^2: 1294 (1571; 1378 with the
+// sweeps alone).
 // ------------------------------------------------------------------------------------------------
 struct BandChunk {
     double ds[kChunk], dl[kChunk], rd[kChunk], du[kChunk], dw[kChunk];
@@ -1240,55 +1165,54 @@ static bool close_apart(const ChConfig& c, const ChWork& w, int sms) {
 }
 
 int ch_launches_per_step(const ChConfig& c, const ChWork& w, int sms) {
-    return (c.rhs_split ? 2 : 1) + (w.n_lines > w.n_general ? 3 + close_apart(c, w, sms) : 0) +
+    return (c.warps2 ? 2 : 1) + (w.n_lines > w.n_general ? 3 + close_apart(c, w, sms) : 0) +
            (w.n_general > 0 ? 3 + few_chains(w.n_general, sms) : 0);
 }
 
 ChConfig ch_config(int index) {
-    // {warps per right-hand-side CTA, right-hand-side passes, x closure}
+    // {warps per right-hand-side CTA, of pass 2 (0: one pass), x closure}
     static const ChConfig tab[kChConfigs] = {
-        {1, 0, 1}, {2, 0, 1}, {4, 0, 1}, {8, 0, 1}, {1, 1, 1}, {2, 1, 1}, {4, 1, 1}, {8, 1, 1}, {2, 2, 1}, {4, 2, 1}, {8, 2, 1},
-        {1, 0, 2}, {4, 0, 0}, {2, 0, 2}, {4, 0, 2}, {8, 0, 2}, {2, 1, 2}, {4, 1, 2}, {8, 1, 2}, {4, 2, 2}, {8, 2, 0}, {8, 2, 2}};
+        {1, 0, 1}, {2, 0, 1}, {4, 0, 1}, {8, 0, 1}, {1, 1, 1}, {2, 2, 1}, {4, 4, 1}, {8, 8, 1}, {4, 2, 1}, {8, 4, 1}, {4, 8, 1},
+        {1, 0, 2}, {4, 0, 0}, {2, 0, 2}, {4, 0, 2}, {8, 0, 2}, {2, 2, 2}, {4, 4, 2}, {8, 8, 2}, {8, 4, 2}, {8, 8, 0}, {4, 4, 0}};
     return tab[(index >= 0 && index < kChConfigs) ? index : 0];
 }
 
 void config_name(const ChConfig& c, char* name, size_t len) {
-    snprintf(name, len, "rhs_warps%d%s%s", c.rhs_warps, c.rhs_split == 2 ? "_2pass_pipe" : (c.rhs_split ? "_2pass" : ""),
-             c.close == 2 ? "_close_apart" : (c.close ? "_close_fused" : ""));
+    char second[16] = "";
+    if (c.warps2) snprintf(second, sizeof(second), "_2pass%d", c.warps2);
+    snprintf(name, len, "rhs_warps%d%s%s", c.rhs_warps, second, c.close == 2 ? "_close_apart" : (c.close ? "_close_fused" : ""));
 }
 
-// The two passes of the split right-hand side. Pass 2 runs in FP64 in both variants: the precision variant's h
-// buffer holds FP32 values, whose FP64 Laplacian is exact, so its mass is conserved to FP64 rounding (the
-// one-pass kernel does the same). Pass 2 pipelined: dynamic shared memory beyond 48 KB, allowed once per device.
-template <typename T, int NW>
-static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, int sms, cudaStream_t s) {
-    // persistent grids over the work list
-    const int n = w.n_blocks, grid = std::max(1, std::min(n, sms * 32 / NW));
-    if (!c.rhs_split) {
-        return launch_overlapped(ch_rhs_kernel<T, NW>, grid, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
+// The two passes of the right-hand side run one CTA per block. Pass 2 runs in FP64 in both variants: the precision
+// variant's h buffer holds FP32 values, whose FP64 Laplacian is exact, so its mass is conserved to FP64 rounding (the
+// one-pass kernel does the same).
+template <typename F>
+static cudaError_t with_warps(int warps, F f) {
+    switch (warps) {
+    case 1: return f(std::integral_constant<int, 1>{});
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    default: return f(std::integral_constant<int, 8>{});
     }
-    // 48 warps per SM in FP64: three CTAs of 8 warps are resident beside the L1 the stencil's halos use, so 32 leave a
-    // third of an SM's work to a second wave (96 grids of 64^2 .. 1024^2: 1319 us a step, 32 warps 1474; a larger
-    // shared-memory carve-out, which makes all of them resident, 1327 and 1481; a CTA per block 1309 .. 1328). Over FP32
-    // values, bound by memory, 32 warps (1330; 48 warps 1382).
-    const int per_sm = std::is_same<T, double>::value ? std::min(48 / NW, 8) : 32 / NW;
-    const int split = std::max(1, std::min(n, sms * per_sm));
-    const cudaError_t e = launch_overlapped(ch_h_kernel<T, NW>, split, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
-    if (e != cudaSuccess) return e;
-    if (c.rhs_split == 2)   // four CTAs per SM fit the double buffer
-        return launch_overlapped(ch_rhs2_pipe_kernel<T, NW>, std::max(1, std::min(n, sms * 4)), dim3(NW * BLK), 0, s, w.grids,
-                                 w.blocks, n, parity);
-    return launch_overlapped(ch_rhs2_kernel<T, NW>, split, dim3(NW * BLK), 0, s, w.grids, w.blocks, n, parity);
 }
 
 template <typename T>
 static cudaError_t launch_rhs(const ChConfig& c, const ChWork& w, int parity, int sms, cudaStream_t s) {
-    switch (c.rhs_warps) {
-    case 1: return launch_rhs<T, 1>(c, w, parity, sms, s);
-    case 2: return launch_rhs<T, 2>(c, w, parity, sms, s);
-    case 4: return launch_rhs<T, 4>(c, w, parity, sms, s);
-    default: return launch_rhs<T, 8>(c, w, parity, sms, s);
-    }
+    if (!c.warps2)
+        return with_warps(c.rhs_warps, [&](auto nw) {
+            constexpr int NW = decltype(nw)::value;   // persistent over the work list
+            return launch_overlapped(ch_rhs_kernel<T, NW>, std::max(1, std::min(w.n_blocks, sms * 32 / NW)), dim3(NW * BLK), 0, s,
+                                     w.grids, w.blocks, w.n_blocks, parity);
+        });
+    const cudaError_t e = with_warps(c.rhs_warps, [&](auto nw) {
+        constexpr int NW = decltype(nw)::value;
+        return launch_overlapped(ch_h_kernel<T, NW>, w.n_blocks, dim3(NW * BLK), 0, s, w.grids, w.blocks, parity);
+    });
+    if (e != cudaSuccess) return e;
+    return with_warps(c.warps2, [&](auto nw) {
+        constexpr int NW = decltype(nw)::value;
+        return launch_overlapped(ch_rhs2_kernel<T, NW>, w.n_blocks, dim3(NW * BLK), 0, s, w.grids, w.blocks, parity);
+    });
 }
 
 cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, int parity, int sms, cudaStream_t s) {

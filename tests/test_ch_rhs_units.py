@@ -1,5 +1,5 @@
 """The FP64 right-hand side in units of sigma_nl and 2/3 where those units are extreme (no time step, a tiny one, no
-biharmonic), in its three kernels (one pass, two passes, pass 2 pipelined): against the scheme in Fourier space, and
+biharmonic), in one pass and in two with 8 and with 4 and 2 warps per CTA: against the scheme in Fourier space, and
 the three against one another bit for bit (GPU)."""
 import numpy as np
 import pytest
@@ -29,7 +29,7 @@ def fourier_step(c, old, gamma, dt_factor):
 def test_units(gpu, n, gamma, dt_factor):
     old, cur = np.random.default_rng(n).uniform(-0.1, 0.1, (2, n, n))
     fields = []
-    for config in (3, 7, 20):
+    for config in (3, 7, 8):
         b = cs.CahnHilliardBatch([n], gamma=gamma, dt_factor=dt_factor)
         b.set_config(config)
         b.set_state(0, cur, old)
