@@ -1157,8 +1157,8 @@ __global__ void __launch_bounds__(256) ch_update_general_kernel(const GridDev* _
 // Whether the element-wise parts of a sweep run as kernels of their own. With fewer chains than FP64 sub-partitions (4
 // per SM) a sweep takes as long as one chain, so they are taken out of it; for lines in two segments, which the
 // closure reaches everywhere, that is no slower with many chains either. Measured (us per step, x closure in the y
-// sweep / apart): 24 grids of 96^2 .. 384^2 (672 chains) 131 / 125, of 512^2 (1536) 418 / 412; 8 grids of 1024^2 (512
-// chains) 551 / 569, 24 (1536) 1448 / 1519; one of 1024^2 (64) 294 / 242.
+// sweep / apart): 24 grids of 96^2 .. 384^2 (672 chains) 123 / 116, of 512^2 (1536) 372 / 367; 8 grids of 1024^2 (512
+// chains) 474 / 485, 24 (1536) 1201 / 1252; one of 1024^2 (64) 262 / 231.
 static bool few_chains(int chains, int sms) { return chains < 4 * sms; }
 static bool close_apart(const ChConfig& c, const ChWork& w, int sms) {
     return c.close == 2 || (c.close == 0 && (w.n_whole == 0 || 2 * (w.n_lines - w.n_general) < 3 * sms));
@@ -1321,7 +1321,7 @@ static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
 
 // Two segments halve a chain, which is the time of a sweep when few lines are resident, and add up to two
 // multiply-adds per point and sweep where the closure's reach is long against half a line, which is the time when
-// many are. Measured (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
+// many are. Measured with the persistent right-hand side (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
 // 384^2 152 / 123, 96 grids of 64^2 .. 1024^2 with those up to 512^2 cut 1466 / 1488; one grid of 1024^2 242 / 161, but the
 // 96 grids 1488 / 1570 with the 1024^2 ones cut as well; 2048^2: one grid 547 / 388, four 1092 / 1039, eight 1909 / 2054.
 // Grids of 1024^2 come in the large batches, larger ones do not, so those between the two sizes keep one segment.

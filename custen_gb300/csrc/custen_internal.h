@@ -165,7 +165,7 @@ struct StreamBlock {
 constexpr uint32_t kPlanMagic = 0xC5E7B300u;
 
 // Launch entry points implemented in the kernel translation units.
-// *path is set to 1 when the TMA-staged kernel ran, 0 for the plain-load kernel.
+// *path is set to 1 when the TMA-staged kernel ran, 0 for the cp.async kernel.
 cudaError_t launch_stencil_f64(const StencilArgs& a, cudaStream_t s, int* path);
 cudaError_t launch_stencil_f32(const StencilArgs& a, cudaStream_t s, int* path);
 cudaError_t launch_weno_adv(const StencilArgs& a, cudaStream_t s);

@@ -42,7 +42,7 @@ constexpr StencilConfig kConfigsF32[kNumConfigs] = {
 };
 
 // One launch with configuration `cfg` (0 .. kNumConfigs-1) of element type `dtype`; *path = 1 when
-// the TMA-staged kernel ran, 0 for the plain-load kernel.
+// the TMA-staged kernel ran, 0 for the cp.async kernel.
 cudaError_t launch_stencil_cfg(const StencilArgs& a, int dtype, int cfg, cudaStream_t s, int* path);
 
 // Upper bound on the CTAs of a persistent stencil launch (0: none, the default). Lowering it makes each

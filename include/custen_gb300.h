@@ -66,7 +66,7 @@ void custen_set_tune_cache(const char* path);
 int custen_tune_cache_path(char* buf, size_t len);
 int custen_autotune(cuSten_t* h, int reps);
 int custen_handle_config(const cuSten_t* h, char* name, size_t len);
-/* Pin a handle to configuration `index` (0 .. 4; -1: choose again at the next Compute). */
+/* Pin a handle to configuration `index` (0 .. 5; -1: choose again at the next Compute). */
 int custen_set_config(cuSten_t* h, int index);
 
 /* Which shipped function (0..5) `f` is on the current device, or -1. */
@@ -233,7 +233,7 @@ int custen_ch_batch_step(void* batch, int steps, int use_graph);   /* asynchrono
 int custen_ch_batch_synchronize(void* batch);
 int custen_ch_batch_mean(void* batch, int sim, double* mean);     /* compensated FP64 sum */
 unsigned long long custen_ch_batch_launches(void* batch);
-/* Kernel configuration of the batch's steps (warps per right-hand-side CTA, rows per y-sweep batch):
+/* Kernel configuration of the batch's steps (warps per right-hand-side CTA and passes, where the x closure is applied):
  * custen_ch_batch_autotune times every configuration over `steps` steps of the batch itself, restores
  * the fields, and keeps the fastest; results do not depend on it. No reference counterpart. */
 int custen_ch_batch_autotune(void* batch, int steps, char* name, size_t len);
