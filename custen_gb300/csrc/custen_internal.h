@@ -134,6 +134,8 @@ struct PlanPrivate {
     int H, V, L, R, T, B;
     int ncoef;            // weights or coefficients read per Compute
     int mem_kind;         // -1 unknown, 0 device, 1 managed, 2 host-accessible system memory
+    bool group_own;       // the last group Compute ran on the handle's own stream
+    unsigned long long id, last_owner;   // this handle (never 0); the one on whose first stream its last work was queued, 0: none
     cudaStream_t user_stream;
     int use_user_stream;
     unsigned long long launches;   // kernels launched by this handle (for instrumentation)

@@ -93,12 +93,13 @@ int custen_create_slab(cuSten_t* h, int variant, int dtype, int deviceNum, int s
                        void* func);
 int custen_compute(cuSten_t* h, int offload);                       /* cuStenCompute2D*(h, offload) */
 int custen_compute_on_stream(cuSten_t* h, int offload, void* stream); /* same, all work on `stream` */
-/* One Compute of each of `count` distinct handles, free to run at the same time: each handle's work runs
- * on its own first stream, after the work already queued on `stream` and before any work queued on
- * `stream` later. Use it for independent operators (e.g. several derivatives of one field into separate
- * outputs): on small fields one launch's tail then overlaps the next launch. All handles and `stream`
- * belong to one device. Handles that write a buffer another member reads must not be grouped. The reference computes one handle per call
- * (stencil_kernels.h:52-183); this has no counterpart there. */
+/* One Compute of each of `count` distinct handles, free to run at the same time, after the work already queued
+ * on `stream` and before any work queued on `stream` later: members with device-resident fields share the
+ * first streams of up to three of the handles, others run on their own first stream. Use it for independent
+ * operators (e.g. several derivatives of one field into separate outputs): one launch's tail then overlaps
+ * the next launch. All handles and `stream` belong to one device. Handles that write a buffer another member
+ * reads must not be grouped. The reference computes one handle per call (stencil_kernels.h:52-183); this has
+ * no counterpart there. */
 int custen_compute_group(cuSten_t* const* handles, int count, int offload, void* stream);
 int custen_swap(cuSten_t* h, void* dataInput);                      /* cuStenSwap2D*(h, dataInput) */
 int custen_destroy(cuSten_t* h);                                    /* cuStenDestroy2D*(h) */
