@@ -5,12 +5,12 @@
 // box of SW = LP + TW + RP columns by SR = T + TH + B rows starting at (x0 - LP, y0 - T), landing at a
 // 128-byte aligned stage. Completion is signalled on the stage's mbarrier (complete_tx); the next
 // tiles' copies run while the current tile computes. Rows and columns outside the launch arrive
-// zero-filled; the last tile column and row may be partial. Periodic variants add wrap-around boxes on the first
-// and last tile columns: the LP
-// columns left of x = 0 come from x = nx - LP, the RP columns right of nx from x = 0, each into a
+// zero-filled; the last tile column and row may be partial. Periodic variants add wrap-around boxes on the tiles
+// whose window leaves the field (the first and last columns, and those behind them that a halo longer than a tile
+// reaches): the LP columns left of x = 0 come from x = nx - LP, the RP columns right of nx from x = 0, each into a
 // side area of the stage on the same mbarrier, from where the edge tile copies them into place.
-// Edge tiles of the first and last tile row fetch their halo rows through the halo pointers with
-// plain (coalesced) loads.
+// Tiles whose window leaves the launch's rows fetch the halo rows through the halo pointers with plain
+// (coalesced) loads.
 //
 // Every mbarrier wait is bounded: on expiry the CTA records an error in g_custen_device_error, waits
 // (bounded) for its own copies still in flight, and returns.
@@ -72,15 +72,23 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Whether the window of the tile at x0 reaches columns left of the field / right of it, or rows outside the launch: the
+// first and last tiles, those next to a narrow last one, and with a halo longer than a tile those behind the first.
+__device__ __forceinline__ bool reaches_left(const StencilArgs& a, int x0) { return x0 < a.L; }
+__device__ __forceinline__ bool reaches_right(const StencilArgs& a, int x0, int tw) { return x0 + tw + a.R > a.nx; }
+__device__ __forceinline__ bool reaches_halo_rows(const StencilArgs& a, int y0, int th) {
+    return (y0 < a.T && a.has_top) || (y0 + th + a.B > a.rows && a.B > 0 && a.has_bot);
+}
+
 // Issue the copies of one tile window into the (128-byte aligned) stage `dst`: the window box, and on
-// the first / last tile column of a periodic launch the wrap-around boxes into the stage's side areas
+// a tile of a periodic launch that reaches beyond the field the wrap-around boxes into the stage's side areas
 // `side` (LP x SR elements, then RP x SR from `side + wl_elems`).
 template <typename T, int TW, int TH>
 __device__ __forceinline__ void issue_window(const StencilArgs& a, const TmaMaps& m, T* dst, T* side, int wl_elems,
                                              int wr_elems, uint64_t* bar, int x0, int y0,
                                              const TileGeom<T, TW, TH>& g) {
-    const bool left = wl_elems > 0 && x0 == 0;
-    const bool right = wr_elems > 0 && x0 + TW + a.R > a.nx;   // the last column, and the one before a narrow last
+    const bool left = wl_elems > 0 && reaches_left(a, x0);
+    const bool right = wr_elems > 0 && reaches_right(a, x0, TW);
     uint32_t bytes = (uint32_t)(g.SR * g.SW * sizeof(T));
     if (left) bytes += (uint32_t)(g.SR * g.LP * sizeof(T));
     if (right) bytes += (uint32_t)(g.SR * g.RP * sizeof(T));
@@ -118,10 +126,10 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
         }
     }
     if (cols_fix) {
-        // wrapped halo columns of the rows inside the launch, from the side areas: column k < LP of row r is
+        // wrapped halo columns of the rows inside the launch, from the side areas: the column of x = -LP + k is
         // side[r * LP + k] (x = nx - LP + k), the column of x = nx + k is side_r[r * RP + k] (x = k); the boxes
         // zero-fill x outside [0, nx) as a too-narrow field needs
-        const bool left = x0 == 0, right = x0 + TW + a.R > a.nx;
+        const bool left = reaches_left(a, x0), right = reaches_right(a, x0, TW);
         const T* side_r = side + wl_elems;
         const int c_end = g.LP + a.nx - x0;   // window column of x = nx
         const int ncols = g.LP + g.RP;
@@ -132,9 +140,10 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
             if (gyl < 0 || gyl >= a.rows) continue;
             const int k = e - r * ncols;
             if (k < g.LP) {
-                if (!left) continue;
-                if (!in_bounds((long long)r * g.SW + k, 0, (long long)g.SR * g.SW)) continue;
-                tile[r * g.SW + k] = side[r * g.LP + k];
+                const int c = k - x0;   // window column of x = -LP + k
+                if (!left || c < 0) continue;
+                if (!in_bounds((long long)r * g.SW + c, 0, (long long)g.SR * g.SW)) continue;
+                tile[r * g.SW + c] = side[r * g.LP + k];
             } else {
                 const int kk = k - g.LP;
                 if (!right || c_end + kk >= g.SW) continue;
@@ -209,8 +218,8 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
         const bool ok = mbar_wait(&full[s], parity);
         const int tyi = t / tiles_x, txi = t - tyi * tiles_x;
         const int x0 = txi * TW, y0 = tyi * TH;
-        const bool rows_fix = (y0 == 0 && a.T > 0 && a.has_top) || (y0 + TH + a.B > a.rows && a.B > 0 && a.has_bot);
-        const bool cols_fix = WRAP && (x0 == 0 || x0 + TW + a.R > a.nx);
+        const bool rows_fix = reaches_halo_rows(a, y0, TH);
+        const bool cols_fix = WRAP && (reaches_left(a, x0) || reaches_right(a, x0, TW));
         if (rows_fix || cols_fix) {
             edge_fixup<T, TW, TH, NT>(a, tile, side, wl_elems, g, x0, y0, tid, rows_fix, cols_fix);
             __syncthreads();
