@@ -122,7 +122,7 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
                 x = x < 0 ? x + a.nx : x - a.nx;
                 if (x < 0 || x >= a.nx) continue;
             }
-            tile[e] = __ldg(rowp + x);
+            tile[e] = rowp[x];   // not the read-only path: the kernel before may still write the row as this one starts
         }
     }
     if (cols_fix) {
