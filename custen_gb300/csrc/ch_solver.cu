@@ -458,6 +458,7 @@ __device__ __forceinline__ void run_chain(int nchunk, ChainBars& bars, double (*
         solve(st, u1, u2, Forward{});
         if (c < nchunk - kStages) solved(st);
     }
+    __syncwarp();   // the y sweep's exchange lies where other lanes may still read the first stage's amplitudes
     own[0][lane] = u1;
     own[1][lane] = u2;
     pair_barrier();
