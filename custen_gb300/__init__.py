@@ -249,6 +249,15 @@ def selftest_wait_expiry(rounds: int = 1 << 12) -> int:
     return int(f.value)
 
 
+def selftest_ring_expiry(nchunk: int, lost: int, rounds: int = 1 << 12) -> tuple:
+    """Run two chains of the Cahn-Hilliard sweeps' ring over `nchunk` chunks, the copy of chunk `lost` of the first never
+    arriving (none: -1). Returns the device error flags seen afterwards (bit 0 after an expiry; left set for device_error())
+    and the copies started and stored back, by either chain's copy warp."""
+    f, c = ctypes.c_uint(0), (ctypes.c_int * 4)()
+    _ch_check(lib().custen_selftest_ring_expiry(ctypes.c_longlong(rounds), nchunk, lost, ctypes.byref(f), c))
+    return int(f.value), list(c)
+
+
 def selftest_fp64(samples: int = 1 << 24, seed: int = 1) -> list:
     """Mismatches of the kernels' own conversions, divisions, sums and products against the hardware's (all
     expected 0)."""

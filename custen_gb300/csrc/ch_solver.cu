@@ -389,9 +389,10 @@ __device__ __forceinline__ double mid_value(const double* q, double own1, double
 }
 
 // The ring of one chain: full[s] completes when a chunk has arrived in stage s, done[s] when it has been solved
-// there and may be copied out.
+// there and may be copied out. failed: a wait for a chunk has expired.
 struct ChainBars {
     uint64_t full[kStages], done[kStages];
+    unsigned failed;
 };
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -399,12 +400,15 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 }
 
 // Waits on the stages' barriers in turn; after one has expired (stencil_tma.cuh) none waits any more, so the
-// warps of a CTA run to their end and meet at its barriers whatever happened; the results are void then.
+// warps of a CTA run to their end and meet at its barriers whatever happened; the results are void then. The copy
+// warp then starts no further copy and stays until those in flight have landed (bounded as well).
 struct RingWait {
+    long long limit;
     unsigned parity = 0;   // per stage: the phase its next completion ends
     bool ok = true;
+    __device__ __forceinline__ explicit RingWait(long long limit_) : limit(limit_) {}
     __device__ __forceinline__ void operator()(uint64_t* bars, int st) {
-        if (ok) ok = mbar_wait(&bars[st], (parity >> st) & 1u);
+        if (ok) ok = mbar_wait(&bars[st], (parity >> st) & 1u, limit);
         parity ^= 1u << st;
     }
     __device__ __forceinline__ void report() const {
@@ -412,32 +416,49 @@ struct RingWait {
     }
 };
 
+// The chain is done with a chunk in stage st (by every lane).
+__device__ __forceinline__ void chunk_solved(ChainBars& bars, const RingWait& full, int st, int lane) {
+    if (!full.ok) *(volatile unsigned*)&bars.failed = 1u;
+    __syncwarp();   // every lane's writes
+    if (lane == 0) mbar_arrive(&bars.done[st]);
+}
+
 // The copy warp of a chain (one lane): load(c, stage, pass) starts the copy of chunk c on the stage's full
 // barrier, store(c, stage) the copy back. A stage is refilled once its store has read it.
 template <class Load, class Store>
-__device__ __forceinline__ void run_copies(int nchunk, ChainBars& bars, Load load, Store store) {
-    RingWait done;
+__device__ __forceinline__ void run_copies(int nchunk, ChainBars& bars, Load load, Store store, long long limit = kWaitLimit) {
+    RingWait done(limit);
+    auto solved = [&](int st) {
+        done(bars.done, st);
+        return done.ok && *(const volatile unsigned*)&bars.failed == 0u;
+    };
     for (int c = 0; c < kStages && c < nchunk; ++c) load(c, c, Forward{});
+    unsigned last = 0;   // per stage: the phase that its last copy ends
+    bool ok = true;
     for (int c = 0; c < nchunk - kStages; ++c) {
         const int st = c % kStages;
-        done(bars.done, st);
+        if (!(ok = solved(st))) break;
         fence_proxy_async_smem();
         store(c, st);
         bulk_wait_read_all();
         load(c + kStages, st, Forward{});
+        last ^= 1u << st;
     }
     bulk_wait_all();   // the backward pass reads the forward pass's chunks again
-    for (int c = nchunk - 1; c >= 0; --c) {
+    for (int c = nchunk - 1; ok && c >= 0; --c) {
         const int st = c % kStages;
-        done(bars.done, st);
+        if (!(ok = solved(st))) break;
         fence_proxy_async_smem();
         store(c, st);
         if (c >= kStages) {
             bulk_wait_read_all();
             load(c - kStages, st, Backward{});
+            last ^= 1u << st;
         }
     }
     bulk_wait_all();
+    if (!ok)
+        for (int st = 0; st < kStages && st < nchunk; ++st) mbar_wait(&bars.full[st], (last >> st) & 1u, limit);
     done.report();
 }
 
@@ -445,12 +466,10 @@ __device__ __forceinline__ void run_copies(int nchunk, ChainBars& bars, Load loa
 // the last two values; v1, v2: the values at the chain's outer end.
 template <class Solve>
 __device__ __forceinline__ void run_chain(int nchunk, ChainBars& bars, double (*own)[BLK], double (*other)[BLK], int lane,
-                                          const double* mid, double& v1, double& v2, Solve solve) {
-    RingWait full;
-    auto solved = [&](int st) {
-        __syncwarp();   // every lane's writes
-        if (lane == 0) mbar_arrive(&bars.done[st]);
-    };
+                                          const double* mid, double& v1, double& v2, Solve solve,
+                                          long long limit = kWaitLimit) {
+    RingWait full(limit);
+    auto solved = [&](int st) { chunk_solved(bars, full, st, lane); };
     double u1 = 0.0, u2 = 0.0;
     for (int c = 0; c < nchunk; ++c) {
         const int st = c % kStages;
@@ -471,7 +490,7 @@ __device__ __forceinline__ void run_chain(int nchunk, ChainBars& bars, double (*
         solve(st, v1, v2, Backward{});
         solved(st);
     }
-    if (lane == 0) full.report();
+    full.report();
 }
 
 // The recurrence over kChunk values in registers, w[0] first: v = w + np1 v1 + np2 v2.
@@ -584,6 +603,7 @@ __device__ __forceinline__ void init_ring(ChainBars (&bars)[2]) {
             for (int st = 0; st < kStages; ++st) {
                 mbar_init(&bars[k].full[st], 1);
                 mbar_init(&bars[k].done[st], 1);
+                bars[k].failed = 0u;
             }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -870,11 +890,8 @@ template <class Get, class Put>
 __device__ __forceinline__ void run_band(const GridDev& gd, const BandTable& bt, ChainBars& bars, const BandChunk* band,
                                          int lane, double& x2, double& x1, Get get, Put put) {
     const int nchunk = gd.n / kChunk;
-    RingWait full;
-    auto solved = [&](int st) {
-        __syncwarp();   // every lane's writes
-        if (lane == 0) mbar_arrive(&bars.done[st]);
-    };
+    RingWait full(kWaitLimit);
+    auto solved = [&](int st) { chunk_solved(bars, full, st, lane); };
     const double* tc = bt.t + min(bt.const_lo, nchunk - 1) * kChunk;
     const double cs = tc[0], cl = tc[bt.m], cr = tc[2 * bt.m], cu = tc[3 * bt.m], cw = tc[4 * bt.m];
     double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
@@ -960,7 +977,7 @@ __device__ __forceinline__ void run_band(const GridDev& gd, const BandTable& bt,
     const double nx1 = r1 - (d * y0v + e * y1v + a * ym1);
     x2 = om[0] * nx2 + om[1] * nx1;
     x1 = om[2] * nx2 + om[3] * nx1;
-    if (lane == 0) full.report();
+    full.report();
 }
 
 constexpr int kBandThreads = 2 * BLK;   // warps: the chain, its copies
@@ -972,6 +989,7 @@ __device__ __forceinline__ void init_bars(ChainBars& bars) {
         for (int st = 0; st < kStages; ++st) {
             mbar_init(&bars.full[st], 1);
             mbar_init(&bars.done[st], 1);
+            bars.failed = 0u;
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1246,6 +1264,28 @@ cudaError_t launch_ch_step(const ChConfig& c, bool rhs_fp32, const ChWork& w, in
         then(ch_update_general_kernel, w.n_blocks, block, 0, w.grids, w.blocks, parity);
     }
     return e;
+}
+
+// Self-test of the rings' failure path (custen_selftest_ring_expiry): two chains of `nchunk` chunks whose copies are plain
+// arrivals, but the copy of chunk `lost` of chain A never arrives (a byte count that nothing delivers; no copy is in flight).
+// counts: copies started and stored back by chain A, then by chain B.
+__global__ void __launch_bounds__(kSweepThreads) ch_ring_expiry_kernel(long long limit, int nchunk, int lost, int* counts) {
+    __shared__ double ex[2][2][BLK], mid[8];
+    __shared__ __align__(8) ChainBars bars[2];
+    if (threadIdx.x < 8) mid[threadIdx.x] = 0.0;
+    init_ring(bars);
+    const int lane = threadIdx.x & (BLK - 1), warp = threadIdx.x / BLK, chain = warp & 1;
+    if (warp < 2) {
+        double v1, v2;
+        run_chain(nchunk, bars[chain], ex[chain], ex[chain ^ 1], lane, mid, v1, v2, [](int, double&, double&, auto) {}, limit);
+    } else if (lane == 0) {
+        auto load = [&](int c, int st, auto) {
+            ++counts[2 * chain];
+            mbar_arrive_expect_tx(&bars[chain].full[st], chain == 0 && c == lost ? 16 : 0);
+        };
+        auto store = [&](int, int) { ++counts[2 * chain + 1]; };
+        run_copies(nchunk, bars[chain], load, store, limit);
+    }
 }
 
 // Compensated (Neumaier) sum of one grid: every thread, then every CTA, then the CTA that finishes last over the
@@ -1655,6 +1695,22 @@ using namespace custen::ch;
 extern "C" {
 
 const char* custen_ch_last_error(void) { return g_ch_err.c_str(); }
+
+int custen_selftest_ring_expiry(long long rounds, int nchunk, int lost, unsigned int* flags, int* counts) {
+    if (rounds < 1 || rounds > custen::kWaitLimit || nchunk < 1 || nchunk > 4096 || !flags || !counts)
+        return ch_fail_arg("invalid arguments");
+    int* d = nullptr;
+    CH_TRY(cudaMalloc(&d, 4 * sizeof(int)), "Allocating the self-test's counts");
+    cudaError_t e = cudaMemset(d, 0, 4 * sizeof(int));
+    if (e == cudaSuccess) {
+        ch_ring_expiry_kernel<<<1, kSweepThreads>>>(rounds, nchunk, lost, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(counts, d, 4 * sizeof(int), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e == cudaSuccess) e = cudaMemcpyFromSymbol(flags, custen::g_custen_device_error, sizeof(unsigned int));
+    return e == cudaSuccess ? 0 : ch_fail(e, "Running the ring's self-test");
+}
 
 int custen_ch_batch_create(void** out, int nsims, const int* n, const double* lx, double gamma, double dt_factor,
                            int rhs_dtype, void* stream) {

@@ -191,6 +191,10 @@ int custen_device_error(unsigned int* flags, int clear);
  * raised and the kernel returns. *flags receives the flags afterwards (left set). No copy fails and
  * nothing traps; the context stays usable. */
 int custen_selftest_wait_expiry(long long rounds, unsigned int* flags);
+/* The same for the rings of the Cahn-Hilliard sweeps: two chains of `nchunk` chunks (1 .. 4096), the copy of chunk `lost`
+ * of the first never arriving (none when `lost` is out of range). counts[0], [1]: copies the first chain's copy warp
+ * started and stored back; [2], [3]: the second's. After an expired wait no further copy is started. */
+int custen_selftest_ring_expiry(long long rounds, int nchunk, int lost, unsigned int* flags, int* counts);
 /* Self-test of the kernels' conversions, divisions, sums and products that spare the FP64 pipe
  * (csrc/fp64_offload.cuh) against the compiler's operators on `samples` generated operands (1 .. 2^34):
  * mismatches[0..5] receive the counts for double -> float, float -> double, c / float, 1 / x, a / b, and a + b,
