@@ -100,6 +100,7 @@ def lib() -> ctypes.CDLL:
             getattr(L, name).argtypes = [vp, vp, vp, vp, vp, vp, i, i, vp]
         L.custen_pent_invert_pivots.argtypes = [vp, i, i, vp]
         L.custen_pent_set_depth.argtypes = [i, i]
+        L.custen_pent_depth.argtypes = [i, i]
         L.custen_ch_last_error.restype = ctypes.c_char_p
         L.custen_ch_batch_create.argtypes = [ctypes.POINTER(vp), i, ctypes.POINTER(i), dp, ctypes.c_double,
                                              ctypes.c_double, i, vp]

@@ -239,15 +239,20 @@ extern "C" {
 
 const char* custen_pent_last_error(void) { return g_err.c_str(); }
 
-// Prefetch depth (rows in flight ahead of the chain: 2, 4 or 8) of the factorisation (which = 0),
+// Rows in flight ahead of the chain (2, 4 or 8; 0: by the batch size) of the factorisation (which = 0),
 // the exact solve (1) and the inverted-pivot solve (2). Results do not depend on it.
 int custen_pent_set_depth(int which, int rows) {
-    if (which < 0 || which > 2 || (rows != 2 && rows != 4 && rows != 8)) {
+    if (which < 0 || which > 2 || (rows != 0 && rows != 2 && rows != 4 && rows != 8)) {
         g_err = "invalid prefetch depth";
         return 2;
     }
     g_kr[which] = rows;
     return 0;
+}
+
+// Rows in flight that a call for `batch` systems on the current device takes; 0 for invalid arguments.
+int custen_pent_depth(int which, int batch) {
+    return which < 0 || which > 2 || batch < 1 ? 0 : rows_in_flight(which, (batch - 1) / kLine + 1);
 }
 
 int custen_pent_factor_batch(double* ds, double* dl, double* d, double* du, double* dw, int m, int batch,

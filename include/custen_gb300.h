@@ -220,8 +220,10 @@ int custen_pent_solve_batch_rcp(const double* ds, const double* dl, const double
                                 const double* dw, double* b, int m, int batch, void* stream);
 const char* custen_pent_last_error(void);
 /* Rows in flight ahead of the recurrence (2, 4 or 8) in the factorisation (which = 0), the exact solve (1)
- * and the inverted-pivot solve (2); chosen by the batch size unless set. Results do not depend on it. */
+ * and the inverted-pivot solve (2); chosen by the batch size unless set, and again after rows = 0. Results do
+ * not depend on it. custen_pent_depth: the rows a call for `batch` systems takes. */
 int custen_pent_set_depth(int which, int rows);
+int custen_pent_depth(int which, int batch);
 
 /* ---- Cahn-Hilliard ADI solver: batches of periodic grids of different sizes ----
  * The method of cuPentCahnADI (cuPentCahnADI/src/cuPentCahnADI.cu:197-627 with BatchHyper.cu and
