@@ -133,6 +133,7 @@ struct PlanPrivate {
     int dtype;
     int H, V, L, R, T, B;
     int ncoef;            // weights or coefficients read per Compute
+    int launch_rows;      // rows of the last launch, 0 before the first
     int mem_kind;         // -1 unknown, 0 device, 1 managed, 2 host-accessible system memory
     bool group_own;       // the last group Compute ran on the handle's own stream
     unsigned long long id, last_owner;   // this handle (never 0); the one on whose first stream its last work was queued, 0: none
@@ -171,5 +172,6 @@ constexpr uint32_t kPlanMagic = 0xC5E7B300u;
 cudaError_t launch_stencil_f64(const StencilArgs& a, cudaStream_t s, int* path);
 cudaError_t launch_stencil_f32(const StencilArgs& a, cudaStream_t s, int* path);
 cudaError_t launch_weno_adv(const StencilArgs& a, cudaStream_t s);
+int weno_tile_rows(int nx, int rows);   // rows per tile of such a launch
 
 }  // namespace custen

@@ -171,6 +171,7 @@ int create_plan(cuSten_t* h, int variant, int dtype, int dev, int numTiles, int 
     p.user_stream = nullptr;
     p.use_user_stream = 0;
     p.launches = 0;
+    p.launch_rows = 0;
     p.fused_func = nullptr;
     p.fused_pre = 0;
     p.cfg = -1;
@@ -350,6 +351,7 @@ static cudaError_t launch(const StencilArgs& a, int dtype, cudaStream_t s, PlanP
                                              : launch_stencil_cfg(a, dtype, p->cfg < 0 ? 0 : p->cfg, s, &path);
     if (e == cudaSuccess) {
         ++p->launches;
+        p->launch_rows = a.rows;
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (path == 1) g_launches_tma.fetch_add(1, std::memory_order_relaxed);
     }
@@ -914,7 +916,10 @@ int custen_handle_config(const cuSten_t* h, char* name, size_t len) {
     PlanPrivate* p = priv_of(h);
     if (!p) return fail_arg("cuSten handle was not created by this library (or was destroyed)");
     if (!name || len == 0) return fail_arg("buffer is NULL");
-    snprintf(name, len, "%s", p->variant == V_XYWENOADVP ? "weno_tw64_th32" : config_name(p->dtype, p->cfg < 0 ? 0 : p->cfg));
+    if (p->variant == V_XYWENOADVP)   // of the last launch, before the first that of the whole field
+        snprintf(name, len, "weno_tw64_th%d", weno_tile_rows(h->nx, p->launch_rows ? p->launch_rows : h->ny));
+    else
+        snprintf(name, len, "%s", config_name(p->dtype, p->cfg < 0 ? 0 : p->cfg));
     return ST_OK;
 }
 void custen_set_stage_chunk_bytes(size_t bytes) { g_stage_chunk_bytes.store(bytes ? bytes : (size_t)32 << 20); }

@@ -228,19 +228,25 @@ cudaError_t launch_tile(const StencilArgs& a, cudaStream_t s, int dev) {
 
 }  // namespace
 
+// Two CTAs are resident per SM (304 on GB300) and each tile is a long stretch of FP64 work, so
+// few tiles leave SMs idle and few waves end in an uneven one; a lower tile forms more differences of its halo
+// twice. Measured (us, 8 / 16 / 32 rows): 300^2 40 / 44 / 77, 600^2 101 / 122 / 123, 1000 x 777 187 / 189 / 201
+// (400 tiles of 32 rows), 1500 x 1400 453 / 431 / 454 (1056), 2048^2 - / 817 / 838 (2048), 4096^2 - / 3199 / 3141.
+int weno_tile_rows(int nx, int rows) {
+    const long long tiles = (long long)((nx + kWenoTW - 1) / kWenoTW) * ((rows + 31) / 32);
+    return tiles < 512 ? 8 : (tiles < 4096 ? 16 : 32);
+}
+
 cudaError_t launch_weno_adv(const StencilArgs& a, cudaStream_t s) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (a.rows <= 0 || a.nx <= 0) return cudaSuccess;
-    // Rows per tile: two CTAs are resident per SM (304 on GB300) and each tile is a long stretch of FP64 work, so
-    // few tiles leave SMs idle and few waves end in an uneven one; a lower tile forms more differences of its halo
-    // twice. Measured (us, 8 / 16 / 32 rows): 300^2 40 / 44 / 77, 600^2 101 / 122 / 123, 1000 x 777 187 / 189 / 201
-    // (400 tiles of 32 rows), 1500 x 1400 453 / 431 / 454 (1056), 2048^2 - / 817 / 838 (2048), 4096^2 - / 3199 / 3141.
-    const long long tiles = (long long)((a.nx + kWenoTW - 1) / kWenoTW) * ((a.rows + 31) / 32);
-    if (tiles < 512) return launch_tile<8>(a, s, dev);
-    if (tiles < 4096) return launch_tile<16>(a, s, dev);
-    return launch_tile<32>(a, s, dev);
+    switch (weno_tile_rows(a.nx, a.rows)) {
+    case 8: return launch_tile<8>(a, s, dev);
+    case 16: return launch_tile<16>(a, s, dev);
+    default: return launch_tile<32>(a, s, dev);
+    }
 }
 
 }  // namespace custen

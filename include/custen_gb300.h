@@ -65,6 +65,8 @@ void custen_set_autotune(int mode);
 void custen_set_tune_cache(const char* path);
 int custen_tune_cache_path(char* buf, size_t len);
 int custen_autotune(cuSten_t* h, int reps);
+/* Name of the kernel configuration the handle uses (WENO: the tile of its last launch, before the first that of the
+ * whole field). */
 int custen_handle_config(const cuSten_t* h, char* name, size_t len);
 /* Pin a handle to configuration `index` (0 .. 5; -1: choose again at the next Compute). */
 int custen_set_config(cuSten_t* h, int index);
