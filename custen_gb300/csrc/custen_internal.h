@@ -134,8 +134,8 @@ struct PlanPrivate {
     int H, V, L, R, T, B;
     int ncoef;            // weights or coefficients read per Compute
     int launch_rows;      // rows of the last launch, 0 before the first
-    int mem_kind;         // -1 unknown, 0 device, 1 managed, 2 host-accessible system memory
-    bool group_own;       // the last group Compute ran on the handle's own stream
+    int mem_kind, mem_kind_out;   // of input and output: -1 unknown, 0 device, 1 managed, 2 host-accessible system memory
+    bool copies() const { return mem_kind != 0 || mem_kind_out == 2; }   // a Compute moves data besides its kernels
     unsigned long long id, last_owner;   // this handle (never 0); the one on whose first stream its last work was queued, 0: none
     cudaStream_t user_stream;
     int use_user_stream;

@@ -165,7 +165,7 @@ int create_plan(cuSten_t* h, int variant, int dtype, int dev, int numTiles, int 
     p.dtype = dtype;
     p.H = H; p.V = V; p.L = L; p.R = R; p.T = T; p.B = B;
     p.ncoef = ncoef;
-    p.mem_kind = -1;
+    p.mem_kind = p.mem_kind_out = -1;
     static std::atomic<unsigned long long> next_id{1};
     p.id = next_id.fetch_add(1, std::memory_order_relaxed);
     p.user_stream = nullptr;
@@ -569,11 +569,10 @@ static int compute_staged(cuSten_t* h, PlanPrivate* p, StencilArgs& a, cudaStrea
     return ST_OK;
 }
 
-// Streams of a group member (custen_compute_group): device-resident fields run on `shared`, the first stream of the
-// handle `owner`, others on the handle's own first stream (PlanPrivate::group_own), which then follows the work queued on
-// `outer`. live: not under capture.
+// Stream of a group member (custen_compute_group): the first stream of the handle `owner`, which may be another one.
+// live: not under capture. The member's memory kinds are known (PlanPrivate).
 struct GroupLane {
-    cudaStream_t shared, outer;
+    cudaStream_t stream;
     unsigned long long owner;
     bool live;
 };
@@ -646,22 +645,19 @@ int compute_plan(cuSten_t* h, int offload, cudaStream_t* explicit_stream, const 
         }
     }
 
-    const int kind = memory_kind(in0);
-    const int kind_out = memory_kind(out0);
-    p->mem_kind = kind;
+    if (!lane) {
+        p->mem_kind = memory_kind(in0);
+        p->mem_kind_out = memory_kind(out0);
+    }
+    const int kind = p->mem_kind, kind_out = p->mem_kind_out;
     if (lane) {
-        p->group_own = kind != 0 || kind_out == 2;
-        if (p->group_own) {
-            CU_TRY(cudaEventRecord(h->events[1], lane->outer), "Recording a group member's fork event");
-            CU_TRY(cudaStreamWaitEvent(h->streams[0], h->events[1], 0), "Ordering a group member");
-        }
-        s = copy_s = p->group_own ? h->streams[0] : lane->shared;
-        if (!p->group_own && lane->live && p->last_owner && p->last_owner != lane->owner && s != h->streams[0]) {
+        s = copy_s = lane->stream;
+        if (lane->live && p->last_owner && p->last_owner != lane->owner && s != h->streams[0]) {
             // the handle's earlier work lies on, or is waited for by, its own first stream
             CU_TRY(cudaEventRecord(h->events[1], h->streams[0]), "Recording a handle's earlier work");
             CU_TRY(cudaStreamWaitEvent(s, h->events[1], 0), "Ordering a group member after its handle's work");
         }
-        if (lane->live) p->last_owner = p->group_own ? p->id : lane->owner;
+        if (lane->live) p->last_owner = lane->owner;
         explicit_stream = &s;
     } else if (!explicit_stream && !p->use_user_stream) {
         p->last_owner = p->id;
@@ -980,35 +976,50 @@ int custen_compute_group(cuSten_t* const* handles, int count, int offload, void*
     if (count == 0) return ST_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     CU_TRY(cudaSetDevice(handles[0]->deviceNum), "Setting current device");
-    // Fork: the first streams of up to three handles follow the work already queued on `stream` and share the members
-    // with device-resident fields between them; the others (copies that should overlap) run on their own streams. Two
+    // Fork: the first streams of up to three members with device-resident fields follow the work already queued on
+    // `stream` and share all such members between them; the others (copies that should overlap) run on their own streams.
+    // One event for all, before any member's work: on the legacy default stream a later record would wait for that
+    // work (six pinned members of 2048^2 there: 2460 us with a record each, 1470 so). Two
     // kernels fill the tails of a third, and every further stream costs three calls and the GPU's waiting on its
     // events: twelve operators at 256^2, FP64, on 12 / 6 / 4 / 3 / 2 streams 69 / 59 / 59 / 55 / 56 us, 1024^2 164 / 162 / 161 /
     // 158 / 160, 8192^2 7905 / 7904 / 7899 / 7900 / 7910; FP32 1024^2 69 / 62 / 59 / 55 / 56, 4096^2 291 / 280 / 284 / 279 / 283;
     // call after call without a pause FP64 1024^2 147 / 145 / 145 / 143 / 145, FP32 4096^2 291 / 285 / 276 / 266 / 278.
     constexpr int kLanes = 3;
-    const int lanes = std::min(count, kLanes);
+    cuSten_t* lane[kLanes];
+    int lanes = 0;
+    for (int k = 0; k < count; ++k) {
+        PlanPrivate* p = priv_of(handles[k]);
+        p->mem_kind = memory_kind(byte_ptr(handles[k]->dataInput[0]));
+        p->mem_kind_out = memory_kind(byte_ptr(handles[k]->dataOutput[0]));
+        if (!p->copies() && lanes < kLanes) lane[lanes++] = handles[k];
+    }
+    auto on_own = [&](int k) {   // on its own first stream
+        return priv_of(handles[k])->copies() || std::find(lane, lane + lanes, handles[k]) != lane + lanes;
+    };
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     CU_TRY(cudaStreamIsCapturing(s, &capture), "Querying the stream's capture");
     const bool live = capture == cudaStreamCaptureStatusNone;
     CU_TRY(cudaEventRecord(handles[0]->events[1], s), "Recording the group's fork event");
-    for (int k = 0; k < lanes; ++k)
-        CU_TRY(cudaStreamWaitEvent(handles[k]->streams[0], handles[0]->events[1], 0), "Ordering a group member");
-    for (int k = 0; k < count; ++k) {
-        const GroupLane lane = {handles[k % lanes]->streams[0], s, priv_of(handles[k % lanes])->id, live};
-        const int st = compute_plan(handles[k], offload, nullptr, &lane);
+    for (int k = 0; k < count; ++k)
+        if (on_own(k)) CU_TRY(cudaStreamWaitEvent(handles[k]->streams[0], handles[0]->events[1], 0), "Ordering a group member");
+    for (int k = 0, next = 0; k < count; ++k) {
+        const cuSten_t* on = priv_of(handles[k])->copies() ? handles[k] : lane[next++ % lanes];
+        const GroupLane to = {on->streams[0], priv_of(on)->id, live};
+        const int st = compute_plan(handles[k], offload, nullptr, &to);
         if (st != ST_OK) return st;
     }
     // join: later work on `stream` follows every member
     for (int k = 0; k < count; ++k) {
-        if (k >= lanes && !priv_of(handles[k])->group_own) continue;
+        if (!on_own(k)) continue;
         CU_TRY(cudaEventRecord(handles[k]->events[0], handles[k]->streams[0]), "Recording a group member's end");
         CU_TRY(cudaStreamWaitEvent(s, handles[k]->events[0], 0), "Joining the group");
     }
     // and so does later work on the members' own streams, as when each member ran on its own
-    for (int k = lanes; live && k < count; ++k)
-        if (!priv_of(handles[k])->group_own)
-            CU_TRY(cudaStreamWaitEvent(handles[k]->streams[0], handles[k % lanes]->events[0], 0), "Ordering a handle's stream");
+    for (int k = 0, next = 0; live && k < count; ++k) {
+        if (priv_of(handles[k])->copies()) continue;
+        const cuSten_t* on = lane[next++ % lanes];
+        if (on != handles[k]) CU_TRY(cudaStreamWaitEvent(handles[k]->streams[0], on->events[0], 0), "Ordering a handle's stream");
+    }
     return ST_OK;
 }
 int custen_compute_on_stream(cuSten_t* h, int offload, void* stream) {
