@@ -178,9 +178,16 @@ __global__ void __launch_bounds__(kLine) solve_kernel(const double* __restrict__
 }
 
 __global__ void __launch_bounds__(kThreads) invert_kernel(double* __restrict__ d, size_t count) {
+    const size_t step = (size_t)gridDim.x * blockDim.x;
+    size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (q >= count) return;
+    double x = d[q];   // on its way while the constants are read
     const f64::F64 f;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < count; q += (size_t)gridDim.x * blockDim.x)
-        d[q] = f64::reciprocal(f, d[q]);
+    for (;;) {
+        d[q] = f64::reciprocal(f, x);
+        if ((q += step) >= count) return;
+        x = d[q];
+    }
 }
 
 thread_local std::string g_err;
