@@ -96,9 +96,11 @@ inline int persistent_grid(int tiles_total, int per_sm) {
 }
 
 // Launch with programmatic stream serialization: the kernel may start before the previous kernel of the stream has
-// ended and waits for it itself (launch_wait). Each CTA allows that when it starts its last tile: 256^2, twelve FP64
-// operators in stream order, 99 us when allowed from the start, 55 us so (116 us without, and with the former set-up
-// and tiles); 4096^2 FP32 in four tiles: 352, 324 and 343 us.
+// ended and waits for it itself (launch_wait). Each CTA allows that when its first warp has computed its last tile:
+// 256^2, twelve FP64 operators in stream order, 99 us when allowed from the kernel's start, 56 us from the last tile's
+// start, 49 us so (116 us without, and with the former set-up and tiles); 4096^2 FP32 in four tiles: 352, 322, 316 and
+// 343 us. Any earlier, the next launch's CTAs take the room beside the running ones, several on one SM and none on
+// another: a 33-point Y window at 512^2 28.3 us against 19.7.
 template <typename... P, typename... A>
 cudaError_t launch_overlapped(void (*kern)(P...), int grid, dim3 block, size_t smem, cudaStream_t s, const A&... args) {
     cudaLaunchAttribute attr;

@@ -207,7 +207,6 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
     for (int it = 0;; ++it) {
         const int t = blockIdx.x + it * gridDim.x;
         if (t >= tiles_total) break;
-        if (t + gridDim.x >= tiles_total) launch_dependents();   // the CTA's last tile
         const int s = it % S;
         const uint32_t parity = (uint32_t)((it / S) & 1);
         T* tile = ring + (size_t)s * stage_bytes / sizeof(T);
@@ -231,6 +230,7 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
         const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
         if (ok)
             compute_tile<T, TW, TH, RPT, VEC, MODE>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
+        if (t + gridDim.x >= tiles_total) launch_dependents();   // a warp is done with the CTA's last tile
         fence_proxy_async_smem();
         // every thread is done with stage s; a copy that never completed ends the CTA here: record it,
         // wait (bounded) for the copies this CTA still has in flight, and leave
