@@ -185,14 +185,27 @@ int tune(const StencilArgs& a, int dtype, cudaStream_t s, int reps, std::vector<
 // The configuration of a launch nothing has been tuned for, by its number of points: small fields need many small
 // tiles to occupy the SMs, large ones amortise a tile's halo and barrier over more points. Measured, twelve operators
 // in us, configurations 0 (64 x 32 points in FP64, 128 x 32 in FP32), 1 (half as wide) and 5 (32 x 16, 64 x 16):
-//   FP64  256^2 92 / 78 / 60   1024^2 209 / 194 / 192   1536^2 364 / 355 / 361   3072^2 1266 / 1258 / 1273
-//         4096^2 2144 / 2165 / 2204   8192^2 8207 / 8298 / -
-//   FP32  256^2 65 / 63 / 51   1536^2 83 / 81 / 74   2048^2 120 / 113 / 118   3000^2 228 / 176 / 187
-//         4096^2 314 / 306 / 359   6000^2 624 / 641 / 684
+//   FP64  256^2 80 / 65 / 48   1024^2 201 / 185 / 180   1536^2 354 / 342 / 346   3072^2 1254 / 1241 / 1263
+//         4096^2 2135 / 2140 / 2198   6000^2 4472 / 4501 / 4640
+//   FP32  256^2 53 / 51 / 38   1536^2 76 / 80 / 76   2048^2 115 / 114 / 118   3000^2 199 / 174 / 186
+//         4096^2 330 / 309 / 364   6000^2 627 / 644 / 660
+// Configuration 1 only where two of its CTAs (4 warps each) fit an SM beside each other: with halos so long that one
+// fills it, configuration 5 keeps three and configuration 0 has 8 warps (81-point X, FP64, 1 / 5 / 0: 1536^2 464 /
+// 324 / 338, 2048^2 784 / 560 / 588, 3000 x 2800 1576 / 1117 / 1162).
+static bool two_fit(const StencilArgs& a, int dtype, const StencilConfig& c) {
+    const int size = dtype == DT_F64 ? 8 : 4, pad = 16 / size, stages = 3;
+    const auto padded = [&](int n) { return (n + pad - 1) / pad * pad; };
+    const size_t halo = padded(a.L) + padded(a.R);   // once in the window, once in the side areas of a wrapped row
+    const size_t row = (halo + c.tw + (a.wrap_x ? halo : 0)) * size;
+    const size_t cta = stages * (c.th + a.T + a.B) * row + a.ncoef * (2 * size + 4) + 2048;
+    return 2 * cta <= 228 * 1024;
+}
 static int default_config(const StencilArgs& a, int dtype) {
     const double points = (double)a.nx * a.rows;
-    if (dtype == DT_F64) return points < 1.5e6 ? 5 : (points < 1.2e7 ? 1 : 0);
-    return points < 3e6 ? 5 : (points < 2e7 ? 1 : 0);
+    const StencilConfig& half = dtype == DT_F64 ? kConfigsF64[1] : kConfigsF32[1];
+    if (points < (dtype == DT_F64 ? 1.5e6 : 3e6)) return 5;
+    if (points < (dtype == DT_F64 ? 1.2e7 : 2e7)) return two_fit(a, dtype, half) ? 1 : 5;
+    return 0;
 }
 
 // The configuration for a device-resident launch: from the cache, from tuning (modes 1, 2 or force),

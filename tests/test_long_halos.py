@@ -57,3 +57,28 @@ def test_both(gpu, variant, fun, geom, nx, ny, dtype):
 def test_tiles_launched_apart(gpu, variant, mem):
     for config in CONFIGS:
         same(variant, 256, 256, 2, y_window(40, 40), mem=mem, config=config)
+
+
+@pytest.mark.parametrize("geom,config", [(x_window(2, 2), 1), (x_window(16, 16), 1), (x_window(40, 40), 5),
+                                         (y_window(40, 40), 1), (y_window(100, 100), 5)])
+def test_default_configuration(gpu, geom, config, tmp_path):
+    """A field that takes the half-wide tile with short windows, whose ring two CTAs of an SM have to share."""
+    from custen_gb300.buffers import DeviceBuffer
+    H, L, R, V, T, B = geom
+    nx, ny = 1536, 1280
+    cs.set_tune_cache(tmp_path / "none.json")
+    try:
+        inp, out, w = DeviceBuffer(nx * ny * 8), DeviceBuffer(nx * ny * 8), DeviceBuffer.from_array(np.ones(H * V))
+        cs._check(cs.lib().custen_memset(inp.ptr, 0, nx * ny * 8))
+        names = []
+        for pin in (None, config):
+            h = cs.Stencil(cs.XP if H > 1 else cs.YP, nx, ny, out.ptr, inp.ptr, w.ptr, H=H, L=L, R=R, V=V, T=T, B=B)
+            if pin is not None:
+                h.set_config(pin)
+            h.compute()
+            cs._check(cs.lib().custen_device_synchronize())
+            names.append(h.config())
+            h.destroy()
+        assert names[0] == names[1]
+    finally:
+        cs.set_tune_cache(None)
