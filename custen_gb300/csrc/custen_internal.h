@@ -51,6 +51,7 @@ struct StencilArgs {
     int wrap_x;           // 1: columns outside [0,nx) wrap around (periodic variants)
     int has_top, has_bot; // 1: halo rows above / below may be read
     int vec_ok;           // 1: rows are 16-byte aligned, vector loads/stores allowed
+    int keep_zeros;       // 1: exact-zero weights stay in the chain (launch_stencil_cfg); 0: dropped
     // 1: every staged input value c is replaced by c^3 - c (as fma(c*c, c, -c)) and the coefficients then
     // apply as plain weights. Set for the Fun variants when the device function is one of the library's
     // own c^3 - c functions, which compute exactly that (builtin_funs.cuh, ids 1, 3, 5).

@@ -98,7 +98,7 @@ stencil_async_kernel(const __grid_constant__ StencilArgs a, int tiles_x, int til
             __syncthreads();
         }
         const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
-        compute_tile<T, TW, TH, RPT, VEC, MODE>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
+        compute_tile<T, TW, TH, RPT, VEC, MODE, false>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
         if (t + gridDim.x >= tiles_total) launch_dependents();   // a warp is done with the CTA's last tile
         cur = cur + 1 == stages ? 0 : cur + 1;
         next = next + 1 == stages ? 0 : next + 1;

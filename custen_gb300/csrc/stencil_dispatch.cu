@@ -30,7 +30,11 @@ int persistent_grid_cap() { return g_grid_cap.load(std::memory_order_relaxed); }
 
 cudaError_t launch_stencil_cfg(const StencilArgs& a, int dtype, int cfg, cudaStream_t s, int* path) {
     if (cfg < 0 || cfg >= kNumConfigs) cfg = 0;
-    return (dtype == DT_F64 ? kLaunchF64 : kLaunchF32)[cfg](a, s, path);
+    // Exact-zero weights are dropped, except in FP32 fields of whole 128 x 32 tiles with a window that has a loop of its own.
+    // For finite fields the results are the same; an infinity or NaN under a zero weight matters only where it is kept.
+    StencilArgs b = a;
+    b.keep_zeros = dtype == DT_F32 && a.vec_ok && a.nx % kConfigsF32[0].tw == 0 && a.rows % kConfigsF32[0].th == 0;
+    return (dtype == DT_F64 ? kLaunchF64 : kLaunchF32)[cfg](b, s, path);
 }
 
 cudaError_t launch_stencil_f64(const StencilArgs& a, cudaStream_t s, int* path) {

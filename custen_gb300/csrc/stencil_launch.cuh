@@ -140,7 +140,7 @@ cudaError_t launch_async_mode(const StencilArgs& a, cudaStream_t s) {
 }
 
 // TMA path: returns cudaErrorNotSupported (without launching) when the geometry does not allow it.
-template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP>
+template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP, bool KEEP>
 cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     TileGeom<T, TW, TH> g(a);
     // One box per window: at most 256 columns and 256 rows; rows 16-byte aligned (global address and stride
@@ -157,7 +157,7 @@ cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
     const size_t stage_bytes = round_up_int((int)((size_t)g.SR * g.SW * sizeof(T)), 128);
     const size_t smem = S * (stage_bytes + wl_bytes + wr_bytes) + g.coef_bytes(a) +
                         256;   // 128 bytes of alignment slack for the ring base + tail padding
-    auto kern = stencil_tma_kernel<T, TW, TH, RPT, VEC, S, MODE, WRAP>;
+    auto kern = stencil_tma_kernel<T, TW, TH, RPT, VEC, S, MODE, WRAP, KEEP>;
     cudaError_t e = ensure_smem(kern, smem);
     if (e != cudaSuccess) return e == cudaErrorInvalidConfiguration ? cudaErrorNotSupported : e;
     int per_sm = 0;
@@ -171,14 +171,22 @@ cudaError_t launch_tma_mode(const StencilArgs& a, cudaStream_t s) {
                              tiles_x, tiles_total);
 }
 
+// The instantiation that keeps or skips zero weights: FP32 shapes only.
+template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP>
+cudaError_t launch_tma_zeros(const StencilArgs& a, cudaStream_t s) {
+    if constexpr (sizeof(T) == 4 && MODE >= MODE_FIRST_SHAPE)
+        if (a.keep_zeros) return launch_tma_mode<T, TW, TH, RPT, VEC, S, MODE, WRAP, true>(a, s);
+    return launch_tma_mode<T, TW, TH, RPT, VEC, S, MODE, WRAP, false>(a, s);
+}
+
 // The instantiation with or without the wrap-around boxes; the Y shapes have no columns to wrap.
 template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE>
 cudaError_t launch_tma_wrap(const StencilArgs& a, cudaStream_t s, bool wrap) {
     if constexpr (MODE >= 5 && MODE <= 7) {
-        return launch_tma_mode<T, TW, TH, RPT, VEC, S, MODE, false>(a, s);
+        return launch_tma_zeros<T, TW, TH, RPT, VEC, S, MODE, false>(a, s);
     } else {
-        return wrap ? launch_tma_mode<T, TW, TH, RPT, VEC, S, MODE, true>(a, s)
-                    : launch_tma_mode<T, TW, TH, RPT, VEC, S, MODE, false>(a, s);
+        return wrap ? launch_tma_zeros<T, TW, TH, RPT, VEC, S, MODE, true>(a, s)
+                    : launch_tma_zeros<T, TW, TH, RPT, VEC, S, MODE, false>(a, s);
     }
 }
 

@@ -156,7 +156,8 @@ __device__ __forceinline__ void edge_fixup(const StencilArgs& a, T* tile, const 
 
 // WRAP: the launch is periodic in x with a left or right halo (wrap-around boxes and side areas); the
 // other launches run an instantiation without them, which keeps their register allocation.
-template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP>
+// KEEP: FP32 shapes multiply by zero weights (StencilArgs::keep_zeros).
+template <typename T, int TW, int TH, int RPT, int VEC, int S, int MODE, bool WRAP, bool KEEP>
 __global__ void __launch_bounds__((TW / VEC) * (TH / RPT), min_blocks_for((TW / VEC) * (TH / RPT), MODE == MODE_FUN))
 stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__ StencilArgs a, int tiles_x,
                    int tiles_total) {
@@ -229,7 +230,7 @@ stencil_tma_kernel(const __grid_constant__ TmaMaps maps, const __grid_constant__
         }
         const bool all_write = tile_all_write(a, x0, x0 + TW, a.row0 + y0, a.row0 + y0 + TH);
         if (ok)
-            compute_tile<T, TW, TH, RPT, VEC, MODE>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
+            compute_tile<T, TW, TH, RPT, VEC, MODE, KEEP>(a, tile, coef_s, list_off, list_w, nlist, g, x0, y0, all_write, zeros);
         if (t + gridDim.x >= tiles_total) launch_dependents();   // a warp is done with the CTA's last tile
         fence_proxy_async_smem();
         // every thread is done with stage s; a copy that never completed ends the CTA here: record it,
