@@ -404,11 +404,15 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 // warp then starts no further copy and stays until those in flight have landed (bounded as well).
 struct RingWait {
     long long limit;
+    unsigned* failed;      // set at an expiry, or null
     unsigned parity = 0;   // per stage: the phase its next completion ends
     bool ok = true;
-    __device__ __forceinline__ explicit RingWait(long long limit_) : limit(limit_) {}
+    __device__ __forceinline__ explicit RingWait(long long limit_, unsigned* failed_ = nullptr) : limit(limit_), failed(failed_) {}
     __device__ __forceinline__ void operator()(uint64_t* bars, int st) {
-        if (ok) ok = mbar_wait(&bars[st], (parity >> st) & 1u, limit);
+        if (ok && !mbar_wait(&bars[st], (parity >> st) & 1u, limit)) {
+            ok = false;
+            if (failed) *(volatile unsigned*)failed = 1u;
+        }
         parity ^= 1u << st;
     }
     __device__ __forceinline__ void report() const {
@@ -417,8 +421,7 @@ struct RingWait {
 };
 
 // The chain is done with a chunk in stage st (by every lane).
-__device__ __forceinline__ void chunk_solved(ChainBars& bars, const RingWait& full, int st, int lane) {
-    if (!full.ok) *(volatile unsigned*)&bars.failed = 1u;
+__device__ __forceinline__ void chunk_solved(ChainBars& bars, int st, int lane) {
     __syncwarp();   // every lane's writes
     if (lane == 0) mbar_arrive(&bars.done[st]);
 }
@@ -468,8 +471,8 @@ template <class Solve>
 __device__ __forceinline__ void run_chain(int nchunk, ChainBars& bars, double (*own)[BLK], double (*other)[BLK], int lane,
                                           const double* mid, double& v1, double& v2, Solve solve,
                                           long long limit = kWaitLimit) {
-    RingWait full(limit);
-    auto solved = [&](int st) { chunk_solved(bars, full, st, lane); };
+    RingWait full(limit, &bars.failed);
+    auto solved = [&](int st) { chunk_solved(bars, st, lane); };
     double u1 = 0.0, u2 = 0.0;
     for (int c = 0; c < nchunk; ++c) {
         const int st = c % kStages;
@@ -808,7 +811,7 @@ __global__ void __launch_bounds__(256, 4) ch_update_kernel(const GridDev* __rest
     const Item item = items[blockIdx.x];
     const GridDev gd = grids[item.grid];
     launch_wait();
-    if (gd.general) return;   // its y sweep has updated the field
+    if (gd.general) return;   // ch_update_general_kernel does it
     const int n = gd.n;
     const int bpr = n / BLK;
     const int y0 = (item.block / bpr) * BLK, x0 = (item.block % bpr) * BLK;
@@ -890,8 +893,8 @@ template <class Get, class Put>
 __device__ __forceinline__ void run_band(const GridDev& gd, const BandTable& bt, ChainBars& bars, const BandChunk* band,
                                          int lane, double& x2, double& x1, Get get, Put put) {
     const int nchunk = gd.n / kChunk;
-    RingWait full(kWaitLimit);
-    auto solved = [&](int st) { chunk_solved(bars, full, st, lane); };
+    RingWait full(kWaitLimit, &bars.failed);
+    auto solved = [&](int st) { chunk_solved(bars, st, lane); };
     const double* tc = bt.t + min(bt.const_lo, nchunk - 1) * kChunk;
     const double cs = tc[0], cl = tc[bt.m], cr = tc[2 * bt.m], cu = tc[3 * bt.m], cw = tc[4 * bt.m];
     double b1 = 0.0, b2 = 0.0, r2 = 0.0, r1 = 0.0;
@@ -1360,12 +1363,14 @@ static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
     return 2.0 * dt * D * gamma / (3.0 * (dx * dx * dx * dx));
 }
 
-// Two segments halve a chain, which is the time of a sweep when few lines are resident, and add up to two
-// multiply-adds per point and sweep where the closure's reach is long against half a line, which is the time when
-// many are. Measured with the persistent right-hand side (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
+// Two segments halve a chain, which is the time of a sweep when fewer chains than FP64 sub-partitions are resident, and
+// add up to two multiply-adds per point and sweep (of 26 in a step) where the closure's reach is long against half a
+// line, which is the time when more are. A grid's segments may depend on n alone, or its bits would depend on its
+// batch, so each size takes the side that loses less: up to 512 points at most 1.5% in a full chip against up to 1.55x alone;
+// 544 to 1024 one segment, since a full chip would lose 5.5%, at the price of 1.5x for a grid alone; above, where chains
+// are longest and eight grids are needed to fill the chip, two (1.4x alone, 8% lost with eight). Measured with the persistent right-hand side (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
 // 384^2 152 / 123, 96 grids of 64^2 .. 1024^2 with those up to 512^2 cut 1466 / 1488; one grid of 1024^2 242 / 161, but the
 // 96 grids 1488 / 1570 with the 1024^2 ones cut as well; 2048^2: one grid 547 / 388, four 1092 / 1039, eight 1909 / 2054.
-// Grids of 1024^2 come in the large batches, larger ones do not, so those between the two sizes keep one segment.
 constexpr int kCutUpTo = 512, kCutAbove = 1024;
 int line_cuts(int n, bool general) {
     return !general && (n <= kCutUpTo || n > kCutAbove) ? 2 : 1;
