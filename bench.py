@@ -623,8 +623,8 @@ def run_gpu(args, world, rank, local):
             "data": "synthetic: sin(3x)cos(5y)+U(-1e-3,1e-3), seed 1",
             "config": {"workload": f"cuSten stencil sweep FP64 {n}^2: 12 operators (X/Y 5-pt p/np, XY 3x3 "
                                    f"cross p/np, Fun c^3-c X/Y/XY p/np), numTiles=1, device-resident",
-                       "schedule": ("one custen_compute_group call per step: the 12 independent handles, each on "
-                                    "its own stream" if group_ms is not None else
+                       "schedule": ("one custen_compute_group call per step: the 12 independent handles, on "
+                                    "three streams" if group_ms is not None else
                                     "12 Computes per step in stream order"),
                        "nx": n, "ny": n, "numTiles": 1, "l2": f"inputs larger than L2 ({n * n * 8 / 2**30:.3g} GiB per field)" if n * n * 8 > 129e6
                        else f"field of {n * n * 8 / 2**20:.3g} MiB fits in L2 (not the headline size)",
@@ -878,7 +878,7 @@ def run_size_sweep(cs, torch, dev, local, sizes=(1024, 2048, 4096, 8192), tiles=
                                      "ms_per_sweep": round(ms, 4), "timing": "graph replay" if graph else "events"}
             if group:
                 # the twelve operators are independent (one input, twelve outputs): one custen_compute_group
-                # call runs each on its handle's own stream, so that one launch's tail overlaps the next
+                # call runs them on three of the handles' streams, so that one launch's tail overlaps the next
                 g2 = None
                 if graph is not None:
                     g2 = torch.cuda.CUDAGraph()

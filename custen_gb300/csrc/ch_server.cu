@@ -5,7 +5,7 @@
 // field buffers, work field and h field are allocated stream-ordered (cudaMallocAsync, no device
 // synchronisation) and their pre-factored solver table is shared by every resident grid of the same
 // size. All resident grids then advance together, a chunk of steps at a time, through the same
-// persistent kernels as the batch solver (ch_solver.cu): one launch per kernel covers every grid.
+// kernels as the batch solver (ch_solver.cu): one launch per kernel covers every grid.
 // Between chunks, finished grids are read back and their memory is released, and new arrivals join,
 // so work that arrives while others are on the GPU overlaps with them. Each grid is computed by the
 // same operations whatever else is resident, so a result is bit-identical alone and in the mix.

@@ -1363,14 +1363,16 @@ static double sigma_lin(int n, double lx, double gamma, double dt_factor) {
     return 2.0 * dt * D * gamma / (3.0 * (dx * dx * dx * dx));
 }
 
-// Two segments halve a chain, which is the time of a sweep when fewer chains than FP64 sub-partitions are resident, and
-// add up to two multiply-adds per point and sweep (of 26 in a step) where the closure's reach is long against half a
-// line, which is the time when more are. A grid's segments may depend on n alone, or its bits would depend on its
-// batch, so each size takes the side that loses less: up to 512 points at most 1.5% in a full chip against up to 1.55x alone;
-// 544 to 1024 one segment, since a full chip would lose 5.5%, at the price of 1.5x for a grid alone; above, where chains
-// are longest and eight grids are needed to fill the chip, two (1.4x alone, 8% lost with eight). Measured with the persistent right-hand side (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2 116 / 75, 24 grids of 96^2 ..
-// 384^2 152 / 123, 96 grids of 64^2 .. 1024^2 with those up to 512^2 cut 1466 / 1488; one grid of 1024^2 242 / 161, but the
-// 96 grids 1488 / 1570 with the 1024^2 ones cut as well; 2048^2: one grid 547 / 388, four 1092 / 1039, eight 1909 / 2054.
+// Two segments halve a chain, which is the time of a sweep when fewer chains than FP64 sub-partitions are resident,
+// and add up to two multiply-adds per point and sweep (of 26 in a step) where the closure's reach is long against
+// half a line, which is the time when more are. A grid's segments may depend on n alone, or its bits would depend on
+// its batch, so each size takes the side that loses less: up to 512 points at most 1.5% in a full chip against up to
+// 1.55x alone; 544 to 1024 one segment, since a full chip would lose 5.5%, at the price of 1.5x for a grid alone;
+// above, where chains are longest and eight grids are needed to fill the chip, two (1.4x alone, 8% lost with eight).
+// Measured with the persistent right-hand side (us per step, one / two segments): one grid of 256^2 64 / 46, 512^2
+// 116 / 75, 24 grids of 96^2 .. 384^2 152 / 123, 96 grids of 64^2 .. 1024^2 with those up to 512^2 cut 1466 / 1488;
+// one grid of 1024^2 242 / 161, but the 96 grids 1488 / 1570 with the 1024^2 ones cut as well; 2048^2: one grid 547 /
+// 388, four 1092 / 1039, eight 1909 / 2054.
 constexpr int kCutUpTo = 512, kCutAbove = 1024;
 int line_cuts(int n, bool general) {
     return !general && (n <= kCutUpTo || n > kCutAbove) ? 2 : 1;

@@ -1,4 +1,5 @@
-// FP64 work moved off the FP64 pipe or to its cheapest instruction, with bit-identical results.
+// FP64 work moved off the FP64 pipe or to its cheapest instruction, with bit-identical results (of Divider, proved but
+// for about one quotient in 2^90: see there).
 //
 // Sums and products as multiply-adds (F64): a multiply-add whose three operands are registers runs at 597 G/s on
 // GB300, an addition or a multiplication at 503 (as does a multiply-add with a literal, parameter or zero
@@ -12,14 +13,15 @@
 //   to_double / to_float   conversions rewritten on the IEEE 754 encodings           0 instead of 1
 //   div_by_float           correctly rounded c / d, d a float value                  3 instead of 10.4
 //   reciprocal             correctly rounded 1 / x                                   4 instead of 5.6 (+ the range check's)
-//   Divider                correctly rounded a / b; several a share b                2 + 3 per a instead of 9.4 per a
+//   Divider                a / b; several a share b                                  2 + 3 per a instead of 9.4 per a
 // Arguments outside the ranges named at each function take the compiler's own operation, out of line. Measured: WENO
 // 1024^2 with fields of order 1, 100, 1e4, 1e6 and 1e9 (the last four with squared indicators outside div_by_float's
 // range at some or all points) 226, 329, 296, 296 and 498 us, with operators throughout 412 (578 at 1e9).
 //
-// Method: Newton's iteration for the reciprocal (1/b = y (1 + e + e^2 + ...), e = 1 - b y), carried to about 47 bits
-// in pairs of floats, then one residual correction of the quotient with a fused multiply-add (Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor",
-// IBM J. Res. Dev. 34, 1990). The error bounds that make the results correctly rounded stand at each function.
+// Method: Newton's iteration for the reciprocal (1/b = y (1 + e + e^2 + ...), e = 1 - b y), carried to about 47
+// bits in pairs of floats, then one residual correction of the quotient with a fused multiply-add (Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990). The
+// error bounds that make the results correctly rounded stand at each function.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -159,14 +161,15 @@ __device__ __forceinline__ double reciprocal(const F64& f, double x) {
     return fma(fma(-x, y, f.one), y, y);
 }
 
-// Correctly rounded quotients by one divisor. |b| in [2^-200, 2^200) and |a| in [2^-800, 2^800) or zero (the quotient and
-// the residual's last bit, 105 places below a's first, are then normal); anything else takes the operator. q0 = RN(a y) is within one unit of a/b, so the residual is exact, and the
-// corrected quotient is correctly rounded where y is RN(1/b) (Markstein). y is, except where 1/b lies within
-// 2^-92 (relative) of a midpoint, where it may be the other neighbour; q0 + r y then still differs from a/b by at
-// most 2^-105 (relative), which changes a rounding only if a/b lies that near a midpoint as well. Divisors just
-// below a power of two, b = 2^j (1 - k 2^-53) with small odd k, are systematically like that (1/b and quotients
-// of simple numerators fall next to midpoints): fractions whose upper 20 bits are ones take the operator. For
-// the others both coincidences together are about one quotient in 2^90.
+// Quotients by one divisor, correctly rounded but for the coincidence below. |b| in [2^-200, 2^200) and |a| in
+// [2^-800, 2^800) or zero (the quotient and the residual's last bit, 105 places below a's first, are then normal);
+// anything else takes the operator. q0 = RN(a y) is within one unit of a/b, so the residual is exact, and the
+// corrected quotient is correctly rounded where y is RN(1/b) (Markstein). y is, except where 1/b lies within 2^-92
+// (relative) of a midpoint, where it may be the other neighbour; q0 + r y then still differs from a/b by at most
+// 2^-105 (relative), which changes a rounding only if a/b lies that near a midpoint as well. Divisors just below a
+// power of two, b = 2^j (1 - k 2^-53) with small odd k, are systematically like that (1/b and quotients of simple
+// numerators fall next to midpoints): fractions whose upper 20 bits are ones take the operator. For the others
+// both coincidences together are about one quotient in 2^90.
 struct Divider {
     double b, y;
     bool ok;

@@ -981,9 +981,10 @@ int custen_compute_group(cuSten_t* const* handles, int count, int offload, void*
     // One event for all, before any member's work: on the legacy default stream a later record would wait for that
     // work (six pinned members of 2048^2 there: 2460 us with a record each, 1470 so). Two
     // kernels fill the tails of a third, and every further stream costs three calls and the GPU's waiting on its
-    // events: twelve operators at 256^2, FP64, on 12 / 6 / 4 / 3 / 2 streams 69 / 59 / 59 / 55 / 56 us, 1024^2 164 / 162 / 161 /
-    // 158 / 160, 8192^2 7905 / 7904 / 7899 / 7900 / 7910; FP32 1024^2 69 / 62 / 59 / 55 / 56, 4096^2 291 / 280 / 284 / 279 / 283;
-    // call after call without a pause FP64 1024^2 147 / 145 / 145 / 143 / 145, FP32 4096^2 291 / 285 / 276 / 266 / 278.
+    // events: twelve operators at 256^2, FP64, on 12 / 6 / 4 / 3 / 2 streams 63 / 56 / 54 / 56 / 53 us, 1024^2 165 / 161 / 162 /
+    // 164 / 163, 8192^2 7917 / 7914 / 7910 / 7914 / 7912; FP32 1024^2 65 / 57 / 57 / 58 / 61, 4096^2 295 / 284 / 289 / 284 / 283;
+    // call after call without a pause FP64 256^2 58 / 53 / 52 / 50 / 46, 1024^2 144 / 142 / 142 / 141 / 142, FP32 4096^2
+    // 282 / 272 / 258 / 261 / 264.
     constexpr int kLanes = 3;
     cuSten_t* lane[kLanes];
     int lanes = 0;

@@ -5,10 +5,10 @@
 // Like the TMA kernel (stencil_tma.cuh) each CTA walks the tiles tile = blockIdx.x + k * gridDim.x with the next
 // windows in flight in a shared-memory ring and runs the same compute stage on them; the elements are copied one by
 // one (8 or 4 bytes, the alignment such rows have), a warp per window row, from the launch's rows or its halo rows,
-// wrapped (periodic) or zero-filled where a variant has no value. Bound by the FP64 pipe as the TMA kernel is (the
-// copies take issue slots only). Measured, 1999 x 1501, FP64 (FP32): 9-point X 56 (11) us, 5 x 5 with zeros 78 (14), dense
-// 3 x 3 57 (12); the kernel before it, one tile per CTA staged with plain loads and every window through the generic
-// weight list, took 68 (23), 94 (30) and 69 (23). On aligned rows (2000 x 1500) the TMA kernel takes 49, 74 and 50.
+// wrapped (periodic) or zero-filled where a variant has no value. Windows of nine weights or more are
+// bound by the FP64 pipe (77 to 85%), shorter ones by issue slots and the copies themselves (47%). Measured, 1999 x 1501, FP64 (FP32): 9-point X 57 (12) us, 5 x 5 with zeros 81 (14), dense
+// 3 x 3 58 (12); the kernel before it, one tile per CTA staged with plain loads and every window through the generic
+// weight list, took 70 (25), 96 (32) and 70 (25). On aligned rows (2000 x 1500) the TMA kernel takes 50, 70 and 50.
 #pragma once
 
 #include "stencil_kernel.cuh"

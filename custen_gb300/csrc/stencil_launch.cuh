@@ -84,8 +84,8 @@ inline int sm_count() {
 // Resident threads per SM of the persistent FP32 grid. These launches are bound by HBM or L2. Beyond about 2e7 points
 // (input and output exceed L2) more resident CTAs, each keeping S windows in flight, make them slower: over the twelve
 // operators at 16384^2, 650 Gpts/s with every CTA that fits, 730 capped at 768 threads per SM, 624 at 512. Below, a
-// few more keep the SMs busier (768 / 1024 / 1536 threads, us): 1024^2 60 / 52 / 52, 2048^2 118 / 113 / 113, 4096^2
-// 318 / 306 / 306.
+// few more keep the SMs busier (768 / 1024 / 1536 threads, us): 1024^2 58 / 50 / 50, 2048^2 121 / 113 / 115, 4096^2
+// 317 / 310 / 313.
 inline int f32_threads_per_sm(const StencilArgs& a) { return (double)a.nx * a.rows < 2e7 ? 1024 : 768; }
 
 // CTAs of a persistent launch: those that fit, at most one per tile, under the test cap.
